@@ -154,6 +154,10 @@ struct swg_graph {
     float merge_ms = 0;
     unsigned *d_hll_seg = nullptr;
     uint64_t hll_seg_cap = 0;
+    // super-k-mer build: pieces of long reads (offsets | counts | prefix | scan
+    // scratch | range [2] | lengths | samples)
+    uint64_t *d_pieces = nullptr;
+    uint64_t pieces_cap = 0;
     // streamed FASTA build: the copy stream, one event per text piece, and
     // the framing arrays that grow as pieces land
     cudaStream_t copy = nullptr, frame = nullptr;
@@ -254,6 +258,8 @@ swg_status build_partitioned(swg_graph *g, const swg_opts *o, BuildArgs &a, cuda
                              double load);
 swg_status build_bucketed(swg_graph *g, const swg_opts *o, BuildArgs &a, cudaStream_t s,
                           double load, bool counted = false);
+bool super_build(const swg_opts *o, const BuildArgs &a, uint64_t N);
+swg_status build_super(swg_graph *g, const swg_opts *o, BuildArgs &a, cudaStream_t s, double load, uint64_t longest);
 
 // The default algorithm is the bucketed one while its worst-case workspace
 // (two record buffers of at most 1.5 x 8 bytes per occurrence, plus an
@@ -359,6 +365,7 @@ swg_status build_impl(swg_graph *g, const swg_opts *o, const uint32_t *packed, u
         SWG_CUDA(cudaGetLastError(), "tile launch");
     }
     if (o->algorithm == SWG_ALGO_PARTITIONED) return build_partitioned(g, o, a, s, load);
+    if (bucketed && super_build(o, a, a.total_occ)) return build_super(g, o, a, s, load, g->h_ctl->max_len);
     if (bucketed) return build_bucketed(g, o, a, s, load);
     return build_direct(g, o, a, s, load);
 }
@@ -597,14 +604,18 @@ swg_status build_partitioned(swg_graph *g, const swg_opts *o, BuildArgs &a, cuda
 // own sample cutoffs and counts per sample, and a final pass moves the
 // survivors into per-sample ranges with the tag stripped.
 swg_status batch_bucketed(swg_graph *g, const swg_opts *o, const swg_sample *sm, uint32_t S,
-                          BuildArgs &a, cudaStream_t s, double load, int tb) {
+                          BuildArgs &a, cudaStream_t s, double load, int tb, uint64_t longest) {
     swg_status st;
     a.tag_bits = S > 1 ? tb : 0;
     a.cutoff = sm[0].cutoff;  // the single sample's, when untagged
     a.k = sm[0].k;
     SWG_CUDA(cudaMemsetAsync(g->d_ctl, 0, sizeof(Control) - sizeof(uint64_t), s), "clear control");
     SWG_CUDA(cudaMemsetAsync(g->d_seg_counts, 0, 2ull * S * 8, s), "clear counters");
-    if ((st = build_bucketed(g, o, a, s, load))) return st;
+    bool same_k = true;  // one k for all: super-k-mer records
+    for (uint32_t i = 1; i < S; i++) same_k = same_k && sm[i].k == sm[0].k;
+    st = same_k && super_build(o, a, a.total_occ) ? build_super(g, o, a, s, load, longest)
+                                                  : build_bucketed(g, o, a, s, load);
+    if (st) return st;
     g->n_samples = S;
     g->s_tbase.assign(S, 0);
     g->s_tcap.assign(S, 0);
@@ -757,7 +768,12 @@ swg_status batch_impl(swg_graph *g, const swg_opts *o, const swg_sample *sm, uin
     g->launches += swg::launch_seg_setup(a, g->d_seg_meta, g->d_seg_meta + S + 1, g->d_read_seg,
                                          g->d_off, s);
     SWG_CUDA(cudaMemsetAsync(g->d_prefix, 0, sizeof(uint64_t), s), "memset prefix");
+    SWG_CUDA(cudaMemsetAsync(&g->d_ctl->max_len, 0, sizeof(unsigned), s), "clear longest read");
+    a.max_len = &g->d_ctl->max_len;
     g->launches += swg::launch_occ_scan(a, s);
+    a.max_len = nullptr;
+    SWG_CUDA(cudaMemcpyAsync(&g->h_ctl->max_len, &g->d_ctl->max_len, sizeof(unsigned), cudaMemcpyDeviceToHost, s),
+             "read longest read");
     g->launches += swg::launch_gather_prefix(g->d_prefix, g->d_seg_meta, S + 1,
                                              g->d_seg_meta + 2 * (uint64_t)S + 1, s);
     SWG_CUDA(cudaGetLastError(), "batch setup launch");
@@ -778,7 +794,7 @@ swg_status batch_impl(swg_graph *g, const swg_opts *o, const swg_sample *sm, uin
         if ((o->algorithm == SWG_ALGO_DEFAULT || o->algorithm == SWG_ALGO_BUCKETED) &&
             o->read_order == SWG_ORDER_INPUT && S <= swg::kMaxTagSamples && 2 * kmax + tb <= 64 &&
             (o->algorithm == SWG_ALGO_BUCKETED || bucketed_fits(g, a.total_occ)))
-            return batch_bucketed(g, o, sm, S, a, s, load, tb);
+            return batch_bucketed(g, o, sm, S, a, s, load, tb, g->h_ctl->max_len);
     }
     a.n_tiles = (a.total_occ + swg::kTileOcc - 1) / swg::kTileOcc;
     if ((st = ensure(&g->d_tiles, &g->tiles_cap, a.n_tiles, "tile table"))) return st;
@@ -908,7 +924,31 @@ struct BucketPlan {
     swg::PartArgs pa;
     swg::BucketArgs bk;
     unsigned long long *scr = nullptr, *sampled = nullptr;
+    bool super = false;  // sk instead of pa and bk: super-k-mer records
+    swg::SkArgs sk;
 };
+
+// Partition bits b1 and sub-bucket bits b2 for N occurrences.
+void bucket_bits(const swg_opts *o, uint64_t N, double target, int &b1, int &b2) {
+    // level-1 partitions: 256, 512 past 400M occurrences (a level-1 round of
+    // 4096 records still writes runs of 8), 1024 only past 6.4G; the options
+    // (then SWG_PART_BITS) override
+    b1 = N <= (400ull << 20) ? 8 : (N <= (6400ull << 20) ? 9 : 10);
+    if (const char *e = std::getenv("SWG_PART_BITS")) b1 = std::min(10, std::max(8, std::atoi(e)));
+    if (o && o->part_bits) b1 = std::min(10, std::max(8, o->part_bits));
+    // sub-buckets of about `target` occurrences (the options, then SWG_BUCKET_RECORDS, override)
+    if (const char *e = std::getenv("SWG_BUCKET_RECORDS")) target = std::max(64.0, std::atof(e));
+    if (o && o->bucket_records) target = std::min(65535.0, std::max(64.0, (double)o->bucket_records));
+    // more partitions when even 1024 sub-buckets each would leave buckets past
+    // twice the target (they would outgrow the shared-memory tables)
+    while (b1 < 10 && (double)N / (double)((1ull << b1) << 10) > 2 * target) b1++;
+    const uint64_t P = 1ull << b1;
+    b2 = 0;
+    while (b2 < 10 && (double)N / (double)(P << b2) > target) b2++;
+    // at most 512 sub-buckets (level-2 runs of >= 8 records per 4096-record
+    // chunk) while the buckets stay under 4x the target
+    if (b2 == 10 && (double)N / (double)(P << 9) <= 4 * target) b2 = 9;
+}
 
 // Sizes the bucketed build for N occurrences, allocates its workspace and
 // lays out the level-1 partition and bucket regions: from exact counts over
@@ -917,26 +957,9 @@ struct BucketPlan {
 swg_status bucketed_plan(swg_graph *g, const swg_opts *o, const BuildArgs &a, uint64_t N, bool counted,
                          uint32_t stride, cudaStream_t s, BucketPlan &pl) {
     swg_status st;
-    // level-1 partitions: 256, 512 past 400M occurrences (a level-1 round of
-    // 4096 records still writes runs of 8), 1024 only past 6.4G; the options
-    // (then SWG_PART_BITS) override
-    int b1 = N <= (400ull << 20) ? 8 : (N <= (6400ull << 20) ? 9 : 10);
-    if (const char *e = std::getenv("SWG_PART_BITS")) b1 = std::min(10, std::max(8, std::atoi(e)));
-    if (o && o->part_bits) b1 = std::min(10, std::max(8, o->part_bits));
-    // sub-buckets of about `target` records (the options, then SWG_BUCKET_RECORDS, override)
-    double target = 4096.0;
-    if (const char *e = std::getenv("SWG_BUCKET_RECORDS")) target = std::max(64.0, std::atof(e));
-    if (o && o->bucket_records) target = std::min(65535.0, std::max(64.0, (double)o->bucket_records));
-    // more partitions when even 1024 sub-buckets each would leave buckets past
-    // twice the target (they would outgrow the shared-memory tables)
-    while (b1 < 10 && (double)N / (double)((1ull << b1) << 10) > 2 * target) b1++;
-    const uint64_t P = 1ull << b1;
-    int b2 = 0;
-    while (b2 < 10 && (double)N / (double)(P << b2) > target) b2++;
-    // at most 512 sub-buckets (level-2 runs of >= 8 records per 4096-record
-    // chunk) while the buckets stay under 4x the target
-    if (b2 == 10 && (double)N / (double)(P << 9) <= 4 * target) b2 = 9;
-    const uint64_t NB = P << b2;
+    int b1, b2;
+    bucket_bits(o, N, 4096.0, b1, b2);
+    const uint64_t P = 1ull << b1, NB = P << b2;
     // region bounds: partitions <= 1.25 N + 4097 P, buckets <= 1.5 N + 257 NB;
     // the level-1 buffer also stages survivor keys at bucket offsets
     const uint64_t rec1_bound = counted ? N : N + N / 4 + 4097 * P;
@@ -1194,6 +1217,253 @@ swg_status grow_keep(T **p, uint64_t *cap, uint64_t want, uint64_t keep, const c
     return SWG_OK;
 }
 
+// ---- the bucketed build over super-k-mer records (super.cu) ----
+// Smaller inputs are bound by launches and latency, not by the records.
+constexpr uint64_t kSuperMin = 512ull << 10;
+// Longest read a streamed piece's scan takes whole (its records hold 14 bits
+// of position); a one-shot build cuts reads past kSuperWhole bases in pieces.
+constexpr uint64_t kSuperLongest = (1ull << 14) - 1;
+constexpr uint64_t kSuperWhole = 512;
+
+bool super_build(const swg_opts *o, const BuildArgs &a, uint64_t N) {
+    // (the other scatter shapes are shapes of the single-occurrence scatters)
+    return swg::super_window(a.k) && N >= kSuperMin && !swg::level1_shape(o->scatter_shape);
+}
+
+// Sizes the build for N occurrences of n_reads reads, allocates its
+// workspace and lays out the regions from every stride-th batch of a's reads,
+// which hold about `share` of the input.
+swg_status super_plan(swg_graph *g, const swg_opts *o, const BuildArgs &a, uint64_t N, uint64_t n_reads,
+                      uint32_t stride, double share, const swg::SkArgs &reads, cudaStream_t s, BucketPlan &pl) {
+    swg_status st;
+    int b1, b2;
+    // sub-buckets of at most 3072 occurrences on average: the 2048-entry tables
+    // (four CTAs an SM) hold their k-molecules; 524,288 such buckets counted
+    // 2.4G skewed occurrences in 18.8 ms, 262,144 in 4096-entry tables in 20.3
+    bucket_bits(o, N, 3072.0, b1, b2);
+    const uint64_t P = 1ull << b1, NB = P << b2;
+    const double scale_max = 2.0 * stride / share;
+    // a random sequence has 2 / (w + 1) runs per k-mer and one more per read
+    const uint64_t rec_cap =
+        (uint64_t)(1.25 * ((double)n_reads + 2.0 * (double)N / (swg::super_window(a.k) + 1))) + 65536;
+    const uint64_t rec1 = rec_cap + rec_cap / 4 + 1025 * P, rec2 = swg::super_bucket_room(rec_cap, NB, scale_max);
+    if ((st = ensure(&g->d_part, &g->part_cap, 4 * P + 1, "partition table"))) return st;
+    if ((st = ensure(&g->d_records, &g->records_cap, 2 * rec1, "records"))) return st;
+    if ((st = ensure(&g->d_rec2, &g->rec2_cap, 2 * rec2, "bucket records"))) return st;
+    const uint64_t scratch = swg::gscan_scratch(NB);
+    if ((st = ensure(&g->d_bk, &g->bk_cap, 4 * NB + 1 + scratch + 2 + P + 1, "bucket table"))) return st;
+    swg::SkArgs sk = reads;  // off, len, seg, n_pieces, pieces
+    sk.k = a.k;
+    sk.b1 = b1;
+    sk.b2 = b2;
+    sk.n_parts = (uint32_t)P;
+    sk.work = g->d_ctl->work;
+    sk.part_count = g->d_part;
+    sk.part_start = g->d_part + P;
+    sk.part_cursor = g->d_part + 2 * P + 1;
+    sk.part_end = g->d_part + 3 * P + 1;
+    sk.cursor2 = g->d_bk;
+    sk.off2 = g->d_bk + NB;
+    sk.big = sk.off2 + NB + 1;
+    sk.big2 = sk.big + NB;
+    pl.scr = sk.big2 + NB;
+    sk.sampled = pl.scr + scratch;
+    sk.chunk_start = sk.sampled + 2;
+    sk.status = &g->d_ctl->status;
+    sk.rec1 = reinterpret_cast<uint4 *>(g->d_records);
+    sk.rec2 = reinterpret_cast<uint4 *>(g->d_rec2);
+    sk.n_kmers = N;
+    sk.rec_cap = rec_cap;
+    sk.scale_max = scale_max;
+    sk.big_count = &g->d_ctl->pad;
+    sk.big2_count = &g->d_ctl->pad2;
+    sk.big_cap = (uint32_t)std::min<uint64_t>(NB, 0xffffffffu);
+    SWG_CUDA(cudaMemsetAsync(sk.part_count, 0, P * 8, s), "clear partitions");
+    SWG_CUDA(cudaMemsetAsync(sk.cursor2, 0, NB * 8, s), "clear bucket samples");
+    SWG_CUDA(cudaMemsetAsync(sk.sampled, 0, 16, s), "clear sample totals");
+    g->launches += swg::launch_super_scan(a, sk, sk.n_pieces, stride, true, swg::kScatterResident, s);
+    g->launches += swg::launch_super_caps(sk, NB, reinterpret_cast<uint64_t *>(pl.scr), s);
+    SWG_CUDA(cudaMemcpyAsync(sk.cursor2, sk.off2, NB * 8, cudaMemcpyDeviceToDevice, s), "bucket cursors");
+    pl.b1 = b1;
+    pl.b2 = b2;
+    pl.P = P;
+    pl.NB = NB;
+    pl.super = true;
+    pl.sk = sk;
+    return SWG_OK;
+}
+
+swg_status super_finish(swg_graph *g, const swg_opts *o, BuildArgs &a, cudaStream_t s, double load, BucketPlan &pl);
+
+swg_status build_super(swg_graph *g, const swg_opts *o, BuildArgs &a, cudaStream_t s, double load, uint64_t longest) {
+    swg_status st;
+    g->algorithm = SWG_ALGO_BUCKETED;
+    swg::SkArgs reads;
+    std::memset(&reads, 0, sizeof(reads));
+    reads.off = a.read_off;
+    reads.len = a.read_len;
+    reads.seg = a.read_seg;
+    reads.n_pieces = a.n_reads;
+    BuildArgs as = a;
+    if (longest > kSuperWhole) {  // one thread per piece of 256 k-mers instead of one per read
+        const uint64_t NP = swg::super_pieces_bound(a.n_reads, a.total_occ), S = swg::gscan_scratch(a.n_reads);
+        if ((st = ensure(&g->d_pieces, &g->pieces_cap, 2 * NP + 2 * a.n_reads + S + 2, "read pieces"))) return st;
+        uint64_t *off = g->d_pieces, *count = off + NP, *first = count + a.n_reads, *scratch = first + a.n_reads,
+                 *range = scratch + S;
+        uint32_t *len = reinterpret_cast<uint32_t *>(range + 2), *seg = len + NP;
+        SWG_CUDA(cudaMemsetAsync(range, 0, 8, s), "piece range");
+        g->launches += swg::launch_super_pieces(a, count, first, scratch, range + 1, off, len,
+                                                a.read_seg ? seg : nullptr, s);
+        reads.off = off;
+        reads.len = len;
+        reads.seg = seg;
+        reads.n_pieces = NP;
+        reads.pieces = true;
+        as.read_range = reinterpret_cast<unsigned long long *>(range);
+    }
+    BucketPlan pl;
+    // the sample sizes the regions: a sixteenth of the reads, a quarter of small inputs
+    const uint32_t stride = a.total_occ >= (64ull << 20) ? 16 : 4;
+    if ((st = super_plan(g, o, as, a.total_occ, reads.n_pieces, stride, 1.0, reads, s, pl))) return st;
+    SWG_CUDA(cudaEventRecord(g->ev[1], s), "event");
+    g->launches += swg::launch_super_scan(as, pl.sk, reads.n_pieces, 1, false, swg::kScatterResident, s);
+    SWG_CUDA(cudaGetLastError(), "super-k-mer scan launch");
+    SWG_CUDA(cudaEventRecord(g->ev[2], s), "event");
+    return super_finish(g, o, a, s, load, pl);
+}
+
+// Output arrays of at least want k-molecules, the first keep kept.
+swg_status ensure_out(swg_graph *g, uint64_t want, uint64_t keep) {
+    if (g->out_cap >= want && g->d_out_keys && g->d_out_mult) return SWG_OK;
+    swg_status st;
+    uint64_t c1 = 0, c2 = 0;
+    if ((st = grow_keep(&g->d_out_keys, &c1, want, keep, "output keys"))) return st;
+    if ((st = grow_keep(&g->d_out_mult, &c2, want, keep, "output multiplicities"))) {
+        g->out_cap = 0;
+        return st;
+    }
+    g->out_cap = std::min(c1, c2);
+    return SWG_OK;
+}
+
+// Everything after the level-1 scatter. An overflowed region (or queue)
+// reruns the build on single occurrences with exact counts.
+swg_status super_finish(swg_graph *g, const swg_opts *o, BuildArgs &a, cudaStream_t s, double load, BucketPlan &pl) {
+    swg_status st;
+    g->algorithm = SWG_ALGO_BUCKETED;
+    const uint64_t N = a.total_occ, NB = pl.NB;
+    const BuildArgs plain = a;
+    if (g->host_keys && !a.tag_bits) {  // survivors also straight to the caller's host arrays
+        a.host_keys = g->host_keys;
+        a.host_mult = g->host_mult;
+        a.host_cap = g->host_cap;
+        a.host_written = &g->d_ctl->host_written;
+        g->host_out_used = true;
+    }
+    g->launches += swg::launch_super_sub(pl.sk, s);
+    SWG_CUDA(cudaGetLastError(), "bucket scatter launch");
+    SWG_CUDA(cudaEventRecord(g->ev[3], s), "event");
+    swg::BucketArgs mean;  // the table choice looks at the plan's mean bucket
+    std::memset(&mean, 0, sizeof(mean));
+    mean.n_parts = (uint32_t)pl.P;
+    mean.b2 = pl.b2;
+    mean.n_rec = N;
+    g->bucket_table = (uint32_t)swg::bucket_count_table(a, mean);
+    // survivors are written as they are found: room for one per 8 occurrences
+    // first (fewer at any usual coverage), exactly what is needed on a rerun
+    // of the count (the records are still there)
+    const uint64_t c = (uint64_t)std::max(a.cutoff, 1);
+    if ((st = ensure_out(g, std::max<uint64_t>(a.tag_bits ? N / 8 : std::min(N / 8, N / c), 1), 0))) return st;
+    for (int attempt = 0;; ++attempt) {
+        a.out_keys = g->d_out_keys;
+        a.out_mult = g->d_out_mult;
+        a.out_cap = g->out_cap;
+        g->launches += swg::launch_super_count(a, pl.sk, NB, (int)g->bucket_table, s);
+        SWG_CUDA(cudaGetLastError(), "bucket count launch");
+        SWG_CUDA(cudaEventRecord(g->ev[5], s), "event");
+        SWG_CUDA(cudaMemcpyAsync(g->h_ctl, g->d_ctl, sizeof(Control) - sizeof(uint64_t), cudaMemcpyDeviceToHost, s),
+                 "read status");
+        SWG_CUDA(cudaEventRecord(g->ev[4], s), "event");
+        SWG_CUDA(cudaStreamSynchronize(s), "bucket count");
+        const bool again = g->h_ctl->status & swg::kStatusPartOverflow;
+        const uint64_t n = g->h_ctl->counters[1];
+        if (!again && n <= g->out_cap) break;
+        if (attempt) {
+            swg::set_error("bucketed build: the survivors outgrew an exact count (internal error)");
+            return SWG_ERR_CUDA;
+        }
+        SWG_CUDA(cudaMemsetAsync(g->d_ctl, 0, sizeof(Control) - sizeof(uint64_t), s), "clear control");
+        if (a.tag_bits)
+            SWG_CUDA(cudaMemsetAsync(a.seg_counts, 0, 2ull * a.n_segs * 8, s), "clear sample counters");
+        if (again) {
+            a = plain;
+            return build_bucketed(g, o, a, s, load, true);
+        }
+        if ((st = ensure_out(g, n, 0))) return st;
+    }
+    const unsigned nbig = g->h_ctl->pad2;  // buckets no shared-memory table held
+    const unsigned retries = g->h_ctl->pad;
+    if (nbig) {
+        const uint64_t n_small = g->h_ctl->counters[1];
+        std::vector<unsigned long long> big(nbig), off(NB + 1), cur(NB), meta(2 * (uint64_t)nbig + 1);
+        SWG_CUDA(cudaMemcpyAsync(big.data(), pl.sk.big2, nbig * 8, cudaMemcpyDeviceToHost, s), "read big buckets");
+        SWG_CUDA(cudaMemcpyAsync(off.data(), pl.sk.off2, (NB + 1) * 8, cudaMemcpyDeviceToHost, s), "read regions");
+        SWG_CUDA(cudaMemcpyAsync(cur.data(), pl.sk.cursor2, NB * 8, cudaMemcpyDeviceToHost, s), "read cursors");
+        SWG_CUDA(cudaStreamSynchronize(s), "big buckets");
+        uint64_t records = 0;
+        for (unsigned i = 0; i < nbig; i++) {
+            meta[i] = off[big[i]];
+            meta[nbig + i] = records;
+            records += std::min<uint64_t>(cur[big[i]], off[big[i] + 1]) - off[big[i]];
+        }
+        meta[2 * (uint64_t)nbig] = records;
+        const uint64_t kmers = std::min<uint64_t>(17 * records, N);  // at most 17 a record
+        if ((st = ensure_out(g, n_small + (a.tag_bits ? kmers : kmers / c + 1), n_small))) return st;
+        a.out_keys = g->d_out_keys;
+        a.out_mult = g->d_out_mult;
+        a.out_cap = g->out_cap;
+        if ((st = ensure(&g->d_bigmeta, &g->bigmeta_cap, meta.size(), "big-bucket list"))) return st;
+        SWG_CUDA(cudaMemcpyAsync(g->d_bigmeta, meta.data(), meta.size() * 8, cudaMemcpyHostToDevice, s),
+                 "big-bucket list");
+        const uint64_t cap = (uint64_t)std::ceil((double)kmers / load) + 64;
+        if ((st = ensure(&g->d_arena, &g->arena_cap, cap, "big-bucket table"))) return st;
+        SWG_CUDA(cudaMemsetAsync(g->d_arena, 0, cap * sizeof(Entry), s), "clear big-bucket table");
+        g->launches += swg::launch_super_big(a, pl.sk, g->d_bigmeta, nbig, records, g->d_arena, cap, s);
+        g->launches += swg::launch_big_compact(a, g->d_arena, cap, s);
+        SWG_CUDA(cudaGetLastError(), "big-bucket launch");
+        SWG_CUDA(cudaMemcpyAsync(g->h_ctl, g->d_ctl, sizeof(Control) - sizeof(uint64_t), cudaMemcpyDeviceToHost, s),
+                 "read status");
+        SWG_CUDA(cudaEventRecord(g->ev[4], s), "event");
+        SWG_CUDA(cudaStreamSynchronize(s), "build");
+    }
+    if (g->h_ctl->status & swg::kStatusCasLimit) {
+        swg::set_error("a bounded CAS retry loop gave up on the device");
+        return SWG_ERR_TIMEOUT;
+    }
+    if (g->h_ctl->status & swg::kStatusTableFull) {
+        swg::set_error("a big-bucket table reached the probe limit");
+        return SWG_ERR_TABLE_FULL;
+    }
+    g->retries = retries;
+    g->estimate = 0.0;
+    g->parts = (uint32_t)pl.P;
+    g->slots = (uint32_t)(1u << pl.b2);
+    g->waves = nbig;
+    g->cap_used = NB;
+    g->n_distinct = g->h_ctl->counters[0];
+    g->n_out = g->h_ctl->counters[1];
+    g->built = true;
+    float t[5] = {0, 0, 0, 0, 0};
+    // [0] setup, [1] level-1 scatter, [2] level-2 scatter, [3] bucket count
+    cudaEventElapsedTime(&t[0], g->ev[0], g->ev[1]);
+    cudaEventElapsedTime(&t[1], g->ev[1], g->ev[2]);
+    cudaEventElapsedTime(&t[2], g->ev[2], g->ev[3]);
+    cudaEventElapsedTime(&t[3], g->ev[3], g->ev[5]);
+    cudaEventElapsedTime(&t[4], g->ev[0], g->ev[4]);
+    std::memcpy(g->ms, t, sizeof(t));
+    return SWG_OK;
+}
+
 constexpr uint64_t kStreamMin = 96ull << 20;    // shorter texts go up and are framed in one piece
 constexpr uint64_t kStreamPiece = 40ull << 20;  // target bytes per piece
 constexpr uint64_t kStreamMaxPieces = 16;
@@ -1215,6 +1485,16 @@ constexpr uint64_t kStreamMaxPieces = 16;
 // or read order, or a graph the bucketed workspace does not fit, falls back
 // to the one-shot build over the reads framed here. Results are those of the
 // one-shot build.
+// Level-1 scatter of one piece's reads (a.read_range, or all of a's reads).
+int scatter_piece(const BuildArgs &a, const BucketPlan &pl, int grid_mode, cudaStream_t s) {
+    if (!pl.super) return swg::launch_part_scatter(a, pl.pa, s, grid_mode);
+    swg::SkArgs sk = pl.sk;
+    sk.off = a.read_off;
+    sk.len = a.read_len;
+    sk.n_pieces = a.n_reads;
+    return swg::launch_super_scan(a, sk, a.n_reads, 1, false, grid_mode, s);
+}
+
 swg_status build_fasta_streamed(swg_graph *g, const swg_opts *o, const char *first, uint64_t n,
                                 cudaStream_t s, bool synced = false) {
     swg_status st;
@@ -1339,8 +1619,7 @@ swg_status build_fasta_streamed(swg_graph *g, const swg_opts *o, const char *fir
             ac.total_occ = 1;
             ac.read_range = piece_reads + 2 * c;
             SWG_CUDA(cudaMemsetAsync(&g->d_ctl->work[1], 0, sizeof(unsigned long long), s), "clear work");
-            g->launches += swg::launch_part_scatter(ac, pl.pa, s,
-                                                    c + 1 < C ? swg::kScatterShared : swg::kScatterResident);
+            g->launches += scatter_piece(ac, pl, c + 1 < C ? swg::kScatterShared : swg::kScatterResident, s);
             SWG_CUDA(cudaGetLastError(), "scatter launch");
             continue;
         }
@@ -1413,7 +1692,18 @@ swg_status build_fasta_streamed(swg_graph *g, const swg_opts *o, const char *fir
                 g->algorithm = SWG_ALGO_BUCKETED;
                 // every stride-th batch of the first piece: 1/16 to 1/8 of all reads
                 const uint32_t stride = (uint32_t)std::max<uint64_t>(1, 16 * first_blocks / nc);
-                if ((st = bucketed_plan(g, o, a0, N_est, false, stride, s, pl))) return st;
+                if (super_build(o, a0, N_est) && longest <= kSuperLongest) {
+                    swg::SkArgs reads;
+                    std::memset(&reads, 0, sizeof(reads));
+                    reads.off = g->d_off;
+                    reads.len = g->d_len;
+                    reads.n_pieces = reads_c;
+                    st = super_plan(g, o, a0, N_est, (uint64_t)(scale * (double)reads_c * 1.02), stride, 1.0 / scale,
+                                    reads, s, pl);
+                } else {
+                    st = bucketed_plan(g, o, a0, N_est, false, stride, s, pl);
+                }
+                if (st) return st;
                 SWG_CUDA(cudaEventRecord(g->ev[1], s), "event");
             }
         }
@@ -1429,8 +1719,7 @@ swg_status build_fasta_streamed(swg_graph *g, const swg_opts *o, const char *fir
             SWG_CUDA(cudaMemsetAsync(&g->d_ctl->work[1], 0, sizeof(unsigned long long), s), "clear work");
             // all but the last piece leave room for the framing of the next
             // one (its kernels would otherwise wait for this scatter to end)
-            g->launches += swg::launch_part_scatter(ac, pl.pa, s,
-                                                    c + 1 < C ? swg::kScatterShared : swg::kScatterPerBatch);
+            g->launches += scatter_piece(ac, pl, c + 1 < C ? swg::kScatterShared : swg::kScatterPerBatch, s);
             SWG_CUDA(cudaGetLastError(), "scatter launch");
         }
         NL = NLc;
@@ -1472,6 +1761,7 @@ swg_status build_fasta_streamed(swg_graph *g, const swg_opts *o, const char *fir
         return SWG_ERR_BAD_INPUT;
     }
     if (stream && o->algorithm == SWG_ALGO_DEFAULT && !bucketed_fits(g, occ)) stream = false;
+    if (stream && pl.super && longest > kSuperLongest) stream = false;  // cut in pieces by the one-shot build
     if (!stream) {  // the one-shot build over the reads framed here
         st = build_impl(g, o, g->d_packed, words, g->d_off, g->d_len, reads);
         if (st == SWG_OK) g->launches += launches;
@@ -1485,8 +1775,9 @@ swg_status build_fasta_streamed(swg_graph *g, const swg_opts *o, const char *fir
     a.n_reads = reads;
     a.total_occ = occ;
     g->occurrences = occ;
-    pl.bk.n_rec = occ;
     g->launches += launches;
+    if (pl.super) return super_finish(g, o, a, s, load, pl);
+    pl.bk.n_rec = occ;
     return bucketed_finish(g, o, a, s, load, false, pl);
 }
 
@@ -1598,6 +1889,7 @@ void swg_graph_free(swg_graph *g) {
     cudaFree(g->d_bigmeta);
     swg::merged_free(&g->mg);
     cudaFree(g->d_hll_seg);
+    cudaFree(g->d_pieces);
     cudaFree(g->d_bucket);
     cudaFree(g->d_poff);
     cudaFree(g->d_plen);

@@ -135,6 +135,56 @@ struct BucketArgs {
     int shape;                             // scatter block shape (swg_opts::scatter_shape; 0 = default)
 };
 
+// The bucketed build over super-k-mer records (super.cu): runs of k-mers
+// with one minimizer, 16 bytes each, split into partitions and buckets by the
+// minimizer's hash.
+struct SkArgs {
+    int k;
+    int b1, b2;                            // partition bits, sub-bucket bits
+    uint32_t n_parts;                      // 1 << b1
+    bool pieces;                           // off / len are pieces of long reads (flags in len)
+    const uint64_t *off;                   // reads, or pieces
+    const uint32_t *len;
+    const uint32_t *seg;                   // their samples (tagged batch)
+    uint64_t n_pieces;
+    unsigned long long *work;              // [2] batches handed out (sample, scatter), zeroed
+    unsigned long long *part_count;        // [n_parts] sampled records
+    unsigned long long *part_start;        // [n_parts + 1]
+    unsigned long long *part_cursor;       // [n_parts]
+    unsigned long long *part_end;          // [n_parts]
+    unsigned long long *sampled;           // [2] sampled records, sampled k-mers
+    unsigned long long *cursor2;           // [n_buckets] sampled records, then cursors
+    unsigned long long *off2;              // [n_buckets + 1] bucket regions
+    unsigned long long *chunk_start;       // [n_parts + 1]
+    unsigned *status;
+    uint4 *rec1, *rec2;
+    uint64_t n_kmers;                      // occurrences expected in the whole input
+    uint64_t rec_cap;                      // records the buffers are sized for
+    double scale_max;                      // records per sampled record they are sized for
+    unsigned long long *big;               // buckets too large for a tier-1 table
+    unsigned *big_count;
+    unsigned long long *big2;              // ... and for a tier-2 table
+    unsigned *big2_count;
+    uint32_t big_cap;                      // capacity of each list
+};
+
+// Super-k-mer launchers (super.cu).
+int super_window(int k);  // m-mers per k-mer; 0: k has no super-k-mer build
+// Most records that the bucket regions of k_sk_bucket_caps sum to.
+uint64_t super_bucket_room(uint64_t records, uint64_t nb, double scale_max);
+uint64_t super_pieces_bound(uint64_t n_reads, uint64_t occurrences);
+int launch_super_pieces(const BuildArgs &a, uint64_t *count, uint64_t *first, uint64_t *scratch, uint64_t *total,
+                        uint64_t *off, uint32_t *len, uint32_t *seg, cudaStream_t s);
+// bound: reads (pieces) at most; sample: sizes only, of every stride-th batch
+int launch_super_scan(const BuildArgs &a, const SkArgs &sk, uint64_t bound, uint32_t stride, bool sample,
+                      int grid_mode, cudaStream_t s);
+int launch_super_caps(const SkArgs &sk, uint64_t nb, uint64_t *scratch, cudaStream_t s);
+int launch_super_sub(const SkArgs &sk, cudaStream_t s);
+int launch_super_count(const BuildArgs &a, const SkArgs &sk, uint64_t nb, int table, cudaStream_t s);
+int launch_super_big(const BuildArgs &a, const SkArgs &sk, const unsigned long long *meta, uint32_t n,
+                     uint64_t records, Entry *table, uint64_t cap, cudaStream_t s);
+int launch_big_compact(const BuildArgs &a, const Entry *table, uint64_t cap, cudaStream_t s);
+
 // Kernel launchers (kernels.cu). Each returns the number of launches made.
 // The occurrence total (into occ_prefix[n_reads]) and, with write, the
 // per-read prefix; launch_occ_scan_write adds the prefix to a scan made
@@ -169,9 +219,6 @@ int launch_bucket_caps(const unsigned long long *counts, const unsigned long lon
                        uint64_t nb, unsigned long long *caps, cudaStream_t s);
 int launch_big_multi(const BuildArgs &a, const BucketArgs &b, const unsigned long long *meta, uint32_t n,
                      uint64_t records, Entry *table, uint64_t cap, cudaStream_t s);
-// persistent: at most the resident blocks, each taking read batches until
-// none is left; else one block per batch (blocks retire as they finish, so
-// other streams' kernels get SMs during the scatter)
 // Grid of the level-1 scatter: one block per batch of reads (blocks retire
 // as they finish), as many blocks as stay resident (each takes batches until
 // none are left), or one block per SM fewer than that, leaving room on every
