@@ -2199,7 +2199,7 @@ template <int NT, int IT, int MINB, int KC = 0, int B1C = 0>
 int launch_p1_scatter_shape(const BuildArgs &a, const PartArgs &p, cudaStream_t s, int grid_mode) {
     auto kern = k_p1_scatter<NT, IT, MINB, KC, B1C>;
     const size_t smem = p1_scatter_smem(p.n_parts, NT * IT);
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(kern, p1_scatter_smem(1u << kPartBitsMax, NT * IT));
     const uint64_t batches = (a.n_reads + NT - 1) / NT;
     const uint64_t resident = resident_grid(kern, NT, smem), sms = device_sm_count();
     uint64_t grid = batches;  // kScatterPerBatch
@@ -2216,7 +2216,7 @@ int launch_part_scatter(const BuildArgs &a, const PartArgs &p, cudaStream_t s, i
         // warp-cooperative extraction (needs the occurrence prefix and tiles)
         auto kern = k_p1_scatter_wc<256, 16, 3>;
         const size_t smem = p1_scatter_smem(p.n_parts, 256 * 16);
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_smem(kern, p1_scatter_smem(1u << kPartBitsMax, 256 * 16));
         const uint64_t grid = std::min<uint64_t>(a.n_tiles, resident_grid(kern, 256, smem));
         kern<<<(unsigned)grid, 256, smem, s>>>(a, p);
         return 1;
@@ -2287,7 +2287,7 @@ int launch_sub_scatter_shape(const BucketArgs &b, cudaStream_t s) {
     static_assert(NT * IT == kBkChunk, "a level-2 chunk is one block's round");
     auto kern = k_sub_scatter<NT, IT, MINB>;
     const uint64_t chunks = b.n_rec / kBkChunk + b.n_parts;  // bound on the partition-aligned chunks
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSubScatterDyn);
+    allow_smem(kern, kSubScatterDyn);
     const uint64_t grid = std::min<uint64_t>(chunks, resident_grid(kern, NT, kSubScatterDyn));
     kern<<<(unsigned)grid, NT, kSubScatterDyn, s>>>(b);
     return 1;
@@ -2300,7 +2300,7 @@ int launch_sub_scatter2_shape(const BucketArgs &b, cudaStream_t s) {
     auto kern = k_sub_scatter2<NT, IT, MINB>;
     const uint64_t chunks = b.n_rec / kBkChunk + b.n_parts;
     const size_t smem = sub_scatter2_smem(b.b2);
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(kern, sub_scatter2_smem(10));
     const uint64_t grid = std::min<uint64_t>(chunks, resident_grid(kern, NT, smem));
     kern<<<(unsigned)grid, NT, smem, s>>>(b);
     return 1;
@@ -2314,8 +2314,7 @@ int launch_sub_scatter(const BucketArgs &b, cudaStream_t s) {
         default: return launch_sub_scatter2_shape<256, 16, 3>(b, s);
         case 3: {  // bulk-copy staging (measured slower on GB300: 2 blocks/SM instead of 3)
             const uint64_t chunks = b.n_rec / kBkChunk + b.n_parts;
-            cudaFuncSetAttribute(k_sub_scatter_tma, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kSubScatterTmaDyn);
+            allow_smem(k_sub_scatter_tma, kSubScatterTmaDyn);
             const uint64_t grid =
                 std::min<uint64_t>(chunks, resident_grid(k_sub_scatter_tma, 256, kSubScatterTmaDyn));
             k_sub_scatter_tma<<<(unsigned)grid, 256, kSubScatterTmaDyn, s>>>(b);
@@ -2339,15 +2338,15 @@ int launch_bucket_count(const BuildArgs &a, const BucketArgs &b, cudaStream_t s)
     const size_t smem1 = bucket_smem<kBkTable>() + tag, smem2 = bucket_smem<kBkTable2>() + tag;
     if (bucket_count_table(a, b) == kBkTableS) {  // small buckets on average
         const size_t smemS = bucket_smem<kBkTableS>();
-        cudaFuncSetAttribute(k_bucket_count_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemS);
+        allow_smem(k_bucket_count_small, smemS);
         const uint64_t grid = std::min<uint64_t>(nb, resident_grid(k_bucket_count_small, kBkThreadsS, smemS));
         k_bucket_count_small<<<(unsigned)grid, kBkThreadsS, smemS, s>>>(a, b, nb);
     } else {
-        cudaFuncSetAttribute(k_bucket_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
+        allow_smem(k_bucket_count, bucket_smem<kBkTable>() + kBucketTagSmem);
         const uint64_t grid = std::min<uint64_t>(nb, resident_grid(k_bucket_count, kBkThreads, smem1));
         k_bucket_count<<<(unsigned)grid, kBkThreads, smem1, s>>>(a, b, nb);
     }
-    cudaFuncSetAttribute(k_bucket_count_large, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
+    allow_smem(k_bucket_count_large, bucket_smem<kBkTable2>() + kBucketTagSmem);
     k_bucket_count_large<<<(unsigned)device_sm_count(), kBkThreads2, smem2, s>>>(a, b);
     return 2;
 }

@@ -4,6 +4,10 @@
 
 #include <cuda_runtime.h>
 
+#include <mutex>
+#include <set>
+#include <utility>
+
 #include "swg_internal.h"
 
 namespace swg {
@@ -194,6 +198,22 @@ __device__ __forceinline__ uint64_t bucket_mult(const unsigned *cnt, uint32_t s,
 }
 
 }  // namespace
+
+// Lets a kernel use up to `most` bytes of dynamic shared memory (its largest
+// use, not the launch's own), once per device: builds run in several threads,
+// and the attribute of a kernel that another thread is launching must not
+// change under it.
+template <typename K>
+void allow_smem(K kernel, size_t most) {
+    static std::mutex mu;
+    static std::set<std::pair<int, K>> done;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lock(mu);
+    if (!done.count({dev, kernel}) &&
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) == cudaSuccess)
+        done.insert({dev, kernel});
+}
 
 // Blocks of a persistent kernel that are resident at once on the device.
 template <typename K>

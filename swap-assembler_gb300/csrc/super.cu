@@ -869,13 +869,14 @@ int scan_launch(const BuildArgs &a, const SkArgs &s, uint64_t bound, uint32_t st
     const uint64_t sms = device_sm_count();
     if (sample) {
         auto kern = k_sk_scan<M, W, true>;
+        allow_smem(kern, scan_smem(1u << kPartBitsMax, W, true));
         const uint64_t want = (batches + stride - 1) / stride;
         kern<<<(unsigned)std::max<uint64_t>(1, std::min(want, resident_grid(kern, kSkThreads, smem))), kSkThreads, smem,
                st>>>(a, s, stride);
         return 1;
     }
     auto kern = k_sk_scan<M, W, false>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(kern, scan_smem(1u << kPartBitsMax, W, false));
     const uint64_t resident = resident_grid(kern, kSkThreads, smem);
     uint64_t grid = batches;
     if (grid_mode == kScatterResident) grid = std::min(batches, resident);
@@ -942,7 +943,7 @@ int launch_super_caps(const SkArgs &s, uint64_t nb, uint64_t *scratch, cudaStrea
 int launch_super_sub(const SkArgs &s, cudaStream_t st) {
     k_sk_chunks<<<1, 1024, 0, st>>>(s);
     const size_t smem = sub_smem(s.b2);
-    cudaFuncSetAttribute(k_sk_sub, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(k_sk_sub, sub_smem(10));
     const uint64_t chunks = s.rec_cap * 5 / 4 / kSkChunk + s.n_parts;
     k_sk_sub<<<(unsigned)std::min<uint64_t>(chunks, resident_grid(k_sk_sub, 256, smem)), 256, smem, st>>>(s);
     return 2;
@@ -951,20 +952,21 @@ int launch_super_sub(const SkArgs &s, cudaStream_t st) {
 template <int kK>
 int count_launch(const BuildArgs &a, const SkArgs &s, uint64_t nb, int table, cudaStream_t st) {
     const size_t tag = a.tag_bits ? 2 * a.n_segs * sizeof(unsigned) : 0;
+    constexpr size_t tag_most = 2 * kMaxTagSamples * sizeof(unsigned);
     if (table == 2048) {
         auto kern = k_sk_count<2048, 256, kK>;
         const size_t smem = count_smem<2048, 256>() + tag;
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_smem(kern, count_smem<2048, 256>() + tag_most);
         kern<<<(unsigned)std::min<uint64_t>(nb, resident_grid(kern, 256, smem)), 256, smem, st>>>(a, s, nb);
     } else {
         auto kern = k_sk_count<4096, 512, kK>;
         const size_t smem = count_smem<4096, 512>() + tag;
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_smem(kern, count_smem<4096, 512>() + tag_most);
         kern<<<(unsigned)std::min<uint64_t>(nb, resident_grid(kern, 512, smem)), 512, smem, st>>>(a, s, nb);
     }
     auto large = k_sk_count<8192, 1024, kK>;
     const size_t smem = count_smem<8192, 1024>() + tag;
-    cudaFuncSetAttribute(large, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(large, count_smem<8192, 1024>() + tag_most);
     large<<<(unsigned)device_sm_count(), 1024, smem, st>>>(a, s, nb);
     return 2;
 }

@@ -127,3 +127,33 @@ def test_batch_of_one_k(k, lengths):
         keys, mult = g.batch_copy_out(i)
         okeys, omult = oracle.records(t, k, i % 4)
         assert np.array_equal(keys, okeys) and np.array_equal(mult, omult), i
+
+
+def test_builds_of_several_threads():
+    """Builds of different sizes (and so kernels with different shared memory)
+    from several threads, each with its own handle: every one succeeds."""
+    import threading
+    rng = np.random.default_rng(11)
+    jobs = []
+    for genome, n, k in [(5_000, 8_000, 31), (400_000, 150_000, 31), (60_000, 30_000, 21), (400_000, 150_000, 21)]:
+        text = _fasta(_sampled(rng, _random(rng, genome), n, [100]))
+        reads = swapgb.reads_from_fasta(text, k)
+        jobs.append((k, reads, swapgb.Graph().build_reads(swapgb.Opts(k=k, cutoff=2), reads).copy_out()))
+    failed = []
+
+    def work(k, reads, want):
+        g = swapgb.Graph()
+        for _ in range(40):
+            try:
+                got = g.build_reads(swapgb.Opts(k=k, cutoff=2), reads).copy_out()
+                if not (np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])):
+                    failed.append("differs")
+            except swapgb.SwgError as e:
+                failed.append(str(e))
+
+    threads = [threading.Thread(target=work, args=j) for j in jobs for _ in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed[:3]
