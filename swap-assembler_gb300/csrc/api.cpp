@@ -21,6 +21,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <thread>
 #include <vector>
@@ -127,6 +128,7 @@ struct swg_graph {
     // batched build (n_samples == 0 after a single-sample build)
     uint32_t n_samples = 0;
     std::vector<uint64_t> s_tbase, s_tcap, s_out, s_distinct, s_occ;
+    std::vector<int> s_k;
     swg::SegParams *d_segs = nullptr;
     uint64_t segs_cap = 0;
     uint32_t *d_read_seg = nullptr;
@@ -177,6 +179,7 @@ struct swg_graph {
     unsigned long long *host_keys = nullptr, *host_mult = nullptr;
     uint64_t host_cap = 0;
     bool host_out_used = false;
+    std::mutex copy_mu;  // sorted copies of one graph, from several threads, share its scratch
 };
 
 namespace {
@@ -783,6 +786,8 @@ swg_status batch_impl(swg_graph *g, const swg_opts *o, const swg_sample *sm, uin
     const uint64_t *occ_pre = meta.data() + 2 * S + 1;
     a.total_occ = occ_pre[S];
     g->occurrences = a.total_occ;
+    g->s_k.resize(S);
+    for (uint32_t i = 0; i < S; i++) g->s_k[i] = sm[i].k;
     g->s_occ.assign(S, 0);
     for (uint32_t i = 0; i < S; i++) g->s_occ[i] = occ_pre[i + 1] - occ_pre[i];
     {
@@ -1781,23 +1786,38 @@ swg_status build_fasta_streamed(swg_graph *g, const swg_opts *o, const char *fir
     return bucketed_finish(g, o, a, s, load, false, pl);
 }
 
-swg_status fetch_sorted(const swg_graph *g, std::vector<uint64_t> &keys,
-                        std::vector<uint64_t> &mult) {
-    if (!g || !g->built || g->n_samples) {
-        swg::set_error(g && g->n_samples ? "batched build: use the swg_batch_* calls"
-                                         : "graph has not been built");
-        return SWG_ERR_BAD_STATE;
+// n of the graph's records to the host: as they lie, or in key order (on the
+// device; where its scratch does not fit, on the host).
+swg_status copy_records(const swg_graph *g, const unsigned long long *d_keys, const unsigned long long *d_mult,
+                        uint64_t n, int k, bool sorted, uint64_t *keys, uint8_t *mult) {
+    if (!n) return SWG_OK;
+    SWG_CUDA(cudaSetDevice(g->device), "cudaSetDevice");
+    if (sorted) {
+        // scratch: a record buffer of the build, which has no use for it any
+        // more, or else memory of the call's own
+        std::lock_guard<std::mutex> lock(const_cast<swg_graph *>(g)->copy_mu);
+        const uint64_t want = swg::sort_scratch_bytes(n);
+        const bool first = g->records_cap >= g->rec2_cap;
+        void *ws = first ? (void *)g->d_records : (void *)g->d_rec2, *own = nullptr;
+        if (!ws || 8 * (first ? g->records_cap : g->rec2_cap) < want) {
+            if (cudaMalloc(&own, want) != cudaSuccess) cudaGetLastError();
+            ws = own;
+        }
+        if (ws) {
+            const swg_status st = swg::copy_records_sorted(d_keys, d_mult, n, 2 * k, g->own, ws, keys, mult);
+            cudaFree(own);
+            return st;
+        }
+        std::vector<uint64_t> hk(n), hm(n);
+        SWG_CUDA(cudaMemcpy(hk.data(), d_keys, n * 8, cudaMemcpyDeviceToHost), "copy keys");
+        SWG_CUDA(cudaMemcpy(hm.data(), d_mult, n * 8, cudaMemcpyDeviceToHost), "copy multiplicities");
+        swg::sort_records(hk.data(), hm.data(), n);
+        if (keys) std::memcpy(keys, hk.data(), n * 8);
+        if (mult) std::memcpy(mult, hm.data(), n * 8);
+        return SWG_OK;
     }
-    keys.resize(g->n_out);
-    mult.resize(g->n_out);
-    if (g->n_out) {
-        SWG_CUDA(cudaSetDevice(g->device), "cudaSetDevice");
-        SWG_CUDA(cudaMemcpy(keys.data(), g->d_out_keys, g->n_out * 8, cudaMemcpyDeviceToHost),
-                 "copy keys");
-        SWG_CUDA(cudaMemcpy(mult.data(), g->d_out_mult, g->n_out * 8, cudaMemcpyDeviceToHost),
-                 "copy multiplicities");
-    }
-    swg::sort_records(keys.data(), mult.data(), g->n_out);
+    if (keys) SWG_CUDA(cudaMemcpy(keys, d_keys, n * 8, cudaMemcpyDeviceToHost), "copy keys");
+    if (mult) SWG_CUDA(cudaMemcpy(mult, d_mult, n * 8, cudaMemcpyDeviceToHost), "copy multiplicities");
     return SWG_OK;
 }
 
@@ -2188,36 +2208,10 @@ swg_status swg_graph_copy_out(const swg_graph *g, uint64_t *keys, uint8_t *mult,
         swg::set_error("output capacity smaller than the survivor count");
         return SWG_ERR_BAD_INPUT;
     }
-    if (g->n_out == 0) return SWG_OK;
-    if (!sorted) {
-        SWG_CUDA(cudaSetDevice(g->device), "cudaSetDevice");
-        if (keys)
-            SWG_CUDA(cudaMemcpy(keys, g->d_out_keys, g->n_out * 8, cudaMemcpyDeviceToHost),
-                     "copy keys");
-        if (mult)
-            SWG_CUDA(cudaMemcpy(mult, g->d_out_mult, g->n_out * 8, cudaMemcpyDeviceToHost),
-                     "copy multiplicities");
-        return SWG_OK;
-    }
-    std::vector<uint64_t> k, m;
-    swg_status st = fetch_sorted(g, k, m);
-    if (st) return st;
-    if (keys) std::memcpy(keys, k.data(), g->n_out * 8);
-    if (mult) std::memcpy(mult, m.data(), g->n_out * 8);
-    return SWG_OK;
+    return copy_records(g, g->d_out_keys, g->d_out_mult, g->n_out, g->k, sorted != 0, keys, mult);
 }
 
-swg_status swg_graph_stats(const swg_graph *g, int64_t out[5]) {
-    if (!g || !out) return SWG_ERR_BAD_INPUT;
-    std::vector<uint64_t> k, m;
-    swg_status st = fetch_sorted(g, k, m);
-    if (st) return st;
-    swg::graph_stats(reinterpret_cast<const uint8_t *>(m.data()), g->n_out, g->k, out);
-    return SWG_OK;
-}
-
-// Both text outputs are formatted on the device (emit.cu) from the
-// device-resident records and streamed to the file.
+// A single-sample graph has been built.
 static swg_status writable(const swg_graph *g) {
     if (!g->built || g->n_samples) {
         swg::set_error(g->n_samples ? "batched build: use the swg_batch_* calls" : "graph has not been built");
@@ -2226,6 +2220,18 @@ static swg_status writable(const swg_graph *g) {
     return SWG_OK;
 }
 
+swg_status swg_graph_stats(const swg_graph *g, int64_t out[5]) {
+    if (!g || !out) return SWG_ERR_BAD_INPUT;
+    swg_status st = writable(g);
+    if (st) return st;
+    std::vector<uint8_t> m(8 * g->n_out);  // totals: the order does not matter
+    if ((st = copy_records(g, g->d_out_keys, g->d_out_mult, g->n_out, g->k, false, nullptr, m.data()))) return st;
+    swg::graph_stats(m.data(), g->n_out, g->k, out);
+    return SWG_OK;
+}
+
+// Both text outputs are formatted on the device (emit.cu) from the
+// device-resident records and streamed to the file.
 swg_status swg_graph_write_kmer_graph(const swg_graph *g, const char *path) {
     Phase phase("printKmerGraph");
     if (!g || !path) return SWG_ERR_BAD_INPUT;
@@ -2463,17 +2469,8 @@ swg_status swg_batch_copy_out(const swg_graph *g, uint32_t s, uint64_t *keys, ui
         swg::set_error("output capacity smaller than the survivor count");
         return SWG_ERR_BAD_INPUT;
     }
-    if (!cnt) return SWG_OK;
-    std::vector<uint64_t> k(cnt), m(cnt);
-    SWG_CUDA(cudaSetDevice(g->device), "cudaSetDevice");
-    SWG_CUDA(cudaMemcpy(k.data(), g->d_out_keys + g->s_tbase[s], cnt * 8, cudaMemcpyDeviceToHost),
-             "copy keys");
-    SWG_CUDA(cudaMemcpy(m.data(), g->d_out_mult + g->s_tbase[s], cnt * 8, cudaMemcpyDeviceToHost),
-             "copy multiplicities");
-    if (sorted) swg::sort_records(k.data(), m.data(), cnt);
-    if (keys) std::memcpy(keys, k.data(), cnt * 8);
-    if (mult) std::memcpy(mult, m.data(), cnt * 8);
-    return SWG_OK;
+    return copy_records(g, g->d_out_keys + g->s_tbase[s], g->d_out_mult + g->s_tbase[s], cnt, g->s_k[s], sorted != 0,
+                        keys, mult);
 }
 
 swg_status swg_graph_build_info(const swg_graph *g, swg_build_info *info) {

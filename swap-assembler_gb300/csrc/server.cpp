@@ -54,6 +54,8 @@ struct Request {
 
 }  // namespace
 
+constexpr uint64_t kFetchKeep = 256ull << 20;
+
 struct swg_server {
     swg_server_opts opts;
     int device = 0;
@@ -74,6 +76,7 @@ struct swg_server {
     std::string dead_error;     // set when every worker failed its set-up
     std::vector<std::thread> workers;
     cudaStream_t fetch_stream = nullptr;
+    cudaMemPool_t pool = nullptr;  // scratch of sorted fetches; keeps at most kFetchKeep mapped between them
 };
 
 namespace {
@@ -278,6 +281,18 @@ swg_status swg_server_create(const swg_server_opts *o, swg_server **out) {
         swg::set_error("stream creation failed");
         return SWG_ERR_CUDA;
     }
+    cudaMemPoolProps props;
+    std::memset(&props, 0, sizeof(props));
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = srv->device;
+    uint64_t keep = kFetchKeep;
+    if (cudaMemPoolCreate(&srv->pool, &props) != cudaSuccess ||
+        cudaMemPoolSetAttribute(srv->pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+        cudaGetLastError();
+        if (srv->pool) cudaMemPoolDestroy(srv->pool);
+        srv->pool = nullptr;  // the device's default pool instead
+    }
     srv->live_workers = srv->opts.workers;
     for (uint32_t i = 0; i < srv->opts.workers; i++) srv->workers.emplace_back(worker_main, srv);
     *out = srv;
@@ -443,20 +458,32 @@ swg_status swg_server_fetch(swg_server *srv, uint64_t ticket, uint64_t *keys, ui
     swg_status st = SWG_OK;
     cudaSetDevice(srv->device);
     if (r->n_out) {
-        std::vector<uint64_t> k(r->n_out), m(r->n_out);
-        cudaError_t e = cudaMemcpyAsync(k.data(), r->d_keys, r->n_out * 8, cudaMemcpyDeviceToHost,
-                                        srv->fetch_stream);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(m.data(), r->d_mult, r->n_out * 8, cudaMemcpyDeviceToHost,
-                                srv->fetch_stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(srv->fetch_stream);
-        if (e != cudaSuccess) {
-            swg::set_error(std::string("fetch: ") + cudaGetErrorString(e));
-            st = SWG_ERR_CUDA;
-        } else {
-            if (sorted) swg::sort_records(k.data(), m.data(), r->n_out);
-            if (keys) std::memcpy(keys, k.data(), r->n_out * 8);
-            if (mult) std::memcpy(mult, m.data(), r->n_out * 8);
+        void *ws = nullptr;
+        const uint64_t want = swg::sort_scratch_bytes(r->n_out);
+        if (sorted && (srv->pool ? cudaMallocFromPoolAsync(&ws, want, srv->pool, srv->fetch_stream)
+                                 : cudaMallocAsync(&ws, want, srv->fetch_stream)) != cudaSuccess) {
+            cudaGetLastError();
+            ws = nullptr;
+        }
+        if (ws) {
+            st = swg::copy_records_sorted(r->d_keys, r->d_mult, r->n_out, 2 * r->k, srv->fetch_stream, ws, keys, mult);
+            cudaFreeAsync(ws, srv->fetch_stream);
+        } else {  // as they lie (in key order on the host where the device scratch does not fit)
+            std::vector<uint64_t> k(r->n_out), m(r->n_out);
+            cudaError_t e = cudaMemcpyAsync(k.data(), r->d_keys, r->n_out * 8, cudaMemcpyDeviceToHost,
+                                            srv->fetch_stream);
+            if (e == cudaSuccess)
+                e = cudaMemcpyAsync(m.data(), r->d_mult, r->n_out * 8, cudaMemcpyDeviceToHost,
+                                    srv->fetch_stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(srv->fetch_stream);
+            if (e != cudaSuccess) {
+                swg::set_error(std::string("fetch: ") + cudaGetErrorString(e));
+                st = SWG_ERR_CUDA;
+            } else {
+                if (sorted) swg::sort_records(k.data(), m.data(), r->n_out);
+                if (keys) std::memcpy(keys, k.data(), r->n_out * 8);
+                if (mult) std::memcpy(mult, m.data(), r->n_out * 8);
+            }
         }
     }
     free_result(srv, r);
@@ -514,6 +541,7 @@ void swg_server_free(swg_server *srv) {
     }
     cudaStreamSynchronize(srv->fetch_stream);
     cudaStreamDestroy(srv->fetch_stream);
+    if (srv->pool) cudaMemPoolDestroy(srv->pool);
     cudaStreamSynchronize(srv->upload_stream);
     cudaStreamDestroy(srv->upload_stream);
     delete srv;

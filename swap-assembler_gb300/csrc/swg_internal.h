@@ -309,6 +309,11 @@ swg_status write_node_lines(const uint64_t *keys, const uint8_t *mult, uint64_t 
                             const char *path);
 void graph_stats(const uint8_t *mult, uint64_t n, int k, int64_t out[5]);
 void sort_records(uint64_t *keys, uint64_t *mult8, uint64_t n);
+// n device records copied to the host in key order (sort.cu; keys below
+// 2^bits), through ws: sort_scratch_bytes(n) of device scratch.
+uint64_t sort_scratch_bytes(uint64_t n);
+swg_status copy_records_sorted(const unsigned long long *d_keys, const unsigned long long *d_mult, uint64_t n, int bits,
+                               cudaStream_t s, void *ws, uint64_t *keys, uint8_t *mult);
 uint64_t revcomp_host(uint64_t x, int k);
 // Device emission of the text outputs (emit.cu), byte-identical with the host
 // writers: records on the device, any order.
