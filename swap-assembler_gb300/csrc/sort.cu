@@ -22,40 +22,199 @@ constexpr int kDigits = 256;
 constexpr int kItems = 16;              // records per thread of a pass
 constexpr uint32_t kTile = 256 * kItems;
 
-// Bitonic sort of the keys with their index; the multiplicities follow the
-// index. Padded with the largest key.
+// Bitonic sort of m (a power of two, at most 1024 R) keys by 1024 threads;
+// thread t holds keys R t .. R t + R - 1, with an index each. Partners at a
+// distance below R are in the thread, below 32 R in the warp (shuffles), the
+// others go through shared memory (a sort of 4096 has 15 such steps of 78; all
+// 78 through shared memory took 40 us, the launch included).
+template <int R, bool kIdx>
+__device__ __forceinline__ void bitonic(unsigned long long (&v)[R], unsigned (&ix)[R], unsigned long long *sk,
+                                        unsigned short *si, uint32_t m) {
+    const uint32_t t = threadIdx.x, e0 = t * R;
+    for (uint32_t k = 2; k <= m; k <<= 1)
+        for (uint32_t j = k >> 1; j; j >>= 1) {
+            if (j < R) {
+#pragma unroll
+                for (int jj = R / 2; jj; jj >>= 1) {
+                    if (j != (uint32_t)jj) continue;
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        if (r & jj) continue;
+                        if ((v[r] > v[r | jj]) == (((e0 + r) & k) == 0)) {
+                            const unsigned long long x = v[r];
+                            v[r] = v[r | jj];
+                            v[r | jj] = x;
+                            const unsigned u = ix[r];
+                            ix[r] = ix[r | jj];
+                            ix[r | jj] = u;
+                        }
+                    }
+                }
+                continue;
+            }
+            const uint32_t d = j / R;
+            const bool least = ((e0 & k) == 0) == ((t & d) == 0);  // this side keeps the smaller key
+            if (d >= 32) {
+                __syncthreads();
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    sk[r * 1024 + t] = v[r];
+                    if (kIdx) si[r * 1024 + t] = (unsigned short)ix[r];
+                }
+                __syncthreads();
+            }
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const unsigned long long y = d < 32 ? __shfl_xor_sync(0xffffffffu, v[r], d) : sk[r * 1024 + (t ^ d)];
+                const unsigned u = !kIdx ? 0 : (d < 32 ? __shfl_xor_sync(0xffffffffu, ix[r], d) : si[r * 1024 + (t ^ d)]);
+                if ((v[r] > y) == least) {
+                    v[r] = y;
+                    ix[r] = u;
+                }
+            }
+        }
+}
+
+// n <= kOne records ordered by one block: the keys with their index, the
+// multiplicities after it. Padded with the largest key.
+__device__ __forceinline__ void sort_block(unsigned long long *sk, unsigned short *si,
+                                           const unsigned long long *__restrict__ keys,
+                                           const unsigned long long *__restrict__ mult, uint32_t n,
+                                           unsigned long long *__restrict__ okeys,
+                                           unsigned long long *__restrict__ omult) {
+    constexpr int R = kOne / 1024;
+    uint32_t m = 32;
+    while (m < n) m <<= 1;
+    unsigned long long v[R];
+    unsigned ix[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        ix[r] = threadIdx.x * R + r;
+        v[r] = ix[r] < n ? keys[ix[r]] : ~0ull;
+    }
+    bitonic<R, true>(v, ix, sk, si, m);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const uint32_t i = threadIdx.x * R + r;
+        if (i < n) {
+            okeys[i] = v[r];
+            omult[i] = mult[ix[r]];
+        }
+    }
+}
+
 __global__ void __launch_bounds__(1024) k_sort_one(const unsigned long long *__restrict__ keys,
                                                    const unsigned long long *__restrict__ mult, uint32_t n,
                                                    unsigned long long *__restrict__ okeys,
                                                    unsigned long long *__restrict__ omult) {
     __shared__ unsigned long long sk[kOne];
     __shared__ unsigned short si[kOne];
+    sort_block(sk, si, keys, mult, n, okeys, omult);
+}
+
+// ---- splitters: nb buckets of kMean records on average, from a sample of
+// kOver keys a bucket at even strides (the keys are distinct, so that the
+// quantiles of any distribution are splitters; at 8 sampled keys a bucket one
+// of 4 times the mean, which would not fit, has odds of 1e-9). Such a bucket
+// sets *over, and the records take the radix passes.
+constexpr uint32_t kMean = 1024, kOver = 8, kSplitBuckets = 1024;
+constexpr uint64_t kSplitMost = (uint64_t)kMean * kSplitBuckets;
+constexpr uint32_t kSampleMost = kOver * kSplitBuckets;
+
+__global__ void __launch_bounds__(1024) k_sort_split(const unsigned long long *__restrict__ keys, uint64_t n, uint32_t nb,
+                                                     unsigned long long *__restrict__ splitters,
+                                                     unsigned *__restrict__ cursor, unsigned *__restrict__ over) {
+    extern __shared__ __align__(16) unsigned char dyn[];
+    unsigned long long *sk = reinterpret_cast<unsigned long long *>(dyn);
+    constexpr int R = kSampleMost / 1024;
+    const uint32_t count = kOver * nb;
     uint32_t m = 32;
-    while (m < n) m <<= 1;
-    for (uint32_t i = threadIdx.x; i < m; i += 1024) {
-        sk[i] = i < n ? keys[i] : ~0ull;
-        si[i] = (unsigned short)i;
+    while (m < count) m <<= 1;
+    unsigned long long v[R];
+    unsigned ix[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const uint32_t i = threadIdx.x * R + r;
+        v[r] = i < count ? keys[(uint64_t)i * n / count] : ~0ull;
+        ix[r] = 0;
     }
-    for (uint32_t k = 2; k <= m; k <<= 1)
-        for (uint32_t j = k >> 1; j; j >>= 1) {
-            __syncthreads();
-            for (uint32_t t = threadIdx.x; t < m / 2; t += 1024) {
-                const uint32_t a = 2 * t - (t & (j - 1)), b = a + j;  // the pair's lower and upper place
-                const unsigned long long x = sk[a], y = sk[b];
-                if ((x > y) == ((a & k) == 0)) {
-                    sk[a] = y;
-                    sk[b] = x;
-                    const unsigned short u = si[a];
-                    si[a] = si[b];
-                    si[b] = u;
-                }
+    bitonic<R, false>(v, ix, sk, nullptr, m);
+    static_assert(R == kOver, "a thread's first key is a splitter");
+    if (threadIdx.x < nb) {  // bucket b: from splitters[b] (0: from the start) to splitters[b + 1]
+        splitters[threadIdx.x] = v[0];
+        cursor[threadIdx.x] = 0;
+    }
+    if (threadIdx.x == 0) *over = 0;
+}
+
+// Records to their buckets' regions of kOne records each, in any order.
+constexpr int kSplitItems = 8;
+__global__ void __launch_bounds__(256) k_sort_scatter(const unsigned long long *__restrict__ keys,
+                                                      const unsigned long long *__restrict__ mult, uint64_t n, uint32_t nb,
+                                                      const unsigned long long *__restrict__ splitters,
+                                                      unsigned *__restrict__ cursor, unsigned *__restrict__ over,
+                                                      unsigned long long *__restrict__ bkeys,
+                                                      unsigned long long *__restrict__ bmult) {
+    __shared__ unsigned long long sp[kSplitBuckets];
+    __shared__ unsigned hist[kSplitBuckets];
+    for (uint32_t b = threadIdx.x; b < nb; b += 256) {
+        sp[b] = splitters[b];
+        hist[b] = 0;
+    }
+    __syncthreads();
+    unsigned long long kv[kSplitItems];
+    unsigned at[kSplitItems];  // bucket | rank << 10
+    const uint64_t r0 = (uint64_t)blockIdx.x * (256 * kSplitItems) + threadIdx.x;
+#pragma unroll
+    for (int i = 0; i < kSplitItems; ++i) {
+        const uint64_t r = r0 + 256 * i;
+        kv[i] = 0;
+        at[i] = 0;
+        if (r < n) {
+            kv[i] = keys[r];
+            uint32_t lo = 0, hi = nb;
+            while (hi - lo > 1) {
+                const uint32_t mid = (lo + hi) >> 1;
+                if (sp[mid] <= kv[i]) lo = mid;
+                else hi = mid;
+            }
+            at[i] = lo | atomicAdd(&hist[lo], 1u) << 10;
+        }
+    }
+    __syncthreads();
+    for (uint32_t b = threadIdx.x; b < nb; b += 256)
+        if (hist[b]) hist[b] = atomicAdd(&cursor[b], hist[b]);
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kSplitItems; ++i) {
+        const uint64_t r = r0 + 256 * i;
+        if (r < n) {
+            const uint32_t b = at[i] & (kSplitBuckets - 1), p = hist[b] + (at[i] >> 10);
+            if (p < kOne) {
+                bkeys[(uint64_t)b * kOne + p] = kv[i];
+                bmult[(uint64_t)b * kOne + p] = mult[r];
+            } else {
+                *over = 1;
             }
         }
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < n; i += 1024) {
-        okeys[i] = sk[i];
-        omult[i] = mult[si[i]];
     }
+}
+
+// Bucket blockIdx.x ordered to its place: after the buckets before it.
+__global__ void __launch_bounds__(1024) k_sort_buckets(const unsigned *__restrict__ cursor,
+                                                       const unsigned *__restrict__ over,
+                                                       const unsigned long long *__restrict__ bkeys,
+                                                       const unsigned long long *__restrict__ bmult,
+                                                       unsigned long long *__restrict__ okeys,
+                                                       unsigned long long *__restrict__ omult) {
+    __shared__ unsigned long long sk[kOne];
+    __shared__ unsigned short si[kOne];
+    __shared__ uint64_t wb[32];
+    if (*over) return;
+    uint64_t base = 0;  // nb <= 1024: one count a thread
+    block_exclusive_scan<1024>(threadIdx.x < blockIdx.x ? cursor[threadIdx.x] : 0u, wb, &base);
+    const uint64_t r0 = (uint64_t)blockIdx.x * kOne;
+    sort_block(sk, si, bkeys + r0, bmult + r0, cursor[blockIdx.x], okeys + base, omult + base);
 }
 
 // Records per digit of every tile, digit-major.
@@ -147,21 +306,35 @@ __global__ void __launch_bounds__(256) k_sort_pass(const unsigned long long *__r
 
 uint64_t sort_scratch_bytes(uint64_t n) {
     if (n <= kOne) return 16 * n;
+    const uint64_t nb = (n + kMean - 1) / kMean;
+    const uint64_t split = n <= kSplitMost ? 16 * n + 16 * nb * kOne + 16 * nb + 16 : 0;
     const uint64_t nc = (n + kTile - 1) / kTile * kDigits;
-    return 32 * n + 8 * (nc + gscan_scratch(nc) + 1);
+    return std::max(split, 32 * n + 8 * (nc + gscan_scratch(nc) + 1));
 }
 
 // ws: sort_scratch_bytes(n) of device scratch, 8-byte aligned. The inputs are
-// not touched.
+// not touched. radix: the radix passes whatever the size.
 swg_status copy_records_sorted(const unsigned long long *d_keys, const unsigned long long *d_mult, uint64_t n, int bits,
-                               cudaStream_t s, void *ws, uint64_t *keys, uint8_t *mult) {
+                               cudaStream_t s, void *ws, uint64_t *keys, uint8_t *mult, bool radix) {
     if (!n) return SWG_OK;
+    unsigned too_large = 0;
     unsigned long long *k[2], *m[2];
     k[0] = static_cast<unsigned long long *>(ws);
     m[0] = k[0] + n;
     int at = 0;
     if (n <= kOne) {
         k_sort_one<<<1, 1024, 0, s>>>(d_keys, d_mult, (uint32_t)n, k[0], m[0]);
+    } else if (n <= kSplitMost && !radix) {
+        const uint32_t nb = (uint32_t)((n + kMean - 1) / kMean);
+        unsigned long long *bk = m[0] + n, *bm = bk + (uint64_t)nb * kOne, *sp = bm + (uint64_t)nb * kOne;
+        unsigned *cursor = reinterpret_cast<unsigned *>(sp + nb), *over = cursor + nb;
+        allow_smem(k_sort_split, kSampleMost * sizeof(unsigned long long));
+        k_sort_split<<<1, 1024, kSampleMost * sizeof(unsigned long long), s>>>(d_keys, n, nb, sp, cursor, over);
+        k_sort_scatter<<<(unsigned)((n + 256 * kSplitItems - 1) / (256 * kSplitItems)), 256, 0, s>>>(
+            d_keys, d_mult, n, nb, sp, cursor, over, bk, bm);
+        k_sort_buckets<<<nb, 1024, 0, s>>>(cursor, over, bk, bm, k[0], m[0]);
+        EMIT_CUDA(cudaGetLastError(), "sort kernels");
+        EMIT_CUDA(cudaMemcpyAsync(&too_large, over, sizeof(unsigned), cudaMemcpyDeviceToHost, s), "sort status");
     } else {
         k[1] = m[0] + n;
         m[1] = k[1] + n;
@@ -180,7 +353,7 @@ swg_status copy_records_sorted(const unsigned long long *d_keys, const unsigned 
     if (keys) EMIT_CUDA(cudaMemcpyAsync(keys, k[at], n * 8, cudaMemcpyDeviceToHost, s), "copy keys");
     if (mult) EMIT_CUDA(cudaMemcpyAsync(mult, m[at], n * 8, cudaMemcpyDeviceToHost, s), "copy multiplicities");
     EMIT_CUDA(cudaStreamSynchronize(s), "sorted copy");
-    return SWG_OK;
+    return too_large ? copy_records_sorted(d_keys, d_mult, n, bits, s, ws, keys, mult, true) : SWG_OK;
 }
 
 }  // namespace swg

@@ -313,7 +313,7 @@ void sort_records(uint64_t *keys, uint64_t *mult8, uint64_t n);
 // 2^bits), through ws: sort_scratch_bytes(n) of device scratch.
 uint64_t sort_scratch_bytes(uint64_t n);
 swg_status copy_records_sorted(const unsigned long long *d_keys, const unsigned long long *d_mult, uint64_t n, int bits,
-                               cudaStream_t s, void *ws, uint64_t *keys, uint8_t *mult);
+                               cudaStream_t s, void *ws, uint64_t *keys, uint8_t *mult, bool radix = false);
 uint64_t revcomp_host(uint64_t x, int k);
 // Device emission of the text outputs (emit.cu), byte-identical with the host
 // writers: records on the device, any order.
