@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <cstdio>
 #include <string>
 
 #include "swapgb.h"
@@ -317,7 +318,19 @@ swg_status copy_records_sorted(const unsigned long long *d_keys, const unsigned 
 uint64_t revcomp_host(uint64_t x, int k);
 // Device emission of the text outputs (emit.cu), byte-identical with the host
 // writers: records on the device, any order.
-// Device text -> file through two pinned 64 MiB buffers (emit.cu).
+// Device text -> file through two pinned buffers (emit.cu). Opened (and
+// emptied) on its own, so that this can overlap kernels in flight; write
+// closes it.
+struct TextFile {
+    const char *path;
+    FILE *fp = nullptr;
+    explicit TextFile(const char *p) : path(p) {}
+    ~TextFile();
+    TextFile(const TextFile &) = delete;
+    TextFile &operator=(const TextFile &) = delete;
+    swg_status open();
+    swg_status write(const char *d_text, uint64_t bytes, cudaStream_t s);
+};
 swg_status stream_to_file(const char *d_text, uint64_t bytes, const char *path, cudaStream_t s);
 // The merged graph on the device: the -d file's text (gathered node lines in
 // key order + final '\n') and, per line, its node key and per arc slot the
