@@ -1097,7 +1097,7 @@ swg_status bucketed_finish(swg_graph *g, const swg_opts *o, BuildArgs &a, cudaSt
     SWG_CUDA(cudaGetLastError(), "bucket scatter launch");
     SWG_CUDA(cudaEventRecord(g->ev[3], s), "event");
     g->launches += swg::launch_bucket_count(a, bk, s);
-    g->bucket_table = (uint32_t)swg::bucket_count_table(a, bk);
+    g->bucket_table = (uint32_t)swg::bucket_count_table(a.tag_bits != 0, bk.n_rec, (uint64_t)bk.n_parts << bk.b2);
     SWG_CUDA(cudaEventRecord(g->ev[5], s), "event");
     g->launches += swg::launch_gscan(reinterpret_cast<const uint64_t *>(bk.surv),
                                      reinterpret_cast<uint64_t *>(bk.surv_off), NB,
@@ -1368,12 +1368,8 @@ swg_status super_finish(swg_graph *g, const swg_opts *o, BuildArgs &a, cudaStrea
     g->launches += swg::launch_super_sub(pl.sk, s);
     SWG_CUDA(cudaGetLastError(), "bucket scatter launch");
     SWG_CUDA(cudaEventRecord(g->ev[3], s), "event");
-    swg::BucketArgs mean;  // the table choice looks at the plan's mean bucket
-    std::memset(&mean, 0, sizeof(mean));
-    mean.n_parts = (uint32_t)pl.P;
-    mean.b2 = pl.b2;
-    mean.n_rec = N;
-    g->bucket_table = (uint32_t)swg::bucket_count_table(a, mean);
+    // (of a batch's per-sample tallies, only as many as there are samples sit beside the tables)
+    g->bucket_table = (uint32_t)swg::bucket_count_table(false, N, NB);
     // survivors are written as they are found: room for one per 8 occurrences
     // first (fewer at any usual coverage), exactly what is needed on a rerun
     // of the count (the records are still there)

@@ -514,16 +514,18 @@ __device__ __forceinline__ bool bucket_keep(const unsigned *cnt, uint32_t s, uns
 //  1. Equal records are merged: at a coverage of 30 to 50 reads most runs of a
 //     bucket repeat others base for base, so counting each distinct one once,
 //     with a weight, spares most of the expansion and of the table's atomics.
-//     Up to CH records (nearly every bucket's all) sit in the registers of
-//     their threads and in the counter array, which is all zero between
-//     buckets; a small table there maps a record's hash to the first record
-//     with these bases, which collects the others' count.
-//  2. The warps expand their distinct records, 32 k-mers at a time, into the
-//     table: 64-bit CAS on the key, two 32-bit adds on 16-bit halves, every
-//     new slot in the warp's own list.
-//  3. The listed slots give the survivors: counted first (one global atomic
-//     per bucket takes their place in the output), then written; the slots
-//     are cleared on the way.
+//     Up to CH records (nearly every bucket's all) go to the counter array,
+//     which is all zero between buckets; a small table there maps a record's
+//     hash to the first record with these bases, and counts the others.
+//  2. The distinct records are listed, with the k-mers before them, and each
+//     warp takes an even share of the k-mers (the warps wait for each other at
+//     the bucket's end) into registers; the counter array is zero again.
+//  3. The warps expand their records, 32 k-mers at a time, into the table:
+//     64-bit CAS on the key, two 32-bit adds on 16-bit halves, every new slot
+//     in the warp's own list.
+//  4. The listed slots give the survivors: counted first (one global atomic
+//     per warp takes their place in the output, so that no warp waits for
+//     another here), then written; the slots are cleared on the way.
 // Buckets whose keys do not fit go to the overflow list uncounted; their
 // records stay as they are.
 template <int T, int NT, int kK>
@@ -533,19 +535,20 @@ __device__ void count_pass(const BuildArgs &a, const SkArgs &s, uint64_t n_items
     constexpr int NW = NT / 32, SEG = T * 3 / 2 / NW, R = NT == 1024 ? 3 : 4;
     constexpr uint32_t CH = R * NT;
     static_assert((1 << kBits) == T, "table sizes");
-    static_assert(CH <= kSkClamp && CH * 28 <= T * 16, "merged records fit the counters' 16 bits and their array");
+    constexpr uint32_t kEven = 16 * R * NW;  // distinct records shared out by their k-mers
+    static_assert(CH <= kSkClamp && CH * 24 <= T * 16, "merged records fit the counters' 16 bits and their array");
+    static_assert(CH * 4 + kEven * 2 <= NW * SEG * 2, "the distinct records' list fits the slots' lists");
     extern __shared__ __align__(16) unsigned char dyn[];
     unsigned long long *keys = reinterpret_cast<unsigned long long *>(dyn);
     unsigned *cnt = reinterpret_cast<unsigned *>(keys + T);
     unsigned short *lists = reinterpret_cast<unsigned short *>(cnt + 4 * T);
     unsigned *s_dist = reinterpret_cast<unsigned *>(lists + NW * SEG);  // tagged batch only
     unsigned *s_surv = s_dist + a.n_segs;
-    uint4 *srec = reinterpret_cast<uint4 *>(cnt);       // merging: records,
-    unsigned *sdup = cnt + 4 * CH;                      // others equal to each,
-    unsigned *stab = sdup + CH;                         // table of first records (index + 1)
-    __shared__ unsigned s_over, s_nused, s_kept;
-    __shared__ unsigned long long s_out;
-    __shared__ unsigned char s_lane[NT];
+    uint4 *srec = reinterpret_cast<uint4 *>(cnt);                // merging: records,
+    unsigned *stab = cnt + 4 * CH;                               // table: first record (index + 1) | others << 16;
+    unsigned *sdis = reinterpret_cast<unsigned *>(lists);        // distinct records: index | weight << 16,
+    unsigned short *sbefore = reinterpret_cast<unsigned short *>(sdis + CH);  // k-mers before each
+    __shared__ unsigned s_over, s_total;
     const uint32_t lane = threadIdx.x & 31, wp = threadIdx.x >> 5, lt = (1u << lane) - 1;
     unsigned short *const used = lists + wp * SEG;
     const int tb = a.tag_bits, k = s.k;
@@ -560,28 +563,22 @@ __device__ void count_pass(const BuildArgs &a, const SkArgs &s, uint64_t n_items
     const unsigned cbias = (0x8000u - (unsigned)min(max(c, 1), 255)) * 0x00010001u;
     const uint4 none = make_uint4(0, 0, 0, 0);
     uint4 rec[R];
-    // the warp's even share [b0, b1) of a bucket's first min(n, CH) records, in
-    // groups of per <= 32
-    uint32_t b0 = 0, b1 = 0, per = 0;
-    auto share = [&](uint64_t n) {
-        const uint32_t n0 = (uint32_t)umin64(n, CH);
-        b0 = n0 * wp / NW;
-        b1 = n0 * (wp + 1) / NW;
-        per = (b1 - b0 + 31) / 32;
-        per = per ? (b1 - b0 + per - 1) / per : 0;
-    };
-    auto mine = [&](int i) { return lane < per && b0 + per * i + lane < b1; };
-    auto load = [&](uint64_t rb) {
+    // record i * NT + threadIdx.x of a bucket's first min(n, CH)
+    auto load = [&](uint64_t rb, uint64_t n) {
 #pragma unroll
-        for (int i = 0; i < R; ++i) rec[i] = mine(i) ? s.rec2[rb + b0 + per * i + lane] : none;
+        for (int i = 0; i < R; ++i) {
+            const uint32_t r = i * NT + threadIdx.x;
+            rec[i] = r < n ? s.rec2[rb + r] : none;
+        }
     };
     // bucket of item it, its records [rb, rb + nrec)
     uint64_t bk = 0, rb = 0, nrec = 0;
+    bool outgrown = false;
     auto bounds = [&](uint64_t it) {
         bk = list ? list[it] : it;
         rb = s.off2[bk];
         const uint64_t end = s.cursor2[bk], lim = s.off2[bk + 1];
-        if (threadIdx.x == 0 && end > lim) atomicOr(s.status, kStatusPartOverflow);
+        outgrown |= end > lim;
         nrec = umin64(end, lim) - rb;
     };
     uint64_t next_bk = 0, next_rb = 0, next_n = 0;
@@ -590,17 +587,17 @@ __device__ void count_pass(const BuildArgs &a, const SkArgs &s, uint64_t n_items
         next_bk = bk, next_rb = rb, next_n = nrec;
     }
     bool have = false;  // rec holds this bucket's first records
+    unsigned long long distinct = 0;  // keys this warp added to tables
     for (uint64_t it = blockIdx.x; it < n_items; it += gridDim.x) {
         const uint64_t nit = it + gridDim.x;
         {
-            const uint64_t tb_ = next_bk, tr = next_rb, tn = next_n;
+            const uint64_t tk = next_bk, tr = next_rb, tn = next_n;
             if (nit < n_items) bounds(nit);
             else nrec = 0;
             next_bk = bk, next_rb = rb, next_n = nrec;
-            bk = tb_, rb = tr, nrec = tn;
+            bk = tk, rb = tr, nrec = tn;
         }
-        share(nrec);
-        if (!have) load(rb);
+        if (!have) load(rb, nrec);
         have = false;
         if (nrec == 0 || nrec > kSkBigRecords) {
             if (nrec && threadIdx.x == 0) {
@@ -612,50 +609,100 @@ __device__ void count_pass(const BuildArgs &a, const SkArgs &s, uint64_t n_items
         __syncthreads();  // the previous bucket is done: the table is all zero
         if (threadIdx.x == 0) {
             s_over = 0;
-            s_nused = 0;
-            s_kept = 0;
+            s_total = 0;
         }
         // equal records among the first CH merged
-        const int tbits = min(31 - __clz(4 * (uint32_t)umin64(nrec, CH) + 255), 31 - __clz(2 * CH));
+        const uint32_t n0 = (uint32_t)umin64(nrec, CH);
+        const int tbits = min(31 - __clz(4 * n0 + 255), 31 - __clz(2 * CH));
 #pragma unroll
         for (int i = 0; i < R; ++i)
-            if (mine(i)) srec[b0 + per * i + lane] = rec[i];
+            if (i * NT + threadIdx.x < n0) srec[i * NT + threadIdx.x] = rec[i];
         __syncthreads();
-        uint32_t weight[R];
+        uint32_t first[R];   // slot of the table where record i is the first with its bases; ~0: it is not
+        uint32_t own = 0;    // this thread's distinct records << 16 | their k-mers
 #pragma unroll
         for (int i = 0; i < R; ++i) {
-            weight[i] = 0;
-            const uint32_t r = b0 + per * i + lane;
-            if (mine(i)) {
+            first[i] = ~0u;
+            const uint32_t r = i * NT + threadIdx.x;
+            if (r < n0) {
                 uint32_t h = (rec[i].x * 0x9e3779b1u ^ rec[i].y * 0x85ebca6bu) + (rec[i].z * 0xc2b2ae35u ^ rec[i].w * 0x27d4eb2fu);
                 h = (h ^ h >> 15) * 0x2c1b3c6du >> (32 - tbits);
                 for (;;) {  // ends: the table has free slots
                     const unsigned old = atomicCAS(&stab[h], 0u, r + 1);
                     if (old == 0) {
-                        weight[i] = 1;
+                        first[i] = h;
+                        own += 1u << 16 | (rec[i].w & 31u);
                         break;
                     }
-                    const uint4 x = srec[old - 1];
+                    const uint4 x = srec[(old & 0xffffu) - 1];
                     if (x.x == rec[i].x && x.y == rec[i].y && x.z == rec[i].z && x.w == rec[i].w) {
-                        atomicAdd(&sdup[old - 1], 1u);
+                        atomicAdd(&stab[h], 1u << 16);
                         break;
                     }
                     h = (h + 1) & ((1u << tbits) - 1);
                 }
             }
         }
+        uint32_t at = own;  // where this thread's distinct records go in the list << 16 | k-mers before them
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(kFull, at, d);
+            if ((int)lane >= d) at += y;
+        }
+        unsigned base = 0;
+        if (lane == 31 && at) base = atomicAdd(&s_total, at);
+        at += __shfl_sync(kFull, base, 31) - own;
         __syncthreads();
-        for (uint32_t j = threadIdx.x; j < 1u << tbits; j += NT) stab[j] = 0;
 #pragma unroll
         for (int i = 0; i < R; ++i) {
-            const uint32_t r = b0 + per * i + lane;
-            if (mine(i)) {
-                if (weight[i]) weight[i] += sdup[r];
-                sdup[r] = 0;
+            const uint32_t r = i * NT + threadIdx.x;
+            if (first[i] != ~0u) {
+                sdis[at >> 16] = r | (1u + (stab[first[i]] >> 16)) << 16;
+                if (at >> 16 < kEven) sbefore[at >> 16] = (unsigned short)at;
+                stab[first[i]] = 0;
+                at += 1u << 16 | (rec[i].w & 31u);
+            } else if (r < n0) {
                 srec[r] = none;
             }
         }
-        __syncthreads();  // the counter array is zero again
+        __syncthreads();
+        // the warp's share of the distinct records (at most R a lane): an even
+        // number of them if they are many or short, else of their k-mers, by
+        // where the records start
+        const uint32_t nd = s_total >> 16, nk = s_total & 0xffffu;
+        uint32_t p0, p1;
+        if (nd > kEven || nk < 4 * nd) {
+            p0 = nd * wp / NW;
+            p1 = nd * (wp + 1) / NW;
+        } else {
+            const uint32_t want = nk * (wp + (lane & 1)) / NW;  // lane 0: the share's start, lane 1: its end
+            uint32_t lo = 0, hi = nd;
+            while (lo < hi) {
+                const uint32_t mid = (lo + hi) >> 1;
+                if (sbefore[mid] < want) lo = mid + 1;
+                else hi = mid;
+            }
+            p0 = __shfl_sync(kFull, lo, 0);
+            p1 = wp + 1 == NW ? nd : __shfl_sync(kFull, lo, 1);
+        }
+        uint32_t weight[R];
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const uint32_t p = p0 + 32 * i + lane;
+            rec[i] = none;
+            weight[i] = 0;
+            if (p < p1) {
+                const uint32_t x = sdis[p];
+                rec[i] = srec[x & 0xffffu];
+                weight[i] = x >> 16;
+                srec[x & 0xffffu] = none;
+            }
+        }
+        for (uint32_t p = p0 + 32 * R + lane; p < p1; p += 32) {  // (uneven beyond that room: the next tier's)
+            srec[sdis[p] & 0xffffu] = none;
+            s_over = 1;
+        }
+        __syncthreads();  // the counter array is zero again, the list is read
         bool full = false;
         uint32_t nu = 0;  // slots in the warp's list
         auto insert = [&](bool valid, const SkOcc &o, const uint4 &x) {
@@ -689,20 +736,8 @@ __device__ void count_pass(const BuildArgs &a, const SkArgs &s, uint64_t n_items
         };
 #pragma unroll
         for (int i = 0; i < R; ++i) {
-            if (b0 + per * i >= b1) break;
-            const unsigned m = __ballot_sync(kFull, weight[i] != 0);
-            if (weight[i]) s_lane[32 * wp + __popc(m & lt)] = (unsigned char)lane;  // the distinct ones to the lowest lanes
-            __syncwarp();
-            const int src = (int)lane < __popc(m) ? s_lane[threadIdx.x] : 0;
-            __syncwarp();
-            uint4 x;
-            x.x = __shfl_sync(kFull, rec[i].x, src);
-            x.y = __shfl_sync(kFull, rec[i].y, src);
-            x.z = __shfl_sync(kFull, rec[i].z, src);
-            x.w = __shfl_sync(kFull, rec[i].w, src);
-            const uint32_t w = __shfl_sync(kFull, weight[i], src);
-            if ((int)lane >= __popc(m)) x = none;
-            sk_expand<kK>(x, w, k, insert);
+            if (p0 + 32 * i >= p1) break;
+            sk_expand<kK>(rec[i], weight[i], k, insert);
         }
         // a larger bucket's other records, one by one; the counters (which
         // saturate at 255 in the end) are clamped before they can carry
@@ -723,10 +758,8 @@ __device__ void count_pass(const BuildArgs &a, const SkArgs &s, uint64_t n_items
             for (uint64_t g = rb + c0 + cn * wp / NW; g < g1; g += 32)
                 sk_expand<kK>(g + lane < g1 ? s.rec2[g + lane] : none, 1, k, insert);
         }
-        share(next_n);
-        load(next_rb);  // the next bucket's first records load while this one is compacted
+        load(next_rb, next_n);  // the next bucket's first records load while this one is compacted
         have = true;
-        if (lane == 0) atomicAdd(&s_nused, nu);
         __syncthreads();
         if (s_over) {
             for (uint32_t j = threadIdx.x; j < (uint32_t)T; j += NT) {
@@ -766,21 +799,16 @@ __device__ void count_pass(const BuildArgs &a, const SkArgs &s, uint64_t n_items
             if (keep) used[ns + __popc(m & lt)] = (unsigned short)sl;
             ns += __popc(m);
         }
-        unsigned at = 0;
-        if (lane == 0 && ns) at = atomicAdd(&s_kept, ns);
-        at = __shfl_sync(kFull, at, 0);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            atomicAdd(&a.counters[0], (unsigned long long)s_nused);
-            if (s_kept) {
-                s_out = atomicAdd(&a.counters[1], (unsigned long long)s_kept);
-                if (a.host_keys) atomicAdd(a.host_written, (unsigned long long)s_kept);
-            }
+        distinct += nu;
+        unsigned long long out = 0;
+        if (lane == 0 && ns) {
+            out = atomicAdd(&a.counters[1], (unsigned long long)ns);
+            if (a.host_keys) atomicAdd(a.host_written, (unsigned long long)ns);
         }
-        __syncthreads();
+        out = __shfl_sync(kFull, out, 0);
         for (uint32_t i = lane; i < ns; i += 32) {
             const uint32_t sl = used[i];
-            const uint64_t pos = s_out + at + i;
+            const uint64_t pos = out + i;
             const unsigned long long key = keys[sl];
             unsigned bias = cbias;
             if (tb) {
@@ -800,6 +828,8 @@ __device__ void count_pass(const BuildArgs &a, const SkArgs &s, uint64_t n_items
             reinterpret_cast<uint4 *>(cnt)[sl] = none;
         }
     }
+    if (lane == 0 && distinct) atomicAdd(&a.counters[0], distinct);
+    if (outgrown && threadIdx.x == 0) atomicOr(s.status, kStatusPartOverflow);
     if (tb) {
         __syncthreads();
         for (uint32_t j = threadIdx.x; j < a.n_segs; j += NT) {
