@@ -109,7 +109,8 @@ struct MergeArgs {
     unsigned long long *oo;    // per state: its ruler << 32 | distance from it (~0: none)
     unsigned *rpos;            // ruler list position of a ruler state
     unsigned *rlist;
-    unsigned long long *rn0, *rn1, *rl0, *rl1;  // ruler list: next ruler / end arc, states to the end
+    ulonglong2 *rp0, *rp1;     // ruler list: next ruler / end arc, states to the end
+    unsigned *moved;           // per pair of rounds of the ruler list's jumping: a ruler had not arrived
     unsigned *len;             // per state: states from it to the end of its walk
     unsigned long long *term;  // per state: kTerm | end arc reached
     unsigned *clist;
@@ -267,15 +268,13 @@ __global__ void k_mg_walk(MergeArgs a) {
         for (unsigned o = 1; o <= 2 * a.n; ++o) {
             const unsigned long long nx = (cur & 1) ? pr.y : pr.x;
             if (nx & kTerm) {
-                a.rn0[p] = nx;
-                a.rl0[p] = o;
+                a.rp0[p] = make_ulonglong2(nx, o);
                 done = true;
                 break;
             }
             const ulonglong2 pn = succ_pair(a, nx);
             if (ruler_of(a, nx, pn)) {
-                a.rn0[p] = a.rpos[nx];
-                a.rl0[p] = o;
+                a.rp0[p] = make_ulonglong2(a.rpos[nx], o);
                 done = true;
                 break;
             }
@@ -287,33 +286,47 @@ __global__ void k_mg_walk(MergeArgs a) {
     }
 }
 
-__global__ void k_mg_rjump(const unsigned long long *__restrict__ rn_in, const unsigned long long *__restrict__ rl_in,
-                           unsigned long long *__restrict__ rn_out, unsigned long long *__restrict__ rl_out,
-                           const unsigned long long *__restrict__ count) {
-    const uint64_t n_rul = *count;
-    for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n_rul;
-         p += (uint64_t)gridDim.x * blockDim.x) {
-        const unsigned long long nx = rn_in[p];
-        if (nx & kTerm) {
-            rn_out[p] = nx;
-            rl_out[p] = rl_in[p];
-        } else {
-            rn_out[p] = rn_in[nx];
-            rl_out[p] = rl_in[p] + rl_in[nx];
+// Pointer jumping over the ruler list, all rounds in one cooperative launch:
+// a round is bound by its launch and its random loads' latency (one 16-byte
+// load a ruler), and a grid barrier costs less than a launch. Rounds go in
+// pairs, so that the result is in rp0 again, and end once every ruler has
+// reached an end (as many rounds as the longest chain's rulers need, where the
+// bound for any chain was 22 to 25); the rulers of a cycle never do.
+__global__ void __launch_bounds__(256) k_mg_rjump(MergeArgs a, int pairs) {
+    const uint64_t n_rul = a.ctr[0], stride = (uint64_t)gridDim.x * blockDim.x;
+    const uint64_t p0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (int r = 0; r < pairs; ++r) {
+        bool moved = false;
+        for (int half = 0; half < 2; ++half) {
+            const ulonglong2 *in = half ? a.rp1 : a.rp0;
+            ulonglong2 *out = half ? a.rp0 : a.rp1;
+            for (uint64_t p = p0; p < n_rul; p += stride) {
+                ulonglong2 v = __ldcg(in + p);
+                if (!(v.x & kTerm)) {
+                    const ulonglong2 w = __ldcg(in + v.x);
+                    v = make_ulonglong2(w.x, v.y + w.y);
+                    moved |= !(v.x & kTerm);
+                }
+                out[p] = v;
+            }
+            if (half && moved) a.moved[r] = 1;
+            cg::this_grid().sync();
+            moved = false;
         }
+        if (!*(volatile unsigned *)(a.moved + r)) return;
     }
 }
 
-__global__ void k_mg_finish(MergeArgs a, const unsigned long long *__restrict__ rn,
-                            const unsigned long long *__restrict__ rl) {
+__global__ void k_mg_finish(MergeArgs a) {
     const uint64_t st = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (st >= 2 * a.n || !is_m(a, st >> 1)) return;
     const unsigned long long oo = a.oo[st];
     if (oo != ~0ull) {
         const unsigned p = (unsigned)(oo >> 32);
-        if (rn[p] & kTerm) {
-            a.len[st] = (unsigned)(rl[p] - (oo & 0xffffffffull));
-            a.term[st] = rn[p];
+        const ulonglong2 v = a.rp0[p];
+        if (v.x & kTerm) {
+            a.len[st] = (unsigned)(v.y - (oo & 0xffffffffull));
+            a.term[st] = v.x;
             return;
         }
     }
@@ -469,22 +482,47 @@ __global__ void k_mg_entries(MergeArgs a) {
     }
 }
 
-// One level of the pairwise reduction: the node at position (2b+1)*2^t
-// merges segment b (left) with segment b+1 (right), graph.cpp:1322-1324.
-__global__ void k_mg_level(MergeArgs a, uint64_t n_pairs, int t) {
-    const uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= n_pairs) return;
-    const uint64_t e = q << (t + 1);
-    const unsigned id = a.ent_chain[e];
-    if (id == kNone) return;
-    const uint64_t m = a.ch_m[id];
-    const uint64_t b = (e - a.ch_eoff[id]) >> t;
-    if (((b + 1) << t) > m) return;  // no node in the middle: the segment carries over
-    const uint64_t ll = 1ull << t;
-    const uint64_t lr = min((b + 2) << t, m + 1) - ((b + 1) << t);
-    const uint64_t sum = (uint64_t)a.ent[e] * ll + (uint64_t)a.ent[e + ll] * lr;
-    const int pre = (int)(unsigned)sum;
-    a.ent[e] = (unsigned char)((uint64_t)(int64_t)pre / (ll + lr));
+// Levels t0 .. t0 + kLevels - 1 (below top) of the pairwise reduction: at
+// level t the node at position (2b+1)*2^t merges segment b (left) with segment
+// b+1 (right), graph.cpp:1322-1324. Segments are aligned to their size, so a
+// block that holds 2^kLevels entries at stride 2^t0 in shared memory takes all
+// of these levels alone (a launch per level, 21 for a chain of millions, took
+// 4 us each for almost no work past the first few).
+constexpr int kLevels = 12;
+__global__ void __launch_bounds__(512) k_mg_levels(MergeArgs a, uint64_t total, int t0, int top) {
+    constexpr unsigned N = 1u << kLevels;
+    __shared__ unsigned char v[N];
+    __shared__ unsigned cm[N / 2], rel[N / 2];  // of every even entry: its chain's m (kNone: no chain), its position >> t0
+    const uint64_t q0 = (uint64_t)blockIdx.x << kLevels;
+    for (unsigned i = threadIdx.x; i < N; i += 512) {
+        const uint64_t e = (q0 + i) << t0;
+        v[i] = e < total ? a.ent[e] : 0;
+        if (!(i & 1)) {
+            const unsigned id = e < total ? a.ent_chain[e] : kNone;
+            cm[i / 2] = id == kNone ? kNone : a.ch_m[id];
+            rel[i / 2] = id == kNone ? 0 : (unsigned)((e - a.ch_eoff[id]) >> t0);
+        }
+    }
+    for (int l = 0; l < kLevels && t0 + l < top; ++l) {
+        __syncthreads();
+        const int t = t0 + l;
+        for (unsigned q = threadIdx.x; q < (N >> (l + 1)); q += 512) {
+            const unsigned i = q << (l + 1);
+            if (cm[i / 2] == kNone) continue;
+            const uint64_t m = cm[i / 2], b = rel[i / 2] >> l;
+            if (((b + 1) << t) > m) continue;  // no node in the middle: the segment carries over
+            const uint64_t ll = 1ull << t;
+            const uint64_t lr = min((b + 2) << t, m + 1) - ((b + 1) << t);
+            const uint64_t sum = (uint64_t)v[i] * ll + (uint64_t)v[i + (1u << l)] * lr;
+            const int pre = (int)(unsigned)sum;
+            v[i] = (unsigned char)((uint64_t)(int64_t)pre / (ll + lr));
+        }
+    }
+    __syncthreads();
+    for (unsigned i = threadIdx.x; i < N; i += 512) {
+        const uint64_t e = (q0 + i) << t0;
+        if (e < total && !(i & 1)) a.ent[e] = v[i];
+    }
 }
 
 // Merge in a given visiting order. Visiting the node at position p merges the
@@ -560,19 +598,23 @@ __global__ void k_mg_survivors(MergeArgs a) {
     a.sidx[q] = (unsigned)j;
 }
 
+// (eight lanes a line, one per arc slot: a line's arcs are chains of dependent
+// loads, and few lines are left of a graph)
 __global__ void k_mg_line_len(MergeArgs a, const unsigned *__restrict__ order, uint64_t n_lines,
                               uint64_t *__restrict__ out) {
-    const uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= n_lines) return;
-    const uint64_t j = order[q];
-    const uint64_t m = a.mult[j];
-    uint64_t l = 69;
-    for (int s = 0; s < 8; ++s) {
-        if (!mbyte(m, s)) continue;
-        const unsigned v = a.nb[j * 8 + s];
-        l += 1 + (is_m(a, v >> 1) ? a.len[first_state(v)] : 0);
+    const uint64_t q = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+    const int s = threadIdx.x & 7;
+    unsigned long long l = 0;
+    if (q < n_lines) {
+        const uint64_t j = order[q];
+        if (mbyte(a.mult[j], s)) {
+            const unsigned v = a.nb[j * 8 + s];
+            l = 1 + (is_m(a, v >> 1) ? a.len[first_state(v)] : 0);
+        }
     }
-    out[q] = l;
+#pragma unroll
+    for (int d = 4; d; d >>= 1) l += __shfl_xor_sync(0xffffffffu, l, d);
+    if (q < n_lines && s == 0) out[q] = 69 + l;
 }
 
 // Line position of every node left.
@@ -581,62 +623,78 @@ __global__ void k_mg_pos(const unsigned *__restrict__ order, uint64_t n_lines, u
     if (q < n_lines) pos_of[order[q]] = (unsigned)q;
 }
 
-__global__ void k_mg_line_write(MergeArgs a, const unsigned *__restrict__ order, uint64_t n_lines,
+// Eight lanes a line: lane s writes arc s's place, its multiplicity and an
+// eighth of the blanks.
+__global__ void __launch_bounds__(256) k_mg_line_write(MergeArgs a, const unsigned *__restrict__ order, uint64_t n_lines,
                                 const uint64_t *__restrict__ off, char *__restrict__ text,
                                 const unsigned *__restrict__ pos_of, MergedGraph mg) {
-    const uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= n_lines) return;
-    const uint64_t j = order[q];
-    const uint64_t m = a.mult[j];
-    char *const start = text + off[q];
-    char *p = put_u64(start, a.keys[j]);
-    mg.key[q] = a.keys[j];
-    mg.del[q] = 0;
-    unsigned mm[8];
-    uint64_t vlen = 69;
-    const uint64_t key = a.keys[j], rk = rc_dev(key, a.k);
-    for (int s = 0; s < 8; ++s) {
-        *p++ = ' ';
-        mm[s] = mbyte(m, s);
-        uint64_t l = 0;
-        unsigned back = kNone;
-        if (mm[s]) {
-            *p = "ACGT"[s & 3];
-            const unsigned v = a.nb[j * 8 + s];
-            mg.src[8 * q + s] = (unsigned long long)(p - text);
-            l = 1;
-            if (is_m(a, v >> 1)) {
-                const uint64_t st = first_state(v);
-                const uint64_t mine = j * 8 + s, other = a.term[st] & ~kTerm;
-                const bool first = arc_less(a, mine, other);  // this end starts the chain
-                const unsigned id = a.chain_of[first ? mine : other];
-                const unsigned long long dest = (unsigned long long)(p - text);
-                if (first) a.ch_dfwd[id] = dest;
-                else a.ch_drev[id] = dest;
-                mm[s] = a.ent[a.ch_eoff[id]];
-                l += a.len[st];
-                back = pos_of[other >> 3] * 8u + (unsigned)(other & 7);
-            } else {  // one base to the next node left: its arc back, as walk_next finds it
-                const uint64_t o = s < 4 ? key : rk;
-                const unsigned first = (unsigned)(o >> (2 * (a.k - 1))) & 3u;
-                back = pos_of[v >> 1] * 8u + ((v & 1u) ? 4u : 0u) + 3u - first;
-            }
-            p += l;
-            vlen += l;
-        } else {
-            mg.src[8 * q + s] = 0;
+    const uint64_t q = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+    const int s = threadIdx.x & 7;
+    const bool in = q < n_lines;
+    const uint64_t j = in ? order[q] : 0, key = in ? a.keys[j] : 0;
+    unsigned mm = in ? mbyte(a.mult[j], s) : 0;
+    unsigned long long l = 0;  // the arc's length
+    unsigned back = kNone, id = 0;
+    bool chain = false, first = false;
+    if (mm) {
+        const unsigned v = a.nb[j * 8 + s];
+        l = 1;
+        if (is_m(a, v >> 1)) {
+            const uint64_t st = first_state(v);
+            const uint64_t mine = j * 8 + s, other = a.term[st] & ~kTerm;
+            chain = true;
+            first = arc_less(a, mine, other);  // this end starts the chain
+            id = a.chain_of[first ? mine : other];
+            mm = a.ent[a.ch_eoff[id]];
+            l += a.len[st];
+            back = pos_of[other >> 3] * 8u + (unsigned)(other & 7);
+        } else {  // one base to the next node left: its arc back, as walk_next finds it
+            const uint64_t o = s < 4 ? key : rc_dev(key, a.k);
+            const unsigned base = (unsigned)(o >> (2 * (a.k - 1))) & 3u;
+            back = pos_of[v >> 1] * 8u + ((v & 1u) ? 4u : 0u) + 3u - base;
         }
-        mg.len[8 * q + s] = (unsigned)l;
-        mg.mult[8 * q + s] = (unsigned char)mm[s];
-        mg.back[8 * q + s] = back;
-        *p++ = '#';
     }
-    for (int s = 0; s < 8; ++s) {
-        *p++ = ' ';
-        p = put_u64(p, mm[s]);
+    const unsigned dig = 1 + ndig(mm);  // " m"
+    unsigned long long al = l + 2;      // " arc#"
+    unsigned dl = dig;
+#pragma unroll
+    for (int d = 1; d < 8; d <<= 1) {  // the line's arcs and multiplicities up to and with this lane's
+        const unsigned long long x = __shfl_up_sync(0xffffffffu, al, d, 8);
+        const unsigned y = __shfl_up_sync(0xffffffffu, dl, d, 8);
+        if (s >= d) {
+            al += x;
+            dl += y;
+        }
     }
-    while ((uint64_t)(p - start) < vlen - 1) *p++ = ' ';
-    *p = '\n';
+    const unsigned long long arcs = __shfl_sync(0xffffffffu, al, 7, 8);
+    const unsigned digits = __shfl_sync(0xffffffffu, dl, 7, 8);
+    if (!in) return;
+    char *const start = text + off[q];
+    const unsigned head = ndig(key);
+    char *p = start + head + (al - l - 2);  // this lane's " arc#"
+    *p = ' ';
+    p[1 + l] = '#';
+    const unsigned long long dest = (unsigned long long)(p + 1 - text);
+    if (l) p[1] = "ACGT"[s & 3];
+    if (chain) {
+        if (first) a.ch_dfwd[id] = dest;
+        else a.ch_drev[id] = dest;
+    }
+    char *d = start + head + arcs + (dl - dig);  // this lane's " m"
+    *d = ' ';
+    put_u64(d + 1, mm);
+    const uint64_t vlen = off[q + 1] - off[q];
+    for (uint64_t i = head + arcs + digits + s; i < vlen - 1; i += 8) start[i] = ' ';
+    mg.src[8 * q + s] = l ? dest : 0;
+    mg.len[8 * q + s] = (unsigned)l;
+    mg.mult[8 * q + s] = (unsigned char)mm;
+    mg.back[8 * q + s] = back;
+    if (s == 0) {
+        put_u64(start, key);
+        start[vlen - 1] = '\n';
+        mg.key[q] = key;
+        mg.del[q] = 0;
+    }
 }
 
 __global__ void k_mg_chars(MergeArgs a, char *__restrict__ text) {
@@ -779,21 +837,24 @@ swg_status merge_graph(const unsigned long long *d_keys, const unsigned long lon
     k_mg_states<<<blocks(n), 256, 0, s>>>(a);
     launches += 3;
     // rulers: at most one per state; counts stay on the device
-    if (!scr.get(&a.rn0, 2 * n) || !scr.get(&a.rn1, 2 * n) || !scr.get(&a.rl0, 2 * n) || !scr.get(&a.rl1, 2 * n))
+    if (!scr.get(&a.rp0, 2 * n) || !scr.get(&a.rp1, 2 * n) || !scr.get(&a.moved, 64))
         return cuda_err(cudaErrorMemoryAllocation, "ruler list");
-    int sms = 0;
-    EMIT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0), "device attribute");
+    EMIT_CUDA(cudaMemsetAsync(a.moved, 0, 64 * sizeof(unsigned), s), "merge clear");
+    int sms = 0, per_sm = 0, dev = 0;
+    EMIT_CUDA(cudaGetDevice(&dev), "device");
+    EMIT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "device attribute");
+    EMIT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mg_rjump, 256, 0), "occupancy");
     const unsigned wgrid = (unsigned)std::max(1, sms * 8);
     k_mg_rpos<<<wgrid, 256, 0, s>>>(a);
     k_mg_walk<<<wgrid, 256, 0, s>>>(a);
-    const int rounds = ceil_log2(std::max<uint64_t>(2 * n, 1)) + 1;
-    unsigned long long *bn[2] = {a.rn0, a.rn1}, *bl[2] = {a.rl0, a.rl1};
-    for (int r = 0; r < rounds; ++r)
-        k_mg_rjump<<<wgrid, 256, 0, s>>>(bn[r & 1], bl[r & 1], bn[(r + 1) & 1], bl[(r + 1) & 1], ctr);
-    launches += 2 + rounds;
-    const unsigned long long *rn = bn[rounds & 1], *rl = bl[rounds & 1];
-    k_mg_finish<<<blocks(2 * n), 256, 0, s>>>(a, rn, rl);
-    ++launches;
+    {
+        int pairs = (ceil_log2(std::max<uint64_t>(2 * n, 1)) + 2) / 2;
+        void *args[] = {&a, &pairs};
+        const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)std::max(1, std::min(per_sm, 4) * sms), blocks(2 * n));
+        EMIT_CUDA(cudaLaunchCooperativeKernel((const void *)k_mg_rjump, dim3(grid), dim3(256), args, 0, s), "ruler list");
+    }
+    k_mg_finish<<<blocks(2 * n), 256, 0, s>>>(a);
+    launches += 4;
     unsigned long long h[6];
     unsigned herr = 0;
     EMIT_CUDA(cudaMemcpyAsync(h, ctr, sizeof(h), cudaMemcpyDeviceToHost, s), "cycle count");
@@ -859,10 +920,9 @@ swg_status merge_graph(const unsigned long long *d_keys, const unsigned long lon
         if (total) k_mg_cart<<<blocks(total), 256, 0, s>>>(a, total);
         ++launches;
     } else {
-        for (int t = 0; t < top; ++t) {
-            const uint64_t pairs = total >> (t + 1);
-            if (!pairs) break;
-            k_mg_level<<<blocks(pairs), 256, 0, s>>>(a, pairs, t);
+        for (int t = 0; t < top; t += kLevels) {
+            const uint64_t per = 1ull << (t + kLevels);
+            k_mg_levels<<<(unsigned)((total + per - 1) / per), 512, 0, s>>>(a, total, t, top);
             ++launches;
         }
     }
@@ -886,7 +946,7 @@ swg_status merge_graph(const unsigned long long *d_keys, const unsigned long lon
         EMIT_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tb, a.skey, skey2, a.sidx, sidx2, (int64_t)n_lines, 0,
                                                   2 * k, s),
                   "sort");
-        k_mg_line_len<<<blocks(n_lines), 256, 0, s>>>(a, sidx2, n_lines, lens);
+        k_mg_line_len<<<blocks(8 * n_lines), 256, 0, s>>>(a, sidx2, n_lines, lens);
         ++launches;
     }
     swg_status st = scan_lengths(lens, loff, n_lines, scr, s);
@@ -902,7 +962,7 @@ swg_status merge_graph(const unsigned long long *d_keys, const unsigned long lon
     if (!scr.get(&pos_of, n)) return cuda_err(cudaErrorMemoryAllocation, "line positions");
     if (n_lines) {
         k_mg_pos<<<blocks(n_lines), 256, 0, s>>>(sidx2, n_lines, pos_of);
-        k_mg_line_write<<<blocks(n_lines), 256, 0, s>>>(a, sidx2, n_lines, loff, mg->text, pos_of, *mg);
+        k_mg_line_write<<<blocks(8 * n_lines), 256, 0, s>>>(a, sidx2, n_lines, loff, mg->text, pos_of, *mg);
     }
     k_mg_chars<<<blocks(n), 256, 0, s>>>(a, mg->text);
     launches += 3;

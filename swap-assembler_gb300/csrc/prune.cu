@@ -119,32 +119,51 @@ __global__ void k_pr_len(MergedGraph m, uint64_t *__restrict__ out, unsigned lon
     if (sum) agg_add(printed, 1);
 }
 
-__global__ void k_pr_write(MergedGraph m, const uint64_t *__restrict__ off, char *__restrict__ text) {
-    const uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= m.lines || off[q + 1] == off[q]) return;
+// Eight lanes a line, one per arc slot (as the merge writes them).
+__global__ void __launch_bounds__(256) k_pr_write(MergedGraph m, const uint64_t *__restrict__ off, char *__restrict__ text) {
+    const uint64_t q = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+    const int s = threadIdx.x & 7;
+    const bool in = q < m.lines && off[q + 1] != off[q];
+    const unsigned l = in ? m.len[8 * q + s] : 0, mult = in ? m.mult[8 * q + s] : 0;
+    const unsigned dig = 1 + ndig(mult);
+    unsigned long long al = l + 2ull;
+    unsigned dl = dig;
+#pragma unroll
+    for (int d = 1; d < 8; d <<= 1) {
+        const unsigned long long x = __shfl_up_sync(0xffffffffu, al, d, 8);
+        const unsigned y = __shfl_up_sync(0xffffffffu, dl, d, 8);
+        if (s >= d) {
+            al += x;
+            dl += y;
+        }
+    }
+    const unsigned long long arcs = __shfl_sync(0xffffffffu, al, 7, 8);
+    const unsigned digits = __shfl_sync(0xffffffffu, dl, 7, 8);
+    if (!in) return;
     char *const start = text + off[q];
-    char *p = put_u64(start, m.key[q]);
-    uint64_t vlen = 69;
-    for (int s = 0; s < 8; ++s) {
-        *p++ = ' ';
-        const unsigned l = m.len[8 * q + s];
-        m.src2[8 * q + s] = (unsigned long long)(p - text);
-        p += l;
-        vlen += l;
-        *p++ = '#';
+    const uint64_t key = m.key[q];
+    const unsigned head = ndig(key);
+    char *p = start + head + (al - l - 2);  // this lane's " arc#"
+    *p = ' ';
+    p[1 + l] = '#';
+    m.src2[8 * q + s] = (unsigned long long)(p + 1 - text);
+    char *d = start + head + arcs + (dl - dig);  // this lane's " m"
+    *d = ' ';
+    put_u64(d + 1, mult);
+    const uint64_t vlen = off[q + 1] - off[q];
+    for (uint64_t i = head + arcs + digits + s; i < vlen - 1; i += 8) start[i] = ' ';
+    if (s == 0) {
+        put_u64(start, key);
+        start[vlen - 1] = '\n';
     }
-    for (int s = 0; s < 8; ++s) {
-        *p++ = ' ';
-        p = put_u64(p, m.mult[8 * q + s]);
-    }
-    while ((uint64_t)(p - start) < vlen - 1) *p++ = ' ';
-    *p = '\n';
 }
 
-// The arc strings move from the old text to the new one in 4 KiB chunks, a
-// block per chunk, so that a few very long arcs (whole chains) spread over
-// the GPU too: chunk counts per piece, their prefix, then each block finds
-// its piece by binary search in the prefix. A piece is an arc's own string
+// The arc strings move from the old text to the new one, a piece's first 4 KiB
+// by a warp of its own and the rest of a long one in 4 KiB chunks, a block
+// each, so that a few very long arcs (whole chains) spread over the GPU too:
+// chunk counts per piece, their prefix, then each block finds its piece by
+// binary search in the prefix. (Most arcs are short; a block and a search for
+// each of them took three times as long.) A piece is an arc's own string
 // (its first `own` bytes, the whole arc unless a merge lengthened it) or,
 // after a merge, a merged node's arc string placed inside an end's new arc.
 constexpr unsigned kChunk = 4096;
@@ -163,16 +182,55 @@ __device__ __forceinline__ unsigned own_len(const MergedGraph &m, const Pieces &
     return x.own ? x.own[a] : m.len[a];
 }
 
-__global__ void k_pr_chunks(MergedGraph m, Pieces x, uint64_t *__restrict__ chunks) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// Where piece i's string lies and goes, and its length.
+__device__ __forceinline__ unsigned piece(const MergedGraph &m, const Pieces &x, uint64_t i, uint64_t &src, uint64_t &dst) {
     const uint64_t arcs = 8 * m.lines;
-    if (i < arcs) chunks[i] = (own_len(m, x, i) + kChunk - 1) / kChunk;
-    else if (i < arcs + x.n) chunks[i] = (x.len[i - arcs] + kChunk - 1) / kChunk;
+    if (i < arcs) {
+        const unsigned l = own_len(m, x, i);
+        if (l) {
+            src = m.src[i];
+            dst = m.src2[i];
+        }
+        return l;
+    }
+    const uint64_t j = i - arcs;
+    const unsigned l = x.len[j];
+    if (l) {
+        src = x.src[j];
+        dst = m.src2[x.arc[j]] + x.at[j];
+    }
+    return l;
 }
 
-__global__ void k_pr_copy(MergedGraph m, Pieces x, const uint64_t *__restrict__ first, uint64_t n_chunks,
-                          const char *__restrict__ from, char *__restrict__ to) {
-    const uint64_t arcs = 8 * m.lines, pieces = arcs + x.n;
+__device__ __forceinline__ unsigned more_chunks(unsigned len) { return len ? (len - 1) / kChunk : 0; }
+
+// A warp's lanes look at 32 pieces; the warp copies the nonempty ones' first
+// chunks one after the other. chunks: those left of each piece.
+__global__ void __launch_bounds__(256) k_pr_short(MergedGraph m, Pieces x, const char *__restrict__ from,
+                                                  char *__restrict__ to, uint64_t *__restrict__ chunks) {
+    const uint64_t pieces = 8 * m.lines + x.n;
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned lane = threadIdx.x & 31;
+    uint64_t src = 0, dst = 0;
+    unsigned len = 0;
+    if (i < pieces) {
+        len = piece(m, x, i, src, dst);
+        chunks[i] = more_chunks(len);
+        len = len < kChunk ? len : kChunk;
+    }
+    for (unsigned todo = __ballot_sync(0xffffffffu, len != 0); todo; todo &= todo - 1) {
+        const int o = __ffs(todo) - 1;
+        const char *a = from + __shfl_sync(0xffffffffu, src, o);
+        char *b = to + __shfl_sync(0xffffffffu, dst, o);
+        const unsigned l = __shfl_sync(0xffffffffu, len, o);
+        for (unsigned c = lane; c < l; c += 32) b[c] = a[c];
+    }
+}
+
+// The long pieces' other chunks; their number is read on the device.
+__global__ void __launch_bounds__(256) k_pr_long(MergedGraph m, Pieces x, const uint64_t *__restrict__ first,
+                                                 const char *__restrict__ from, char *__restrict__ to) {
+    const uint64_t pieces = 8 * m.lines + x.n, n_chunks = first[pieces];
     for (uint64_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
         uint64_t lo = 0, hi = pieces;  // the last piece whose first chunk is <= c
         while (hi - lo > 1) {
@@ -180,18 +238,9 @@ __global__ void k_pr_copy(MergedGraph m, Pieces x, const uint64_t *__restrict__ 
             if (first[mid] <= c) lo = mid;
             else hi = mid;
         }
-        const uint64_t at = (c - first[lo]) * kChunk;
-        uint64_t src, dst, len;
-        if (lo < arcs) {
-            src = m.src[lo];
-            dst = m.src2[lo];
-            len = own_len(m, x, lo);
-        } else {
-            const uint64_t j = lo - arcs;
-            src = x.src[j];
-            dst = m.src2[x.arc[j]] + x.at[j];
-            len = x.len[j];
-        }
+        uint64_t src = 0, dst = 0;
+        const unsigned len = piece(m, x, lo, src, dst);
+        const uint64_t at = (c - first[lo] + 1) * kChunk;
         const uint64_t rest = len - at;
         const unsigned l = rest < kChunk ? (unsigned)rest : kChunk;
         const char *a = from + src + at;
@@ -229,16 +278,14 @@ swg_status rewrite(MergedGraph *m, cudaStream_t s, Scratch &scr, const Pieces &x
         uint64_t *chunks = nullptr, *first = nullptr;
         if (!scr.get(&chunks, pieces) || !scr.get(&first, pieces + 1))
             return cuda_err(cudaErrorMemoryAllocation, "rewrite workspace");
-        k_pr_write<<<blocks(m->lines), 256, 0, s>>>(*m, off, m->text2);
-        k_pr_chunks<<<blocks(pieces), 256, 0, s>>>(*m, x, chunks);
+        k_pr_write<<<blocks(8 * m->lines), 256, 0, s>>>(*m, off, m->text2);
+        k_pr_short<<<blocks(pieces), 256, 0, s>>>(*m, x, m->text, m->text2, chunks);
         st = scan_lengths(chunks, first, pieces, scr, s);
         if (st) return st;
-        uint64_t n_chunks = 0;
-        EMIT_CUDA(cudaMemcpyAsync(&n_chunks, first + pieces, 8, cudaMemcpyDeviceToHost, s), "chunks");
-        EMIT_CUDA(cudaStreamSynchronize(s), "chunks");
-        if (n_chunks)
-            k_pr_copy<<<(unsigned)std::min<uint64_t>(n_chunks, 1u << 20), 256, 0, s>>>(*m, x, first, n_chunks,
-                                                                                      m->text, m->text2);
+        // at most a chunk per 4 KiB of the new text
+        const uint64_t most = h[0] / kChunk;
+        if (most)
+            k_pr_long<<<(unsigned)std::min<uint64_t>(most, 4096), 256, 0, s>>>(*m, x, first, m->text, m->text2);
     }
     EMIT_CUDA(cudaMemsetAsync(m->text2 + h[0], '\n', 1, s), "merged text");
     EMIT_CUDA(cudaGetLastError(), "rewrite kernels");
@@ -337,21 +384,37 @@ __global__ void k_sm_init(SimplifyArgs a) {
     }
 }
 
-__global__ void k_sm_jump(SimplifyArgs a, int in) {
-    const uint64_t st = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (st >= 2 * a.m.lines || !sm_m(a, st >> 1)) return;
-    const int out = in ^ 1;
-    const unsigned long long nx = a.nx[in][st];
-    if (nx & kTerm) {
-        a.nx[out][st] = nx;
-        a.cn[out][st] = a.cn[in][st];
-        a.ws[out][st] = a.ws[in][st];
-        a.mx[out][st] = a.mx[in][st];
-    } else {
-        a.nx[out][st] = a.nx[in][nx];
-        a.cn[out][st] = a.cn[in][st] + a.cn[in][nx];
-        a.ws[out][st] = a.ws[in][st] + a.ws[in][nx];
-        a.mx[out][st] = max(a.mx[in][st], a.mx[in][nx]);
+// Pointer jumping, all rounds in one cooperative launch (as the merge's ruler
+// list): rounds in pairs, so that the result is in the first buffers again,
+// until every state has reached an end (those of a cycle never do).
+__global__ void __launch_bounds__(256) k_sm_jump(SimplifyArgs a, int pairs, unsigned *moved) {
+    const uint64_t states = 2 * a.m.lines, stride = (uint64_t)gridDim.x * blockDim.x;
+    for (int r = 0; r < pairs; ++r) {
+        for (int in = 0; in < 2; ++in) {
+            const int out = in ^ 1;
+            bool left = false;
+            for (uint64_t st = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; st < states; st += stride) {
+                if (!sm_m(a, st >> 1)) continue;
+                unsigned long long nx = __ldcg(a.nx[in] + st), ws = __ldcg(a.ws[in] + st), mx = __ldcg(a.mx[in] + st);
+                unsigned cn = __ldcg(a.cn[in] + st);
+                if (!(nx & kTerm)) {
+                    const unsigned long long to = nx;
+                    nx = __ldcg(a.nx[in] + to);
+                    cn += __ldcg(a.cn[in] + to);
+                    ws += __ldcg(a.ws[in] + to);
+                    const unsigned long long y = __ldcg(a.mx[in] + to);
+                    mx = y > mx ? y : mx;
+                    left |= !(nx & kTerm);
+                }
+                a.nx[out][st] = nx;
+                a.cn[out][st] = cn;
+                a.ws[out][st] = ws;
+                a.mx[out][st] = mx;
+            }
+            if (in && left) moved[r] = 1;
+            cg::this_grid().sync();
+        }
+        if (!*(volatile unsigned *)(moved + r)) return;
     }
 }
 
@@ -429,19 +492,43 @@ __global__ void k_sm_entries(SimplifyArgs a, int in) {
     }
 }
 
-// One level of the weighted pairwise reduction (graph.cpp:2157-2163).
-__global__ void k_sm_level(SimplifyArgs a, uint64_t n_pairs, int t) {
-    const uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= n_pairs) return;
-    const uint64_t e = q << (t + 1);
-    const unsigned id = a.ent_chain[e];
-    if (id == kNone) return;
-    const uint64_t b = (e - a.ch_eoff[id]) >> t;
-    if (((b + 1) << t) > a.ch_m[id]) return;
-    const uint64_t r = e + (1ull << t);
-    const uint64_t ll = a.ent_l[e], lr = a.ent_l[r];
-    a.ent_m[e] = (unsigned char)(((uint64_t)a.ent_m[e] * ll + (uint64_t)a.ent_m[r] * lr) / (ll + lr));
-    a.ent_l[e] = ll + lr;
+// Levels t0 .. t0 + kLevels - 1 (below top) of the weighted pairwise reduction
+// (graph.cpp:2157-2163), a block's entries in shared memory (as the merge's).
+constexpr int kLevels = 10;
+__global__ void __launch_bounds__(256) k_sm_levels(SimplifyArgs a, uint64_t total, int t0, int top) {
+    constexpr unsigned N = 1u << kLevels;
+    __shared__ unsigned char v[N];
+    __shared__ unsigned long long w[N];
+    __shared__ unsigned cm[N / 2], rel[N / 2];  // of every even entry: its chain's m (kNone: no chain), its position >> t0
+    const uint64_t q0 = (uint64_t)blockIdx.x << kLevels;
+    for (unsigned i = threadIdx.x; i < N; i += 256) {
+        const uint64_t e = (q0 + i) << t0;
+        v[i] = e < total ? a.ent_m[e] : 0;
+        w[i] = e < total ? a.ent_l[e] : 0;
+        if (!(i & 1)) {
+            const unsigned id = e < total ? a.ent_chain[e] : kNone;
+            cm[i / 2] = id == kNone ? kNone : a.ch_m[id];
+            rel[i / 2] = id == kNone ? 0 : (unsigned)((e - a.ch_eoff[id]) >> t0);
+        }
+    }
+    for (int l = 0; l < kLevels && t0 + l < top; ++l) {
+        __syncthreads();
+        for (unsigned q = threadIdx.x; q < (N >> (l + 1)); q += 256) {
+            const unsigned i = q << (l + 1), r = i + (1u << l);
+            if (cm[i / 2] == kNone || (((uint64_t)(rel[i / 2] >> l) + 1) << (t0 + l)) > cm[i / 2]) continue;
+            const uint64_t ll = w[i], lr = w[r];
+            v[i] = (unsigned char)(((uint64_t)v[i] * ll + (uint64_t)v[r] * lr) / (ll + lr));
+            w[i] = ll + lr;
+        }
+    }
+    __syncthreads();
+    for (unsigned i = threadIdx.x; i < N; i += 256) {
+        const uint64_t e = (q0 + i) << t0;
+        if (e < total && !(i & 1)) {
+            a.ent_m[e] = v[i];
+            a.ent_l[e] = w[i];
+        }
+    }
 }
 
 // The two end arcs of every chain take the chain: its total length and
@@ -587,14 +674,22 @@ swg_status simplify_lines(MergedGraph *m, cudaStream_t s, uint64_t *count) {
     EMIT_CUDA(cudaMemsetAsync(a.ctr, 0, (8 + 2 * kCls) * 8, s), "simplify");
     EMIT_CUDA(cudaMemsetAsync(a.xlen, 0, std::max<uint64_t>(2 * L, 1) * 4, s), "simplify");
     if (L == 0) return rewrite(m, s, scr);
-    const int rounds = sm_ceil_log2(2 * L) + 1;
+    int pairs = (sm_ceil_log2(2 * L) + 2) / 2;
+    unsigned *moved = nullptr;
+    if (!scr.get(&moved, 64)) return cuda_err(cudaErrorMemoryAllocation, "simplify workspace");
+    int sms = 0, per_sm = 0, dev = 0;
+    EMIT_CUDA(cudaGetDevice(&dev), "device");
+    EMIT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "device attribute");
+    EMIT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sm_jump, 256, 0), "occupancy");
+    const unsigned jgrid = (unsigned)std::min<uint64_t>((uint64_t)std::max(1, std::min(per_sm, 4) * sms), blocks(2 * L));
     unsigned long long h[4] = {0, 0, 0, 0};
-    int in = 0;
+    const int in = 0;  // the jumps leave their result in the first buffers
     k_sm_classify<<<blocks(L), 256, 0, s>>>(a);
     for (int attempt = 0; attempt < 2; ++attempt) {  // again after cutting cycles
         k_sm_init<<<blocks(L), 256, 0, s>>>(a);
-        in = 0;
-        for (int r = 0; r < rounds; ++r, in ^= 1) k_sm_jump<<<blocks(2 * L), 256, 0, s>>>(a, in);
+        EMIT_CUDA(cudaMemsetAsync(moved, 0, 64 * sizeof(unsigned), s), "simplify");
+        void *args[] = {&a, &pairs, &moved};
+        EMIT_CUDA(cudaLaunchCooperativeKernel((const void *)k_sm_jump, dim3(jgrid), dim3(256), args, 0, s), "simplify");
         if (attempt == 1) break;
         k_sm_cut<<<blocks(L), 256, 0, s>>>(a, in);
         EMIT_CUDA(cudaMemcpyAsync(h, a.ctr, sizeof(h), cudaMemcpyDeviceToHost, s), "simplify");
@@ -623,10 +718,9 @@ swg_status simplify_lines(MergedGraph *m, cudaStream_t s, uint64_t *count) {
     EMIT_CUDA(cudaMemcpyAsync(a.own, m->len, 8 * L * 4, cudaMemcpyDeviceToDevice, s), "simplify");
     k_sm_chain_alloc<<<blocks(L), 256, 0, s>>>(a, in);
     k_sm_entries<<<blocks(L), 256, 0, s>>>(a, in);
-    for (int t = 0; t < top; ++t) {
-        const uint64_t pairs = total >> (t + 1);
-        if (!pairs) break;
-        k_sm_level<<<blocks(pairs), 256, 0, s>>>(a, pairs, t);
+    for (int t = 0; t < top; t += kLevels) {
+        const uint64_t per = 1ull << (t + kLevels);
+        k_sm_levels<<<(unsigned)((total + per - 1) / per), 256, 0, s>>>(a, total, t, top);
     }
     k_sm_apply<<<blocks(L), 256, 0, s>>>(a, in);
     k_sm_delete<<<blocks(L), 256, 0, s>>>(a);
