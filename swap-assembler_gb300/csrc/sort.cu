@@ -17,7 +17,8 @@
 namespace swg {
 namespace {
 
-constexpr uint32_t kOne = 4096;         // records one block orders
+constexpr uint32_t kOne = 1024;         // records one block orders alone
+constexpr uint32_t kRoom = 4096;        // records one block can order
 constexpr int kDigits = 256;
 constexpr int kItems = 16;              // records per thread of a pass
 constexpr uint32_t kTile = 256 * kItems;
@@ -75,16 +76,14 @@ __device__ __forceinline__ void bitonic(unsigned long long (&v)[R], unsigned (&i
         }
 }
 
-// n <= kOne records ordered by one block: the keys with their index, the
+// n <= kRoom records ordered by one block: the keys with their index, the
 // multiplicities after it. Padded with the largest key.
-__device__ __forceinline__ void sort_block(unsigned long long *sk, unsigned short *si,
-                                           const unsigned long long *__restrict__ keys,
-                                           const unsigned long long *__restrict__ mult, uint32_t n,
-                                           unsigned long long *__restrict__ okeys,
-                                           unsigned long long *__restrict__ omult) {
-    constexpr int R = kOne / 1024;
-    uint32_t m = 32;
-    while (m < n) m <<= 1;
+template <int R>
+__device__ __forceinline__ void sort_block_of(unsigned long long *sk, unsigned short *si,
+                                              const unsigned long long *__restrict__ keys,
+                                              const unsigned long long *__restrict__ mult, uint32_t n, uint32_t m,
+                                              unsigned long long *__restrict__ okeys,
+                                              unsigned long long *__restrict__ omult) {
     unsigned long long v[R];
     unsigned ix[R];
 #pragma unroll
@@ -103,51 +102,75 @@ __device__ __forceinline__ void sort_block(unsigned long long *sk, unsigned shor
     }
 }
 
+// As few keys a thread as hold them all: the steps' latency counts here.
+__device__ __forceinline__ void sort_block(unsigned long long *sk, unsigned short *si,
+                                           const unsigned long long *__restrict__ keys,
+                                           const unsigned long long *__restrict__ mult, uint32_t n,
+                                           unsigned long long *__restrict__ okeys,
+                                           unsigned long long *__restrict__ omult) {
+    uint32_t m = 32;
+    while (m < n) m <<= 1;
+    if (m <= 1024) sort_block_of<1>(sk, si, keys, mult, n, m, okeys, omult);
+    else if (m <= 2048) sort_block_of<2>(sk, si, keys, mult, n, m, okeys, omult);
+    else sort_block_of<kRoom / 1024>(sk, si, keys, mult, n, m, okeys, omult);
+}
+
 __global__ void __launch_bounds__(1024) k_sort_one(const unsigned long long *__restrict__ keys,
                                                    const unsigned long long *__restrict__ mult, uint32_t n,
                                                    unsigned long long *__restrict__ okeys,
                                                    unsigned long long *__restrict__ omult) {
-    __shared__ unsigned long long sk[kOne];
-    __shared__ unsigned short si[kOne];
+    __shared__ unsigned long long sk[kRoom];
+    __shared__ unsigned short si[kRoom];
     sort_block(sk, si, keys, mult, n, okeys, omult);
 }
 
-// ---- splitters: nb buckets of kMean records on average, from a sample of
-// kOver keys a bucket at even strides (the keys are distinct, so that the
-// quantiles of any distribution are splitters; at 8 sampled keys a bucket one
-// of 4 times the mean, which would not fit, has odds of 1e-9). Such a bucket
-// sets *over, and the records take the radix passes.
-constexpr uint32_t kMean = 1024, kOver = 8, kSplitBuckets = 1024;
+// ---- splitters: nb buckets of kMean records on average (a block's sort of
+// twice as many takes three times as long: its steps are bound by shuffles),
+// from a sample of kOver keys a bucket at even strides (the keys are distinct,
+// so that the quantiles of any distribution are splitters; at 4 sampled keys a
+// bucket one of 8 times the mean, which would not fit its region, has odds of
+// 1e-10). Such a bucket sets *over, and the records take the radix passes.
+constexpr uint32_t kMean = 512, kOver = 4, kSplitBuckets = 2048;
 constexpr uint64_t kSplitMost = (uint64_t)kMean * kSplitBuckets;
 constexpr uint32_t kSampleMost = kOver * kSplitBuckets;
+
+template <int R>
+__device__ __forceinline__ void split_of(unsigned long long *sk, const unsigned long long *__restrict__ keys, uint64_t n,
+                                         uint32_t count, uint32_t m, unsigned long long *__restrict__ splitters) {
+    const uint64_t step = (n << 20) / count;  // n <= 2^20, the index below 2^13
+    unsigned long long v[R];
+    unsigned ix[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const uint32_t i = threadIdx.x * R + r;
+        v[r] = i < count ? keys[(i * step) >> 20] : ~0ull;
+        ix[r] = 0;
+    }
+    bitonic<R, false>(v, ix, sk, nullptr, m);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {  // bucket b: from splitters[b] (0: from the start) to splitters[b + 1]
+        const uint32_t e = threadIdx.x * R + r;
+        if (e < count && e % kOver == 0) splitters[e / kOver] = v[r];
+    }
+}
 
 __global__ void __launch_bounds__(1024) k_sort_split(const unsigned long long *__restrict__ keys, uint64_t n, uint32_t nb,
                                                      unsigned long long *__restrict__ splitters,
                                                      unsigned *__restrict__ cursor, unsigned *__restrict__ over) {
     extern __shared__ __align__(16) unsigned char dyn[];
     unsigned long long *sk = reinterpret_cast<unsigned long long *>(dyn);
-    constexpr int R = kSampleMost / 1024;
     const uint32_t count = kOver * nb;
     uint32_t m = 32;
     while (m < count) m <<= 1;
-    unsigned long long v[R];
-    unsigned ix[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const uint32_t i = threadIdx.x * R + r;
-        v[r] = i < count ? keys[(uint64_t)i * n / count] : ~0ull;
-        ix[r] = 0;
-    }
-    bitonic<R, false>(v, ix, sk, nullptr, m);
-    static_assert(R == kOver, "a thread's first key is a splitter");
-    if (threadIdx.x < nb) {  // bucket b: from splitters[b] (0: from the start) to splitters[b + 1]
-        splitters[threadIdx.x] = v[0];
-        cursor[threadIdx.x] = 0;
-    }
+    if (m <= 1024) split_of<1>(sk, keys, n, count, m, splitters);
+    else if (m <= 2048) split_of<2>(sk, keys, n, count, m, splitters);
+    else if (m <= 4096) split_of<4>(sk, keys, n, count, m, splitters);
+    else split_of<8>(sk, keys, n, count, m, splitters);
+    for (uint32_t b = threadIdx.x; b < nb; b += 1024) cursor[b] = 0;
     if (threadIdx.x == 0) *over = 0;
 }
 
-// Records to their buckets' regions of kOne records each, in any order.
+// Records to their buckets' regions of kRoom records each, in any order.
 constexpr int kSplitItems = 8;
 __global__ void __launch_bounds__(256) k_sort_scatter(const unsigned long long *__restrict__ keys,
                                                       const unsigned long long *__restrict__ mult, uint64_t n, uint32_t nb,
@@ -163,7 +186,7 @@ __global__ void __launch_bounds__(256) k_sort_scatter(const unsigned long long *
     }
     __syncthreads();
     unsigned long long kv[kSplitItems];
-    unsigned at[kSplitItems];  // bucket | rank << 10
+    unsigned at[kSplitItems];  // bucket | rank << 16
     const uint64_t r0 = (uint64_t)blockIdx.x * (256 * kSplitItems) + threadIdx.x;
 #pragma unroll
     for (int i = 0; i < kSplitItems; ++i) {
@@ -178,7 +201,7 @@ __global__ void __launch_bounds__(256) k_sort_scatter(const unsigned long long *
                 if (sp[mid] <= kv[i]) lo = mid;
                 else hi = mid;
             }
-            at[i] = lo | atomicAdd(&hist[lo], 1u) << 10;
+            at[i] = lo | atomicAdd(&hist[lo], 1u) << 16;
         }
     }
     __syncthreads();
@@ -189,10 +212,10 @@ __global__ void __launch_bounds__(256) k_sort_scatter(const unsigned long long *
     for (int i = 0; i < kSplitItems; ++i) {
         const uint64_t r = r0 + 256 * i;
         if (r < n) {
-            const uint32_t b = at[i] & (kSplitBuckets - 1), p = hist[b] + (at[i] >> 10);
-            if (p < kOne) {
-                bkeys[(uint64_t)b * kOne + p] = kv[i];
-                bmult[(uint64_t)b * kOne + p] = mult[r];
+            const uint32_t b = at[i] & 0xffffu, p = hist[b] + (at[i] >> 16);
+            if (p < kRoom) {
+                bkeys[(uint64_t)b * kRoom + p] = kv[i];
+                bmult[(uint64_t)b * kRoom + p] = mult[r];
             } else {
                 *over = 1;
             }
@@ -207,13 +230,14 @@ __global__ void __launch_bounds__(1024) k_sort_buckets(const unsigned *__restric
                                                        const unsigned long long *__restrict__ bmult,
                                                        unsigned long long *__restrict__ okeys,
                                                        unsigned long long *__restrict__ omult) {
-    __shared__ unsigned long long sk[kOne];
-    __shared__ unsigned short si[kOne];
+    __shared__ unsigned long long sk[kRoom];
+    __shared__ unsigned short si[kRoom];
     __shared__ uint64_t wb[32];
     if (*over) return;
-    uint64_t base = 0;  // nb <= 1024: one count a thread
-    block_exclusive_scan<1024>(threadIdx.x < blockIdx.x ? cursor[threadIdx.x] : 0u, wb, &base);
-    const uint64_t r0 = (uint64_t)blockIdx.x * kOne;
+    uint64_t before = 0, base = 0;
+    for (uint32_t b = threadIdx.x; b < blockIdx.x; b += 1024) before += cursor[b];
+    block_exclusive_scan<1024>(before, wb, &base);
+    const uint64_t r0 = (uint64_t)blockIdx.x * kRoom;
     sort_block(sk, si, bkeys + r0, bmult + r0, cursor[blockIdx.x], okeys + base, omult + base);
 }
 
@@ -307,7 +331,7 @@ __global__ void __launch_bounds__(256) k_sort_pass(const unsigned long long *__r
 uint64_t sort_scratch_bytes(uint64_t n) {
     if (n <= kOne) return 16 * n;
     const uint64_t nb = (n + kMean - 1) / kMean;
-    const uint64_t split = n <= kSplitMost ? 16 * n + 16 * nb * kOne + 16 * nb + 16 : 0;
+    const uint64_t split = n <= kSplitMost ? 16 * n + 16 * nb * kRoom + 16 * nb + 16 : 0;
     const uint64_t nc = (n + kTile - 1) / kTile * kDigits;
     return std::max(split, 32 * n + 8 * (nc + gscan_scratch(nc) + 1));
 }
@@ -326,7 +350,7 @@ swg_status copy_records_sorted(const unsigned long long *d_keys, const unsigned 
         k_sort_one<<<1, 1024, 0, s>>>(d_keys, d_mult, (uint32_t)n, k[0], m[0]);
     } else if (n <= kSplitMost && !radix) {
         const uint32_t nb = (uint32_t)((n + kMean - 1) / kMean);
-        unsigned long long *bk = m[0] + n, *bm = bk + (uint64_t)nb * kOne, *sp = bm + (uint64_t)nb * kOne;
+        unsigned long long *bk = m[0] + n, *bm = bk + (uint64_t)nb * kRoom, *sp = bm + (uint64_t)nb * kRoom;
         unsigned *cursor = reinterpret_cast<unsigned *>(sp + nb), *over = cursor + nb;
         allow_smem(k_sort_split, kSampleMost * sizeof(unsigned long long));
         k_sort_split<<<1, 1024, kSampleMost * sizeof(unsigned long long), s>>>(d_keys, n, nb, sp, cursor, over);

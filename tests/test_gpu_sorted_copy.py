@@ -20,7 +20,7 @@ def _check(g, n=None):
     assert np.array_equal(again[0], keys) and np.array_equal(again[1], mult)  # the graph's own order stays
 
 
-@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 1000, 4095, 4096, 4097, 8191, 8192, 8193, 70_001, 1_048_575, 1_048_576,
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 1000, 1022, 1023, 1024, 1025, 2047, 2048, 2049, 4095, 4096, 4097, 8191, 8192, 8193, 70_001, 1_048_575, 1_048_576,
                                1_048_577, 1_503_001])
 def test_sizes(n):
     rng = np.random.default_rng(n)
