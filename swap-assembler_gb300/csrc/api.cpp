@@ -336,18 +336,12 @@ swg_status build_impl(swg_graph *g, const swg_opts *o, const uint32_t *packed, u
 
     SWG_CUDA(cudaEventRecord(g->ev[0], s), "event");
     SWG_CUDA(cudaMemsetAsync(g->d_ctl, 0, sizeof(Control), s), "memset control");
-    SWG_CUDA(cudaMemsetAsync(g->d_prefix, 0, sizeof(uint64_t), s), "memset prefix");
     a.max_len = &g->d_ctl->max_len;
-    g->launches += swg::launch_occ_scan(a, s, false);  // the total; the per-read prefix below if needed
+    g->launches += swg::launch_occ_total(a, reinterpret_cast<unsigned long long *>(&g->d_ctl->occ_total), s);
     a.max_len = nullptr;
-    SWG_CUDA(cudaGetLastError(), "occurrence scan launch");
-    SWG_CUDA(cudaMemcpyAsync(&g->h_ctl->occ_total, g->d_prefix + n_reads, sizeof(uint64_t),
-                             cudaMemcpyDeviceToHost, s),
-             "read occurrence total");
-    SWG_CUDA(cudaMemcpyAsync(&g->h_ctl->max_len, &g->d_ctl->max_len, sizeof(unsigned),
-                             cudaMemcpyDeviceToHost, s),
-             "read longest read");
-    SWG_CUDA(cudaStreamSynchronize(s), "occurrence scan");
+    SWG_CUDA(cudaGetLastError(), "occurrence total launch");
+    SWG_CUDA(cudaMemcpyAsync(g->h_ctl, g->d_ctl, sizeof(Control), cudaMemcpyDeviceToHost, s), "read occurrence total");
+    SWG_CUDA(cudaStreamSynchronize(s), "occurrence total");
     a.total_occ = g->h_ctl->occ_total;
     g->occurrences = a.total_occ;
     g->retries = 0;
@@ -360,7 +354,8 @@ swg_status build_impl(swg_graph *g, const swg_opts *o, const uint32_t *packed, u
     // the per-read occurrence prefix and the tiles of kTileOcc occurrences:
     // every algorithm but the bucketed build's thread-per-read scatter uses them
     if (!bucketed || swg::level1_shape(o->scatter_shape) == 4) {
-        g->launches += swg::launch_occ_scan_write(a, s);
+        SWG_CUDA(cudaMemsetAsync(g->d_prefix, 0, sizeof(uint64_t), s), "memset prefix");
+        g->launches += swg::launch_occ_scan(a, s);
         a.n_tiles = (a.total_occ + swg::kTileOcc - 1) / swg::kTileOcc;
         if ((st = ensure(&g->d_tiles, &g->tiles_cap, a.n_tiles, "tile table"))) return st;
         a.tile_first_read = g->d_tiles;
@@ -1223,8 +1218,6 @@ swg_status grow_keep(T **p, uint64_t *cap, uint64_t want, uint64_t keep, const c
 }
 
 // ---- the bucketed build over super-k-mer records (super.cu) ----
-// Smaller inputs are bound by launches and latency, not by the records.
-constexpr uint64_t kSuperMin = 512ull << 10;
 // Longest read a streamed piece's scan takes whole (its records hold 14 bits
 // of position); a one-shot build cuts reads past kSuperWhole bases in pieces.
 constexpr uint64_t kSuperLongest = (1ull << 14) - 1;
@@ -1232,7 +1225,7 @@ constexpr uint64_t kSuperWhole = 512;
 
 bool super_build(const swg_opts *o, const BuildArgs &a, uint64_t N) {
     // (the other scatter shapes are shapes of the single-occurrence scatters)
-    return swg::super_window(a.k) && N >= kSuperMin && !swg::level1_shape(o->scatter_shape);
+    return swg::super_window(a.k) && N && !swg::level1_shape(o->scatter_shape);
 }
 
 // Sizes the build for N occurrences of n_reads reads, allocates its
@@ -1249,31 +1242,33 @@ swg_status super_plan(swg_graph *g, const swg_opts *o, const BuildArgs &a, uint6
     const uint64_t P = 1ull << b1, NB = P << b2;
     const double scale_max = 2.0 * stride / share;
     // a random sequence has 2 / (w + 1) runs per k-mer and one more per read
+    // (of those that have a k-mer)
     const uint64_t rec_cap =
-        (uint64_t)(1.25 * ((double)n_reads + 2.0 * (double)N / (swg::super_window(a.k) + 1))) + 65536;
-    const uint64_t rec1 = rec_cap + rec_cap / 4 + 1025 * P, rec2 = swg::super_bucket_room(rec_cap, NB, scale_max);
+        (uint64_t)(1.25 * ((double)std::min(n_reads, N) + 2.0 * (double)N / (swg::super_window(a.k) + 1))) + 65536;
+    // (rec_cap / 1000: the partition regions are worked out in single precision)
+    const uint64_t rec1 = rec_cap + rec_cap / 4 + rec_cap / 1000 + 1025 * P, rec2 = swg::super_bucket_room(rec_cap, NB, scale_max);
     if ((st = ensure(&g->d_part, &g->part_cap, 4 * P + 1, "partition table"))) return st;
     if ((st = ensure(&g->d_records, &g->records_cap, 2 * rec1, "records"))) return st;
     if ((st = ensure(&g->d_rec2, &g->rec2_cap, 2 * rec2, "bucket records"))) return st;
     const uint64_t scratch = swg::gscan_scratch(NB);
-    if ((st = ensure(&g->d_bk, &g->bk_cap, 4 * NB + 1 + scratch + 2 + P + 1, "bucket table"))) return st;
+    // d_bk: bucket samples / cursors [NB] | partition samples [P] | sample totals
+    // [2] (cleared together) | regions [NB+1] | overflow lists [2 NB] | scan scratch
+    if ((st = ensure(&g->d_bk, &g->bk_cap, 4 * NB + 1 + scratch + 2 + P, "bucket table"))) return st;
     swg::SkArgs sk = reads;  // off, len, seg, n_pieces, pieces
     sk.k = a.k;
     sk.b1 = b1;
     sk.b2 = b2;
     sk.n_parts = (uint32_t)P;
     sk.work = g->d_ctl->work;
-    sk.part_count = g->d_part;
     sk.part_start = g->d_part + P;
     sk.part_cursor = g->d_part + 2 * P + 1;
-    sk.part_end = g->d_part + 3 * P + 1;
     sk.cursor2 = g->d_bk;
-    sk.off2 = g->d_bk + NB;
+    sk.part_count = g->d_bk + NB;
+    sk.sampled = sk.part_count + P;
+    sk.off2 = sk.sampled + 2;
     sk.big = sk.off2 + NB + 1;
     sk.big2 = sk.big + NB;
     pl.scr = sk.big2 + NB;
-    sk.sampled = pl.scr + scratch;
-    sk.chunk_start = sk.sampled + 2;
     sk.status = &g->d_ctl->status;
     sk.rec1 = reinterpret_cast<uint4 *>(g->d_records);
     sk.rec2 = reinterpret_cast<uint4 *>(g->d_rec2);
@@ -1283,12 +1278,9 @@ swg_status super_plan(swg_graph *g, const swg_opts *o, const BuildArgs &a, uint6
     sk.big_count = &g->d_ctl->pad;
     sk.big2_count = &g->d_ctl->pad2;
     sk.big_cap = (uint32_t)std::min<uint64_t>(NB, 0xffffffffu);
-    SWG_CUDA(cudaMemsetAsync(sk.part_count, 0, P * 8, s), "clear partitions");
-    SWG_CUDA(cudaMemsetAsync(sk.cursor2, 0, NB * 8, s), "clear bucket samples");
-    SWG_CUDA(cudaMemsetAsync(sk.sampled, 0, 16, s), "clear sample totals");
+    SWG_CUDA(cudaMemsetAsync(sk.cursor2, 0, (NB + P + 2) * 8, s), "clear samples");
     g->launches += swg::launch_super_scan(a, sk, sk.n_pieces, stride, true, swg::kScatterResident, s);
     g->launches += swg::launch_super_caps(sk, NB, reinterpret_cast<uint64_t *>(pl.scr), s);
-    SWG_CUDA(cudaMemcpyAsync(sk.cursor2, sk.off2, NB * 8, cudaMemcpyDeviceToDevice, s), "bucket cursors");
     pl.b1 = b1;
     pl.b2 = b2;
     pl.P = P;
@@ -1299,6 +1291,16 @@ swg_status super_plan(swg_graph *g, const swg_opts *o, const BuildArgs &a, uint6
 }
 
 swg_status super_finish(swg_graph *g, const swg_opts *o, BuildArgs &a, cudaStream_t s, double load, BucketPlan &pl);
+
+// The record buffers given back, for the build over single occurrences to take
+// what it needs: where super-k-mer records do not fit the device (reads hardly
+// longer than k have about one each, 16 bytes against 8), it may.
+void drop_records(swg_graph *g) {
+    cudaFree(g->d_records);
+    cudaFree(g->d_rec2);
+    g->d_records = g->d_rec2 = nullptr;
+    g->records_cap = g->rec2_cap = 0;
+}
 
 swg_status build_super(swg_graph *g, const swg_opts *o, BuildArgs &a, cudaStream_t s, double load, uint64_t longest) {
     swg_status st;
@@ -1312,7 +1314,9 @@ swg_status build_super(swg_graph *g, const swg_opts *o, BuildArgs &a, cudaStream
     BuildArgs as = a;
     if (longest > kSuperWhole) {  // one thread per piece of 256 k-mers instead of one per read
         const uint64_t NP = swg::super_pieces_bound(a.n_reads, a.total_occ), S = swg::gscan_scratch(a.n_reads);
-        if ((st = ensure(&g->d_pieces, &g->pieces_cap, 2 * NP + 2 * a.n_reads + S + 2, "read pieces"))) return st;
+        st = ensure(&g->d_pieces, &g->pieces_cap, 2 * NP + 2 * a.n_reads + S + 2, "read pieces");
+        if (st == SWG_ERR_OOM) return build_bucketed(g, o, a, s, load);
+        if (st) return st;
         uint64_t *off = g->d_pieces, *count = off + NP, *first = count + a.n_reads, *scratch = first + a.n_reads,
                  *range = scratch + S;
         uint32_t *len = reinterpret_cast<uint32_t *>(range + 2), *seg = len + NP;
@@ -1327,9 +1331,15 @@ swg_status build_super(swg_graph *g, const swg_opts *o, BuildArgs &a, cudaStream
         as.read_range = reinterpret_cast<unsigned long long *>(range);
     }
     BucketPlan pl;
-    // the sample sizes the regions: a sixteenth of the reads, a quarter of small inputs
-    const uint32_t stride = a.total_occ >= (64ull << 20) ? 16 : 4;
-    if ((st = super_plan(g, o, as, a.total_occ, reads.n_pieces, stride, 1.0, reads, s, pl))) return st;
+    // the sample sizes the regions: a sixteenth of the reads, more of small
+    // inputs (all below 4M occurrences: a batch of 256 reads is much of them)
+    const uint32_t stride = a.total_occ >= (64ull << 20) ? 16 : (a.total_occ >= (4ull << 20) ? 4 : 1);
+    st = super_plan(g, o, as, a.total_occ, reads.n_pieces, stride, 1.0, reads, s, pl);
+    if (st == SWG_ERR_OOM) {
+        drop_records(g);
+        return build_bucketed(g, o, a, s, load);
+    }
+    if (st) return st;
     SWG_CUDA(cudaEventRecord(g->ev[1], s), "event");
     g->launches += swg::launch_super_scan(as, pl.sk, reads.n_pieces, 1, false, swg::kScatterResident, s);
     SWG_CUDA(cudaGetLastError(), "super-k-mer scan launch");
@@ -1342,6 +1352,12 @@ swg_status ensure_out(swg_graph *g, uint64_t want, uint64_t keep) {
     if (g->out_cap >= want && g->d_out_keys && g->d_out_mult) return SWG_OK;
     swg_status st;
     uint64_t c1 = 0, c2 = 0;
+    if (!keep) {
+        cudaFree(g->d_out_keys);
+        cudaFree(g->d_out_mult);
+        g->d_out_keys = g->d_out_mult = nullptr;
+        g->out_cap = 0;
+    }
     if ((st = grow_keep(&g->d_out_keys, &c1, want, keep, "output keys"))) return st;
     if ((st = grow_keep(&g->d_out_mult, &c2, want, keep, "output multiplicities"))) {
         g->out_cap = 0;
@@ -1374,7 +1390,8 @@ swg_status super_finish(swg_graph *g, const swg_opts *o, BuildArgs &a, cudaStrea
     // first (fewer at any usual coverage), exactly what is needed on a rerun
     // of the count (the records are still there)
     const uint64_t c = (uint64_t)std::max(a.cutoff, 1);
-    if ((st = ensure_out(g, std::max<uint64_t>(a.tag_bits ? N / 8 : std::min(N / 8, N / c), 1), 0))) return st;
+    st = ensure_out(g, std::max<uint64_t>(a.tag_bits ? N / 8 : std::min(N / 8, N / c), 1), 0);
+    if (st && st != SWG_ERR_OOM) return st;  // (no room for the guess: the count alone says how much is needed)
     for (int attempt = 0;; ++attempt) {
         a.out_keys = g->d_out_keys;
         a.out_mult = g->d_out_mult;
@@ -1386,7 +1403,7 @@ swg_status super_finish(swg_graph *g, const swg_opts *o, BuildArgs &a, cudaStrea
                  "read status");
         SWG_CUDA(cudaEventRecord(g->ev[4], s), "event");
         SWG_CUDA(cudaStreamSynchronize(s), "bucket count");
-        const bool again = g->h_ctl->status & swg::kStatusPartOverflow;
+        bool again = g->h_ctl->status & swg::kStatusPartOverflow;
         const uint64_t n = g->h_ctl->counters[1];
         if (!again && n <= g->out_cap) break;
         if (attempt) {
@@ -1396,11 +1413,15 @@ swg_status super_finish(swg_graph *g, const swg_opts *o, BuildArgs &a, cudaStrea
         SWG_CUDA(cudaMemsetAsync(g->d_ctl, 0, sizeof(Control) - sizeof(uint64_t), s), "clear control");
         if (a.tag_bits)
             SWG_CUDA(cudaMemsetAsync(a.seg_counts, 0, 2ull * a.n_segs * 8, s), "clear sample counters");
+        if (!again && (st = ensure_out(g, n, 0))) {
+            if (st != SWG_ERR_OOM) return st;
+            drop_records(g);
+            again = true;
+        }
         if (again) {
             a = plain;
             return build_bucketed(g, o, a, s, load, true);
         }
-        if ((st = ensure_out(g, n, 0))) return st;
     }
     const unsigned nbig = g->h_ctl->pad2;  // buckets no shared-memory table held
     const unsigned retries = g->h_ctl->pad;
@@ -1701,9 +1722,11 @@ swg_status build_fasta_streamed(swg_graph *g, const swg_opts *o, const char *fir
                     reads.n_pieces = reads_c;
                     st = super_plan(g, o, a0, N_est, (uint64_t)(scale * (double)reads_c * 1.02), stride, 1.0 / scale,
                                     reads, s, pl);
+                    if (st == SWG_ERR_OOM) drop_records(g);
                 } else {
-                    st = bucketed_plan(g, o, a0, N_est, false, stride, s, pl);
+                    st = SWG_ERR_OOM;
                 }
+                if (st == SWG_ERR_OOM) st = bucketed_plan(g, o, a0, N_est, false, stride, s, pl);
                 if (st) return st;
                 SWG_CUDA(cudaEventRecord(g->ev[1], s), "event");
             }

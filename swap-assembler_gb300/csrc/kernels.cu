@@ -66,6 +66,26 @@ __global__ void __launch_bounds__(kScanBlock) k_scan_reduce(BuildArgs a) {
     }
 }
 
+// The occurrences of all reads (added to *total) and the longest read, for the
+// builds that need no per-read prefix: one launch of resident blocks.
+__global__ void __launch_bounds__(kScanBlock) k_occ_total(const uint32_t *__restrict__ len, uint64_t n_reads, int k,
+                                                          unsigned long long *total, unsigned *longest) {
+    unsigned long long s = 0;
+    uint32_t most = 0;
+    for (uint64_t r = (uint64_t)blockIdx.x * kScanBlock + threadIdx.x; r < n_reads; r += (uint64_t)gridDim.x * kScanBlock) {
+        const uint32_t L = len[r];
+        s += occ_of(L, k);
+        most = max(most, L);
+    }
+#pragma unroll
+    for (int d = 16; d; d >>= 1) s += __shfl_down_sync(kFull, s, d);
+    most = __reduce_max_sync(kFull, most);
+    if ((threadIdx.x & 31) == 0 && most) {
+        atomicAdd(total, s);
+        atomicMax(longest, most);
+    }
+}
+
 __global__ void __launch_bounds__(1024) k_scan_blocks(uint64_t *block_sums, uint64_t nb,
                                                       uint64_t *occ_total) {
     __shared__ uint64_t wb[32];
@@ -2061,20 +2081,20 @@ int device_sm_count() {
 
 uint64_t scan_block_count(uint64_t n_reads) { return (n_reads + kScanChunk - 1) / kScanChunk; }
 
-int launch_occ_scan(const BuildArgs &a, cudaStream_t s, bool write) {
+int launch_occ_scan(const BuildArgs &a, cudaStream_t s) {
     const uint64_t nb = scan_block_count(a.n_reads);
     if (nb == 0) return 0;
     k_scan_reduce<<<(unsigned)nb, kScanBlock, 0, s>>>(a);
     k_scan_blocks<<<1, 1024, 0, s>>>(a.scan_blocks, nb, a.occ_prefix + a.n_reads);
-    if (!write) return 2;
     k_scan_write<<<(unsigned)nb, kScanBlock, 0, s>>>(a);
     return 3;
 }
 
-int launch_occ_scan_write(const BuildArgs &a, cudaStream_t s) {
-    const uint64_t nb = scan_block_count(a.n_reads);
-    if (nb == 0) return 0;
-    k_scan_write<<<(unsigned)nb, kScanBlock, 0, s>>>(a);
+int launch_occ_total(const BuildArgs &a, unsigned long long *total, cudaStream_t s) {
+    if (!a.n_reads) return 0;
+    const uint64_t blocks = (a.n_reads + 4 * kScanBlock - 1) / (4 * kScanBlock);
+    k_occ_total<<<(unsigned)std::min<uint64_t>(blocks, (uint64_t)device_sm_count() * 8), kScanBlock, 0, s>>>(
+        a.read_len, a.n_reads, a.k, total, a.max_len);
     return 1;
 }
 

@@ -14,7 +14,7 @@
 //   k_sk_pieces_*  long reads cut into pieces of kSkPiece k-mers
 //   k_sk_scan      minimizers, runs; level-1 scatter of the records (or, on a
 //                  sample of the reads, sizes per partition and bucket)
-//   k_sk_caps, k_sk_bucket_caps, k_sk_chunks   regions and chunks
+//   k_sk_regions (or k_sk_caps, k_sk_bucket_caps)   regions
 //   k_sk_sub       level-2 scatter into buckets
 //   k_sk_count*    per-bucket counting, cutoff, survivors
 //   k_sk_big       buckets no shared-memory table holds
@@ -295,9 +295,42 @@ __device__ __forceinline__ double sk_records(const SkArgs &s, uint64_t sampled) 
     return r < (double)s.rec_cap ? r : (double)s.rec_cap;
 }
 
-// Partition regions: 1.25 x the partition's share of the expected records +
-// 1024, laid out by exclusive prefix (one block). The sampled total goes to
-// sampled[0].
+// What the regions follow from: the records expected and those per sampled
+// record (worked out once a block: 64-bit arithmetic is slow here, and regions
+// of single-precision sizes are as good).
+struct SkScale {
+    float r, f;
+    bool sampled;
+};
+__device__ __forceinline__ SkScale sk_scale(const SkArgs &s, uint64_t sampled, SkScale *shared) {
+    if (threadIdx.x == 0) {
+        const double r = sk_records(s, sampled);
+        shared->r = (float)r;
+        shared->f = sampled ? (float)fmin(r / (double)sampled, s.scale_max) : 0.0f;
+        shared->sampled = sampled != 0;
+    }
+    __syncthreads();
+    return *shared;
+}
+
+// A partition's region: 1.25 x its share of the expected records + 1024.
+__device__ __forceinline__ uint64_t part_cap(const SkArgs &s, uint64_t count, const SkScale &x) {
+    return (uint64_t)(1.25f * (x.sampled ? (float)count * x.f : x.r / (float)s.n_parts)) + 1024;
+}
+
+// A bucket's region. Its sample is a few dozen records, so the region covers
+// the mean that is six standard deviations of a Poisson count above what was
+// seen, and a quarter more for tandem repeats, whose reads bring several
+// records each to one bucket: 1.25 c + 18 + 6 sqrt(c + 9) sampled records,
+// times the input's records per sampled one (at most scale_max, which the
+// buffers are sized for).
+__device__ __forceinline__ uint64_t bucket_cap(uint64_t count, const SkScale &x, uint64_t nb) {
+    const float c = (float)count;
+    return (uint64_t)(x.sampled ? x.f * (1.25f * c + 18.0f + 6.0f * sqrtf(c + 9.0f)) : x.r / (float)nb);
+}
+
+// Partition regions, laid out by exclusive prefix (one block). The sampled
+// total goes to sampled[0].
 __global__ void __launch_bounds__(1024) k_sk_caps(SkArgs s) {
     __shared__ uint64_t wb[32];
     const uint32_t j = threadIdx.x;
@@ -305,10 +338,9 @@ __global__ void __launch_bounds__(1024) k_sk_caps(SkArgs s) {
     uint64_t total;
     block_exclusive_scan<1024>(c, wb, &total);
     uint64_t cap = 0;
-    if (j < s.n_parts) {
-        const double share = total ? (double)c / (double)total : 1.0 / (double)s.n_parts;
-        cap = (uint64_t)(share * sk_records(s, total) * 1.25) + 1024;
-    }
+    __shared__ SkScale sc;
+    const SkScale x = sk_scale(s, total, &sc);
+    if (j < s.n_parts) cap = part_cap(s, c, x);
     uint64_t all;
     const uint64_t ex = block_exclusive_scan<1024>(cap, wb, &all);
     if (j < s.n_parts) {
@@ -321,46 +353,64 @@ __global__ void __launch_bounds__(1024) k_sk_caps(SkArgs s) {
     }
 }
 
-// Bucket regions (counts and caps may be the same array). A bucket's sample is
-// a few dozen records, so its region covers the mean that is six standard
-// deviations of a Poisson count above what was seen, and a quarter more for
-// tandem repeats, whose reads bring several records each to one bucket:
-// 1.25 c + 18 + 6 sqrt(c + 9) sampled records, times the input's records per
-// sampled one (at most scale_max, which the buffers are sized for).
+// Bucket regions (counts and caps may be the same array).
 __global__ void __launch_bounds__(256) k_sk_bucket_caps(SkArgs s, const unsigned long long *counts, uint64_t nb,
                                                         unsigned long long *caps) {
+    __shared__ SkScale sc;
+    const SkScale x = sk_scale(s, s.sampled[0], &sc);
     const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= nb) return;
-    const uint64_t t = s.sampled[0];
-    const double r = sk_records(s, t), c = (double)counts[j];
-    const double f = t ? fmin(r / (double)t, s.scale_max) : 0.0;
-    caps[j] = (uint64_t)(t ? f * (1.25 * c + 18.0 + 6.0 * sqrt(c + 9.0)) : r / (double)nb);
+    if (j < nb) caps[j] = bucket_cap(counts[j], x, nb);
 }
 
-// End of every partition's records (an overflow flagged) and its level-2
-// chunks as an exclusive prefix.
-__global__ void __launch_bounds__(1024) k_sk_chunks(SkArgs s) {
+// Both kinds of regions of a plan of at most 1024 kRegionItems buckets, and
+// the cursors at their starts, by one block (six launches otherwise, most of a
+// small build's preparation).
+constexpr int kRegionItems = 16;
+__global__ void __launch_bounds__(1024) k_sk_regions(SkArgs s, uint32_t nb) {
     __shared__ uint64_t wb[32];
     const uint32_t j = threadIdx.x;
-    uint64_t c = 0;
+    const uint64_t pc = j < s.n_parts ? s.part_count[j] : 0;
+    uint64_t sampled;
+    block_exclusive_scan<1024>(pc, wb, &sampled);
+    __shared__ SkScale sc;
+    const SkScale x = sk_scale(s, sampled, &sc);
+    uint64_t cap = 0, all;
+    if (j < s.n_parts) cap = part_cap(s, pc, x);
+    const uint64_t ex = block_exclusive_scan<1024>(cap, wb, &all);
     if (j < s.n_parts) {
-        uint64_t end = s.part_cursor[j];
-        if (end > s.part_start[j + 1]) {
-            atomicOr(s.status, kStatusPartOverflow);
-            end = s.part_start[j + 1];
-        }
-        s.part_end[j] = end;
-        c = (end - s.part_start[j] + kSkChunk - 1) / kSkChunk;
+        s.part_start[j] = ex;
+        s.part_cursor[j] = ex;
     }
-    uint64_t total;
-    const uint64_t ex = block_exclusive_scan<1024>(c, wb, &total);
-    if (j < s.n_parts) s.chunk_start[j] = ex;
-    if (j == 0) s.chunk_start[s.n_parts] = total;
+    if (j == 0) s.part_start[s.n_parts] = all;
+    const uint32_t per = (nb + 1023) / 1024;
+    uint64_t c[kRegionItems], sum = 0;
+#pragma unroll
+    for (int i = 0; i < kRegionItems; ++i) {
+        const uint32_t b = j * per + i;
+        c[i] = i < (int)per && b < nb ? bucket_cap(s.cursor2[b], x, nb) : 0;
+        sum += c[i];
+    }
+    uint64_t at = block_exclusive_scan<1024>(sum, wb, &all);
+#pragma unroll
+    for (int i = 0; i < kRegionItems; ++i) {
+        const uint32_t b = j * per + i;
+        if (i < (int)per && b < nb) {
+            s.off2[b] = at;
+            s.cursor2[b] = at;
+        }
+        at += c[i];
+    }
+    if (j == 0) s.off2[nb] = all;
 }
 
 // Level-2 scatter: a chunk of one partition's records is held in registers,
 // ordered by sub-bucket in shared memory and written as one run per bucket.
-size_t sub_smem(int b2) { return kSkChunk * sizeof(uint4) + ((size_t)1 << b2) * (sizeof(unsigned long long) + 3 * sizeof(unsigned)); }
+// Every block works out the partitions' chunks for itself (and flags a
+// partition that outgrew its region).
+size_t sub_smem(int b2, uint32_t n_parts) {
+    return kSkChunk * sizeof(uint4) + ((size_t)1 << b2) * (sizeof(unsigned long long) + 3 * sizeof(unsigned)) +
+           (n_parts + 1) * sizeof(unsigned);
+}
 
 __global__ void __launch_bounds__(256, 4) k_sk_sub(SkArgs s) {
     constexpr int NT = 256, IT = kSubItems;
@@ -370,19 +420,46 @@ __global__ void __launch_bounds__(256, 4) k_sk_sub(SkArgs s) {
     unsigned long long *dst = reinterpret_cast<unsigned long long *>(sorted + kSkChunk);
     unsigned *hist = reinterpret_cast<unsigned *>(dst + P2);
     unsigned *loff = hist + P2, *lim = loff + P2;
+    unsigned *chunk_start = lim + P2;
     __shared__ uint64_t wb[NT / 32];
     const uint32_t per = (P2 + NT - 1) / NT, submask = P2 - 1;
-    const uint64_t nq = *s.status & kStatusPartOverflow ? 0 : s.chunk_start[s.n_parts];
     for (uint32_t j = threadIdx.x; j < P2; j += NT) hist[j] = 0;
+    const uint32_t pp = (s.n_parts + NT - 1) / NT;
+    unsigned chunks = 0;
+    bool outgrown = false;
+    for (uint32_t x = 0; x < pp; ++x) {
+        const uint32_t j = threadIdx.x * pp + x;
+        if (j < s.n_parts) {
+            const uint64_t end = s.part_cursor[j], lim2 = s.part_start[j + 1];
+            outgrown |= end > lim2;
+            const unsigned c = (unsigned)((umin64(end, lim2) - s.part_start[j] + kSkChunk - 1) / kSkChunk);
+            chunk_start[j] = c;
+            chunks += c;
+        }
+    }
+    uint64_t nq;
+    unsigned run0 = (unsigned)block_exclusive_scan<NT>(chunks, wb, &nq);
+    for (uint32_t x = 0; x < pp; ++x) {
+        const uint32_t j = threadIdx.x * pp + x;
+        if (j < s.n_parts) {
+            const unsigned c = chunk_start[j];
+            chunk_start[j] = run0;
+            run0 += c;
+        }
+    }
+    if (__syncthreads_or(outgrown || (*s.status & kStatusPartOverflow))) {  // the build recounts
+        if (threadIdx.x == 0) atomicOr(s.status, kStatusPartOverflow);
+        return;
+    }
     for (uint64_t q = blockIdx.x; q < nq; q += gridDim.x) {
         uint32_t lo = 0, hi = s.n_parts;
         while (hi - lo > 1) {
             const uint32_t mid = (lo + hi) >> 1;
-            if (s.chunk_start[mid] <= q) lo = mid;
+            if (chunk_start[mid] <= q) lo = mid;
             else hi = mid;
         }
-        const uint64_t r0 = s.part_start[lo] + (q - s.chunk_start[lo]) * kSkChunk;
-        const uint32_t n = (uint32_t)umin64(kSkChunk, s.part_end[lo] - r0);
+        const uint64_t r0 = s.part_start[lo] + (q - chunk_start[lo]) * kSkChunk;
+        const uint32_t n = (uint32_t)umin64(kSkChunk, umin64(s.part_cursor[lo], s.part_start[lo + 1]) - r0);
         uint4 v[IT];
 #pragma unroll
         for (int it = 0; it < IT; ++it) {
@@ -844,7 +921,7 @@ __device__ void count_pass(const BuildArgs &a, const SkArgs &s, uint64_t n_items
 // CTA of 1024 threads an SM with 8192 entries, over tier 1's overflow list.
 template <int T, int NT, int kK>
 __global__ void __launch_bounds__(NT, 1024 / NT) k_sk_count(BuildArgs a, SkArgs s, uint64_t n) {
-    if (*s.status & kStatusPartOverflow) return;
+    if ((*s.status & kStatusPartOverflow) || (T == 8192 && blockIdx.x >= *s.big_count)) return;
     if (T == 8192) count_pass<T, NT, kK>(a, s, umin64(*s.big_count, s.big_cap), s.big, s.big2, s.big2_count);
     else count_pass<T, NT, kK>(a, s, n, nullptr, s.big, s.big_count);
 }
@@ -950,7 +1027,8 @@ int launch_super_scan(const BuildArgs &a, const SkArgs &s, uint64_t bound, uint3
 // sum over the buckets, by the square root's concavity
 uint64_t super_bucket_room(uint64_t records, uint64_t nb, double scale_max) {
     const double mean = (double)records / (double)nb / scale_max;
-    return records + records / 4 + (uint64_t)((double)nb * scale_max * (18.0 + 6.0 * std::sqrt(mean + 9.0))) + nb;
+    const double most = 1.25 * (double)records + (double)nb * scale_max * (18.0 + 6.0 * std::sqrt(mean + 9.0));
+    return (uint64_t)(1.001 * most) + nb;  // (the regions are worked out in single precision)
 }
 
 uint64_t super_pieces_bound(uint64_t n_reads, uint64_t occurrences) { return n_reads + occurrences / kSkPiece + 1; }
@@ -964,19 +1042,24 @@ int launch_super_pieces(const BuildArgs &a, uint64_t *count, uint64_t *first, ui
 }
 
 int launch_super_caps(const SkArgs &s, uint64_t nb, uint64_t *scratch, cudaStream_t st) {
+    if (nb <= 1024 * kRegionItems) {
+        k_sk_regions<<<1, 1024, 0, st>>>(s, (uint32_t)nb);
+        return 1;
+    }
     k_sk_caps<<<1, 1024, 0, st>>>(s);
     k_sk_bucket_caps<<<(unsigned)((nb + 255) / 256), 256, 0, st>>>(s, s.cursor2, nb, s.cursor2);
-    return 2 + launch_gscan(reinterpret_cast<const uint64_t *>(s.cursor2), reinterpret_cast<uint64_t *>(s.off2), nb,
-                            scratch, reinterpret_cast<uint64_t *>(s.off2 + nb), st);
+    const int n = launch_gscan(reinterpret_cast<const uint64_t *>(s.cursor2), reinterpret_cast<uint64_t *>(s.off2), nb,
+                               scratch, reinterpret_cast<uint64_t *>(s.off2 + nb), st);
+    cudaMemcpyAsync(s.cursor2, s.off2, nb * 8, cudaMemcpyDeviceToDevice, st);
+    return 2 + n;
 }
 
 int launch_super_sub(const SkArgs &s, cudaStream_t st) {
-    k_sk_chunks<<<1, 1024, 0, st>>>(s);
-    const size_t smem = sub_smem(s.b2);
-    allow_smem(k_sk_sub, sub_smem(10));
+    const size_t smem = sub_smem(s.b2, s.n_parts);
+    allow_smem(k_sk_sub, sub_smem(10, 1u << kPartBitsMax));
     const uint64_t chunks = s.rec_cap * 5 / 4 / kSkChunk + s.n_parts;
     k_sk_sub<<<(unsigned)std::min<uint64_t>(chunks, resident_grid(k_sk_sub, 256, smem)), 256, smem, st>>>(s);
-    return 2;
+    return 1;
 }
 
 template <int kK>

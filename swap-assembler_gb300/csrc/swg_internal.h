@@ -152,11 +152,9 @@ struct SkArgs {
     unsigned long long *part_count;        // [n_parts] sampled records
     unsigned long long *part_start;        // [n_parts + 1]
     unsigned long long *part_cursor;       // [n_parts]
-    unsigned long long *part_end;          // [n_parts]
     unsigned long long *sampled;           // [2] sampled records, sampled k-mers
     unsigned long long *cursor2;           // [n_buckets] sampled records, then cursors
     unsigned long long *off2;              // [n_buckets + 1] bucket regions
-    unsigned long long *chunk_start;       // [n_parts + 1]
     unsigned *status;
     uint4 *rec1, *rec2;
     uint64_t n_kmers;                      // occurrences expected in the whole input
@@ -187,11 +185,11 @@ int launch_super_big(const BuildArgs &a, const SkArgs &sk, const unsigned long l
 int launch_big_compact(const BuildArgs &a, const Entry *table, uint64_t cap, cudaStream_t s);
 
 // Kernel launchers (kernels.cu). Each returns the number of launches made.
-// The occurrence total (into occ_prefix[n_reads]) and, with write, the
-// per-read prefix; launch_occ_scan_write adds the prefix to a scan made
-// without it.
-int launch_occ_scan(const BuildArgs &a, cudaStream_t s, bool write = true);
-int launch_occ_scan_write(const BuildArgs &a, cudaStream_t s);
+// The per-read occurrence prefix, its total in occ_prefix[n_reads] (and the
+// longest read maxed into max_len, if set).
+int launch_occ_scan(const BuildArgs &a, cudaStream_t s);
+// The total alone (one k), added to *total, and the longest read.
+int launch_occ_total(const BuildArgs &a, unsigned long long *total, cudaStream_t s);
 // The level-1 scatter's block shape for swg_opts::scatter_shape (0: the
 // SWG_SCATTER_SHAPE default).
 int level1_shape(int opt_shape);
