@@ -623,8 +623,8 @@ __device__ __forceinline__ bool bucket_keep(const unsigned *cnt, uint32_t s, uns
 // Buckets whose keys do not fit go to the overflow list uncounted; their
 // records stay as they are.
 template <int T, int NT, int kK>
-__device__ void count_pass(const BuildArgs &a, const SkArgs &s, uint64_t n_items, const unsigned long long *list,
-                           unsigned long long *ovf, unsigned *ovf_count) {
+__device__ void count_pass(const BuildArgs &a, const SkArgs &s, uint64_t n_items, uint32_t set,
+                           const unsigned long long *list, unsigned long long *ovf, unsigned *ovf_count) {
     constexpr int kBits = T == 2048 ? 11 : (T == 4096 ? 12 : 13);
     constexpr int NW = NT / 32, SEG = T * 3 / 2 / NW, R = NT == 1024 ? 3 : 4;
     constexpr uint32_t CH = R * NT;
@@ -642,7 +642,9 @@ __device__ void count_pass(const BuildArgs &a, const SkArgs &s, uint64_t n_items
     unsigned *stab = cnt + 4 * CH;                               // table: first record (index + 1) | others << 16;
     unsigned *sdis = reinterpret_cast<unsigned *>(lists);        // distinct records: index | weight << 16,
     unsigned short *sbefore = reinterpret_cast<unsigned short *>(sdis + CH);  // k-mers before each
-    __shared__ unsigned s_over, s_total;
+    __shared__ unsigned s_over, s_total, s_added;
+    __shared__ uint64_t s_start[2][4];
+    __shared__ unsigned s_n[2][4];
     const uint32_t lane = threadIdx.x & 31, wp = threadIdx.x >> 5, lt = (1u << lane) - 1;
     unsigned short *const used = lists + wp * SEG;
     const int tb = a.tag_bits, k = s.k;
@@ -656,57 +658,108 @@ __device__ void count_pass(const BuildArgs &a, const SkArgs &s, uint64_t n_items
     // (a cutoff of 0 keeps what 1 keeps: a multiplicity of 0 is no arc)
     const unsigned cbias = (0x8000u - (unsigned)min(max(c, 1), 255)) * 0x00010001u;
     const uint4 none = make_uint4(0, 0, 0, 0);
+    // The CTA's buckets come in sets of `set` neighbours; it counts as many of a
+    // set at once as it expects to fit its table (by the distinct keys a record
+    // that it has seen) and the merging's CH records: what is done once per
+    // pass, half the time of a pass over a bucket of few distinct k-molecules,
+    // is then shared. Two sets' bounds are kept, the later one read ahead.
+    const uint32_t n_sets = (uint32_t)((n_items + set - 1) / set);  // (at most 2^20 buckets)
+    bool outgrown = false;
+    auto fetch = [&](uint32_t q, int buf) {
+        if (threadIdx.x < set) {
+            const uint64_t it = (uint64_t)q * set + threadIdx.x;
+            uint64_t start = 0, n = 0;
+            if (it < n_items) {
+                const uint64_t bk = list ? list[it] : it;
+                start = s.off2[bk];
+                const uint64_t end = s.cursor2[bk], lim = s.off2[bk + 1];
+                outgrown |= end > lim;
+                n = umin64(end, lim) - start;
+            }
+            s_start[buf][threadIdx.x] = start;
+            s_n[buf][threadIdx.x] = (unsigned)umin64(n, 1u << 30);
+        }
+    };
+    uint32_t per_record = 32 << 8;  // distinct keys a record so far, 8 fraction bits (before the first pass: one bucket)
+    uint32_t cur = blockIdx.x;      // set, its buffer, the pass's first bucket in it, how many, their records
+    int buf = 0;
+    uint32_t i0 = 0, nb = 0, nrec = 0;
+    auto pick = [&]() {
+        nb = 1;
+        nrec = s_n[buf][i0];
+        while (i0 + nb < set) {
+            const uint32_t n = nrec + s_n[buf][i0 + nb];
+            if (n > CH || (n * per_record) >> 8 > (uint32_t)T * 15 / 32) break;  // (no overflow: n <= CH, a record's 17 k-mers)
+            nrec = n;
+            ++nb;
+        }
+    };
     uint4 rec[R];
-    // record i * NT + threadIdx.x of a bucket's first min(n, CH)
-    auto load = [&](uint64_t rb, uint64_t n) {
+    auto load = [&]() {  // record i * NT + threadIdx.x of the pass's first min(nrec, CH)
+        if (nb == 1) {
+            const uint4 *from = s.rec2 + s_start[buf][i0];
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const uint32_t r = i * NT + threadIdx.x;
+                rec[i] = r < nrec ? from[r] : none;
+            }
+            return;
+        }
 #pragma unroll
         for (int i = 0; i < R; ++i) {
-            const uint32_t r = i * NT + threadIdx.x;
-            rec[i] = r < n ? s.rec2[rb + r] : none;
-        }
-    };
-    // bucket of item it, its records [rb, rb + nrec)
-    uint64_t bk = 0, rb = 0, nrec = 0;
-    bool outgrown = false;
-    auto bounds = [&](uint64_t it) {
-        bk = list ? list[it] : it;
-        rb = s.off2[bk];
-        const uint64_t end = s.cursor2[bk], lim = s.off2[bk + 1];
-        outgrown |= end > lim;
-        nrec = umin64(end, lim) - rb;
-    };
-    uint64_t next_bk = 0, next_rb = 0, next_n = 0;
-    if (blockIdx.x < n_items) {
-        bounds(blockIdx.x);
-        next_bk = bk, next_rb = rb, next_n = nrec;
-    }
-    bool have = false;  // rec holds this bucket's first records
-    unsigned long long distinct = 0;  // keys this warp added to tables
-    for (uint64_t it = blockIdx.x; it < n_items; it += gridDim.x) {
-        const uint64_t nit = it + gridDim.x;
-        {
-            const uint64_t tk = next_bk, tr = next_rb, tn = next_n;
-            if (nit < n_items) bounds(nit);
-            else nrec = 0;
-            next_bk = bk, next_rb = rb, next_n = nrec;
-            bk = tk, rb = tr, nrec = tn;
-        }
-        if (!have) load(rb, nrec);
-        have = false;
-        if (nrec == 0 || nrec > kSkBigRecords) {
-            if (nrec && threadIdx.x == 0) {
-                const unsigned i = atomicAdd(ovf_count, 1u);
-                if (i < s.big_cap) ovf[i] = bk;
+            uint32_t r = i * NT + threadIdx.x, j = i0;
+            rec[i] = none;
+            if (r < nrec) {
+                while (j + 1 < i0 + nb && r >= s_n[buf][j]) r -= s_n[buf][j++];
+                rec[i] = s.rec2[s_start[buf][j] + r];
             }
+        }
+    };
+    auto overflow = [&]() {  // the pass's buckets to the overflow list (one thread)
+        for (uint32_t j = i0; j < i0 + nb; ++j) {
+            const uint64_t it = (uint64_t)cur * set + j;
+            if (!s_n[buf][j]) continue;
+            const unsigned i = atomicAdd(ovf_count, 1u);
+            if (i < s.big_cap) ovf[i] = list ? list[it] : it;
+        }
+    };
+    fetch(cur, 0);
+    fetch(cur + gridDim.x, 1);
+    __syncthreads();
+    pick();
+    load();
+    unsigned long long distinct = 0;  // keys this warp added to tables
+    // to the next pass's buckets; the set after the next one is fetched at the
+    // top of the first pass over a set, which is past all reads of its buffer
+    bool fresh_set = false;
+    auto advance = [&]() {
+        i0 += nb;
+        if (i0 >= set) {
+            i0 = 0;
+            cur += gridDim.x;
+            buf ^= 1;
+            fresh_set = true;
+        }
+        pick();
+    };
+    while (cur < n_sets) {
+        __syncthreads();  // the previous pass is done: the table is all zero
+        if (fresh_set) fetch(cur + gridDim.x, buf ^ 1);
+        fresh_set = false;
+        if (nrec > kSkBigRecords) {
+            if (threadIdx.x == 0) overflow();
+            __syncthreads();  // (the bounds fetched above are read from here on)
+            advance();
+            load();
             continue;
         }
-        __syncthreads();  // the previous bucket is done: the table is all zero
         if (threadIdx.x == 0) {
             s_over = 0;
             s_total = 0;
+            s_added = 0;
         }
         // equal records among the first CH merged
-        const uint32_t n0 = (uint32_t)umin64(nrec, CH);
+        const uint32_t n0 = min(nrec, CH);
         const int tbits = min(31 - __clz(4 * n0 + 255), 31 - __clz(2 * CH));
 #pragma unroll
         for (int i = 0; i < R; ++i)
@@ -839,7 +892,7 @@ __device__ void count_pass(const BuildArgs &a, const SkArgs &s, uint64_t n_items
         }
         // a larger bucket's other records, one by one; the counters (which
         // saturate at 255 in the end) are clamped before they can carry
-        for (uint64_t c0 = CH; c0 < nrec; c0 += kSkClamp) {
+        for (uint32_t c0 = CH; c0 < nrec; c0 += kSkClamp) {
             __syncthreads();
             for (uint32_t j = threadIdx.x; j < (uint32_t)T; j += NT) {
                 uint4 *e = reinterpret_cast<uint4 *>(cnt) + j;
@@ -851,22 +904,26 @@ __device__ void count_pass(const BuildArgs &a, const SkArgs &s, uint64_t n_items
                 *e = v;
             }
             __syncthreads();
-            const uint64_t cn = umin64(nrec - c0, kSkClamp);
+            const uint32_t cn = min(nrec - c0, kSkClamp);
+            const uint64_t rb = s_start[buf][i0];  // (a pass with more than CH records has one bucket)
             const uint64_t g1 = rb + c0 + cn * (wp + 1) / NW;
             for (uint64_t g = rb + c0 + cn * wp / NW; g < g1; g += 32)
                 sk_expand<kK>(g + lane < g1 ? s.rec2[g + lane] : none, 1, k, insert);
         }
-        load(next_rb, next_n);  // the next bucket's first records load while this one is compacted
-        have = true;
+        if (lane == 0) atomicAdd(&s_added, nu);
         __syncthreads();
-        if (s_over) {
+        const bool over = s_over != 0;
+        if (over && threadIdx.x == 0) overflow();
+        if (nrec >= 32) {  // a pass weighs a quarter; an eighth more for the spread
+            const uint32_t seen = (s_added * 288u) / nrec;
+            per_record = over ? min(2 * per_record, 32u << 8) : (per_record == 32 << 8 ? seen : (3 * per_record + seen) / 4);
+        }
+        advance();
+        load();  // the next pass's records load while this one is compacted
+        if (over) {
             for (uint32_t j = threadIdx.x; j < (uint32_t)T; j += NT) {
                 keys[j] = 0;
                 reinterpret_cast<uint4 *>(cnt)[j] = none;
-            }
-            if (threadIdx.x == 0) {
-                const unsigned i = atomicAdd(ovf_count, 1u);
-                if (i < s.big_cap) ovf[i] = bk;
             }
             continue;
         }
@@ -927,7 +984,7 @@ __device__ void count_pass(const BuildArgs &a, const SkArgs &s, uint64_t n_items
         }
     }
     if (lane == 0 && distinct) atomicAdd(&a.counters[0], distinct);
-    if (outgrown && threadIdx.x == 0) atomicOr(s.status, kStatusPartOverflow);
+    if (outgrown) atomicOr(s.status, kStatusPartOverflow);
     if (tb) {
         __syncthreads();
         for (uint32_t j = threadIdx.x; j < a.n_segs; j += NT) {
@@ -943,8 +1000,12 @@ __device__ void count_pass(const BuildArgs &a, const SkArgs &s, uint64_t n_items
 template <int T, int NT, int kK>
 __global__ void __launch_bounds__(NT, 1024 / NT) k_sk_count(BuildArgs a, SkArgs s, uint64_t n) {
     if ((*s.status & kStatusPartOverflow) || (T == 8192 && blockIdx.x >= *s.big_count)) return;
-    if (T == 8192) count_pass<T, NT, kK>(a, s, umin64(*s.big_count, s.big_cap), s.big, s.big2, s.big2_count);
-    else count_pass<T, NT, kK>(a, s, n, nullptr, s.big, s.big_count);
+    if (T == 8192) {
+        count_pass<T, NT, kK>(a, s, umin64(*s.big_count, s.big_cap), 1, s.big, s.big2, s.big2_count);
+    } else {  // sets of four buckets, fewer where the CTAs would not get a dozen sets each
+        const uint32_t set = n >= 48ull * gridDim.x ? 4 : (n >= 12ull * gridDim.x ? 2 : 1);
+        count_pass<T, NT, kK>(a, s, n, set, nullptr, s.big, s.big_count);
+    }
 }
 
 // Buckets no shared-memory table holds, in one global-memory table of record
