@@ -1225,7 +1225,7 @@ constexpr uint64_t kSuperWhole = 512;
 
 bool super_build(const swg_opts *o, const BuildArgs &a, uint64_t N) {
     // (the other scatter shapes are shapes of the single-occurrence scatters)
-    return swg::super_window(a.k) && N && !swg::level1_shape(o->scatter_shape);
+    return swg::super_window(a.k, N) && N && !swg::level1_shape(o->scatter_shape);
 }
 
 // Sizes the build for N occurrences of n_reads reads, allocates its
@@ -1244,7 +1244,7 @@ swg_status super_plan(swg_graph *g, const swg_opts *o, const BuildArgs &a, uint6
     // a random sequence has 2 / (w + 1) runs per k-mer and one more per read
     // (of those that have a k-mer)
     const uint64_t rec_cap =
-        (uint64_t)(1.25 * ((double)std::min(n_reads, N) + 2.0 * (double)N / (swg::super_window(a.k) + 1))) + 65536;
+        (uint64_t)(1.25 * ((double)std::min(n_reads, N) + 2.0 * (double)N / (swg::super_window(a.k, N) + 1))) + 65536;
     // (rec_cap / 1000: the partition regions are worked out in single precision)
     const uint64_t rec1 = rec_cap + rec_cap / 4 + rec_cap / 1000 + 1025 * P, rec2 = swg::super_bucket_room(rec_cap, NB, scale_max);
     if ((st = ensure(&g->d_part, &g->part_cap, 4 * P + 1, "partition table"))) return st;
@@ -1256,6 +1256,7 @@ swg_status super_plan(swg_graph *g, const swg_opts *o, const BuildArgs &a, uint6
     if ((st = ensure(&g->d_bk, &g->bk_cap, 4 * NB + 1 + scratch + 2 + P, "bucket table"))) return st;
     swg::SkArgs sk = reads;  // off, len, seg, n_pieces, pieces
     sk.k = a.k;
+    sk.w = swg::super_window(a.k, N);
     sk.b1 = b1;
     sk.b2 = b2;
     sk.n_parts = (uint32_t)P;

@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(kSkThreads, 4) k_sk_scan(BuildArgs a, SkArgs s
 #pragma unroll
                     for (int j = 0; j < W; ++j) {
                         if (j && j % 4 == 0 && pos && p + j >= nk) break;  // past the read's last k-mer
-                        // (bits below the m-mer only break ties, and M is odd: no m-mer is its own reverse)
+                        // (bits below the m-mer only break ties)
                         const uint32_t f = j < 16 ? __funnelshift_l(w0, w1, 2 * j) : w0;
                         const uint32_t v = W - 1 - j < 16 ? __funnelshift_l(r0, r1, 2 * (W - 1 - j)) : r0;
                         const uint32_t h = (min(f, v) & kTop) * 0x9e3779b1u + 0x7f4a7c15u;
@@ -1076,18 +1076,20 @@ int scan_launch(const BuildArgs &a, const SkArgs &s, uint64_t bound, uint32_t st
 
 }  // namespace
 
-// Window of m-mers per k-mer (0: no super-k-mer build for this k). m = k - w +
-// 1: as long as 15 bases (a 32-bit hash), so that a large genome still has
-// enough distinct minimizers, but w at least 7 so that runs stay long.
-int super_window(int k) {
+// Window w of m-mers per k-mer (0: no super-k-mer build for this k), m = k - w
+// + 1. Short m-mers make long runs, fewer records and more k-mers per block of
+// the scan (up to the record's 17): but 4^m / 2 minimizers have to be several
+// per bucket, or single ones make buckets uneven and too full. Builds at k =
+// 21: of 216M occurrences of a 5 Mbp genome 2.13 ms with m = 11, 2.24 with 12,
+// 2.37 with 13; of 693M of 40 Mbp 10.0 (329 buckets recounted), 7.8 and 8.2.
+int super_window(int k, uint64_t occurrences) {
+    const int m = occurrences <= (256ull << 20) ? 11 : (occurrences <= (2048ull << 20) ? 12 : 13);
     switch (k) {
         case 31: return 17;
-        case 29: return 15;
-        case 27: return 13;
-        case 25: return 13;
-        case 23: return 11;
-        case 21: return 9;
-        case 19: return 7;
+        case 29: return 17;
+        case 27: return 15;
+        case 25: return m == 13 ? 13 : 14;
+        case 23: case 21: case 19: return k - m + 1;
         default: return 0;
     }
 }
@@ -1095,15 +1097,24 @@ int super_window(int k) {
 int launch_super_scan(const BuildArgs &a, const SkArgs &s, uint64_t bound, uint32_t stride, bool sample, int grid_mode,
                       cudaStream_t st) {
     if (!bound) return 0;
-    switch (s.k) {
-        case 31: return scan_launch<15, 17>(a, s, bound, stride, sample, grid_mode, st);
-        case 29: return scan_launch<15, 15>(a, s, bound, stride, sample, grid_mode, st);
-        case 27: return scan_launch<15, 13>(a, s, bound, stride, sample, grid_mode, st);
-        case 25: return scan_launch<13, 13>(a, s, bound, stride, sample, grid_mode, st);
-        case 23: return scan_launch<13, 11>(a, s, bound, stride, sample, grid_mode, st);
-        case 21: return scan_launch<13, 9>(a, s, bound, stride, sample, grid_mode, st);
-        default: return scan_launch<13, 7>(a, s, bound, stride, sample, grid_mode, st);
-    }
+#define SWG_SCAN(M, W) \
+    if (s.k == M + W - 1 && s.w == W) return scan_launch<M, W>(a, s, bound, stride, sample, grid_mode, st)
+    SWG_SCAN(15, 17);
+    SWG_SCAN(13, 17);
+    SWG_SCAN(13, 15);
+    SWG_SCAN(12, 14);
+    SWG_SCAN(13, 13);
+    SWG_SCAN(11, 13);
+    SWG_SCAN(12, 12);
+    SWG_SCAN(13, 11);
+    SWG_SCAN(11, 11);
+    SWG_SCAN(12, 10);
+    SWG_SCAN(13, 9);
+    SWG_SCAN(11, 9);
+    SWG_SCAN(12, 8);
+    SWG_SCAN(13, 7);
+#undef SWG_SCAN
+    return 0;  // (super_window names no other)
 }
 
 // sum over the buckets, by the square root's concavity

@@ -140,7 +140,7 @@ struct BucketArgs {
 // with one minimizer, 16 bytes each, split into partitions and buckets by the
 // minimizer's hash.
 struct SkArgs {
-    int k;
+    int k, w;                              // w: m-mers per k-mer
     int b1, b2;                            // partition bits, sub-bucket bits
     uint32_t n_parts;                      // 1 << b1
     bool pieces;                           // off / len are pieces of long reads (flags in len)
@@ -168,7 +168,7 @@ struct SkArgs {
 };
 
 // Super-k-mer launchers (super.cu).
-int super_window(int k);  // m-mers per k-mer; 0: k has no super-k-mer build
+int super_window(int k, uint64_t occurrences);  // m-mers per k-mer; 0: k has no super-k-mer build
 // Most records that the bucket regions of k_sk_bucket_caps sum to.
 uint64_t super_bucket_room(uint64_t records, uint64_t nb, double scale_max);
 uint64_t super_pieces_bound(uint64_t n_reads, uint64_t occurrences);
