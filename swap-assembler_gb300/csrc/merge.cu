@@ -18,7 +18,7 @@
 // mergeable nodes is cut at its largest key, which is visited last and keeps
 // the whole cycle on its two arcs.
 //
-// Steps (one stream): open-addressing index key -> node (16-byte entries);
+// Steps (one stream): open-addressing index key -> node (4-byte entries);
 // per node the neighbour of each arc; for every mergeable node two
 // directed walk states; list ranking of the walks with a sparse ruling set
 // (one state in 16..256 — up to about 2^20 rulers — plus every walk head starts a ruler; a ruler
@@ -48,7 +48,7 @@ namespace {
 
 constexpr unsigned long long kTerm = 1ull << 63;  // walk successor: end arc code (node * 8 + slot)
 constexpr unsigned kNone = 0xffffffffu;
-constexpr unsigned long long kEmptyKey = ~0ull;
+constexpr unsigned kNodeMask = (1u << 29) - 1;
 constexpr int kClasses = 40;  // chain segment size classes 2^0 .. 2^39
 
 // error bits
@@ -101,7 +101,7 @@ struct MergeArgs {
     uint64_t rmask;  // ruler sampling: one state in rmask + 1
     const unsigned long long *keys;
     const unsigned long long *mult;  // byte s = multiplicity of slot s
-    ulonglong2 *ht;                  // index: x = key (kEmptyKey when free), y = node
+    unsigned *ht;                    // index: the key's hash's top 3 bits << 29 | node (kNone when free)
     uint64_t hmask;
     unsigned *nb;              // n*8: (neighbour << 1) | arrival side, kNone for an empty slot
     unsigned char *fl;         // bit0 mergeable, bits1-2 right slot, bits3-4 left slot - 4
@@ -122,7 +122,7 @@ struct MergeArgs {
     unsigned char *ent;        // chain unit-arc multiplicities, reduced in place
     unsigned *ent_chain;
     unsigned long long *cls_count, *cls_cursor;
-    unsigned long long *ctr;   // [0] rulers [1] cycle states [2] chains [3] cycles cut [4] merged nodes
+    unsigned long long *ctr;   // [0] rulers [1] cycle states [2] chains' first nodes [3] cycles cut [4] merged nodes
                                // [5] surviving nodes
     unsigned long long *skey;  // surviving nodes: keys, then (sorted) node indices
     unsigned *sidx;
@@ -132,12 +132,19 @@ struct MergeArgs {
     CartSlot *cart;            // per chain position (the ent layout)
 };
 
+// The index holds nodes, not keys: 4 bytes a slot keep it, and the keys, in L2
+// for ten times the nodes that 16-byte slots did (5M nodes: 67 MB where it was
+// 268, and 67 MB to clear). A key is read where the slot's 3 bits of its hash
+// agree, so probes past other keys seldom read one. (n < 2^29: an entry is
+// never kNone.)
 __device__ __forceinline__ unsigned lookup(const MergeArgs &a, uint64_t key) {
-    uint64_t h = fmix64(key) & a.hmask;
+    const uint64_t f = fmix64(key);
+    const unsigned tag = (unsigned)(f >> 61);
+    uint64_t h = f & a.hmask;
     for (uint64_t probe = 0; probe <= a.hmask; ++probe) {
-        const ulonglong2 e = a.ht[h];
-        if (e.x == key) return (unsigned)e.y;
-        if (e.x == kEmptyKey) return kNone;
+        const unsigned e = a.ht[h];
+        if (e == kNone) return kNone;
+        if (e >> 29 == tag && a.keys[e & kNodeMask] == key) return e & kNodeMask;
         h = (h + 1) & a.hmask;
     }
     return kNone;
@@ -152,13 +159,12 @@ __global__ void k_mg_index(MergeArgs a) {
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.n) return;
     const unsigned long long key = a.keys[i];
-    uint64_t h = fmix64(key) & a.hmask;
+    const uint64_t f = fmix64(key);
+    const unsigned tag = (unsigned)(f >> 61);
+    uint64_t h = f & a.hmask;
     for (uint64_t probe = 0; probe <= a.hmask; ++probe) {
-        const unsigned long long prev = atomicCAS(&a.ht[h].x, kEmptyKey, key);
-        if (prev == kEmptyKey || prev == key) {
-            a.ht[h].y = i;
-            return;
-        }
+        const unsigned prev = atomicCAS(&a.ht[h], kNone, tag << 29 | (unsigned)i);
+        if (prev == kNone || (prev >> 29 == tag && a.keys[prev & kNodeMask] == key)) return;
         h = (h + 1) & a.hmask;
     }
     atomicOr(a.err, kErrIndex);
@@ -166,37 +172,44 @@ __global__ void k_mg_index(MergeArgs a) {
 
 // Neighbour of every arc (node::getNodeID, graph.cpp:164-196: oriented k-mer
 // plus the arc base, last k bases, canonical id and the side reached) and
-// whether the node is merged away.
-__global__ void k_mg_classify(MergeArgs a) {
+// whether the node is merged away. A thread goes through its node's arcs, not
+// through the eight slots: the lanes of a warp have theirs in different slots,
+// and a warp then waits for two lookups where it waited for eight. One counter
+// update a block: one a warp, all of them to the same word, took longer than
+// the lookups. 5M nodes: 325 us with 16-byte index slots, eight
+// rounds and a counter update a warp, 141 now (4.2 TB/s of DRAM traffic).
+__global__ void __launch_bounds__(256) k_mg_classify(MergeArgs a) {
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.n) return;
-    const int k = a.k;
-    const uint64_t kmask = (1ull << (2 * k)) - 1;
-    const uint64_t key = a.keys[i], m = a.mult[i], rk = rc_dev(key, k);
-    int rc = 0, lc = 0, rs = 0, ls = 4;
-    bool self = false;
-#pragma unroll
-    for (int s = 0; s < 8; ++s) {
-        unsigned v = kNone;
-        if (mbyte(m, s)) {
+    bool merged = false;
+    if (i < a.n) {
+        const int k = a.k;
+        const uint64_t kmask = (1ull << (2 * k)) - 1;
+        const uint64_t key = a.keys[i], m = a.mult[i], rk = rc_dev(key, k);
+        const uint64_t full = (((m & 0x7f7f7f7f7f7f7f7full) + 0x7f7f7f7f7f7f7f7full) | m) & 0x8080808080808080ull;
+        uint4 *nb = reinterpret_cast<uint4 *>(a.nb + i * 8);
+        nb[0] = nb[1] = make_uint4(kNone, kNone, kNone, kNone);
+        bool ok = true;  // every neighbour is there and none is the node itself
+        for (uint64_t left = full; left; left &= left - 1) {
+            const int s = (__ffsll((long long)left) - 1) >> 3;
             const uint64_t e = (((s < 4 ? key : rk) << 2) | (uint64_t)(s & 3)) & kmask;
             const uint64_t r = rc_dev(e, k);
             const unsigned side = e >= r;
             const unsigned j = lookup(a, side ? e : r);
             if (j == kNone) {
                 atomicOr(a.err, kErrNeighbour);
+                ok = false;
             } else {
-                v = (j << 1) | side;
-                self |= (uint64_t)j == i;
+                a.nb[i * 8 + s] = (j << 1) | side;
+                ok &= (uint64_t)j != i;
             }
-            if (s < 4) ++rc, rs = s;
-            else ++lc, ls = s;
         }
-        a.nb[i * 8 + s] = v;
+        const unsigned right = (unsigned)full, l = (unsigned)(full >> 32);
+        merged = ok && __popc(right) == 1 && __popc(l) == 1;
+        const int rs = right ? (31 - __clz(right)) >> 3 : 0, ls = l ? (31 - __clz(l)) >> 3 : 0;
+        a.fl[i] = (unsigned char)((merged ? 1 : 0) | (rs << 1) | (ls << 3));
     }
-    const bool merged = rc == 1 && lc == 1 && !self;
-    a.fl[i] = (unsigned char)((merged ? 1 : 0) | (rs << 1) | ((ls - 4) << 3));
-    if (merged) agg_inc(&a.ctr[4]);
+    const int c = __syncthreads_count(merged);
+    if (threadIdx.x == 0 && c) atomicAdd(&a.ctr[4], (unsigned long long)c);
 }
 
 // Walk state 2i+d of a merged node: d = 0 traverses it as its key (leaves by
@@ -217,17 +230,29 @@ __device__ __forceinline__ unsigned long long walk_next(const MergeArgs &a, uint
 
 __device__ __forceinline__ bool ruler_of(const MergeArgs &a, uint64_t st, const ulonglong2 &pair);
 
-// Both walk states of a merged node, and which of them start rulers.
-__global__ void k_mg_states(MergeArgs a) {
+// Both walk states of a merged node, and which of them start rulers. The
+// block's rulers get their places with one counter update (one a warp took
+// most of the kernel's time: 5M nodes 251 us, 64 now).
+__global__ void __launch_bounds__(256) k_mg_states(MergeArgs a) {
+    __shared__ unsigned rulers;
+    __shared__ unsigned long long base;
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.n || !is_m(a, i)) return;
-    const ulonglong2 pair = make_ulonglong2(walk_next(a, i, 0), walk_next(a, i, 1));
-    *reinterpret_cast<ulonglong2 *>(a.succ + 2 * i) = pair;
-    for (int d = 0; d < 2; ++d) {
-        if (!ruler_of(a, 2 * i + d, pair)) continue;
-        const unsigned p = (unsigned)agg_inc(&a.ctr[0]);
-        a.rlist[p] = (unsigned)(2 * i + d);
+    if (threadIdx.x == 0) rulers = 0;
+    __syncthreads();
+    bool first = false, second = false;
+    if (i < a.n && is_m(a, i)) {
+        const ulonglong2 pair = make_ulonglong2(walk_next(a, i, 0), walk_next(a, i, 1));
+        *reinterpret_cast<ulonglong2 *>(a.succ + 2 * i) = pair;
+        *reinterpret_cast<ulonglong2 *>(a.oo + 2 * i) = make_ulonglong2(~0ull, ~0ull);
+        first = ruler_of(a, 2 * i, pair);
+        second = ruler_of(a, 2 * i + 1, pair);
     }
+    unsigned at = first || second ? atomicAdd(&rulers, (unsigned)first + second) : 0;
+    __syncthreads();
+    if (threadIdx.x == 0 && rulers) base = atomicAdd(&a.ctr[0], (unsigned long long)rulers);
+    __syncthreads();
+    if (first) a.rlist[base + at++] = (unsigned)(2 * i);
+    if (second) a.rlist[base + at] = (unsigned)(2 * i + 1);
 }
 
 // The successors of a node's two states sit side by side: one 16-byte load.
@@ -441,16 +466,17 @@ __global__ void k_mg_chain_count(MergeArgs a) {
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.n || !is_m(a, i)) return;
     const ChainPos c = chain_pos(a, i);
-    if (c.pos == 1) agg_add_labeled(a.cls_count, size_class(c.m), 1);
+    if (c.pos != 1) return;
+    agg_add_labeled(a.cls_count, size_class(c.m), 1);
+    a.clist[agg_inc(&a.ctr[2])] = (unsigned)i;  // (the cycles' list is done with)
 }
 
-__global__ void k_mg_chain_alloc(MergeArgs a) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.n || !is_m(a, i)) return;
-    const ChainPos c = chain_pos(a, i);
-    if (c.pos != 1) return;
+__global__ void k_mg_chain_alloc(MergeArgs a, uint64_t n_chains) {
+    const uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= n_chains) return;
+    const ChainPos c = chain_pos(a, a.clist[q]);
     const int cl = size_class(c.m);
-    const unsigned id = (unsigned)agg_inc(&a.ctr[2]);
+    const unsigned id = (unsigned)q;
     a.ch_eoff[id] = agg_add_labeled(a.cls_cursor, cl, 1ull << cl);
     a.ch_m[id] = c.m;
     a.chain_of[c.start] = id;
@@ -807,8 +833,7 @@ swg_status merge_graph(const unsigned long long *d_keys, const unsigned long lon
     a.mult = d_mult;
     EMIT_CUDA(cudaMemsetAsync(ctr, 0, (8 + 2 * kClasses) * sizeof(unsigned long long), s), "merge clear");
     EMIT_CUDA(cudaMemsetAsync(a.err, 0, sizeof(unsigned), s), "merge clear");
-    EMIT_CUDA(cudaMemsetAsync(a.ht, 0xff, hcap * sizeof(ulonglong2), s), "merge clear");
-    EMIT_CUDA(cudaMemsetAsync(a.oo, 0xff, 2 * n * sizeof(unsigned long long), s), "merge clear");
+    EMIT_CUDA(cudaMemsetAsync(a.ht, 0xff, hcap * sizeof(unsigned), s), "merge clear");
     int launches = 0;
     k_mg_index<<<blocks(n), 256, 0, s>>>(a);
     if (h_order) {  // visit times from the caller's order
@@ -913,7 +938,7 @@ swg_status merge_graph(const unsigned long long *d_keys, const unsigned long lon
         return cuda_err(cudaErrorMemoryAllocation, "chain workspace");
     EMIT_CUDA(cudaMemsetAsync(a.ent_chain, 0xff, std::max<uint64_t>(total, 1) * sizeof(unsigned), s), "chain clear");
     if (a.vt && !scr.get(&a.cart, total)) return cuda_err(cudaErrorMemoryAllocation, "merge tree");
-    k_mg_chain_alloc<<<blocks(n), 256, 0, s>>>(a);
+    k_mg_chain_alloc<<<blocks(n_chains), 256, 0, s>>>(a, n_chains);
     k_mg_entries<<<blocks(n), 256, 0, s>>>(a);
     launches += 2;
     if (a.vt) {
