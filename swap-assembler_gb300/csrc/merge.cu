@@ -47,6 +47,7 @@ namespace swg {
 namespace {
 
 constexpr unsigned long long kTerm = 1ull << 63;  // walk successor: end arc code (node * 8 + slot)
+constexpr unsigned kEnd = 1u << 31;               // 32-bit successor or ruler list entry: an end arc is reached
 constexpr unsigned kNone = 0xffffffffu;
 constexpr unsigned kNodeMask = (1u << 29) - 1;
 constexpr int kClasses = 40;  // chain segment size classes 2^0 .. 2^39
@@ -105,14 +106,13 @@ struct MergeArgs {
     uint64_t hmask;
     unsigned *nb;              // n*8: (neighbour << 1) | arrival side, kNone for an empty slot
     unsigned char *fl;         // bit0 mergeable, bits1-2 right slot, bits3-4 left slot - 4
-    unsigned long long *succ;  // 2n walk states: next state or kTerm | end arc
+    uint2 *succ;               // per node, its two walk states': next state, kEnd if an end arc is next
     unsigned long long *oo;    // per state: its ruler << 32 | distance from it (~0: none)
     unsigned *rpos;            // ruler list position of a ruler state
     unsigned *rlist;
-    ulonglong2 *rp0, *rp1;     // ruler list: next ruler / end arc, states to the end
+    uint2 *rp0, *rp1;          // ruler list: next ruler or end arc, states to it | kEnd at an end arc
     unsigned *moved;           // per pair of rounds of the ruler list's jumping: a ruler had not arrived
-    unsigned *len;             // per state: states from it to the end of its walk
-    unsigned long long *term;  // per state: kTerm | end arc reached
+    uint2 *lt;                 // per state: states from it to the end of its walk, end arc reached
     unsigned *clist;
     unsigned long long *cx0, *cx1, *cy0, *cy1;  // cycle pointer jumping
     unsigned *chain_of;        // per arc code: chain id (set at the chain's start arc)
@@ -222,13 +222,19 @@ __device__ __forceinline__ unsigned long long walk_next(const MergeArgs &a, uint
     const unsigned v = a.nb[i * 8 + (d ? lslot(f) : rslot(f))];
     const uint64_t j = v >> 1;
     const unsigned side = v & 1u;
-    if (is_m(a, j)) return 2 * j + (side ? 0 : 1);
+    if (is_m(a, j)) return v ^ 1u;  // state 2 * j + (side ? 0 : 1)
     const uint64_t o = d ? rc_dev(a.keys[i], a.k) : a.keys[i];
     const unsigned first = (unsigned)(o >> (2 * (a.k - 1))) & 3u;
     return kTerm | (j * 8 + (side ? 4 : 0) + 3 - first);
 }
 
-__device__ __forceinline__ bool ruler_of(const MergeArgs &a, uint64_t st, const ulonglong2 &pair);
+// The same, with kEnd for any end arc.
+__device__ __forceinline__ unsigned walk_state(const MergeArgs &a, unsigned char f, uint64_t i, int d) {
+    const unsigned v = a.nb[i * 8 + (d ? lslot(f) : rslot(f))];
+    return is_m(a, v >> 1) ? v ^ 1u : kEnd;  // state 2 * j + (side ? 0 : 1)
+}
+
+__device__ __forceinline__ bool ruler_of(const MergeArgs &a, unsigned st, uint2 pair);
 
 // Both walk states of a merged node, and which of them start rulers. The
 // block's rulers get their places with one counter update (one a warp took
@@ -241,8 +247,9 @@ __global__ void __launch_bounds__(256) k_mg_states(MergeArgs a) {
     __syncthreads();
     bool first = false, second = false;
     if (i < a.n && is_m(a, i)) {
-        const ulonglong2 pair = make_ulonglong2(walk_next(a, i, 0), walk_next(a, i, 1));
-        *reinterpret_cast<ulonglong2 *>(a.succ + 2 * i) = pair;
+        const unsigned char f = a.fl[i];
+        const uint2 pair = make_uint2(walk_state(a, f, i, 0), walk_state(a, f, i, 1));
+        a.succ[i] = pair;
         *reinterpret_cast<ulonglong2 *>(a.oo + 2 * i) = make_ulonglong2(~0ull, ~0ull);
         first = ruler_of(a, 2 * i, pair);
         second = ruler_of(a, 2 * i + 1, pair);
@@ -251,88 +258,106 @@ __global__ void __launch_bounds__(256) k_mg_states(MergeArgs a) {
     __syncthreads();
     if (threadIdx.x == 0 && rulers) base = atomicAdd(&a.ctr[0], (unsigned long long)rulers);
     __syncthreads();
-    if (first) a.rlist[base + at++] = (unsigned)(2 * i);
-    if (second) a.rlist[base + at] = (unsigned)(2 * i + 1);
-}
-
-// The successors of a node's two states sit side by side: one 16-byte load.
-__device__ __forceinline__ ulonglong2 succ_pair(const MergeArgs &a, uint64_t st) {
-    return *reinterpret_cast<const ulonglong2 *>(a.succ + (st & ~1ull));
+    if (first) {
+        a.rpos[2 * i] = (unsigned)base + at;
+        a.rlist[base + at++] = (unsigned)(2 * i);
+    }
+    if (second) {
+        a.rpos[2 * i + 1] = (unsigned)base + at;
+        a.rlist[base + at] = (unsigned)(2 * i + 1);
+    }
 }
 
 // A ruler: the first state of a walk (its twin leaves to an end) or, on
 // average, one state in rmask + 1 (16..256, chosen for at most about 2^20 rulers:
 // enough walkers to keep the SMs' warp slots busy while each walk's loads
 // wait on memory one after the other, and a ruler list small enough for L2).
-__device__ __forceinline__ bool ruler_of(const MergeArgs &a, uint64_t st, const ulonglong2 &pair) {
-    const unsigned long long twin = (st & 1) ? pair.x : pair.y;
-    return (twin & kTerm) || (fmix64(st) & a.rmask) == 0;
-}
-
-// The ruler list position of every ruler state (read when a walk meets it).
-__global__ void k_mg_rpos(MergeArgs a) {
-    const uint64_t n_rul = a.ctr[0];
-    for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n_rul;
-         p += (uint64_t)gridDim.x * blockDim.x)
-        a.rpos[a.rlist[p]] = (unsigned)p;
+__device__ __forceinline__ bool ruler_of(const MergeArgs &a, unsigned st, uint2 pair) {
+    return ((st & 1 ? pair.x : pair.y) & kEnd) || (fmix64(st) & a.rmask) == 0;
 }
 
 // Each ruler walks to the next ruler or the walk's end, labelling the states
-// on the way with (its list position, distance); per step one 16-byte load
-// and one 8-byte store. Grid-stride over the ruler count on the device.
-__global__ void k_mg_walk(MergeArgs a) {
-    const uint64_t n_rul = a.ctr[0];
-    for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n_rul;
-         p += (uint64_t)gridDim.x * blockDim.x) {
-        const unsigned r = a.rlist[p];
-        const unsigned long long tag = p << 32;
-        a.oo[r] = tag;
-        uint64_t cur = r;
-        ulonglong2 pr = succ_pair(a, r);
-        bool done = false;
-        for (unsigned o = 1; o <= 2 * a.n; ++o) {
-            const unsigned long long nx = (cur & 1) ? pr.y : pr.x;
-            if (nx & kTerm) {
-                a.rp0[p] = make_ulonglong2(nx, o);
-                done = true;
-                break;
-            }
-            const ulonglong2 pn = succ_pair(a, nx);
-            if (ruler_of(a, nx, pn)) {
-                a.rp0[p] = make_ulonglong2(a.rpos[nx], o);
-                done = true;
-                break;
-            }
-            a.oo[nx] = tag | o;
+// on the way with (its list position, distance); per step one 8-byte load
+// (a node's two successors: 40 MB for 5M nodes, half of L2's reach) and one
+// 8-byte store. Bound by those loads' latency, one after the other, so a lane
+// that has arrived takes its next ruler at once, its first load issued while
+// the walk before was under way, and does not wait for its warp's longest walk
+// (of 32 walks of 16 states on average, the longest has 65). The next ruler
+// is noted as a state; the ruler list's kernel looks its position up.
+// 5M nodes: 237 us with a warp waiting for its 32 walks and 16-byte pairs, 182 now.
+__global__ void __launch_bounds__(256) k_mg_walk(MergeArgs a) {
+    const uint64_t n_rul = a.ctr[0], stride = (uint64_t)gridDim.x * blockDim.x;
+    uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= n_rul) return;
+    unsigned cur = a.rlist[p], ahead = p + stride < n_rul ? a.rlist[p + stride] : 0;
+    uint2 pr = a.succ[cur >> 1], pr_ahead = a.succ[ahead >> 1];
+    unsigned later = p + 2 * stride < n_rul ? a.rlist[p + 2 * stride] : 0;
+    a.oo[cur] = p << 32;
+    for (unsigned o = 1; o <= 2 * a.n;) {
+        const unsigned nx = cur & 1 ? pr.y : pr.x;
+        const bool end = nx & kEnd;
+        uint2 pn = make_uint2(0, 0);
+        if (!end) pn = a.succ[nx >> 1];
+        if (!end && !ruler_of(a, nx, pn)) {
+            a.oo[nx] = p << 32 | o;
             cur = nx;
             pr = pn;
+            ++o;
+            continue;
         }
-        if (!done) atomicOr(a.err, kErrWalk);
+        a.rp0[p] = end ? make_uint2((unsigned)walk_next(a, cur >> 1, cur & 1), o | kEnd) : make_uint2(nx, o);
+        p += stride;
+        if (p >= n_rul) return;
+        cur = ahead;
+        pr = pr_ahead;
+        a.oo[cur] = p << 32;
+        o = 1;
+        ahead = later;
+        pr_ahead = a.succ[ahead >> 1];
+        later = p + 2 * stride < n_rul ? a.rlist[p + 2 * stride] : 0;
     }
+    for (; p < n_rul; p += stride) a.rp0[p] = make_uint2(0, kEnd);  // (the host stops at the error)
+    atomicOr(a.err, kErrWalk);
 }
 
 // Pointer jumping over the ruler list, all rounds in one cooperative launch:
-// a round is bound by its launch and its random loads' latency (one 16-byte
-// load a ruler), and a grid barrier costs less than a launch. Rounds go in
+// a round is bound by its random loads' latency (so a thread has four rulers'
+// under way) and a grid barrier, which costs less than a launch. Rounds go in
 // pairs, so that the result is in rp0 again, and end once every ruler has
 // reached an end (as many rounds as the longest chain's rulers need, where the
-// bound for any chain was 22 to 25); the rulers of a cycle never do.
-__global__ void __launch_bounds__(256) k_mg_rjump(MergeArgs a, int pairs) {
+// bound for any chain was 22 to 25); the rulers of a cycle never do. 5M nodes,
+// 700,000 rulers: 140 us with four blocks of 256 an SM and a ruler at a time,
+// 108 with one of 1024 an SM and four (eight of 256 an SM: 138, the barrier).
+constexpr int kJump = 4;
+__global__ void __launch_bounds__(1024) k_mg_rjump(MergeArgs a, int pairs) {
     const uint64_t n_rul = a.ctr[0], stride = (uint64_t)gridDim.x * blockDim.x;
     const uint64_t p0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (uint64_t p = p0; p < n_rul; p += stride) {  // states to list positions
+        const uint2 v = a.rp0[p];
+        if (!(v.y & kEnd)) a.rp0[p].x = a.rpos[v.x];
+    }
+    cg::this_grid().sync();
     for (int r = 0; r < pairs; ++r) {
         bool moved = false;
         for (int half = 0; half < 2; ++half) {
-            const ulonglong2 *in = half ? a.rp1 : a.rp0;
-            ulonglong2 *out = half ? a.rp0 : a.rp1;
-            for (uint64_t p = p0; p < n_rul; p += stride) {
-                ulonglong2 v = __ldcg(in + p);
-                if (!(v.x & kTerm)) {
-                    const ulonglong2 w = __ldcg(in + v.x);
-                    v = make_ulonglong2(w.x, v.y + w.y);
-                    moved |= !(v.x & kTerm);
+            const uint2 *in = half ? a.rp1 : a.rp0;
+            uint2 *out = half ? a.rp0 : a.rp1;
+            for (uint64_t p = p0; p < n_rul; p += kJump * stride) {
+                uint2 v[kJump], w[kJump];
+#pragma unroll
+                for (int j = 0; j < kJump; ++j)
+                    v[j] = p + j * stride < n_rul ? __ldcg(in + p + j * stride) : make_uint2(0, kEnd);
+#pragma unroll
+                for (int j = 0; j < kJump; ++j)
+                    if (!(v[j].y & kEnd)) w[j] = __ldcg(in + v[j].x);
+#pragma unroll
+                for (int j = 0; j < kJump; ++j) {
+                    if (!(v[j].y & kEnd)) {  // (a cycle's sums mean nothing, and stay below kEnd)
+                        v[j] = make_uint2(w[j].x, ((v[j].y + (w[j].y & ~kEnd)) & ~kEnd) | (w[j].y & kEnd));
+                        moved |= !(v[j].y & kEnd);
+                    }
+                    if (p + j * stride < n_rul) out[p + j * stride] = v[j];
                 }
-                out[p] = v;
             }
             if (half && moved) a.moved[r] = 1;
             cg::this_grid().sync();
@@ -343,21 +368,20 @@ __global__ void __launch_bounds__(256) k_mg_rjump(MergeArgs a, int pairs) {
 }
 
 __global__ void k_mg_finish(MergeArgs a) {
-    const uint64_t st = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (st >= 2 * a.n || !is_m(a, st >> 1)) return;
-    const unsigned long long oo = a.oo[st];
-    if (oo != ~0ull) {
-        const unsigned p = (unsigned)(oo >> 32);
-        const ulonglong2 v = a.rp0[p];
-        if (v.x & kTerm) {
-            a.len[st] = (unsigned)(v.y - (oo & 0xffffffffull));
-            a.term[st] = v.x;
-            return;
-        }
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= a.n || !is_m(a, i)) return;
+    const ulonglong2 oo = *reinterpret_cast<const ulonglong2 *>(a.oo + 2 * i);
+    uint2 lt[2];
+#pragma unroll
+    for (int d = 0; d < 2; ++d) {
+        const unsigned long long o = d ? oo.y : oo.x;
+        uint2 v = make_uint2(0, 0);
+        if (o != ~0ull) v = a.rp0[o >> 32];
+        const bool ends = v.y & kEnd;
+        lt[d] = ends ? make_uint2((v.y & ~kEnd) - (unsigned)o, v.x) : make_uint2(0, 0);
+        if (!ends) a.clist[agg_inc(&a.ctr[1])] = (unsigned)(2 * i + d);
     }
-    a.len[st] = 0;
-    a.term[st] = 0;
-    a.clist[agg_inc(&a.ctr[1])] = (unsigned)st;
+    *reinterpret_cast<uint4 *>(a.lt + 2 * i) = make_uint4(lt[0].x, lt[0].y, lt[1].x, lt[1].y);
 }
 
 // ---- cycles of merged nodes: largest key by pointer jumping, cut there
@@ -372,7 +396,7 @@ __global__ void k_mg_cyc_init(MergeArgs a, uint64_t c) {
     if (t >= c) return;
     const unsigned st = a.clist[t];
     a.cx0[st] = cut_rank(a, st >> 1);
-    a.cy0[st] = a.succ[st];
+    a.cy0[st] = st & 1 ? a.succ[st >> 1].y : a.succ[st >> 1].x;  // (no end arc in a cycle)
 }
 
 __global__ void k_mg_cyc_max(MergeArgs a, uint64_t c, const unsigned long long *__restrict__ mx_in,
@@ -429,8 +453,7 @@ __global__ void k_mg_cyc_done(MergeArgs a, uint64_t c, const unsigned long long 
     const unsigned st = a.clist[t];
     if (!is_m(a, st >> 1)) return;
     if (!(nx[st] & kTerm)) atomicOr(a.err, kErrCycle);
-    a.len[st] = (unsigned)ln[st];
-    a.term[st] = nx[st];
+    a.lt[st] = make_uint2((unsigned)ln[st], (unsigned)nx[st]);
 }
 
 // ---- chains
@@ -449,8 +472,9 @@ struct ChainPos {
 
 __device__ __forceinline__ ChainPos chain_pos(const MergeArgs &a, uint64_t i) {
     ChainPos c;
-    const unsigned la = a.len[2 * i], lb = a.len[2 * i + 1];
-    const uint64_t beta = a.term[2 * i] & ~kTerm, alpha = a.term[2 * i + 1] & ~kTerm;
+    const uint4 lt = *reinterpret_cast<const uint4 *>(a.lt + 2 * i);
+    const unsigned la = lt.x, lb = lt.z;
+    const uint64_t beta = lt.y, alpha = lt.w;
     c.m = la + lb - 1;
     c.fwd = arc_less(a, alpha, beta);
     c.pos = c.fwd ? lb : la;
@@ -635,7 +659,7 @@ __global__ void k_mg_line_len(MergeArgs a, const unsigned *__restrict__ order, u
         const uint64_t j = order[q];
         if (mbyte(a.mult[j], s)) {
             const unsigned v = a.nb[j * 8 + s];
-            l = 1 + (is_m(a, v >> 1) ? a.len[first_state(v)] : 0);
+            l = 1 + (is_m(a, v >> 1) ? a.lt[first_state(v)].x : 0);
         }
     }
 #pragma unroll
@@ -667,12 +691,12 @@ __global__ void __launch_bounds__(256) k_mg_line_write(MergeArgs a, const unsign
         l = 1;
         if (is_m(a, v >> 1)) {
             const uint64_t st = first_state(v);
-            const uint64_t mine = j * 8 + s, other = a.term[st] & ~kTerm;
+            const uint64_t mine = j * 8 + s, other = a.lt[st].y;
             chain = true;
             first = arc_less(a, mine, other);  // this end starts the chain
             id = a.chain_of[first ? mine : other];
             mm = a.ent[a.ch_eoff[id]];
-            l += a.len[st];
+            l += a.lt[st].x;
             back = pos_of[other >> 3] * 8u + (unsigned)(other & 7);
         } else {  // one base to the next node left: its arc back, as walk_next finds it
             const uint64_t o = s < 4 ? key : rc_dev(key, a.k);
@@ -821,9 +845,9 @@ swg_status merge_graph(const unsigned long long *d_keys, const unsigned long lon
     uint64_t hcap = 1024;
     while (hcap < 2 * n) hcap *= 2;
     a.hmask = hcap - 1;
-    if (!scr.get(&a.ht, hcap) || !scr.get(&a.nb, 8 * n) || !scr.get(&a.fl, n) || !scr.get(&a.succ, 2 * n) ||
+    if (!scr.get(&a.ht, hcap) || !scr.get(&a.nb, 8 * n) || !scr.get(&a.fl, n) || !scr.get(&a.succ, n) ||
         !scr.get(&a.oo, 2 * n) || !scr.get(&a.rpos, 2 * n) || !scr.get(&a.rlist, 2 * n) ||
-        !scr.get(&a.len, 2 * n) || !scr.get(&a.term, 2 * n) || !scr.get(&a.clist, 2 * n) ||
+        !scr.get(&a.lt, 2 * n) || !scr.get(&a.clist, 2 * n) ||
         !scr.get(&a.chain_of, 8 * n) || !scr.get(&ctr, 8 + 2 * kClasses) || !scr.get(&a.err, 1))
         return cuda_err(cudaErrorMemoryAllocation, "merge workspace");
     a.ctr = ctr;
@@ -865,21 +889,20 @@ swg_status merge_graph(const unsigned long long *d_keys, const unsigned long lon
     if (!scr.get(&a.rp0, 2 * n) || !scr.get(&a.rp1, 2 * n) || !scr.get(&a.moved, 64))
         return cuda_err(cudaErrorMemoryAllocation, "ruler list");
     EMIT_CUDA(cudaMemsetAsync(a.moved, 0, 64 * sizeof(unsigned), s), "merge clear");
-    int sms = 0, per_sm = 0, dev = 0;
+    int sms = 0, dev = 0;
     EMIT_CUDA(cudaGetDevice(&dev), "device");
     EMIT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "device attribute");
-    EMIT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mg_rjump, 256, 0), "occupancy");
     const unsigned wgrid = (unsigned)std::max(1, sms * 8);
-    k_mg_rpos<<<wgrid, 256, 0, s>>>(a);
     k_mg_walk<<<wgrid, 256, 0, s>>>(a);
     {
         int pairs = (ceil_log2(std::max<uint64_t>(2 * n, 1)) + 2) / 2;
         void *args[] = {&a, &pairs};
-        const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)std::max(1, std::min(per_sm, 4) * sms), blocks(2 * n));
-        EMIT_CUDA(cudaLaunchCooperativeKernel((const void *)k_mg_rjump, dim3(grid), dim3(256), args, 0, s), "ruler list");
+        const uint64_t rulers = 2 * n / (a.rmask + 1);  // (about; and the walks' first states)
+        const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)std::max(1, sms), rulers / 1024 + 1);
+        EMIT_CUDA(cudaLaunchCooperativeKernel((const void *)k_mg_rjump, dim3(grid), dim3(1024), args, 0, s), "ruler list");
     }
-    k_mg_finish<<<blocks(2 * n), 256, 0, s>>>(a);
-    launches += 4;
+    k_mg_finish<<<blocks(n), 256, 0, s>>>(a);
+    launches += 3;
     unsigned long long h[6];
     unsigned herr = 0;
     EMIT_CUDA(cudaMemcpyAsync(h, ctr, sizeof(h), cudaMemcpyDeviceToHost, s), "cycle count");
