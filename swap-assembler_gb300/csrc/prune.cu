@@ -158,15 +158,33 @@ __global__ void __launch_bounds__(256) k_pr_write(MergedGraph m, const uint64_t 
     }
 }
 
-// The arc strings move from the old text to the new one, a piece's first 4 KiB
-// by a warp of its own and the rest of a long one in 4 KiB chunks, a block
-// each, so that a few very long arcs (whole chains) spread over the GPU too:
-// chunk counts per piece, their prefix, then each block finds its piece by
-// binary search in the prefix. (Most arcs are short; a block and a search for
-// each of them took three times as long.) A piece is an arc's own string
-// (its first `own` bytes, the whole arc unless a merge lengthened it) or,
-// after a merge, a merged node's arc string placed inside an end's new arc.
-constexpr unsigned kChunk = 4096;
+// The arc strings move from the old text to the new one, a piece's first KiB
+// by eight lanes and the rest of a long one in chunks of a KiB, a warp each,
+// so that a few very long arcs (whole chains) spread over the GPU too: chunk
+// counts per piece, their prefix, then each warp finds its piece by binary
+// search in the prefix. (Most arcs are short; a search for each of them took
+// three times as long.) Bound by the loads' latency, so every lane has sixteen
+// bytes under way. A piece is an arc's own string (its first `own` bytes, the
+// whole arc unless a merge lengthened it) or, after a merge, a merged node's
+// arc string placed inside an end's new arc. 50,000 pieces, 1 MB: first parts
+// of 4 KiB by a warp, a byte a lane at a time, took 29 to 62 us and the rest by
+// blocks 2 to 15 (four rewrites of a pipeline: 208); now 17 to 30 and 13 (146).
+constexpr unsigned kPart = 1024;   // bytes of a piece moved at a time
+constexpr unsigned kChunk = 4096;  // of a contig
+constexpr int kBytes = 16;         // a lane's under way
+
+// `l` bytes by `lanes` neighbouring lanes, of which this one is `lane`.
+__device__ __forceinline__ void move_bytes(char *b, const char *a, unsigned l, unsigned lane, unsigned lanes) {
+    for (unsigned c = lane; c < l; c += kBytes * lanes) {
+        char v[kBytes];
+#pragma unroll
+        for (int j = 0; j < kBytes; ++j)
+            if (c + j * lanes < l) v[j] = a[c + j * lanes];
+#pragma unroll
+        for (int j = 0; j < kBytes; ++j)
+            if (c + j * lanes < l) b[c + j * lanes] = v[j];
+    }
+}
 
 struct Pieces {
     const unsigned *own;                    // per arc slot: bytes of its old string (nullptr: len)
@@ -202,10 +220,10 @@ __device__ __forceinline__ unsigned piece(const MergedGraph &m, const Pieces &x,
     return l;
 }
 
-__device__ __forceinline__ unsigned more_chunks(unsigned len) { return len ? (len - 1) / kChunk : 0; }
+__device__ __forceinline__ unsigned more_parts(unsigned len) { return len ? (len - 1) / kPart : 0; }
 
-// A warp's lanes look at 32 pieces; the warp copies the nonempty ones' first
-// chunks one after the other. chunks: those left of each piece.
+// A warp's lanes look at 32 pieces; its four groups of eight lanes move the
+// nonempty ones' first parts. chunks: the parts left of each piece.
 __global__ void __launch_bounds__(256) k_pr_short(MergedGraph m, Pieces x, const char *__restrict__ from,
                                                   char *__restrict__ to, uint64_t *__restrict__ chunks) {
     const uint64_t pieces = 8 * m.lines + x.n;
@@ -215,23 +233,30 @@ __global__ void __launch_bounds__(256) k_pr_short(MergedGraph m, Pieces x, const
     unsigned len = 0;
     if (i < pieces) {
         len = piece(m, x, i, src, dst);
-        chunks[i] = more_chunks(len);
-        len = len < kChunk ? len : kChunk;
+        chunks[i] = more_parts(len);
+        len = len < kPart ? len : kPart;
     }
-    for (unsigned todo = __ballot_sync(0xffffffffu, len != 0); todo; todo &= todo - 1) {
-        const int o = __ffs(todo) - 1;
-        const char *a = from + __shfl_sync(0xffffffffu, src, o);
-        char *b = to + __shfl_sync(0xffffffffu, dst, o);
-        const unsigned l = __shfl_sync(0xffffffffu, len, o);
-        for (unsigned c = lane; c < l; c += 32) b[c] = a[c];
+    for (unsigned todo = __ballot_sync(0xffffffffu, len != 0); todo;) {
+        int o = -1;
+#pragma unroll
+        for (unsigned g = 0; g < 4; ++g) {  // the next four pieces, one a group
+            if (g == lane >> 3) o = __ffs(todo) - 1;
+            todo &= todo - 1;
+        }
+        const char *a = from + __shfl_sync(0xffffffffu, src, o & 31);
+        char *b = to + __shfl_sync(0xffffffffu, dst, o & 31);
+        const unsigned l = __shfl_sync(0xffffffffu, len, o & 31);
+        if (o >= 0) move_bytes(b, a, l, lane & 7, 8);
+        __syncwarp();
     }
 }
 
-// The long pieces' other chunks; their number is read on the device.
+// The long pieces' other parts; their number is read on the device.
 __global__ void __launch_bounds__(256) k_pr_long(MergedGraph m, Pieces x, const uint64_t *__restrict__ first,
                                                  const char *__restrict__ from, char *__restrict__ to) {
     const uint64_t pieces = 8 * m.lines + x.n, n_chunks = first[pieces];
-    for (uint64_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
+    const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
+    for (uint64_t c = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < n_chunks; c += warps) {
         uint64_t lo = 0, hi = pieces;  // the last piece whose first chunk is <= c
         while (hi - lo > 1) {
             const uint64_t mid = (lo + hi) / 2;
@@ -240,12 +265,9 @@ __global__ void __launch_bounds__(256) k_pr_long(MergedGraph m, Pieces x, const 
         }
         uint64_t src = 0, dst = 0;
         const unsigned len = piece(m, x, lo, src, dst);
-        const uint64_t at = (c - first[lo] + 1) * kChunk;
+        const uint64_t at = (c - first[lo] + 1) * kPart;
         const uint64_t rest = len - at;
-        const unsigned l = rest < kChunk ? (unsigned)rest : kChunk;
-        const char *a = from + src + at;
-        char *b = to + dst + at;
-        for (unsigned i = threadIdx.x; i < l; i += blockDim.x) b[i] = a[i];
+        move_bytes(to + dst + at, from + src + at, rest < kPart ? (unsigned)rest : kPart, threadIdx.x & 31, 32);
     }
 }
 
@@ -282,10 +304,10 @@ swg_status rewrite(MergedGraph *m, cudaStream_t s, Scratch &scr, const Pieces &x
         k_pr_short<<<blocks(pieces), 256, 0, s>>>(*m, x, m->text, m->text2, chunks);
         st = scan_lengths(chunks, first, pieces, scr, s);
         if (st) return st;
-        // at most a chunk per 4 KiB of the new text
-        const uint64_t most = h[0] / kChunk;
+        // at most a part per KiB of the new text, eight a block
+        const uint64_t most = h[0] / kPart;
         if (most)
-            k_pr_long<<<(unsigned)std::min<uint64_t>(most, 4096), 256, 0, s>>>(*m, x, first, m->text, m->text2);
+            k_pr_long<<<(unsigned)std::min<uint64_t>((most + 7) / 8, 4096), 256, 0, s>>>(*m, x, first, m->text, m->text2);
     }
     EMIT_CUDA(cudaMemsetAsync(m->text2 + h[0], '\n', 1, s), "merged text");
     EMIT_CUDA(cudaGetLastError(), "rewrite kernels");
