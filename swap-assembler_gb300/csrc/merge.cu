@@ -126,7 +126,7 @@ struct MergeArgs {
                                // [5] surviving nodes
     unsigned long long *skey;  // surviving nodes: keys, then (sorted) node indices
     unsigned *sidx;
-    unsigned *err;
+    unsigned *err;             // (the word after the counters [0] to [6])
     // merge in a given visiting order (null: the fixed tree order)
     unsigned long long *vt;    // per node: its visit time
     CartSlot *cart;            // per chain position (the ent layout)
@@ -492,13 +492,13 @@ __global__ void k_mg_chain_count(MergeArgs a) {
     const ChainPos c = chain_pos(a, i);
     if (c.pos != 1) return;
     agg_add_labeled(a.cls_count, size_class(c.m), 1);
-    a.clist[agg_inc(&a.ctr[2])] = (unsigned)i;  // (the cycles' list is done with)
+    a.rlist[agg_inc(&a.ctr[2])] = (unsigned)i;  // (the rulers' list is done with)
 }
 
 __global__ void k_mg_chain_alloc(MergeArgs a, uint64_t n_chains) {
     const uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= n_chains) return;
-    const ChainPos c = chain_pos(a, a.clist[q]);
+    const ChainPos c = chain_pos(a, a.rlist[q]);
     const int cl = size_class(c.m);
     const unsigned id = (unsigned)q;
     a.ch_eoff[id] = agg_add_labeled(a.cls_cursor, cl, 1ull << cl);
@@ -848,15 +848,15 @@ swg_status merge_graph(const unsigned long long *d_keys, const unsigned long lon
     if (!scr.get(&a.ht, hcap) || !scr.get(&a.nb, 8 * n) || !scr.get(&a.fl, n) || !scr.get(&a.succ, n) ||
         !scr.get(&a.oo, 2 * n) || !scr.get(&a.rpos, 2 * n) || !scr.get(&a.rlist, 2 * n) ||
         !scr.get(&a.lt, 2 * n) || !scr.get(&a.clist, 2 * n) ||
-        !scr.get(&a.chain_of, 8 * n) || !scr.get(&ctr, 8 + 2 * kClasses) || !scr.get(&a.err, 1))
+        !scr.get(&a.chain_of, 8 * n) || !scr.get(&ctr, 8 + 2 * kClasses))
         return cuda_err(cudaErrorMemoryAllocation, "merge workspace");
     a.ctr = ctr;
+    a.err = reinterpret_cast<unsigned *>(ctr + 7);
     a.cls_count = ctr + 8;
     a.cls_cursor = ctr + 8 + kClasses;
     a.keys = d_keys;
     a.mult = d_mult;
     EMIT_CUDA(cudaMemsetAsync(ctr, 0, (8 + 2 * kClasses) * sizeof(unsigned long long), s), "merge clear");
-    EMIT_CUDA(cudaMemsetAsync(a.err, 0, sizeof(unsigned), s), "merge clear");
     EMIT_CUDA(cudaMemsetAsync(a.ht, 0xff, hcap * sizeof(unsigned), s), "merge clear");
     int launches = 0;
     k_mg_index<<<blocks(n), 256, 0, s>>>(a);
@@ -902,12 +902,12 @@ swg_status merge_graph(const unsigned long long *d_keys, const unsigned long lon
         EMIT_CUDA(cudaLaunchCooperativeKernel((const void *)k_mg_rjump, dim3(grid), dim3(1024), args, 0, s), "ruler list");
     }
     k_mg_finish<<<blocks(n), 256, 0, s>>>(a);
-    launches += 3;
-    unsigned long long h[6];
-    unsigned herr = 0;
-    EMIT_CUDA(cudaMemcpyAsync(h, ctr, sizeof(h), cudaMemcpyDeviceToHost, s), "cycle count");
-    EMIT_CUDA(cudaMemcpyAsync(&herr, a.err, sizeof(unsigned), cudaMemcpyDeviceToHost, s), "merge status");
-    EMIT_CUDA(cudaStreamSynchronize(s), "cycle count");
+    k_mg_chain_count<<<blocks(n), 256, 0, s>>>(a);  // (a cycle's states, at 0, are no chain's: counted again below)
+    launches += 4;
+    unsigned long long h[8 + kClasses];
+    EMIT_CUDA(cudaMemcpyAsync(h, ctr, sizeof(h), cudaMemcpyDeviceToHost, s), "merge counts");
+    EMIT_CUDA(cudaStreamSynchronize(s), "merge counts");
+    unsigned herr = (unsigned)h[7];
     if (herr & (kErrIndex | kErrNeighbour)) {
         set_error("merge: node index or neighbour lookup failed (arc without its neighbour k-molecule)");
         return SWG_ERR_BAD_INPUT;
@@ -932,19 +932,18 @@ swg_status merge_graph(const unsigned long long *d_keys, const unsigned long lon
         for (int r = 0; r < rounds; ++r)
             k_mg_cyc_rank<<<blocks(c), 256, 0, s>>>(a, c, bx[r & 1], by[r & 1], bx[(r + 1) & 1], by[(r + 1) & 1]);
         k_mg_cyc_done<<<blocks(c), 256, 0, s>>>(a, c, bx[rounds & 1], by[rounds & 1]);
-        launches += 4 + 2 * rounds;
+        EMIT_CUDA(cudaMemsetAsync(a.cls_count, 0, kClasses * sizeof(unsigned long long), s), "cycle chains");
+        EMIT_CUDA(cudaMemsetAsync(&a.ctr[2], 0, sizeof(unsigned long long), s), "cycle chains");
+        k_mg_chain_count<<<blocks(n), 256, 0, s>>>(a);
+        launches += 5 + 2 * rounds;
+        EMIT_CUDA(cudaMemcpyAsync(h, ctr, sizeof(h), cudaMemcpyDeviceToHost, s), "cycle chains");
+        EMIT_CUDA(cudaStreamSynchronize(s), "cycle chains");
+        if (h[7]) {
+            set_error("merge: a walk did not end (internal error)");
+            return SWG_ERR_TIMEOUT;
+        }
     }
-    k_mg_chain_count<<<blocks(n), 256, 0, s>>>(a);
-    ++launches;
-    unsigned long long cls[kClasses];
-    EMIT_CUDA(cudaMemcpyAsync(cls, a.cls_count, sizeof(cls), cudaMemcpyDeviceToHost, s), "chain classes");
-    EMIT_CUDA(cudaMemcpyAsync(h, ctr, sizeof(h), cudaMemcpyDeviceToHost, s), "cycle cuts");
-    EMIT_CUDA(cudaMemcpyAsync(&herr, a.err, sizeof(unsigned), cudaMemcpyDeviceToHost, s), "merge status");
-    EMIT_CUDA(cudaStreamSynchronize(s), "chain classes");
-    if (herr) {
-        set_error("merge: a walk did not end (internal error)");
-        return SWG_ERR_TIMEOUT;
-    }
+    const unsigned long long *cls = h + 8;
     // segments of 2^c entries, largest class first: every offset is aligned
     unsigned long long cursor[kClasses];
     uint64_t total = 0, n_chains = 0;

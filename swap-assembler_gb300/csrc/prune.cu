@@ -277,15 +277,15 @@ inline unsigned blocks(uint64_t n) { return (unsigned)std::max<uint64_t>((n + 25
 swg_status rewrite(MergedGraph *m, cudaStream_t s, Scratch &scr, const Pieces &x = Pieces{}) {
     uint64_t *len = nullptr, *off = nullptr;
     unsigned long long *printed = nullptr;
-    if (!scr.get(&len, m->lines) || !scr.get(&off, m->lines + 1) || !scr.get(&printed, 1))
+    if (!scr.get(&len, m->lines) || !scr.get(&off, m->lines + 2))
         return cuda_err(cudaErrorMemoryAllocation, "rewrite workspace");
+    printed = reinterpret_cast<unsigned long long *>(off + m->lines + 1);  // (read together with the text's size)
     EMIT_CUDA(cudaMemsetAsync(printed, 0, 8, s), "rewrite");
     if (m->lines) k_pr_len<<<blocks(m->lines), 256, 0, s>>>(*m, len, printed);
     swg_status st = scan_lengths(len, off, m->lines, scr, s);
     if (st) return st;
     uint64_t h[2] = {0, 0};
-    EMIT_CUDA(cudaMemcpyAsync(&h[0], off + m->lines, 8, cudaMemcpyDeviceToHost, s), "text size");
-    EMIT_CUDA(cudaMemcpyAsync(&h[1], printed, 8, cudaMemcpyDeviceToHost, s), "text size");
+    EMIT_CUDA(cudaMemcpyAsync(h, off + m->lines, 16, cudaMemcpyDeviceToHost, s), "text size");
     EMIT_CUDA(cudaStreamSynchronize(s), "text size");
     const uint64_t bytes = h[0] + 1;
     if (bytes > m->text2_cap) {
@@ -704,7 +704,7 @@ swg_status simplify_lines(MergedGraph *m, cudaStream_t s, uint64_t *count) {
     EMIT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "device attribute");
     EMIT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sm_jump, 256, 0), "occupancy");
     const unsigned jgrid = (unsigned)std::min<uint64_t>((uint64_t)std::max(1, std::min(per_sm, 4) * sms), blocks(2 * L));
-    unsigned long long h[4] = {0, 0, 0, 0};
+    unsigned long long h[8 + kCls] = {0};
     const int in = 0;  // the jumps leave their result in the first buffers
     k_sm_classify<<<blocks(L), 256, 0, s>>>(a);
     for (int attempt = 0; attempt < 2; ++attempt) {  // again after cutting cycles
@@ -714,15 +714,18 @@ swg_status simplify_lines(MergedGraph *m, cudaStream_t s, uint64_t *count) {
         EMIT_CUDA(cudaLaunchCooperativeKernel((const void *)k_sm_jump, dim3(jgrid), dim3(256), args, 0, s), "simplify");
         if (attempt == 1) break;
         k_sm_cut<<<blocks(L), 256, 0, s>>>(a, in);
+        k_sm_chain_count<<<blocks(L), 256, 0, s>>>(a, in);  // (of no use if there are cycles: counted again below)
         EMIT_CUDA(cudaMemcpyAsync(h, a.ctr, sizeof(h), cudaMemcpyDeviceToHost, s), "simplify");
         EMIT_CUDA(cudaStreamSynchronize(s), "simplify");
         if (!h[3]) break;
     }
-    k_sm_chain_count<<<blocks(L), 256, 0, s>>>(a, in);
-    unsigned long long cls[kCls];
-    EMIT_CUDA(cudaMemcpyAsync(cls, a.cls_count, sizeof(cls), cudaMemcpyDeviceToHost, s), "simplify");
-    EMIT_CUDA(cudaMemcpyAsync(h, a.ctr, sizeof(h), cudaMemcpyDeviceToHost, s), "simplify");
-    EMIT_CUDA(cudaStreamSynchronize(s), "simplify");
+    if (h[3]) {
+        EMIT_CUDA(cudaMemsetAsync(a.cls_count, 0, kCls * 8, s), "simplify");
+        k_sm_chain_count<<<blocks(L), 256, 0, s>>>(a, in);
+        EMIT_CUDA(cudaMemcpyAsync(h, a.ctr, sizeof(h), cudaMemcpyDeviceToHost, s), "simplify");
+        EMIT_CUDA(cudaStreamSynchronize(s), "simplify");
+    }
+    const unsigned long long *cls = h + 8;
     unsigned long long cursor[kCls];
     uint64_t total = 0, n_chains = 0;
     int top = 0;

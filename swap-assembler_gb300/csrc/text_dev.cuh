@@ -57,25 +57,44 @@ __device__ __forceinline__ uint64_t neighbour_dev(uint64_t key, int slot, int k)
 }
 
 // Stream-ordered device scratch, freed on every return path.
-// With a pool, from that pool (one that keeps its memory for reuse).
+// With a pool, from that pool (one that keeps its memory for reuse). Small
+// requests share slabs: a pass over a merged graph's lines makes some thirty
+// of them, and an allocation and its release cost the host 2 us.
 struct Scratch {
+    static constexpr size_t kSlab = 4u << 20;
     cudaStream_t s;
     cudaMemPool_t pool;
     void *p[48] = {};
     int n = 0;
+    char *slab = nullptr;
+    size_t left = 0;  // of the slab
     explicit Scratch(cudaStream_t st, cudaMemPool_t mp = nullptr) : s(st), pool(mp) {}
+    void *take(size_t bytes) {
+        void *q = nullptr;
+        if (n == 48) return nullptr;
+        const cudaError_t e = pool ? cudaMallocFromPoolAsync(&q, bytes, pool, s) : cudaMallocAsync(&q, bytes, s);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        return p[n++] = q;
+    }
     template <typename T>
     bool get(T **out, uint64_t count) {
         *out = nullptr;
-        if (n == 48) return false;
-        const size_t bytes = std::max<uint64_t>(count, 1) * sizeof(T);
-        const cudaError_t e = pool ? cudaMallocFromPoolAsync((void **)out, bytes, pool, s)
-                                   : cudaMallocAsync((void **)out, bytes, s);
-        if (e != cudaSuccess) {
-            cudaGetLastError();
-            return false;
+        const size_t bytes = (std::max<uint64_t>(count, 1) * sizeof(T) + 255) & ~(size_t)255;
+        if (bytes > kSlab / 4) {
+            *out = static_cast<T *>(take(bytes));
+            return *out != nullptr;
         }
-        p[n++] = *out;
+        if (left < bytes) {
+            slab = static_cast<char *>(take(kSlab));
+            left = slab ? kSlab : 0;
+            if (!slab) return false;
+        }
+        *out = reinterpret_cast<T *>(slab);
+        slab += bytes;
+        left -= bytes;
         return true;
     }
     ~Scratch() {
