@@ -107,13 +107,15 @@ __global__ void __launch_bounds__(kFBlock) k_nl_pos(const unsigned long long *__
     }
 }
 
-// Exclusive scan of at most a few kGChunk items by one block (in place
-// allowed): one launch where the three-kernel scan would take three.
-__global__ void __launch_bounds__(kFBlock) k_gscan_small(const uint64_t *in, uint64_t n, uint64_t *out,
+// Exclusive scan of at most 8 * kGChunk items by one block (in place allowed):
+// one launch where the three-kernel scan would take three. 6,300 items:
+// 10 us with 256 threads, 7 with 1024; three launches 11 and the gaps between.
+constexpr int kSmallScan = 1024;
+__global__ void __launch_bounds__(kSmallScan) k_gscan_small(const uint64_t *in, uint64_t n, uint64_t *out,
                                                          uint64_t *total) {
-    __shared__ uint64_t wb[kFBlock / 32];
+    __shared__ uint64_t wb[kSmallScan / 32];
     uint64_t carry = 0;
-    for (uint64_t b0 = 0; b0 < n; b0 += kGChunk) {
+    for (uint64_t b0 = 0; b0 < n; b0 += kSmallScan * kGItems) {
         const uint64_t base = b0 + (uint64_t)threadIdx.x * kGItems;
         uint64_t v[kGItems];
         uint64_t s = 0;
@@ -123,7 +125,7 @@ __global__ void __launch_bounds__(kFBlock) k_gscan_small(const uint64_t *in, uin
             s += v[it];
         }
         uint64_t t;
-        uint64_t run = carry + block_exclusive_scan<kFBlock>(s, wb, &t);
+        uint64_t run = carry + block_exclusive_scan<kSmallScan>(s, wb, &t);
 #pragma unroll
         for (int it = 0; it < kGItems; ++it) {
             if (base + it < n) out[base + it] = run;
@@ -480,8 +482,8 @@ int launch_gscan(const uint64_t *in, uint64_t *out, uint64_t n, uint64_t *scratc
         cudaMemsetAsync(total, 0, sizeof(uint64_t), s);
         return 0;
     }
-    if (nb <= 2) {
-        k_gscan_small<<<1, kFBlock, 0, s>>>(in, n, out, total);
+    if (nb <= 8) {  // two rounds of the block; beyond, it would take longer than three launches
+        k_gscan_small<<<1, kSmallScan, 0, s>>>(in, n, out, total);
         return 1;
     }
     k_gscan_reduce<<<(unsigned)nb, kFBlock, 0, s>>>(in, n, scratch);

@@ -125,7 +125,7 @@ struct MergeArgs {
     unsigned long long *ctr;   // [0] rulers [1] cycle states [2] chains' first nodes [3] cycles cut [4] merged nodes
                                // [5] surviving nodes
     unsigned long long *skey;  // surviving nodes: keys, then (sorted) node indices
-    unsigned *sidx;
+    unsigned long long *sidx;
     unsigned *err;             // (the word after the counters [0] to [6])
     // merge in a given visiting order (null: the fixed tree order)
     unsigned long long *vt;    // per node: its visit time
@@ -645,13 +645,14 @@ __global__ void k_mg_survivors(MergeArgs a) {
     if (j >= a.n || is_m(a, j)) return;
     const unsigned long long q = agg_inc(&a.ctr[5]);
     a.skey[q] = a.keys[j];
-    a.sidx[q] = (unsigned)j;
+    a.sidx[q] = j;
 }
 
 // (eight lanes a line, one per arc slot: a line's arcs are chains of dependent
-// loads, and few lines are left of a graph)
-__global__ void k_mg_line_len(MergeArgs a, const unsigned *__restrict__ order, uint64_t n_lines,
-                              uint64_t *__restrict__ out) {
+// loads, and few lines are left of a graph; unordered: nothing to read yet)
+__global__ void k_mg_line_len(MergeArgs a, const unsigned long long *__restrict__ order, uint64_t n_lines,
+                              uint64_t *__restrict__ out, const unsigned *__restrict__ unordered) {
+    if (unordered && *unordered) return;
     const uint64_t q = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
     const int s = threadIdx.x & 7;
     unsigned long long l = 0;
@@ -668,14 +669,14 @@ __global__ void k_mg_line_len(MergeArgs a, const unsigned *__restrict__ order, u
 }
 
 // Line position of every node left.
-__global__ void k_mg_pos(const unsigned *__restrict__ order, uint64_t n_lines, unsigned *__restrict__ pos_of) {
+__global__ void k_mg_pos(const unsigned long long *__restrict__ order, uint64_t n_lines, unsigned *__restrict__ pos_of) {
     const uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (q < n_lines) pos_of[order[q]] = (unsigned)q;
 }
 
 // Eight lanes a line: lane s writes arc s's place, its multiplicity and an
 // eighth of the blanks.
-__global__ void __launch_bounds__(256) k_mg_line_write(MergeArgs a, const unsigned *__restrict__ order, uint64_t n_lines,
+__global__ void __launch_bounds__(256) k_mg_line_write(MergeArgs a, const unsigned long long *__restrict__ order, uint64_t n_lines,
                                 const uint64_t *__restrict__ off, char *__restrict__ text,
                                 const unsigned *__restrict__ pos_of, MergedGraph mg) {
     const uint64_t q = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
@@ -975,32 +976,47 @@ swg_status merge_graph(const unsigned long long *d_keys, const unsigned long lon
     }
     // the nodes left, in key order
     const uint64_t n_lines = n - h[4] + h[3];
-    unsigned long long *skey2 = nullptr;
-    unsigned *sidx2 = nullptr;
+    unsigned long long *skey2 = nullptr, *sidx2 = nullptr;
     uint64_t *lens = nullptr, *loff = nullptr;
-    if (!scr.get(&a.skey, n_lines) || !scr.get(&a.sidx, n_lines) || !scr.get(&skey2, n_lines) ||
-        !scr.get(&sidx2, n_lines) || !scr.get(&lens, n_lines) || !scr.get(&loff, n_lines + 1))
+    if (!scr.get(&a.skey, n_lines) || !scr.get(&a.sidx, n_lines) || !scr.get(&lens, n_lines) || !scr.get(&loff, n_lines + 1))
         return cuda_err(cudaErrorMemoryAllocation, "line workspace");
     k_mg_survivors<<<blocks(n), 256, 0, s>>>(a);
     ++launches;
-    if (n_lines) {
-        size_t tb = 0;
-        EMIT_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, a.skey, skey2, a.sidx, sidx2, (int64_t)n_lines, 0,
-                                                  2 * k, s),
-                  "sort size");
-        unsigned char *tmp = nullptr;
-        if (!scr.get(&tmp, tb)) return cuda_err(cudaErrorMemoryAllocation, "sort scratch");
-        EMIT_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tb, a.skey, skey2, a.sidx, sidx2, (int64_t)n_lines, 0,
-                                                  2 * k, s),
-                  "sort");
-        k_mg_line_len<<<blocks(8 * n_lines), 256, 0, s>>>(a, sidx2, n_lines, lens);
-        ++launches;
-    }
-    swg_status st = scan_lengths(lens, loff, n_lines, scr, s);
-    if (st) return st;
     uint64_t bytes = 0;
-    EMIT_CUDA(cudaMemcpyAsync(&bytes, loff + n_lines, 8, cudaMemcpyDeviceToHost, s), "text size");
-    EMIT_CUDA(cudaStreamSynchronize(s), "text size");
+    // by splitters (three launches, 37 us for 6,000 lines; the library's passes
+    // took eight and 61), or by the library's passes if there are more lines
+    // than those take or one of their buckets runs full
+    for (bool library = n_lines > sort_device_most();; library = true) {
+        unsigned *over = nullptr;
+        unsigned unordered = 0;
+        if (n_lines && !library) {
+            unsigned char *ws = nullptr;
+            if (!scr.get(&ws, sort_scratch_bytes(n_lines))) return cuda_err(cudaErrorMemoryAllocation, "sort scratch");
+            sort_records_device(a.skey, a.sidx, n_lines, s, ws, &skey2, &sidx2, &over);
+        } else if (n_lines) {
+            if (!scr.get(&skey2, n_lines) || !scr.get(&sidx2, n_lines))
+                return cuda_err(cudaErrorMemoryAllocation, "line workspace");
+            size_t tb = 0;
+            EMIT_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, a.skey, skey2, a.sidx, sidx2, (int64_t)n_lines, 0,
+                                                      2 * k, s),
+                      "sort size");
+            unsigned char *tmp = nullptr;
+            if (!scr.get(&tmp, tb)) return cuda_err(cudaErrorMemoryAllocation, "sort scratch");
+            EMIT_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tb, a.skey, skey2, a.sidx, sidx2, (int64_t)n_lines, 0,
+                                                      2 * k, s),
+                      "sort");
+        }
+        if (over) EMIT_CUDA(cudaMemcpyAsync(&unordered, over, sizeof(unsigned), cudaMemcpyDeviceToHost, s), "sort status");
+        if (n_lines) {
+            k_mg_line_len<<<blocks(8 * n_lines), 256, 0, s>>>(a, sidx2, n_lines, lens, over);
+            ++launches;
+        }
+        swg_status st = scan_lengths(lens, loff, n_lines, scr, s);
+        if (st) return st;
+        EMIT_CUDA(cudaMemcpyAsync(&bytes, loff + n_lines, 8, cudaMemcpyDeviceToHost, s), "text size");
+        EMIT_CUDA(cudaStreamSynchronize(s), "text size");
+        if (!unordered) break;
+    }
     swg_status gst = merged_reserve(mg, bytes + 1, n_lines);
     if (gst) return gst;
     mg->k = k;

@@ -159,16 +159,14 @@ __global__ void __launch_bounds__(256) k_pr_write(MergedGraph m, const uint64_t 
 }
 
 // The arc strings move from the old text to the new one, a piece's first KiB
-// by eight lanes and the rest of a long one in chunks of a KiB, a warp each,
-// so that a few very long arcs (whole chains) spread over the GPU too: chunk
-// counts per piece, their prefix, then each warp finds its piece by binary
-// search in the prefix. (Most arcs are short; a search for each of them took
-// three times as long.) Bound by the loads' latency, so every lane has sixteen
-// bytes under way. A piece is an arc's own string (its first `own` bytes, the
-// whole arc unless a merge lengthened it) or, after a merge, a merged node's
-// arc string placed inside an end's new arc. 50,000 pieces, 1 MB: first parts
-// of 4 KiB by a warp, a byte a lane at a time, took 29 to 62 us and the rest by
-// blocks 2 to 15 (four rewrites of a pipeline: 208); now 17 to 30 and 13 (146).
+// by eight lanes; the rest of a long one is listed in parts of a KiB, a warp
+// each, so that a few very long arcs (whole chains) spread over the GPU too.
+// Bound by the loads' latency, so every lane has sixteen bytes under way. A
+// piece is an arc's own string (its first `own` bytes, the whole arc unless a
+// merge lengthened it) or, after a merge, a merged node's arc string placed
+// inside an end's new arc. 50,000 pieces, 1 MB: first parts of 4 KiB by a warp,
+// a byte a lane at a time, took 29 to 62 us, parts' counts scanned and searched
+// 13 to 27; now 17 to 26 and 8.
 constexpr unsigned kPart = 1024;   // bytes of a piece moved at a time
 constexpr unsigned kChunk = 4096;  // of a contig
 constexpr int kBytes = 16;         // a lane's under way
@@ -220,21 +218,30 @@ __device__ __forceinline__ unsigned piece(const MergedGraph &m, const Pieces &x,
     return l;
 }
 
-__device__ __forceinline__ unsigned more_parts(unsigned len) { return len ? (len - 1) / kPart : 0; }
-
 // A warp's lanes look at 32 pieces; its four groups of eight lanes move the
-// nonempty ones' first parts. chunks: the parts left of each piece.
+// nonempty ones' first parts, and the warp lists the other parts of the long
+// ones (piece << 24 | part; a part's number is below 2^22), counted in *listed.
 __global__ void __launch_bounds__(256) k_pr_short(MergedGraph m, Pieces x, const char *__restrict__ from,
-                                                  char *__restrict__ to, uint64_t *__restrict__ chunks) {
+                                                  char *__restrict__ to, unsigned long long *__restrict__ parts,
+                                                  unsigned long long *__restrict__ listed) {
     const uint64_t pieces = 8 * m.lines + x.n;
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const unsigned lane = threadIdx.x & 31;
     uint64_t src = 0, dst = 0;
-    unsigned len = 0;
+    unsigned len = 0, more = 0;
     if (i < pieces) {
         len = piece(m, x, i, src, dst);
-        chunks[i] = more_parts(len);
+        more = len ? (len - 1) / kPart : 0;
         len = len < kPart ? len : kPart;
+    }
+    for (unsigned todo = __ballot_sync(0xffffffffu, more != 0); todo; todo &= todo - 1) {
+        const int o = __ffs(todo) - 1;
+        const unsigned count = __shfl_sync(0xffffffffu, more, o);
+        unsigned long long at = 0;
+        if (lane == 0) at = atomicAdd(listed, (unsigned long long)count);
+        at = __shfl_sync(0xffffffffu, at, 0);
+        const unsigned long long id = (i - lane + o) << 24;
+        for (unsigned c = lane; c < count; c += 32) parts[at + c] = id | (c + 1);
     }
     for (unsigned todo = __ballot_sync(0xffffffffu, len != 0); todo;) {
         int o = -1;
@@ -251,21 +258,15 @@ __global__ void __launch_bounds__(256) k_pr_short(MergedGraph m, Pieces x, const
     }
 }
 
-// The long pieces' other parts; their number is read on the device.
-__global__ void __launch_bounds__(256) k_pr_long(MergedGraph m, Pieces x, const uint64_t *__restrict__ first,
+// The listed parts, a warp each; their number is read on the device.
+__global__ void __launch_bounds__(256) k_pr_long(MergedGraph m, Pieces x, const unsigned long long *__restrict__ parts,
+                                                 const unsigned long long *__restrict__ listed,
                                                  const char *__restrict__ from, char *__restrict__ to) {
-    const uint64_t pieces = 8 * m.lines + x.n, n_chunks = first[pieces];
-    const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
-    for (uint64_t c = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < n_chunks; c += warps) {
-        uint64_t lo = 0, hi = pieces;  // the last piece whose first chunk is <= c
-        while (hi - lo > 1) {
-            const uint64_t mid = (lo + hi) / 2;
-            if (first[mid] <= c) lo = mid;
-            else hi = mid;
-        }
+    const uint64_t n = *listed, warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
+    for (uint64_t c = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < n; c += warps) {
         uint64_t src = 0, dst = 0;
-        const unsigned len = piece(m, x, lo, src, dst);
-        const uint64_t at = (c - first[lo] + 1) * kPart;
+        const unsigned len = piece(m, x, parts[c] >> 24, src, dst);
+        const uint64_t at = (parts[c] & 0xffffffu) * kPart;
         const uint64_t rest = len - at;
         move_bytes(to + dst + at, from + src + at, rest < kPart ? (unsigned)rest : kPart, threadIdx.x & 31, 32);
     }
@@ -277,10 +278,11 @@ inline unsigned blocks(uint64_t n) { return (unsigned)std::max<uint64_t>((n + 25
 swg_status rewrite(MergedGraph *m, cudaStream_t s, Scratch &scr, const Pieces &x = Pieces{}) {
     uint64_t *len = nullptr, *off = nullptr;
     unsigned long long *printed = nullptr;
-    if (!scr.get(&len, m->lines) || !scr.get(&off, m->lines + 2))
+    if (!scr.get(&len, m->lines) || !scr.get(&off, m->lines + 3))
         return cuda_err(cudaErrorMemoryAllocation, "rewrite workspace");
-    printed = reinterpret_cast<unsigned long long *>(off + m->lines + 1);  // (read together with the text's size)
-    EMIT_CUDA(cudaMemsetAsync(printed, 0, 8, s), "rewrite");
+    // (the count of printed lines is read together with the text's size; the listed parts' comes after it)
+    printed = reinterpret_cast<unsigned long long *>(off + m->lines + 1);
+    EMIT_CUDA(cudaMemsetAsync(printed, 0, 16, s), "rewrite");
     if (m->lines) k_pr_len<<<blocks(m->lines), 256, 0, s>>>(*m, len, printed);
     swg_status st = scan_lengths(len, off, m->lines, scr, s);
     if (st) return st;
@@ -297,17 +299,14 @@ swg_status rewrite(MergedGraph *m, cudaStream_t s, Scratch &scr, const Pieces &x
     }
     if (m->lines) {
         const uint64_t pieces = 8 * m->lines + x.n;
-        uint64_t *chunks = nullptr, *first = nullptr;
-        if (!scr.get(&chunks, pieces) || !scr.get(&first, pieces + 1))
-            return cuda_err(cudaErrorMemoryAllocation, "rewrite workspace");
+        const uint64_t most = h[0] / kPart;  // a part per KiB of the new text
+        unsigned long long *parts = nullptr;
+        if (!scr.get(&parts, most)) return cuda_err(cudaErrorMemoryAllocation, "rewrite workspace");
         k_pr_write<<<blocks(8 * m->lines), 256, 0, s>>>(*m, off, m->text2);
-        k_pr_short<<<blocks(pieces), 256, 0, s>>>(*m, x, m->text, m->text2, chunks);
-        st = scan_lengths(chunks, first, pieces, scr, s);
-        if (st) return st;
-        // at most a part per KiB of the new text, eight a block
-        const uint64_t most = h[0] / kPart;
+        k_pr_short<<<blocks(pieces), 256, 0, s>>>(*m, x, m->text, m->text2, parts, printed + 1);
         if (most)
-            k_pr_long<<<(unsigned)std::min<uint64_t>((most + 7) / 8, 4096), 256, 0, s>>>(*m, x, first, m->text, m->text2);
+            k_pr_long<<<(unsigned)std::min<uint64_t>((most + 7) / 8, 4096), 256, 0, s>>>(*m, x, parts, printed + 1,
+                                                                                        m->text, m->text2);
     }
     EMIT_CUDA(cudaMemsetAsync(m->text2 + h[0], '\n', 1, s), "merged text");
     EMIT_CUDA(cudaGetLastError(), "rewrite kernels");

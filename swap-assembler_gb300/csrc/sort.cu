@@ -336,6 +336,29 @@ uint64_t sort_scratch_bytes(uint64_t n) {
     return std::max(split, 32 * n + 8 * (nc + gscan_scratch(nc) + 1));
 }
 
+uint64_t sort_device_most() { return kSplitMost; }
+
+void sort_records_device(const unsigned long long *d_keys, const unsigned long long *d_mult, uint64_t n, cudaStream_t s,
+                         void *ws, unsigned long long **keys, unsigned long long **mult, unsigned **over) {
+    unsigned long long *k = static_cast<unsigned long long *>(ws), *m = k + n;
+    *keys = k;
+    *mult = m;
+    *over = nullptr;
+    if (n <= kOne) {
+        k_sort_one<<<1, 1024, 0, s>>>(d_keys, d_mult, (uint32_t)n, k, m);
+        return;
+    }
+    const uint32_t nb = (uint32_t)((n + kMean - 1) / kMean);
+    unsigned long long *bk = m + n, *bm = bk + (uint64_t)nb * kRoom, *sp = bm + (uint64_t)nb * kRoom;
+    unsigned *cursor = reinterpret_cast<unsigned *>(sp + nb);
+    *over = cursor + nb;
+    allow_smem(k_sort_split, kSampleMost * sizeof(unsigned long long));
+    k_sort_split<<<1, 1024, kSampleMost * sizeof(unsigned long long), s>>>(d_keys, n, nb, sp, cursor, *over);
+    k_sort_scatter<<<(unsigned)((n + 256 * kSplitItems - 1) / (256 * kSplitItems)), 256, 0, s>>>(d_keys, d_mult, n, nb, sp,
+                                                                                                cursor, *over, bk, bm);
+    k_sort_buckets<<<nb, 1024, 0, s>>>(cursor, *over, bk, bm, k, m);
+}
+
 // ws: sort_scratch_bytes(n) of device scratch, 8-byte aligned. The inputs are
 // not touched. radix: the radix passes whatever the size.
 swg_status copy_records_sorted(const unsigned long long *d_keys, const unsigned long long *d_mult, uint64_t n, int bits,
@@ -346,19 +369,12 @@ swg_status copy_records_sorted(const unsigned long long *d_keys, const unsigned 
     k[0] = static_cast<unsigned long long *>(ws);
     m[0] = k[0] + n;
     int at = 0;
-    if (n <= kOne) {
-        k_sort_one<<<1, 1024, 0, s>>>(d_keys, d_mult, (uint32_t)n, k[0], m[0]);
-    } else if (n <= kSplitMost && !radix) {
-        const uint32_t nb = (uint32_t)((n + kMean - 1) / kMean);
-        unsigned long long *bk = m[0] + n, *bm = bk + (uint64_t)nb * kRoom, *sp = bm + (uint64_t)nb * kRoom;
-        unsigned *cursor = reinterpret_cast<unsigned *>(sp + nb), *over = cursor + nb;
-        allow_smem(k_sort_split, kSampleMost * sizeof(unsigned long long));
-        k_sort_split<<<1, 1024, kSampleMost * sizeof(unsigned long long), s>>>(d_keys, n, nb, sp, cursor, over);
-        k_sort_scatter<<<(unsigned)((n + 256 * kSplitItems - 1) / (256 * kSplitItems)), 256, 0, s>>>(
-            d_keys, d_mult, n, nb, sp, cursor, over, bk, bm);
-        k_sort_buckets<<<nb, 1024, 0, s>>>(cursor, over, bk, bm, k[0], m[0]);
+    if (n <= kOne || (n <= kSplitMost && !radix)) {
+        unsigned *over = nullptr;
+        sort_records_device(d_keys, d_mult, n, s, ws, &k[0], &m[0], &over);
         EMIT_CUDA(cudaGetLastError(), "sort kernels");
-        EMIT_CUDA(cudaMemcpyAsync(&too_large, over, sizeof(unsigned), cudaMemcpyDeviceToHost, s), "sort status");
+        if (over)
+            EMIT_CUDA(cudaMemcpyAsync(&too_large, over, sizeof(unsigned), cudaMemcpyDeviceToHost, s), "sort status");
     } else {
         k[1] = m[0] + n;
         m[1] = k[1] + n;

@@ -311,6 +311,12 @@ void sort_records(uint64_t *keys, uint64_t *mult8, uint64_t n);
 // n device records copied to the host in key order (sort.cu; keys below
 // 2^bits), through ws: sort_scratch_bytes(n) of device scratch.
 uint64_t sort_scratch_bytes(uint64_t n);
+// The same left on the device: the launches for n <= sort_device_most() records
+// (*keys, *mult: where they lie in ws). *over, if not null: read after the
+// stream has come this far, nonzero if they are not ordered (a bucket ran full).
+uint64_t sort_device_most();
+void sort_records_device(const unsigned long long *d_keys, const unsigned long long *d_mult, uint64_t n, cudaStream_t s,
+                         void *ws, unsigned long long **keys, unsigned long long **mult, unsigned **over);
 swg_status copy_records_sorted(const unsigned long long *d_keys, const unsigned long long *d_mult, uint64_t n, int bits,
                                cudaStream_t s, void *ws, uint64_t *keys, uint8_t *mult, bool radix = false);
 uint64_t revcomp_host(uint64_t x, int k);
