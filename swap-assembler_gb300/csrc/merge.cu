@@ -20,10 +20,10 @@
 //
 // Steps (one stream): open-addressing index key -> node (4-byte entries);
 // per node the neighbour of each arc; for every mergeable node two
-// directed walk states; list ranking of the walks with a sparse ruling set
-// (one state in 16..256 — up to about 2^20 rulers — plus every walk head starts a ruler; a ruler
-// walks to the next one, then the rulers' own list is ranked by pointer
-// jumping); cycles (states no ruler reaches, or rulers whose list never
+// directed walk states; list ranking of the walks in three steps (within
+// tiles of neighbouring nodes, in shared memory; over the states where walks
+// enter tiles, each eighth walking to the next; over those by pointer
+// jumping); cycles (states that are not reached so, or whose list never
 // ends) are found, cut and ranked by pointer jumping; chains are laid out in
 // power-of-two aligned segments so the tree reduction runs level by level in
 // place; finally the surviving nodes are ordered by key, each formats its
@@ -47,7 +47,8 @@ namespace swg {
 namespace {
 
 constexpr unsigned long long kTerm = 1ull << 63;  // walk successor: end arc code (node * 8 + slot)
-constexpr unsigned kEnd = 1u << 31;               // 32-bit successor or ruler list entry: an end arc is reached
+constexpr unsigned kEnd = 1u << 31;               // 32-bit successor or list entry: an end arc is reached
+constexpr unsigned kHead = 1u << 30;              // ruler list entry: the walk's first
 constexpr unsigned kNone = 0xffffffffu;
 constexpr unsigned kNodeMask = (1u << 29) - 1;
 constexpr int kClasses = 40;  // chain segment size classes 2^0 .. 2^39
@@ -99,19 +100,19 @@ __device__ __forceinline__ unsigned long long agg_add_labeled(unsigned long long
 struct MergeArgs {
     int k;
     uint64_t n;
-    uint64_t rmask;  // ruler sampling: one state in rmask + 1
     const unsigned long long *keys;
     const unsigned long long *mult;  // byte s = multiplicity of slot s
     unsigned *ht;                    // index: the key's hash's top 3 bits << 29 | node (kNone when free)
     uint64_t hmask;
     unsigned *nb;              // n*8: (neighbour << 1) | arrival side, kNone for an empty slot
     unsigned char *fl;         // bit0 mergeable, bits1-2 right slot, bits3-4 left slot - 4
-    uint2 *succ;               // per node, its two walk states': next state, kEnd if an end arc is next
     unsigned long long *oo;    // per state: its ruler << 32 | distance from it (~0: none)
     unsigned *rpos;            // ruler list position of a ruler state
-    unsigned *rlist;
-    uint2 *rp0, *rp1;          // ruler list: next ruler or end arc, states to it | kEnd at an end arc
-    unsigned *moved;           // per pair of rounds of the ruler list's jumping: a ruler had not arrived
+    uint2 *rp0;                // ruler list: next ruler or end arc, states to it | kEnd at an end arc, kHead
+    uint2 *ro;                 // per ruler: its pole, distance from it (kNone: none)
+    uint2 *pp0, *pp1;          // pole list: next pole or end arc, states to it | kEnd at an end arc
+    unsigned *heads;           // poles that are walks' first rulers (then: chains' first nodes)
+    unsigned *moved;           // per pair of rounds of the pole list's jumping: a pole had not arrived
     uint2 *lt;                 // per state: states from it to the end of its walk, end arc reached
     unsigned *clist;
     unsigned long long *cx0, *cx1, *cy0, *cy1;  // cycle pointer jumping
@@ -123,7 +124,7 @@ struct MergeArgs {
     unsigned *ent_chain;
     unsigned long long *cls_count, *cls_cursor;
     unsigned long long *ctr;   // [0] rulers [1] cycle states [2] chains' first nodes [3] cycles cut [4] merged nodes
-                               // [5] surviving nodes
+                               // [5] surviving nodes [6] poles listed
     unsigned long long *skey;  // surviving nodes: keys, then (sorted) node indices
     unsigned long long *sidx;
     unsigned *err;             // (the word after the counters [0] to [6])
@@ -234,136 +235,168 @@ __device__ __forceinline__ unsigned walk_state(const MergeArgs &a, unsigned char
     return is_m(a, v >> 1) ? v ^ 1u : kEnd;  // state 2 * j + (side ? 0 : 1)
 }
 
-__device__ __forceinline__ bool ruler_of(const MergeArgs &a, unsigned st, uint2 pair);
-
-// Both walk states of a merged node, and which of them start rulers. The
-// block's rulers get their places with one counter update (one a warp took
-// most of the kernel's time: 5M nodes 251 us, 64 now).
-__global__ void __launch_bounds__(256) k_mg_states(MergeArgs a) {
+// Both walk states of a merged node, ranked within the block's 512 nodes. The
+// build leaves the k-molecules of a bucket side by side, and a walk stays in a
+// bucket for six to nine nodes, so most of it is a matter of shared memory
+// here, with coalesced reads and writes around it, where walking node by node
+// through memory took as long as all else together. A state whose predecessor
+// (its twin's successor's twin) lies in another tile, or which has none, is a
+// ruler; the others are ranked from theirs by pointer jumping, as many rounds
+// as the tile's longest stretch needs (states of a cycle within the tile never
+// get there). Per state in shared memory: predecessor | distance << 11 | rooted.
+// 5M nodes: 103 us (116 with tiles of 1024 nodes, fewer of them an SM); with
+// the ruler list's kernel 236 where states, walks and list took 347.
+constexpr int kTile = 512;
+__global__ void __launch_bounds__(kTile, 4) k_mg_states(MergeArgs a) {
+    constexpr unsigned kRooted = 1u << 31, kDist = 0xffffu << 11;
+    __shared__ unsigned v[2 * kTile], pos[2 * kTile];
     __shared__ unsigned rulers;
     __shared__ unsigned long long base;
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (threadIdx.x == 0) rulers = 0;
-    __syncthreads();
-    bool first = false, second = false;
-    if (i < a.n && is_m(a, i)) {
-        const unsigned char f = a.fl[i];
-        const uint2 pair = make_uint2(walk_state(a, f, i, 0), walk_state(a, f, i, 1));
-        a.succ[i] = pair;
-        *reinterpret_cast<ulonglong2 *>(a.oo + 2 * i) = make_ulonglong2(~0ull, ~0ull);
-        first = ruler_of(a, 2 * i, pair);
-        second = ruler_of(a, 2 * i + 1, pair);
+    const unsigned t = threadIdx.x;
+    const uint64_t first = (uint64_t)blockIdx.x * kTile, i = first + t;
+    if (t == 0) rulers = 0;
+    const unsigned char f = i < a.n ? a.fl[i] : 0;
+    const bool in = f & 1u;
+    unsigned nx[2] = {kEnd, kEnd}, w[2];
+    if (in) {
+        nx[0] = walk_state(a, f, i, 0);
+        nx[1] = walk_state(a, f, i, 1);
     }
-    unsigned at = first || second ? atomicAdd(&rulers, (unsigned)first + second) : 0;
     __syncthreads();
-    if (threadIdx.x == 0 && rulers) base = atomicAdd(&a.ctr[0], (unsigned long long)rulers);
+#pragma unroll
+    for (int d = 0; d < 2; ++d) {
+        const unsigned pred = nx[d ^ 1] ^ 1u;  // (if the twin has a successor)
+        const bool here = in && !(nx[d ^ 1] & kEnd) && (pred >> 1) - first < (uint64_t)kTile;
+        w[d] = here ? (pred - (unsigned)(2 * first)) | 1u << 11 : (2 * t + d) | kRooted;
+        v[2 * t + d] = w[d];
+        if (in && !here) pos[2 * t + d] = atomicAdd(&rulers, 1u);
+    }
     __syncthreads();
-    if (first) {
-        a.rpos[2 * i] = (unsigned)base + at;
-        a.rlist[base + at++] = (unsigned)(2 * i);
-    }
-    if (second) {
-        a.rpos[2 * i + 1] = (unsigned)base + at;
-        a.rlist[base + at] = (unsigned)(2 * i + 1);
-    }
-}
-
-// A ruler: the first state of a walk (its twin leaves to an end) or, on
-// average, one state in rmask + 1 (16..256, chosen for at most about 2^20 rulers:
-// enough walkers to keep the SMs' warp slots busy while each walk's loads
-// wait on memory one after the other, and a ruler list small enough for L2).
-__device__ __forceinline__ bool ruler_of(const MergeArgs &a, unsigned st, uint2 pair) {
-    return ((st & 1 ? pair.x : pair.y) & kEnd) || (fmix64(st) & a.rmask) == 0;
-}
-
-// Each ruler walks to the next ruler or the walk's end, labelling the states
-// on the way with (its list position, distance); per step one 8-byte load
-// (a node's two successors: 40 MB for 5M nodes, half of L2's reach) and one
-// 8-byte store. Bound by those loads' latency, one after the other, so a lane
-// that has arrived takes its next ruler at once, its first load issued while
-// the walk before was under way, and does not wait for its warp's longest walk
-// (of 32 walks of 16 states on average, the longest has 65). The next ruler
-// is noted as a state; the ruler list's kernel looks its position up.
-// 5M nodes: 237 us with a warp waiting for its 32 walks and 16-byte pairs, 182 now.
-__global__ void __launch_bounds__(256) k_mg_walk(MergeArgs a) {
-    const uint64_t n_rul = a.ctr[0], stride = (uint64_t)gridDim.x * blockDim.x;
-    uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n_rul) return;
-    unsigned cur = a.rlist[p], ahead = p + stride < n_rul ? a.rlist[p + stride] : 0;
-    uint2 pr = a.succ[cur >> 1], pr_ahead = a.succ[ahead >> 1];
-    unsigned later = p + 2 * stride < n_rul ? a.rlist[p + 2 * stride] : 0;
-    a.oo[cur] = p << 32;
-    for (unsigned o = 1; o <= 2 * a.n;) {
-        const unsigned nx = cur & 1 ? pr.y : pr.x;
-        const bool end = nx & kEnd;
-        uint2 pn = make_uint2(0, 0);
-        if (!end) pn = a.succ[nx >> 1];
-        if (!end && !ruler_of(a, nx, pn)) {
-            a.oo[nx] = p << 32 | o;
-            cur = nx;
-            pr = pn;
-            ++o;
-            continue;
+    if (t == 0 && rulers) base = atomicAdd(&a.ctr[0], (unsigned long long)rulers);
+    for (int r = 0; r < 12; ++r) {  // stretches are at most 2 * kTile - 1 states
+        bool open = false;
+#pragma unroll
+        for (int d = 0; d < 2; ++d) {
+            if (w[d] & kRooted) continue;
+            const unsigned u = v[w[d] & (2 * kTile - 1)];
+            w[d] = (u & (kRooted | (2 * kTile - 1))) | (((w[d] & kDist) + (u & kDist)) & kDist);
+            open |= !(w[d] & kRooted);
         }
-        a.rp0[p] = end ? make_uint2((unsigned)walk_next(a, cur >> 1, cur & 1), o | kEnd) : make_uint2(nx, o);
-        p += stride;
-        if (p >= n_rul) return;
-        cur = ahead;
-        pr = pr_ahead;
-        a.oo[cur] = p << 32;
-        o = 1;
-        ahead = later;
-        pr_ahead = a.succ[ahead >> 1];
-        later = p + 2 * stride < n_rul ? a.rlist[p + 2 * stride] : 0;
+        const bool more = __syncthreads_or(open);
+        v[2 * t] = w[0];
+        v[2 * t + 1] = w[1];
+        __syncthreads();
+        if (!more) break;
     }
-    for (; p < n_rul; p += stride) a.rp0[p] = make_uint2(0, kEnd);  // (the host stops at the error)
-    atomicOr(a.err, kErrWalk);
+#pragma unroll
+    for (int d = 0; d < 2; ++d) {
+        if (!in || w[d] != ((2 * t + d) | kRooted)) continue;
+        const unsigned at = (unsigned)base + pos[2 * t + d];
+        a.rpos[2 * i + d] = at;
+        a.rp0[at] = make_uint2(0, kEnd);  // (stays if arcs do not lead back)
+    }
+    __syncthreads();
+    if (!in) return;
+    unsigned long long o[2];
+#pragma unroll
+    for (int d = 0; d < 2; ++d) {
+        const unsigned root = w[d] & (2 * kTile - 1), dist = (w[d] & kDist) >> 11;
+        const unsigned at = (unsigned)base + pos[root];
+        o[d] = w[d] & kRooted ? (unsigned long long)at << 32 | dist : ~0ull;
+        if (!(w[d] & kRooted)) continue;
+        // the stretch's last state knows where it leads, and whether it is a walk's first stretch
+        const bool end = nx[d] & kEnd;
+        if (end || (nx[d] >> 1) - first >= (uint64_t)kTile) {
+            const uint64_t r = first + (root >> 1);
+            const bool head = root == 2 * t + d ? nx[d ^ 1] & kEnd : walk_state(a, a.fl[r], r, (root & 1) ^ 1) & kEnd;
+            a.rp0[at] = make_uint2(end ? (unsigned)walk_next(a, i, d) : nx[d], (dist + 1) | (end ? kEnd : 0) | (head ? kHead : 0));
+        }
+    }
+    *reinterpret_cast<ulonglong2 *>(a.oo + 2 * i) = make_ulonglong2(o[0], o[1]);
 }
 
-// Pointer jumping over the ruler list, all rounds in one cooperative launch:
-// a round is bound by its random loads' latency (so a thread has four rulers'
-// under way) and a grid barrier, which costs less than a launch. Rounds go in
-// pairs, so that the result is in rp0 again, and end once every ruler has
-// reached an end (as many rounds as the longest chain's rulers need, where the
-// bound for any chain was 22 to 25); the rulers of a cycle never do. 5M nodes,
-// 700,000 rulers: 140 us with four blocks of 256 an SM and a ruler at a time,
-// 108 with one of 1024 an SM and four (eight of 256 an SM: 138, the barrier).
-constexpr int kJump = 4;
-__global__ void __launch_bounds__(1024) k_mg_rjump(MergeArgs a, int pairs) {
+// The ruler list ranked, in one cooperative launch (a grid barrier costs less
+// than a launch, and one block of 1024 an SM less than more): every eighth
+// ruler and every walk's first is a pole; the poles walk to the next pole,
+// noting the rulers on the way; the poles' list is ranked by pointer jumping;
+// the rulers take over their pole's result. Bound by the latency of random
+// loads, all of L2: so as few rounds over as short a list as walks of some
+// twenty steps leave. Jumping rounds go in pairs, so that the result is in pp0
+// again, and end once every pole has reached an end (the poles of a cycle never
+// do). 5M nodes: 133 us. (A longest walk has twelve times the mean: every fourth
+// ruler a pole shortens it, but doubles the list, 25 us more in all; blocks for
+// n / 8192, up to one an SM, because a barrier's time grows with them.)
+constexpr unsigned kPole = 8;
+__global__ void __launch_bounds__(1024) k_mg_rank(MergeArgs a, int pairs) {
     const uint64_t n_rul = a.ctr[0], stride = (uint64_t)gridDim.x * blockDim.x;
-    const uint64_t p0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    for (uint64_t p = p0; p < n_rul; p += stride) {  // states to list positions
-        const uint2 v = a.rp0[p];
-        if (!(v.y & kEnd)) a.rp0[p].x = a.rpos[v.x];
+    const uint64_t p0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, every = (n_rul + kPole - 1) / kPole;
+    for (uint64_t q = p0; q < n_rul; q += stride) {  // next rulers from states to list positions
+        const uint2 v = __ldcg(a.rp0 + q);
+        if (!(v.y & kEnd)) {
+            const unsigned next = a.rpos[v.x];
+            if (next >= n_rul) atomicOr(a.err, kErrWalk);  // (arcs that do not lead back)
+            a.rp0[q].x = next < n_rul ? next : 0;
+        }
+        uint2 o = make_uint2(kNone, 0);
+        if (q % kPole == 0) {
+            o.x = (unsigned)(q / kPole);
+        } else if (v.y & kHead) {
+            const uint64_t h = agg_inc(&a.ctr[6]);
+            a.heads[h] = (unsigned)q;
+            o.x = (unsigned)(every + h);
+        }
+        a.ro[q] = o;
+    }
+    cg::this_grid().sync();
+    const uint64_t n_pole = every + __ldcg(&a.ctr[6]);
+    for (uint64_t p = p0; p < n_pole; p += stride) {
+        uint64_t cur = p < every ? p * kPole : __ldcg(a.heads + (p - every));
+        uint2 out = make_uint2(0, kEnd);
+        bool done = false;
+        unsigned o = 0;
+        for (uint64_t step = 0; step <= n_rul && !done; ++step) {
+            const uint2 v = __ldcg(a.rp0 + cur);
+            o += v.y & (kHead - 1);
+            done = (v.y & kEnd) || v.x % kPole == 0;
+            if (done) {
+                out = v.y & kEnd ? make_uint2(v.x, o | kEnd) : make_uint2(v.x / kPole, o);
+            } else {
+                a.ro[v.x] = make_uint2((unsigned)p, o);
+                cur = v.x;
+            }
+        }
+        if (!done) atomicOr(a.err, kErrWalk);
+        a.pp0[p] = out;
     }
     cg::this_grid().sync();
     for (int r = 0; r < pairs; ++r) {
         bool moved = false;
         for (int half = 0; half < 2; ++half) {
-            const uint2 *in = half ? a.rp1 : a.rp0;
-            uint2 *out = half ? a.rp0 : a.rp1;
-            for (uint64_t p = p0; p < n_rul; p += kJump * stride) {
-                uint2 v[kJump], w[kJump];
-#pragma unroll
-                for (int j = 0; j < kJump; ++j)
-                    v[j] = p + j * stride < n_rul ? __ldcg(in + p + j * stride) : make_uint2(0, kEnd);
-#pragma unroll
-                for (int j = 0; j < kJump; ++j)
-                    if (!(v[j].y & kEnd)) w[j] = __ldcg(in + v[j].x);
-#pragma unroll
-                for (int j = 0; j < kJump; ++j) {
-                    if (!(v[j].y & kEnd)) {  // (a cycle's sums mean nothing, and stay below kEnd)
-                        v[j] = make_uint2(w[j].x, ((v[j].y + (w[j].y & ~kEnd)) & ~kEnd) | (w[j].y & kEnd));
-                        moved |= !(v[j].y & kEnd);
-                    }
-                    if (p + j * stride < n_rul) out[p + j * stride] = v[j];
+            const uint2 *in = half ? a.pp1 : a.pp0;
+            uint2 *out = half ? a.pp0 : a.pp1;
+            for (uint64_t p = p0; p < n_pole; p += stride) {
+                uint2 v = __ldcg(in + p);
+                if (!(v.y & kEnd)) {  // (a cycle's sums mean nothing, and stay below kEnd)
+                    const uint2 w = __ldcg(in + v.x);
+                    v = make_uint2(w.x, ((v.y + (w.y & ~kEnd)) & ~kEnd) | (w.y & kEnd));
+                    moved |= !(v.y & kEnd);
                 }
+                out[p] = v;
             }
             if (half && moved) a.moved[r] = 1;
             cg::this_grid().sync();
             moved = false;
         }
-        if (!*(volatile unsigned *)(a.moved + r)) return;
+        if (!*(volatile unsigned *)(a.moved + r)) break;
+    }
+    for (uint64_t q = p0; q < n_rul; q += stride) {
+        const uint2 o = __ldcg(a.ro + q);
+        uint2 v = make_uint2(0, 0);
+        if (o.x != kNone) {
+            const uint2 w = __ldcg(a.pp0 + o.x);
+            if (w.y & kEnd) v = make_uint2(w.x, w.y - o.y);
+        }
+        a.rp0[q] = v;
     }
 }
 
@@ -396,7 +429,7 @@ __global__ void k_mg_cyc_init(MergeArgs a, uint64_t c) {
     if (t >= c) return;
     const unsigned st = a.clist[t];
     a.cx0[st] = cut_rank(a, st >> 1);
-    a.cy0[st] = st & 1 ? a.succ[st >> 1].y : a.succ[st >> 1].x;  // (no end arc in a cycle)
+    a.cy0[st] = walk_next(a, st >> 1, (int)(st & 1));  // (no end arc in a cycle)
 }
 
 __global__ void k_mg_cyc_max(MergeArgs a, uint64_t c, const unsigned long long *__restrict__ mx_in,
@@ -492,13 +525,13 @@ __global__ void k_mg_chain_count(MergeArgs a) {
     const ChainPos c = chain_pos(a, i);
     if (c.pos != 1) return;
     agg_add_labeled(a.cls_count, size_class(c.m), 1);
-    a.rlist[agg_inc(&a.ctr[2])] = (unsigned)i;  // (the rulers' list is done with)
+    a.heads[agg_inc(&a.ctr[2])] = (unsigned)i;  // (the poles' list is done with)
 }
 
 __global__ void k_mg_chain_alloc(MergeArgs a, uint64_t n_chains) {
     const uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= n_chains) return;
-    const ChainPos c = chain_pos(a, a.rlist[q]);
+    const ChainPos c = chain_pos(a, a.heads[q]);
     const int cl = size_class(c.m);
     const unsigned id = (unsigned)q;
     a.ch_eoff[id] = agg_add_labeled(a.cls_cursor, cl, 1ull << cl);
@@ -840,14 +873,12 @@ swg_status merge_graph(const unsigned long long *d_keys, const unsigned long lon
     std::memset(&a, 0, sizeof(a));
     a.k = k;
     a.n = n;
-    a.rmask = 15;
-    while (a.rmask < 255 && 2 * n / (a.rmask + 1) > (1ull << 20)) a.rmask = 2 * a.rmask + 1;
     unsigned long long *ctr = nullptr;
     uint64_t hcap = 1024;
     while (hcap < 2 * n) hcap *= 2;
     a.hmask = hcap - 1;
-    if (!scr.get(&a.ht, hcap) || !scr.get(&a.nb, 8 * n) || !scr.get(&a.fl, n) || !scr.get(&a.succ, n) ||
-        !scr.get(&a.oo, 2 * n) || !scr.get(&a.rpos, 2 * n) || !scr.get(&a.rlist, 2 * n) ||
+    if (!scr.get(&a.ht, hcap) || !scr.get(&a.nb, 8 * n) || !scr.get(&a.fl, n) ||
+        !scr.get(&a.oo, 2 * n) || !scr.get(&a.rpos, 2 * n) || !scr.get(&a.heads, 2 * n) ||
         !scr.get(&a.lt, 2 * n) || !scr.get(&a.clist, 2 * n) ||
         !scr.get(&a.chain_of, 8 * n) || !scr.get(&ctr, 8 + 2 * kClasses))
         return cuda_err(cudaErrorMemoryAllocation, "merge workspace");
@@ -884,27 +915,25 @@ swg_status merge_graph(const unsigned long long *d_keys, const unsigned long lon
         ++launches;
     }
     k_mg_classify<<<blocks(n), 256, 0, s>>>(a);
-    k_mg_states<<<blocks(n), 256, 0, s>>>(a);
-    launches += 3;
     // rulers: at most one per state; counts stay on the device
-    if (!scr.get(&a.rp0, 2 * n) || !scr.get(&a.rp1, 2 * n) || !scr.get(&a.moved, 64))
+    if (!scr.get(&a.rp0, 2 * n) || !scr.get(&a.ro, 2 * n) || !scr.get(&a.pp0, 2 * n) || !scr.get(&a.pp1, 2 * n) ||
+        !scr.get(&a.moved, 64))
         return cuda_err(cudaErrorMemoryAllocation, "ruler list");
     EMIT_CUDA(cudaMemsetAsync(a.moved, 0, 64 * sizeof(unsigned), s), "merge clear");
+    k_mg_states<<<(unsigned)std::max<uint64_t>((n + kTile - 1) / kTile, 1), kTile, 0, s>>>(a);
+    launches += 3;
     int sms = 0, dev = 0;
     EMIT_CUDA(cudaGetDevice(&dev), "device");
     EMIT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "device attribute");
-    const unsigned wgrid = (unsigned)std::max(1, sms * 8);
-    k_mg_walk<<<wgrid, 256, 0, s>>>(a);
     {
         int pairs = (ceil_log2(std::max<uint64_t>(2 * n, 1)) + 2) / 2;
         void *args[] = {&a, &pairs};
-        const uint64_t rulers = 2 * n / (a.rmask + 1);  // (about; and the walks' first states)
-        const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)std::max(1, sms), rulers / 1024 + 1);
-        EMIT_CUDA(cudaLaunchCooperativeKernel((const void *)k_mg_rjump, dim3(grid), dim3(1024), args, 0, s), "ruler list");
+        const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)std::max(1, sms), n / 8192 + 1);
+        EMIT_CUDA(cudaLaunchCooperativeKernel((const void *)k_mg_rank, dim3(grid), dim3(1024), args, 0, s), "ruler list");
     }
     k_mg_finish<<<blocks(n), 256, 0, s>>>(a);
     k_mg_chain_count<<<blocks(n), 256, 0, s>>>(a);  // (a cycle's states, at 0, are no chain's: counted again below)
-    launches += 4;
+    launches += 3;
     unsigned long long h[8 + kClasses];
     EMIT_CUDA(cudaMemcpyAsync(h, ctr, sizeof(h), cudaMemcpyDeviceToHost, s), "merge counts");
     EMIT_CUDA(cudaStreamSynchronize(s), "merge counts");
