@@ -1219,10 +1219,16 @@ swg_status grow_keep(T **p, uint64_t *cap, uint64_t want, uint64_t keep, const c
 
 // ---- the bucketed build over super-k-mer records (super.cu) ----
 // Longest read a streamed piece's scan takes whole (its records hold 14 bits
-// of position); a one-shot build cuts reads past kSuperWhole bases in pieces.
+// of position); a one-shot build cuts reads past kSuperWhole bases in pieces
+// (a block is done when its longest read is; most short-read sets have none).
 constexpr uint64_t kSuperLongest = (1ull << 14) - 1;
 constexpr uint64_t kSuperWhole = 512;
 
+// Super-k-mers for every odd k that their records and minimizers serve (19 to
+// 31: a record holds 47 bases, and a shorter k has too few m-mers), at every
+// size: builds of 0.2M occurrences take 126 us, by single occurrences 178; of
+// 175M 2.14 ms and 3.01; of 2.4G, with repeats, 28.9 and 46.5. An even k-mer can
+// be its own reverse complement, and a batch may mix k: single occurrences.
 bool super_build(const swg_opts *o, const BuildArgs &a, uint64_t N) {
     // (the other scatter shapes are shapes of the single-occurrence scatters)
     return swg::super_window(a.k, N) && N && !swg::level1_shape(o->scatter_shape);
@@ -1236,8 +1242,10 @@ swg_status super_plan(swg_graph *g, const swg_opts *o, const BuildArgs &a, uint6
     swg_status st;
     int b1, b2;
     // sub-buckets of at most 3072 occurrences on average: the 2048-entry tables
-    // (four CTAs an SM) hold their k-molecules; 524,288 such buckets counted
-    // 2.4G skewed occurrences in 18.8 ms, 262,144 in 4096-entry tables in 20.3
+    // (four CTAs an SM) hold their k-molecules. (Past 800M occurrences they are
+    // larger and 4096-entry tables count them: 2.4G skewed ones in 262,144
+    // buckets 17.5 ms, 524,288 16.7, in 1,048,576 and the small tables 17.4, but
+    // the scan's and the preparation's share grows with them.)
     bucket_bits(o, N, 3072.0, b1, b2);
     const uint64_t P = 1ull << b1, NB = P << b2;
     const double scale_max = 2.0 * stride / share;
@@ -1428,16 +1436,17 @@ swg_status super_finish(swg_graph *g, const swg_opts *o, BuildArgs &a, cudaStrea
     const unsigned retries = g->h_ctl->pad;
     if (nbig) {
         const uint64_t n_small = g->h_ctl->counters[1];
-        std::vector<unsigned long long> big(nbig), off(NB + 1), cur(NB), meta(2 * (uint64_t)nbig + 1);
-        SWG_CUDA(cudaMemcpyAsync(big.data(), pl.sk.big2, nbig * 8, cudaMemcpyDeviceToHost, s), "read big buckets");
-        SWG_CUDA(cudaMemcpyAsync(off.data(), pl.sk.off2, (NB + 1) * 8, cudaMemcpyDeviceToHost, s), "read regions");
-        SWG_CUDA(cudaMemcpyAsync(cur.data(), pl.sk.cursor2, NB * 8, cudaMemcpyDeviceToHost, s), "read cursors");
+        std::vector<unsigned long long> meta(2 * (uint64_t)nbig + 1);
+        if ((st = ensure(&g->d_bigmeta, &g->bigmeta_cap, meta.size(), "big-bucket list"))) return st;
+        g->launches += swg::launch_super_big_bounds(pl.sk, nbig, g->d_bigmeta, s);
+        SWG_CUDA(cudaMemcpyAsync(meta.data(), g->d_bigmeta, 2 * (uint64_t)nbig * 8, cudaMemcpyDeviceToHost, s),
+                 "big buckets");
         SWG_CUDA(cudaStreamSynchronize(s), "big buckets");
         uint64_t records = 0;
         for (unsigned i = 0; i < nbig; i++) {
-            meta[i] = off[big[i]];
+            const uint64_t m = meta[nbig + i];
             meta[nbig + i] = records;
-            records += std::min<uint64_t>(cur[big[i]], off[big[i] + 1]) - off[big[i]];
+            records += m;
         }
         meta[2 * (uint64_t)nbig] = records;
         const uint64_t kmers = std::min<uint64_t>(17 * records, N);  // at most 17 a record
@@ -1445,7 +1454,6 @@ swg_status super_finish(swg_graph *g, const swg_opts *o, BuildArgs &a, cudaStrea
         a.out_keys = g->d_out_keys;
         a.out_mult = g->d_out_mult;
         a.out_cap = g->out_cap;
-        if ((st = ensure(&g->d_bigmeta, &g->bigmeta_cap, meta.size(), "big-bucket list"))) return st;
         SWG_CUDA(cudaMemcpyAsync(g->d_bigmeta, meta.data(), meta.size() * 8, cudaMemcpyHostToDevice, s),
                  "big-bucket list");
         const uint64_t cap = (uint64_t)std::ceil((double)kmers / load) + 64;

@@ -14,9 +14,10 @@
 //   k_compact     K2: the -c cutoff (graph.cpp:1092-1114) as one streaming
 //                 pass over the table with block-level stream compaction
 //   k_p1_*, k_sub_*, k_bucket_*
-//                 bucketed build: two hash-partition scatters group the
-//                 occurrence records by bucket, then one CTA per bucket
-//                 counts it in a shared-memory table
+//                 bucketed build over single occurrences: two hash-partition
+//                 scatters group their records by bucket, then one CTA per
+//                 bucket counts it in a shared-memory table (super.cu has the
+//                 one over super-k-mers, for odd k from 19)
 //   k_probe       random-access roofline probe
 //
 // Every device-side retry loop is bounded; on exhaustion the kernel sets a
@@ -41,7 +42,6 @@ constexpr uint64_t kScanChunk = (uint64_t)kScanBlock * kScanItems;
 constexpr int kCBlock = 256;
 constexpr int kCItems = 8;
 
-// ---------------------------------------------------------------------
 // ---------------------------------------------------------------------
 // Occurrence prefix: occ_prefix[r] = sum_{q<r} max(0, len[q]-k+1).
 __global__ void __launch_bounds__(kScanBlock) k_scan_reduce(BuildArgs a) {
@@ -2242,6 +2242,8 @@ int launch_part_scatter(const BuildArgs &a, const PartArgs &p, cudaStream_t s, i
         return 1;
     }
     const bool single = !a.segs && !a.read_seg && !a.tag_bits;
+    // (Odd k from 19 to 31 come here for shapes 1 to 4, and to be counted again
+    // exactly; otherwise they go by super-k-mers.)
     // Single-sample builds with 256 partitions and a common k: the walk's
     // shifts and masks and the record layout are compile-time constants, and
     // rounds of 12 records a thread fit 64 registers, so four blocks share an

@@ -1014,13 +1014,12 @@ swg_status merge_graph(const unsigned long long *d_keys, const unsigned long lon
     uint64_t bytes = 0;
     // by splitters (three launches, 37 us for 6,000 lines; the library's passes
     // took eight and 61), or by the library's passes if there are more lines
-    // than those take or one of their buckets runs full
+    // than those take, one of their buckets runs full or there is no room
     for (bool library = n_lines > sort_device_most();; library = true) {
         unsigned *over = nullptr;
         unsigned unordered = 0;
-        if (n_lines && !library) {
-            unsigned char *ws = nullptr;
-            if (!scr.get(&ws, sort_scratch_bytes(n_lines))) return cuda_err(cudaErrorMemoryAllocation, "sort scratch");
+        unsigned char *ws = nullptr;
+        if (n_lines && !library && scr.get(&ws, sort_scratch_bytes(n_lines))) {
             sort_records_device(a.skey, a.sidx, n_lines, s, ws, &skey2, &sidx2, &over);
         } else if (n_lines) {
             if (!scr.get(&skey2, n_lines) || !scr.get(&sidx2, n_lines))

@@ -54,7 +54,9 @@ __device__ __forceinline__ uint32_t sk_mix(uint32_t x) {  // bucket of a minimiz
 }
 
 // ---- pieces of long reads: a piece's length word has bit 30 / 31 set when a
-// base precedes / follows it in its read.
+// base precedes / follows it in its read. A thread per read left 80 blocks for
+// 20,000 reads of 3 to 15 kbp; level 1 over pieces takes 0.40 ms there (setup
+// included 0.78), the single-occurrence scatter took 5.5 (7.3).
 __global__ void __launch_bounds__(256) k_sk_pieces_count(BuildArgs a, uint64_t *__restrict__ n) {
     const uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= a.n_reads) return;
@@ -97,6 +99,11 @@ __global__ void __launch_bounds__(256) k_sk_pieces_fill(BuildArgs a, const uint6
 // k-mers (5), thread (8); high word the minimizer, then partition (10 bits),
 // sub-bucket (10), rank (12).
 // kSample: only counts, per partition and per bucket.
+// Bound by the ALU pipe (80% busy: shifts, minima and selects at half rate).
+// 2.5M reads of 100 bp, 175M occurrences, k = 31: 0.38 ms, where the scatter of
+// single occurrences took 0.81 and wrote four times the bytes. With runs pushed
+// from inside the block 0.61 (a warp's few lanes at a time); with every load
+// checked against the read's end 0.40.
 template <int M, int W, bool kSample>
 __global__ void __launch_bounds__(kSkThreads, 4) k_sk_scan(BuildArgs a, SkArgs s, uint32_t stride) {
     constexpr int K = M + W - 1, NT = kSkThreads, NW = NT / 32;
@@ -381,7 +388,8 @@ __global__ void __launch_bounds__(256) k_sk_bucket_caps(SkArgs s, const unsigned
 
 // Both kinds of regions of a plan of at most 1024 kRegionItems buckets, and
 // the cursors at their starts, by one block (six launches otherwise, most of a
-// small build's preparation).
+// small build's preparation). Single precision: 9 us for 2048 buckets, 25 in
+// double.
 constexpr int kRegionItems = 16;
 __global__ void __launch_bounds__(1024) k_sk_regions(SkArgs s, uint32_t nb) {
     __shared__ uint64_t wb[32];
@@ -423,7 +431,9 @@ __global__ void __launch_bounds__(1024) k_sk_regions(SkArgs s, uint32_t nb) {
 // Level-2 scatter: a chunk of one partition's records is held in registers,
 // ordered by sub-bucket in shared memory and written as one run per bucket.
 // Every block works out the partitions' chunks for itself (and flags a
-// partition that outgrew its region).
+// partition that outgrew its region). Bound by memory latency and bandwidth:
+// 175M occurrences 0.145 ms, 0.68 for the records of single ones (8 B each,
+// where these take 2 an occurrence).
 size_t sub_smem(int b2, uint32_t n_parts) {
     return kSkChunk * sizeof(uint4) + ((size_t)1 << b2) * (sizeof(unsigned long long) + 3 * sizeof(unsigned)) +
            (n_parts + 1) * sizeof(unsigned);
@@ -622,6 +632,14 @@ __device__ __forceinline__ bool bucket_keep(const unsigned *cnt, uint32_t s, uns
 //     another here), then written; the slots are cleared on the way.
 // Buckets whose keys do not fit go to the overflow list uncounted; their
 // records stay as they are.
+// Bound on chip, by the table's shared-memory atomics and what feeds them.
+// 2.5M reads of 100 bp at 1% errors (175M occurrences, 50M of them distinct):
+// 1.49 ms, of which inserting 0.86 (the probes past a slot that is taken 0.38,
+// the adds 0.14), cutting the k-mers out of the records 0.34, the rest 0.30.
+// Without merging equal records 2.05. The count of single occurrences took
+// 1.27, after scatters that took 1.0 ms more than the records' do. A load
+// before the CAS, or 32-bit CAS on the halves of a key, took longer (1.68,
+// 1.75 to 1.89 against 1.62 with 131072 buckets).
 template <int T, int NT, int kK>
 __device__ void count_pass(const BuildArgs &a, const SkArgs &s, uint64_t n_items, uint32_t set,
                            const unsigned long long *list, unsigned long long *ovf, unsigned *ovf_count) {
@@ -1008,45 +1026,107 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_sk_count(BuildArgs a, SkArgs 
     }
 }
 
-// Buckets no shared-memory table holds, in one global-memory table of record
-// hashes (rmix64 of the key, as k_big_compact reads it): meta = first record
-// [n] | record prefix [n+1]. Equal keys of a warp's step are merged first.
+// First record and records of the buckets no shared-memory table holds.
+__global__ void k_sk_big_bounds(SkArgs s, uint32_t n, unsigned long long *meta) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const unsigned long long b = s.big2[i], start = s.off2[b];
+    meta[i] = start;
+    meta[n + i] = umin64(s.cursor2[b], s.off2[b + 1]) - start;
+}
+
+// Those buckets, in one global-memory table of record hashes (rmix64 of the
+// key, as k_big_compact reads it): meta = first record [n] | record prefix
+// [n+1]. They are tandem repeats, so their k-mers are few and hot, and updates
+// of the same entry go one after the other: equal records of a chunk are merged
+// first, as in the tables' count, then equal keys of a warp's step. 2.4G
+// occurrences with 2% tandem repeats, 31 such buckets: 1.0 ms, 2.9 record by
+// record.
+constexpr uint32_t kSkBigChunk = 1024;
 __global__ void __launch_bounds__(256) k_sk_big(BuildArgs a, SkArgs s, const unsigned long long *meta, uint32_t n,
                                                 Entry *table, uint64_t cap) {
-    const int lane = threadIdx.x & 31;
+    constexpr int R = kSkBigChunk / 256, kSlotBits = 11;
+    __shared__ uint4 srec[kSkBigChunk];
+    __shared__ unsigned stab[1 << kSlotBits], sdis[kSkBigChunk];  // first record (index + 1) | others << 16; distinct ones
+    __shared__ unsigned s_distinct;
+    const uint32_t lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
     const unsigned long long *rbs = meta, *pre = meta + n;
     const uint64_t total = pre[n];
-    const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t g = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; g * 32 < total; g += warps) {
-        const uint64_t i = g * 32 + lane;
-        uint4 rec = make_uint4(0, 0, 0, 0);
-        if (i < total) {
-            uint32_t lo = 0, hi = n;
-            while (hi - lo > 1) {
-                const uint32_t mid = (lo + hi) >> 1;
-                if (pre[mid] <= i) lo = mid;
-                else hi = mid;
-            }
-            rec = s.rec2[rbs[lo] + (i - pre[lo])];
-        }
-        sk_expand<0>(rec, 1, s.k, [&](bool valid, const SkOcc &o, const uint4 &x) {
-            const unsigned vmask = __ballot_sync(kFull, valid);
-            if (!valid) return;
-            uint64_t key = o.key;
-            if (a.tag_bits) key |= (uint64_t)((x.w >> 17) & 1023u) << (64 - a.tag_bits);
-            uint64_t inc = (uint64_t)o.radd << (8 * o.rs) | (uint64_t)o.ladd << (8 * o.ls);
-            const unsigned peers = __match_any_sync(vmask, key);
-            if (__any_sync(vmask, peers != (1u << lane))) {
-                uint64_t tot = 0;
+    for (uint64_t g0 = (uint64_t)blockIdx.x * kSkBigChunk; g0 < total; g0 += (uint64_t)gridDim.x * kSkBigChunk) {
+        for (uint32_t j = threadIdx.x; j < 1u << kSlotBits; j += 256) stab[j] = 0;
+        if (threadIdx.x == 0) s_distinct = 0;
+        uint4 rec[R];
 #pragma unroll
-                for (int sl = 0; sl < 8; ++sl) {
-                    const unsigned b = __ballot_sync(vmask, (unsigned)(inc >> (8 * sl)) & 1u);
-                    tot |= (uint64_t)__popc(b & peers) << (8 * sl);
+        for (int i = 0; i < R; ++i) {
+            const uint64_t g = g0 + i * 256 + threadIdx.x;
+            if (g < total) {
+                uint32_t lo = 0, hi = n;
+                while (hi - lo > 1) {
+                    const uint32_t mid = (lo + hi) >> 1;
+                    if (pre[mid] <= g) lo = mid;
+                    else hi = mid;
                 }
-                inc = tot;
+                srec[i * 256 + threadIdx.x] = rec[i] = s.rec2[rbs[lo] + (g - pre[lo])];
             }
-            if (lane == __ffs(peers) - 1) insert_or_update(table, cap, rmix64(key), inc, a.status);
-        });
+        }
+        __syncthreads();
+        uint32_t first[R];
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            first[i] = ~0u;
+            if (g0 + i * 256 + threadIdx.x >= total) continue;
+            uint32_t h = (rec[i].x * 0x9e3779b1u ^ rec[i].y * 0x85ebca6bu) + (rec[i].z * 0xc2b2ae35u ^ rec[i].w * 0x27d4eb2fu);
+            h = (h ^ h >> 15) * 0x2c1b3c6du >> (32 - kSlotBits);
+            for (;;) {  // ends: the table has twice the chunk's slots
+                const unsigned old = atomicCAS(&stab[h], 0u, i * 256 + threadIdx.x + 1);
+                if (old == 0) {
+                    first[i] = h;
+                    break;
+                }
+                const uint4 x = srec[(old & 0xffffu) - 1];
+                if (x.x == rec[i].x && x.y == rec[i].y && x.z == rec[i].z && x.w == rec[i].w) {
+                    atomicAdd(&stab[h], 1u << 16);
+                    break;
+                }
+                h = (h + 1) & ((1u << kSlotBits) - 1);
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+            if (first[i] != ~0u)
+                sdis[atomicAdd(&s_distinct, 1u)] = i * 256 + threadIdx.x | (1u + (stab[first[i]] >> 16)) << 16;
+        __syncthreads();
+        const uint32_t nd = s_distinct;
+        for (uint32_t p0 = wp * 32; p0 < nd; p0 += 256) {
+            uint4 one = make_uint4(0, 0, 0, 0);
+            uint32_t weight = 0;
+            if (p0 + lane < nd) {
+                one = srec[sdis[p0 + lane] & 0xffffu];
+                weight = sdis[p0 + lane] >> 16;
+            }
+            sk_expand<0>(one, weight, s.k, [&](bool valid, const SkOcc &o, const uint4 &x) {
+                const unsigned vmask = __ballot_sync(kFull, valid);
+                if (!valid) return;
+                uint64_t key = o.key;
+                if (a.tag_bits) key |= (uint64_t)((x.w >> 17) & 1023u) << (64 - a.tag_bits);
+                // (counts saturate at 255: so may the sums on the way)
+                const uint64_t inc = (uint64_t)min(o.radd, 255u) << (8 * o.rs) | (uint64_t)min(o.ladd, 255u) << (8 * o.ls);
+                const unsigned peers = __match_any_sync(vmask, key);
+                unsigned low = 0, high = 0;
+                for (unsigned left = peers; __any_sync(vmask, left); left &= left - 1) {  // a round per lane of the largest group
+                    const int from = left ? __ffs(left) - 1 : (int)lane;
+                    const unsigned l = __shfl_sync(vmask, (unsigned)inc, from), h = __shfl_sync(vmask, (unsigned)(inc >> 32), from);
+                    if (left) {
+                        low = __vaddus4(low, l);
+                        high = __vaddus4(high, h);
+                    }
+                }
+                if (lane == (uint32_t)__ffs(peers) - 1)
+                    insert_or_update(table, cap, rmix64(key), (uint64_t)high << 32 | low, a.status);
+            });
+        }
+        __syncthreads();
     }
 }
 
@@ -1189,9 +1269,15 @@ int launch_super_count(const BuildArgs &a, const SkArgs &s, uint64_t nb, int tab
     }
 }
 
+int launch_super_big_bounds(const SkArgs &s, uint32_t n, unsigned long long *meta, cudaStream_t st) {
+    k_sk_big_bounds<<<(n + 255) / 256, 256, 0, st>>>(s, n, meta);
+    return 1;
+}
+
 int launch_super_big(const BuildArgs &a, const SkArgs &s, const unsigned long long *meta, uint32_t n, uint64_t records,
                      Entry *table, uint64_t cap, cudaStream_t st) {
-    const uint64_t blocks = std::min<uint64_t>((records + 255) / 256, (uint64_t)device_sm_count() * 8);
+    const uint64_t blocks =
+        std::min<uint64_t>((records + kSkBigChunk - 1) / kSkBigChunk, (uint64_t)device_sm_count() * 6);
     k_sk_big<<<(unsigned)std::max<uint64_t>(blocks, 1), 256, 0, st>>>(a, s, meta, n, table, cap);
     return 1;
 }

@@ -180,6 +180,7 @@ int launch_super_scan(const BuildArgs &a, const SkArgs &sk, uint64_t bound, uint
 int launch_super_caps(const SkArgs &sk, uint64_t nb, uint64_t *scratch, cudaStream_t s);
 int launch_super_sub(const SkArgs &sk, cudaStream_t s);
 int launch_super_count(const BuildArgs &a, const SkArgs &sk, uint64_t nb, int table, cudaStream_t s);
+int launch_super_big_bounds(const SkArgs &s, uint32_t n, unsigned long long *meta, cudaStream_t st);
 int launch_super_big(const BuildArgs &a, const SkArgs &sk, const unsigned long long *meta, uint32_t n,
                      uint64_t records, Entry *table, uint64_t cap, cudaStream_t s);
 int launch_big_compact(const BuildArgs &a, const Entry *table, uint64_t cap, cudaStream_t s);

@@ -42,7 +42,7 @@ def _check(reads, k, c, **opts):
     text = _fasta(reads)
     g = swapgb.Graph().build_reads(swapgb.Opts(k=k, cutoff=c, **opts), swapgb.reads_from_fasta(text, k))
     assert g.info()["algorithm"] == swapgb.ALGO_BUCKETED
-    assert g.info()["occurrences"] >= 600_000  # smaller builds scatter single occurrences
+    assert g.info()["occurrences"] >= 600_000  # several buckets a block
     keys, mult = g.copy_out(sorted=True)
     okeys, omult = oracle.records(text, k, c)
     assert np.array_equal(keys, okeys) and np.array_equal(mult, omult)
@@ -75,6 +75,22 @@ def test_low_complexity_and_identical_reads(k):
     reads += [b"ACG" * 40 + _random(rng, 30) for _ in range(2_000)]
     g = _check(reads, k, 2)
     assert (g.copy_out()[1] == 255).any()
+
+
+@pytest.mark.parametrize("copies", [16_385, 17_408, 17_409, 60_000])
+def test_hot_buckets(copies):
+    """Buckets for the global-memory table, around a whole number of its chunks
+    of 1024 records: copies of one short read, of another with one of three
+    last bases, and of a read within a tandem repeat (equal k-molecules in one
+    record, weights past 255)."""
+    rng = np.random.default_rng(copies)
+    k = 21
+    hot = _random(rng, k + 2)
+    other = _random(rng, k + 1)
+    reads = [hot] * copies + [other[:k] + b"ACG"[i % 3:i % 3 + 1] for i in range(copies)] + [b"AC" * 30] * (copies // 10)
+    reads += _sampled(rng, _random(rng, 40_000), 8_000, [100])
+    reads = [reads[i] for i in rng.permutation(len(reads))]
+    assert _check(reads, k, 2).info()["waves"] >= 1
 
 
 def test_few_survivors_and_many():
