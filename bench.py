@@ -167,6 +167,13 @@ def traffic_per_occ(kernel: str) -> tuple[float | None, str | None]:
     return d.get("dram_bytes_per_occurrence"), d.get("source")
 
 
+def super_kmer_window(k: int, occurrences: int) -> int:
+    """Windows of m-mers in a k-mer of the super-k-mer build, 0 where the build
+    scatters single k-mers (super_window in csrc/super.cu)."""
+    m = 11 if occurrences <= 256 << 20 else 12 if occurrences <= 2048 << 20 else 13
+    return {31: 17, 29: 17, 27: 15, 25: 13 if m == 13 else 14, 23: 24 - m, 21: 22 - m, 19: 20 - m}.get(k, 0)
+
+
 def cpu_baseline(text: bytes, n_bases: int, budget_s: float = 20.0) -> dict:
     """The oracle port timed on this host's cores on a bounded prefix sample."""
     sys.path.insert(0, str(ROOT / "oracle"))
@@ -190,9 +197,9 @@ def cpu_baseline(text: bytes, n_bases: int, budget_s: float = 20.0) -> dict:
 
 
 # Random accesses per k-molecule the GPU merge makes (merge.cu): index insert
-# 1, one neighbour lookup per arc (about 2), the two neighbours' flags 2, per
-# walk state one 16-byte successor load and one label store (4), the chain
-# entry 1 and the two arc-string bases 2.
+# 1, per arc (about 2) the index slot and the key it names (4), the two
+# neighbours' flags 2, the results of its two walk states 2, the chain entry 1
+# and the two arc-string bases 2.
 MERGE_RANDOM_PER_NODE = 12
 
 
@@ -776,19 +783,27 @@ def main() -> int:
                  "written back) + 0.25 B per base + 12 B per read")
     elif used == swapgb.ALGO_BUCKETED:
         # the longer of the two single-kernel phases, each timed by events
-        # around that kernel's launch on the build stream
-        if mean_ms[1] >= mean_ms[3]:
-            kname, k_ms, kfile = "k_p1_scatter", mean_ms[1], "k_p1_scatter"
-            algo_bytes = n_bases / 4 + reads.n_reads * 12 + n_occ * 8
-            model = ("packed reads in (0.25 B per base + 12 B per read), one 8 B record per "
-                     "k-mer occurrence out")
+        # around that kernel's launch on the build stream (the counting phase
+        # includes the recount of buckets that outgrew their table)
+        w = super_kmer_window(K, n_occ)
+        packed_in = n_bases / 4 + reads.n_reads * 12
+        if w:  # odd k from 19 to 31: records of runs of k-mers that share a minimizer
+            rec_bytes = 16 * (2 * n_occ / (w + 1) + n_with_occ)
+            rec_what = ("16 B per super-k-mer record (2 / (%d + 1) of the k-mer occurrences, the density of "
+                        "minimizers of %d windows, and one per read)" % (w, w))
         else:
-            # the tier-1 configuration the build chose (2048-entry tables for
-            # small buckets); the tier-2 recount is part of the same phase
-            kname = "k_bucket_count_small" if info.get("bucket_table") == 2048 else "k_bucket_count"
-            k_ms, kfile = mean_ms[3], kname
-            algo_bytes = n_occ * 8 + survivors * 16
-            model = "one 8 B record per k-mer occurrence in, 16 B per surviving k-molecule staged"
+            rec_bytes, rec_what = 8 * n_occ, "8 B per k-mer occurrence"
+        if mean_ms[1] >= mean_ms[3]:
+            kname, k_ms = "k_sk_scan" if w else "k_p1_scatter", mean_ms[1]
+            algo_bytes = packed_in + rec_bytes
+            model = "packed reads in (0.25 B per base + 12 B per read), out " + rec_what
+        else:
+            small = info.get("bucket_table") == 2048
+            kname = "k_sk_count" if w else ("k_bucket_count_small" if small else "k_bucket_count")
+            k_ms = mean_ms[3]
+            algo_bytes = rec_bytes + survivors * 16
+            model = "in " + rec_what + "; 16 B per surviving k-molecule out"
+        kfile = kname
     else:
         # the whole partitioned build: every kernel, DRAM bytes it cannot avoid
         kname, k_ms = "partitioned build (all kernels)", mean_ms[4]
@@ -802,21 +817,6 @@ def main() -> int:
                 "unit": "GB/s", "frac": achieved / hbm, "peak_source": peak_src,
                 "traffic": (tpo * n_occ) if tpo else None, "traffic_source": tsrc,
                 "algorithmic_bytes": algo_bytes, "bytes_model": model, "kernel_ms": k_ms}
-    if kname.startswith("k_bucket_count") and not args.no_probe:
-        # the kernel's own ceiling is on chip: one 64-bit shared CAS per record
-        # (a lower bound: linear probing adds some) and one 32-bit shared add
-        # per arc, at the rates this GPU's shared-memory atomics reach
-        r_add = swapgb.probe_shared_atomics("add_u32", 1 << 31, stream.cuda_stream)
-        r_cas = swapgb.probe_shared_atomics("cas_u64", 1 << 30, stream.cuda_stream)
-        n_arcs = 2 * n_occ - 2 * n_with_occ
-        floor_ms = 1e3 * (n_occ / r_cas + n_arcs / r_add)
-        roofline["on_chip"] = {"bound": "shared-memory atomics", "floor_ms": floor_ms,
-                               "frac": floor_ms / k_ms, "cas64_lane_ops_per_s": r_cas,
-                               "add32_lane_ops_per_s": r_add, "cas_per_build": n_occ,
-                               "adds_per_build": n_arcs,
-                               "model": "one 64-bit shared atomicCAS per record + one 32-bit shared "
-                                        "atomicAdd per arc, at the rates swg_probe_shared_atomics "
-                                        "measures in the same table layout (this run)"}
     atomic = None
     if not args.no_probe and rank == 0:
         table_bytes = 16 << 30

@@ -56,7 +56,7 @@ __device__ __forceinline__ uint32_t sk_mix(uint32_t x) {  // bucket of a minimiz
 // ---- pieces of long reads: a piece's length word has bit 30 / 31 set when a
 // base precedes / follows it in its read. A thread per read left 80 blocks for
 // 20,000 reads of 3 to 15 kbp; level 1 over pieces takes 0.40 ms there (setup
-// included 0.78), the single-occurrence scatter took 5.5 (7.3).
+// included 0.53), the single-occurrence scatter took 5.5 (7.3).
 __global__ void __launch_bounds__(256) k_sk_pieces_count(BuildArgs a, uint64_t *__restrict__ n) {
     const uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= a.n_reads) return;
