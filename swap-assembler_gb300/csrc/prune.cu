@@ -109,8 +109,11 @@ __global__ void k_pr_low(MergedGraph m, const unsigned long long *sums, unsigned
 }
 
 // ---- rewrite of the text
-__global__ void k_pr_len(MergedGraph m, uint64_t *__restrict__ out, unsigned long long *printed) {
+// (count: what the pass before counted, put beside what the host reads next)
+__global__ void k_pr_len(MergedGraph m, uint64_t *__restrict__ out, unsigned long long *printed,
+                         const unsigned long long *__restrict__ count) {
     const uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (q == 0 && count) printed[1] = *count;
     if (q >= m.lines) return;
     uint64_t sum = 0;
     if (!m.del[q])
@@ -166,7 +169,7 @@ __global__ void __launch_bounds__(256) k_pr_write(MergedGraph m, const uint64_t 
 // merge lengthened it) or, after a merge, a merged node's arc string placed
 // inside an end's new arc. 50,000 pieces, 1 MB: first parts of 4 KiB by a warp,
 // a byte a lane at a time, took 29 to 62 us, parts' counts scanned and searched
-// 13 to 27; now 17 to 26 and 8.
+// 13 to 27; now 14 and 8.
 constexpr unsigned kPart = 1024;   // bytes of a piece moved at a time
 constexpr unsigned kChunk = 4096;  // of a contig
 constexpr int kBytes = 16;         // a lane's under way
@@ -218,44 +221,24 @@ __device__ __forceinline__ unsigned piece(const MergedGraph &m, const Pieces &x,
     return l;
 }
 
-// A warp's lanes look at 32 pieces; its four groups of eight lanes move the
-// nonempty ones' first parts, and the warp lists the other parts of the long
-// ones (piece << 24 | part; a part's number is below 2^22), counted in *listed.
+// Eight lanes a piece: they move its first part, and list the other parts of a
+// long one (piece << 24 | part; a part's number is below 2^22), counted in
+// *listed. (A warp that looked at 32 pieces and moved four at a time waited for
+// eight rounds of loads: 17 to 26 us for 50,000 pieces, 14 now.)
 __global__ void __launch_bounds__(256) k_pr_short(MergedGraph m, Pieces x, const char *__restrict__ from,
                                                   char *__restrict__ to, unsigned long long *__restrict__ parts,
                                                   unsigned long long *__restrict__ listed) {
     const uint64_t pieces = 8 * m.lines + x.n;
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const unsigned lane = threadIdx.x & 31;
+    const uint64_t i = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+    const unsigned lane = threadIdx.x & 7;
     uint64_t src = 0, dst = 0;
-    unsigned len = 0, more = 0;
-    if (i < pieces) {
-        len = piece(m, x, i, src, dst);
-        more = len ? (len - 1) / kPart : 0;
-        len = len < kPart ? len : kPart;
-    }
-    for (unsigned todo = __ballot_sync(0xffffffffu, more != 0); todo; todo &= todo - 1) {
-        const int o = __ffs(todo) - 1;
-        const unsigned count = __shfl_sync(0xffffffffu, more, o);
-        unsigned long long at = 0;
-        if (lane == 0) at = atomicAdd(listed, (unsigned long long)count);
-        at = __shfl_sync(0xffffffffu, at, 0);
-        const unsigned long long id = (i - lane + o) << 24;
-        for (unsigned c = lane; c < count; c += 32) parts[at + c] = id | (c + 1);
-    }
-    for (unsigned todo = __ballot_sync(0xffffffffu, len != 0); todo;) {
-        int o = -1;
-#pragma unroll
-        for (unsigned g = 0; g < 4; ++g) {  // the next four pieces, one a group
-            if (g == lane >> 3) o = __ffs(todo) - 1;
-            todo &= todo - 1;
-        }
-        const char *a = from + __shfl_sync(0xffffffffu, src, o & 31);
-        char *b = to + __shfl_sync(0xffffffffu, dst, o & 31);
-        const unsigned l = __shfl_sync(0xffffffffu, len, o & 31);
-        if (o >= 0) move_bytes(b, a, l, lane & 7, 8);
-        __syncwarp();
-    }
+    const unsigned len = i < pieces ? piece(m, x, i, src, dst) : 0;
+    const unsigned more = len ? (len - 1) / kPart : 0;
+    unsigned long long at = 0;
+    if (lane == 0 && more) at = atomicAdd(listed, (unsigned long long)more);
+    at = __shfl_sync(0xffffffffu, at, 0, 8);
+    for (unsigned c = lane; c < more; c += 8) parts[at + c] = i << 24 | (c + 1);
+    if (len) move_bytes(to + dst, from + src, len < kPart ? len : kPart, lane, 8);
 }
 
 // The listed parts, a warp each; their number is read on the device.
@@ -275,20 +258,22 @@ __global__ void __launch_bounds__(256) k_pr_long(MergedGraph m, Pieces x, const 
 inline unsigned blocks(uint64_t n) { return (unsigned)std::max<uint64_t>((n + 255) / 256, 1); }
 
 // Writes the lines into the spare text, then swaps it in.
-swg_status rewrite(MergedGraph *m, cudaStream_t s, Scratch &scr, const Pieces &x = Pieces{}) {
+swg_status rewrite(MergedGraph *m, cudaStream_t s, Scratch &scr, const Pieces &x = Pieces{},
+                   const unsigned long long *d_count = nullptr, uint64_t *count = nullptr) {
     uint64_t *len = nullptr, *off = nullptr;
     unsigned long long *printed = nullptr;
-    if (!scr.get(&len, m->lines) || !scr.get(&off, m->lines + 3))
+    if (!scr.get(&len, m->lines) || !scr.get(&off, m->lines + 4))
         return cuda_err(cudaErrorMemoryAllocation, "rewrite workspace");
-    // (the count of printed lines is read together with the text's size; the listed parts' comes after it)
+    // read together with the text's size: printed lines, the pass's count; the listed parts' comes after them
     printed = reinterpret_cast<unsigned long long *>(off + m->lines + 1);
-    EMIT_CUDA(cudaMemsetAsync(printed, 0, 16, s), "rewrite");
-    if (m->lines) k_pr_len<<<blocks(m->lines), 256, 0, s>>>(*m, len, printed);
+    EMIT_CUDA(cudaMemsetAsync(printed, 0, 24, s), "rewrite");
+    if (m->lines) k_pr_len<<<blocks(m->lines), 256, 0, s>>>(*m, len, printed, d_count);
     swg_status st = scan_lengths(len, off, m->lines, scr, s);
     if (st) return st;
-    uint64_t h[2] = {0, 0};
-    EMIT_CUDA(cudaMemcpyAsync(h, off + m->lines, 16, cudaMemcpyDeviceToHost, s), "text size");
+    uint64_t h[3] = {0, 0, 0};
+    EMIT_CUDA(cudaMemcpyAsync(h, off + m->lines, 24, cudaMemcpyDeviceToHost, s), "text size");
     EMIT_CUDA(cudaStreamSynchronize(s), "text size");
+    if (count) *count = h[2];
     const uint64_t bytes = h[0] + 1;
     if (bytes > m->text2_cap) {
         cudaFree(m->text2);
@@ -303,9 +288,9 @@ swg_status rewrite(MergedGraph *m, cudaStream_t s, Scratch &scr, const Pieces &x
         unsigned long long *parts = nullptr;
         if (!scr.get(&parts, most)) return cuda_err(cudaErrorMemoryAllocation, "rewrite workspace");
         k_pr_write<<<blocks(8 * m->lines), 256, 0, s>>>(*m, off, m->text2);
-        k_pr_short<<<blocks(pieces), 256, 0, s>>>(*m, x, m->text, m->text2, parts, printed + 1);
+        k_pr_short<<<blocks(8 * pieces), 256, 0, s>>>(*m, x, m->text, m->text2, parts, printed + 2);
         if (most)
-            k_pr_long<<<(unsigned)std::min<uint64_t>((most + 7) / 8, 4096), 256, 0, s>>>(*m, x, parts, printed + 1,
+            k_pr_long<<<(unsigned)std::min<uint64_t>((most + 7) / 8, 4096), 256, 0, s>>>(*m, x, parts, printed + 2,
                                                                                         m->text, m->text2);
     }
     EMIT_CUDA(cudaMemsetAsync(m->text2 + h[0], '\n', 1, s), "merged text");
@@ -672,8 +657,7 @@ swg_status prune_tips(MergedGraph *m, cudaStream_t s, uint64_t *count) {
         k_pr_tipslot<<<blocks(m->lines), 256, 0, s>>>(*m, tip);
         k_pr_tips<<<blocks(m->lines), 256, 0, s>>>(*m, tip, ctr);
     }
-    EMIT_CUDA(cudaMemcpyAsync(count, ctr, 8, cudaMemcpyDeviceToHost, s), "tips");
-    return rewrite(m, s, scr);
+    return rewrite(m, s, scr, Pieces{}, ctr, count);
 }
 
 swg_status simplify_lines(MergedGraph *m, cudaStream_t s, uint64_t *count) {
@@ -805,8 +789,7 @@ swg_status prune_low_coverage(MergedGraph *m, cudaStream_t s, uint64_t *count) {
         k_pr_cov<<<blocks(m->lines), 256, 0, s>>>(*m, ctr);
         k_pr_low<<<blocks(m->lines), 256, 0, s>>>(*m, ctr, ctr + 2);
     }
-    EMIT_CUDA(cudaMemcpyAsync(count, ctr + 2, 8, cudaMemcpyDeviceToHost, s), "low coverage");
-    return rewrite(m, s, scr);
+    return rewrite(m, s, scr, Pieces{}, ctr + 2, count);
 }
 
 }  // namespace swg
