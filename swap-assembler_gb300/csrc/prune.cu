@@ -356,50 +356,83 @@ __device__ __forceinline__ unsigned long long agg_add_labeled(unsigned long long
     return g.shfl(base, 0) + step * g.thread_rank();
 }
 
-__global__ void k_sm_classify(SimplifyArgs a) {
-    const uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= a.m.lines) return;
-    int rc = 0, lc = 0, rs = 0, ls = 4;
-    if (!a.m.del[q])
-        for (int s = 0; s < 8; ++s)
-            if (a.m.len[8 * q + s]) {
-                if (s < 4) ++rc, rs = s;
-                else ++lc, ls = s;
-            }
-    const bool merged = rc == 1 && lc == 1 && (a.m.back[8 * q + rs] >> 3) != q && (a.m.back[8 * q + ls] >> 3) != q;
-    a.fl[q] = (unsigned char)((merged ? 1 : 0) | (rs << 1) | ((ls - 4) << 3));
-    if (merged) agg_inc(&a.ctr[0]);
+__device__ __forceinline__ bool sm_arc_less(const SimplifyArgs &a, uint64_t x, uint64_t y) {
+    const unsigned long long kx = a.m.key[x >> 3], ky = a.m.key[y >> 3];
+    return kx < ky || (kx == ky && (x & 7) < (y & 7));
 }
 
-// Walk state 2q+d leaves line q by its right (d = 0) or left (d = 1) arc; the
-// next line is entered by the slot the back link names: entered from the
-// left (slot >= 4), it is traversed leaving by its right arc.
-__global__ void k_sm_init(SimplifyArgs a) {
-    const uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= a.m.lines || !sm_m(a, q)) return;
-    const unsigned char f = a.fl[q];
-    for (int d = 0; d < 2; ++d) {
-        const int slot = d ? sm_ls(f) : sm_rs(f);
-        const unsigned b = a.m.back[8 * q + slot];
-        const uint64_t far = b >> 3;
-        const uint64_t st = 2 * q + d;
-        a.nx[0][st] = sm_m(a, far) ? 2 * far + ((b & 7) >= 4 ? 0 : 1) : (kTerm | b);
-        a.cn[0][st] = 1;
-        a.ws[0][st] = a.m.len[8 * q + slot];
-        a.mx[0][st] = a.m.key[q];
+struct SmPos {
+    unsigned m, pos;
+    uint64_t alpha, beta;  // end arcs reached going back / forward
+    bool fwd;              // the chain runs through the node leaving by its right arc
+};
+
+__device__ __forceinline__ SmPos sm_pos(const SimplifyArgs &a, int in, uint64_t q) {
+    SmPos c;
+    const unsigned la = __ldcg(a.cn[in] + 2 * q), lb = __ldcg(a.cn[in] + 2 * q + 1);
+    c.beta = __ldcg(a.nx[in] + 2 * q) & ~kTerm;
+    c.alpha = __ldcg(a.nx[in] + 2 * q + 1) & ~kTerm;
+    c.m = la + lb - 1;
+    c.fwd = sm_arc_less(a, c.alpha, c.beta);
+    c.pos = c.fwd ? lb : la;
+    return c;
+}
+
+__device__ __forceinline__ int sm_class(unsigned m) { return m == 0 ? 0 : 64 - __clzll((unsigned long long)m); }
+
+// Lines merged away, their walk states ranked by pointer jumping, cycles and
+// chains counted: all in one cooperative launch, since each step is a few
+// microseconds over a few thousand lines and a grid barrier costs less than a
+// launch (one block of 1024 an SM at most: a barrier's time grows with them).
+//  - A line with one arc on each side that does not lead back to it is merged.
+//  - Walk state 2q+d leaves line q by its right (d = 0) or left (d = 1) arc; the
+//    next line is entered by the slot the back link names: entered from the
+//    left (slot >= 4), it is traversed leaving by its right arc.
+//  - Jumping rounds go in pairs, so that the result is in the first buffers
+//    again, until every state has reached an end (those of a cycle never do).
+//  - Lines still in a cycle then (ctr[3]): the cycle's largest key ends it, and
+//    the host launches this again (first = 0); the chains are counted anew.
+// 6,300 lines: the five kernels 37 and 55 us (after tips, after low coverage),
+// this 26 and 42.
+__global__ void __launch_bounds__(1024) k_sm_rank(SimplifyArgs a, int pairs, unsigned *moved, int first) {
+    const uint64_t lines = a.m.lines, states = 2 * lines, stride = (uint64_t)gridDim.x * blockDim.x;
+    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (first) {
+        for (uint64_t q = t; q < lines; q += stride) {
+            int rc = 0, lc = 0, rs = 0, ls = 4;
+            if (!a.m.del[q])
+                for (int s = 0; s < 8; ++s)
+                    if (a.m.len[8 * q + s]) {
+                        if (s < 4) ++rc, rs = s;
+                        else ++lc, ls = s;
+                    }
+            const bool merged =
+                rc == 1 && lc == 1 && (a.m.back[8 * q + rs] >> 3) != q && (a.m.back[8 * q + ls] >> 3) != q;
+            a.fl[q] = (unsigned char)((merged ? 1 : 0) | (rs << 1) | ((ls - 4) << 3));
+            if (merged) agg_inc(&a.ctr[0]);
+        }
+        cg::this_grid().sync();
     }
-}
-
-// Pointer jumping, all rounds in one cooperative launch (as the merge's ruler
-// list): rounds in pairs, so that the result is in the first buffers again,
-// until every state has reached an end (those of a cycle never do).
-__global__ void __launch_bounds__(256) k_sm_jump(SimplifyArgs a, int pairs, unsigned *moved) {
-    const uint64_t states = 2 * a.m.lines, stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t q = t; q < lines; q += stride) {
+        if (!sm_m(a, q)) continue;
+        const unsigned char f = a.fl[q];
+        for (int d = 0; d < 2; ++d) {
+            const int slot = d ? sm_ls(f) : sm_rs(f);
+            const unsigned b = a.m.back[8 * q + slot];
+            const uint64_t far = b >> 3;
+            const uint64_t st = 2 * q + d;
+            a.nx[0][st] = sm_m(a, far) ? 2 * far + ((b & 7) >= 4 ? 0 : 1) : (kTerm | b);
+            a.cn[0][st] = 1;
+            a.ws[0][st] = a.m.len[8 * q + slot];
+            a.mx[0][st] = a.m.key[q];
+        }
+    }
+    cg::this_grid().sync();
     for (int r = 0; r < pairs; ++r) {
         for (int in = 0; in < 2; ++in) {
             const int out = in ^ 1;
             bool left = false;
-            for (uint64_t st = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; st < states; st += stride) {
+            for (uint64_t st = t; st < states; st += stride) {
                 if (!sm_m(a, st >> 1)) continue;
                 unsigned long long nx = __ldcg(a.nx[in] + st), ws = __ldcg(a.ws[in] + st), mx = __ldcg(a.mx[in] + st);
                 unsigned cn = __ldcg(a.cn[in] + st);
@@ -420,50 +453,22 @@ __global__ void __launch_bounds__(256) k_sm_jump(SimplifyArgs a, int pairs, unsi
             if (in && left) moved[r] = 1;
             cg::this_grid().sync();
         }
-        if (!*(volatile unsigned *)(moved + r)) return;
+        if (!*(volatile unsigned *)(moved + r)) break;
     }
-}
-
-// States still in a cycle after the jumps: the cycle's largest key ends it.
-__global__ void k_sm_cut(SimplifyArgs a, int in) {
-    const uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= a.m.lines || !sm_m(a, q) || (a.nx[in][2 * q] & kTerm)) return;
-    agg_inc(&a.ctr[3]);
-    if (a.m.key[q] == a.mx[in][2 * q]) {
-        a.fl[q] &= (unsigned char)~1u;
-        agg_inc(&a.ctr[1]);
+    for (uint64_t q = t; q < lines; q += stride) {
+        if (!sm_m(a, q)) continue;
+        if (!(__ldcg(a.nx[0] + 2 * q) & kTerm)) {
+            if (!first) continue;
+            agg_inc(&a.ctr[3]);
+            if (a.m.key[q] == __ldcg(a.mx[0] + 2 * q)) {
+                a.fl[q] &= (unsigned char)~1u;
+                agg_inc(&a.ctr[1]);
+            }
+            continue;
+        }
+        const SmPos c = sm_pos(a, 0, q);
+        if (c.pos == 1) agg_add_labeled(a.cls_count, sm_class(c.m), 1);
     }
-}
-
-__device__ __forceinline__ bool sm_arc_less(const SimplifyArgs &a, uint64_t x, uint64_t y) {
-    const unsigned long long kx = a.m.key[x >> 3], ky = a.m.key[y >> 3];
-    return kx < ky || (kx == ky && (x & 7) < (y & 7));
-}
-
-struct SmPos {
-    unsigned m, pos;
-    uint64_t alpha, beta;  // end arcs reached going back / forward
-    bool fwd;              // the chain runs through the node leaving by its right arc
-};
-
-__device__ __forceinline__ SmPos sm_pos(const SimplifyArgs &a, int in, uint64_t q) {
-    SmPos c;
-    const unsigned la = a.cn[in][2 * q], lb = a.cn[in][2 * q + 1];
-    c.beta = a.nx[in][2 * q] & ~kTerm;
-    c.alpha = a.nx[in][2 * q + 1] & ~kTerm;
-    c.m = la + lb - 1;
-    c.fwd = sm_arc_less(a, c.alpha, c.beta);
-    c.pos = c.fwd ? lb : la;
-    return c;
-}
-
-__device__ __forceinline__ int sm_class(unsigned m) { return m == 0 ? 0 : 64 - __clzll((unsigned long long)m); }
-
-__global__ void k_sm_chain_count(SimplifyArgs a, int in) {
-    const uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= a.m.lines || !sm_m(a, q)) return;
-    const SmPos c = sm_pos(a, in, q);
-    if (c.pos == 1) agg_add_labeled(a.cls_count, sm_class(c.m), 1);
 }
 
 __global__ void k_sm_chain_alloc(SimplifyArgs a, int in) {
@@ -545,6 +550,7 @@ __global__ void __launch_bounds__(256) k_sm_levels(SimplifyArgs a, uint64_t tota
 __global__ void k_sm_apply(SimplifyArgs a, int in) {
     const uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= a.m.lines || !sm_m(a, q)) return;
+    a.m.del[q] = 1;
     const SmPos c = sm_pos(a, in, q);
     const uint64_t start = c.fwd ? c.alpha : c.beta, end = c.fwd ? c.beta : c.alpha;
     const unsigned id = a.chain_of[start];
@@ -574,12 +580,6 @@ __global__ void k_sm_apply(SimplifyArgs a, int in) {
             a.m.back[end] = (unsigned)start;
         }
     }
-}
-
-__global__ void k_sm_delete(SimplifyArgs a) {
-    const uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= a.m.lines || !sm_m(a, q)) return;
-    a.m.del[q] = 1;
 }
 
 int sm_ceil_log2(uint64_t v) {
@@ -682,31 +682,20 @@ swg_status simplify_lines(MergedGraph *m, cudaStream_t s, uint64_t *count) {
     int pairs = (sm_ceil_log2(2 * L) + 2) / 2;
     unsigned *moved = nullptr;
     if (!scr.get(&moved, 64)) return cuda_err(cudaErrorMemoryAllocation, "simplify workspace");
-    int sms = 0, per_sm = 0, dev = 0;
+    int sms = 0, dev = 0;
     EMIT_CUDA(cudaGetDevice(&dev), "device");
     EMIT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "device attribute");
-    EMIT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sm_jump, 256, 0), "occupancy");
-    const unsigned jgrid = (unsigned)std::min<uint64_t>((uint64_t)std::max(1, std::min(per_sm, 4) * sms), blocks(2 * L));
+    const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)std::max(1, sms), (2 * L + 1023) / 1024);
     unsigned long long h[8 + kCls] = {0};
     const int in = 0;  // the jumps leave their result in the first buffers
-    k_sm_classify<<<blocks(L), 256, 0, s>>>(a);
-    for (int attempt = 0; attempt < 2; ++attempt) {  // again after cutting cycles
-        k_sm_init<<<blocks(L), 256, 0, s>>>(a);
+    for (int first = 1; first >= 0; --first) {  // again after cutting cycles
         EMIT_CUDA(cudaMemsetAsync(moved, 0, 64 * sizeof(unsigned), s), "simplify");
-        void *args[] = {&a, &pairs, &moved};
-        EMIT_CUDA(cudaLaunchCooperativeKernel((const void *)k_sm_jump, dim3(jgrid), dim3(256), args, 0, s), "simplify");
-        if (attempt == 1) break;
-        k_sm_cut<<<blocks(L), 256, 0, s>>>(a, in);
-        k_sm_chain_count<<<blocks(L), 256, 0, s>>>(a, in);  // (of no use if there are cycles: counted again below)
+        if (!first) EMIT_CUDA(cudaMemsetAsync(a.cls_count, 0, kCls * 8, s), "simplify");
+        void *args[] = {&a, &pairs, &moved, &first};
+        EMIT_CUDA(cudaLaunchCooperativeKernel((const void *)k_sm_rank, dim3(grid), dim3(1024), args, 0, s), "simplify");
         EMIT_CUDA(cudaMemcpyAsync(h, a.ctr, sizeof(h), cudaMemcpyDeviceToHost, s), "simplify");
         EMIT_CUDA(cudaStreamSynchronize(s), "simplify");
         if (!h[3]) break;
-    }
-    if (h[3]) {
-        EMIT_CUDA(cudaMemsetAsync(a.cls_count, 0, kCls * 8, s), "simplify");
-        k_sm_chain_count<<<blocks(L), 256, 0, s>>>(a, in);
-        EMIT_CUDA(cudaMemcpyAsync(h, a.ctr, sizeof(h), cudaMemcpyDeviceToHost, s), "simplify");
-        EMIT_CUDA(cudaStreamSynchronize(s), "simplify");
     }
     const unsigned long long *cls = h + 8;
     unsigned long long cursor[kCls];
@@ -731,7 +720,6 @@ swg_status simplify_lines(MergedGraph *m, cudaStream_t s, uint64_t *count) {
         k_sm_levels<<<(unsigned)((total + per - 1) / per), 256, 0, s>>>(a, total, t, top);
     }
     k_sm_apply<<<blocks(L), 256, 0, s>>>(a, in);
-    k_sm_delete<<<blocks(L), 256, 0, s>>>(a);
     EMIT_CUDA(cudaGetLastError(), "simplify kernels");
     *count = h[0] - h[1];
     Pieces x;
