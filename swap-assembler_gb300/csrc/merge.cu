@@ -400,6 +400,49 @@ __global__ void __launch_bounds__(1024) k_mg_rank(MergeArgs a, int pairs) {
     }
 }
 
+// ---- chains
+// End arcs compare by (key of the end node, slot). Only end nodes' keys are
+// read here: a small, cache-resident set.
+__device__ __forceinline__ bool arc_less(const MergeArgs &a, uint64_t x, uint64_t y) {
+    const unsigned long long kx = a.keys[x >> 3], ky = a.keys[y >> 3];
+    return kx < ky || (kx == ky && (x & 7) < (y & 7));
+}
+
+struct ChainPos {
+    unsigned m, pos;
+    uint64_t start;  // the smaller end arc code: the chain's start
+    bool fwd;        // the chain runs through this node as its key (state 2i)
+};
+
+__device__ __forceinline__ ChainPos chain_pos_of(const MergeArgs &a, uint4 lt) {
+    ChainPos c;
+    const unsigned la = lt.x, lb = lt.z;
+    const uint64_t beta = lt.y, alpha = lt.w;
+    c.m = la + lb - 1;
+    c.fwd = arc_less(a, alpha, beta);
+    c.pos = c.fwd ? lb : la;
+    c.start = c.fwd ? alpha : beta;
+    return c;
+}
+
+__device__ __forceinline__ ChainPos chain_pos(const MergeArgs &a, uint64_t i) {
+    return chain_pos_of(a, *reinterpret_cast<const uint4 *>(a.lt + 2 * i));
+}
+
+__device__ __forceinline__ int size_class(unsigned m) {  // ceil(log2(m + 1))
+    return m == 0 ? 0 : 64 - __clzll((unsigned long long)m);
+}
+
+// A chain's first node counts it by size and lists itself.
+__device__ __forceinline__ void count_chain(const MergeArgs &a, uint64_t i, const ChainPos &c) {
+    if (c.pos != 1) return;
+    agg_add_labeled(a.cls_count, size_class(c.m), 1);
+    a.heads[agg_inc(&a.ctr[2])] = (unsigned)i;  // (the poles' list is done with)
+}
+
+// Per state the distance to its walk's end and the end arc, and the chains
+// counted while both are at hand (again by k_mg_chain_count once cycles are
+// cut; their states, at 0, are no chain's). 5M nodes: 40 us, two kernels took 62.
 __global__ void k_mg_finish(MergeArgs a) {
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.n || !is_m(a, i)) return;
@@ -414,7 +457,9 @@ __global__ void k_mg_finish(MergeArgs a) {
         lt[d] = ends ? make_uint2((v.y & ~kEnd) - (unsigned)o, v.x) : make_uint2(0, 0);
         if (!ends) a.clist[agg_inc(&a.ctr[1])] = (unsigned)(2 * i + d);
     }
-    *reinterpret_cast<uint4 *>(a.lt + 2 * i) = make_uint4(lt[0].x, lt[0].y, lt[1].x, lt[1].y);
+    const uint4 both = make_uint4(lt[0].x, lt[0].y, lt[1].x, lt[1].y);
+    *reinterpret_cast<uint4 *>(a.lt + 2 * i) = both;
+    count_chain(a, i, chain_pos_of(a, both));
 }
 
 // ---- cycles of merged nodes: largest key by pointer jumping, cut there
@@ -489,43 +534,10 @@ __global__ void k_mg_cyc_done(MergeArgs a, uint64_t c, const unsigned long long 
     a.lt[st] = make_uint2((unsigned)ln[st], (unsigned)nx[st]);
 }
 
-// ---- chains
-// End arcs compare by (key of the end node, slot). Only end nodes' keys are
-// read here: a small, cache-resident set.
-__device__ __forceinline__ bool arc_less(const MergeArgs &a, uint64_t x, uint64_t y) {
-    const unsigned long long kx = a.keys[x >> 3], ky = a.keys[y >> 3];
-    return kx < ky || (kx == ky && (x & 7) < (y & 7));
-}
-
-struct ChainPos {
-    unsigned m, pos;
-    uint64_t start;  // the smaller end arc code: the chain's start
-    bool fwd;        // the chain runs through this node as its key (state 2i)
-};
-
-__device__ __forceinline__ ChainPos chain_pos(const MergeArgs &a, uint64_t i) {
-    ChainPos c;
-    const uint4 lt = *reinterpret_cast<const uint4 *>(a.lt + 2 * i);
-    const unsigned la = lt.x, lb = lt.z;
-    const uint64_t beta = lt.y, alpha = lt.w;
-    c.m = la + lb - 1;
-    c.fwd = arc_less(a, alpha, beta);
-    c.pos = c.fwd ? lb : la;
-    c.start = c.fwd ? alpha : beta;
-    return c;
-}
-
-__device__ __forceinline__ int size_class(unsigned m) {  // ceil(log2(m + 1))
-    return m == 0 ? 0 : 64 - __clzll((unsigned long long)m);
-}
-
 __global__ void k_mg_chain_count(MergeArgs a) {
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.n || !is_m(a, i)) return;
-    const ChainPos c = chain_pos(a, i);
-    if (c.pos != 1) return;
-    agg_add_labeled(a.cls_count, size_class(c.m), 1);
-    a.heads[agg_inc(&a.ctr[2])] = (unsigned)i;  // (the poles' list is done with)
+    count_chain(a, i, chain_pos(a, i));
 }
 
 __global__ void k_mg_chain_alloc(MergeArgs a, uint64_t n_chains) {
@@ -544,7 +556,13 @@ __global__ void k_mg_chain_alloc(MergeArgs a, uint64_t n_chains) {
 // also the arc it enters by.
 __global__ void k_mg_entries(MergeArgs a) {
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.n || !is_m(a, i)) return;
+    if (i >= a.n) return;
+    if (!is_m(a, i)) {  // a node left: listed for the key-order sort
+        const unsigned long long q = agg_inc(&a.ctr[5]);
+        a.skey[q] = a.keys[i];
+        a.sidx[q] = i;
+        return;
+    }
     const ChainPos c = chain_pos(a, i);
     const unsigned id = a.chain_of[c.start];
     const uint64_t e = a.ch_eoff[id];
@@ -672,19 +690,11 @@ __device__ __forceinline__ uint64_t first_state(unsigned v) {
     return 2 * (uint64_t)(v >> 1) + ((v & 1u) ? 0 : 1);
 }
 
-// The nodes left (not merged away), listed for the key-order sort.
-__global__ void k_mg_survivors(MergeArgs a) {
-    const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= a.n || is_m(a, j)) return;
-    const unsigned long long q = agg_inc(&a.ctr[5]);
-    a.skey[q] = a.keys[j];
-    a.sidx[q] = j;
-}
-
 // (eight lanes a line, one per arc slot: a line's arcs are chains of dependent
 // loads, and few lines are left of a graph; unordered: nothing to read yet)
 __global__ void k_mg_line_len(MergeArgs a, const unsigned long long *__restrict__ order, uint64_t n_lines,
-                              uint64_t *__restrict__ out, const unsigned *__restrict__ unordered) {
+                              uint64_t *__restrict__ out, const unsigned *__restrict__ unordered,
+                              unsigned *__restrict__ pos_of) {
     if (unordered && *unordered) return;
     const uint64_t q = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
     const int s = threadIdx.x & 7;
@@ -698,13 +708,10 @@ __global__ void k_mg_line_len(MergeArgs a, const unsigned long long *__restrict_
     }
 #pragma unroll
     for (int d = 4; d; d >>= 1) l += __shfl_xor_sync(0xffffffffu, l, d);
-    if (q < n_lines && s == 0) out[q] = 69 + l;
-}
-
-// Line position of every node left.
-__global__ void k_mg_pos(const unsigned long long *__restrict__ order, uint64_t n_lines, unsigned *__restrict__ pos_of) {
-    const uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q < n_lines) pos_of[order[q]] = (unsigned)q;
+    if (q < n_lines && s == 0) {
+        out[q] = 69 + l;
+        pos_of[order[q]] = (unsigned)q;  // the line's position, for the arcs back
+    }
 }
 
 // Eight lanes a line: lane s writes arc s's place, its multiplicity and an
@@ -932,8 +939,7 @@ swg_status merge_graph(const unsigned long long *d_keys, const unsigned long lon
         EMIT_CUDA(cudaLaunchCooperativeKernel((const void *)k_mg_rank, dim3(grid), dim3(1024), args, 0, s), "ruler list");
     }
     k_mg_finish<<<blocks(n), 256, 0, s>>>(a);
-    k_mg_chain_count<<<blocks(n), 256, 0, s>>>(a);  // (a cycle's states, at 0, are no chain's: counted again below)
-    launches += 3;
+    launches += 2;
     unsigned long long h[8 + kClasses];
     EMIT_CUDA(cudaMemcpyAsync(h, ctr, sizeof(h), cudaMemcpyDeviceToHost, s), "merge counts");
     EMIT_CUDA(cudaStreamSynchronize(s), "merge counts");
@@ -984,9 +990,11 @@ swg_status merge_graph(const unsigned long long *d_keys, const unsigned long lon
         n_chains += cls[c];
         if (cls[c] && !top) top = c;
     }
+    const uint64_t n_lines = n - h[4] + h[3];  // nodes left
     EMIT_CUDA(cudaMemcpyAsync(a.cls_cursor, cursor, sizeof(cursor), cudaMemcpyHostToDevice, s), "chain layout");
     if (!scr.get(&a.ch_eoff, n_chains) || !scr.get(&a.ch_m, n_chains) || !scr.get(&a.ch_dfwd, n_chains) ||
-        !scr.get(&a.ch_drev, n_chains) || !scr.get(&a.ent, total) || !scr.get(&a.ent_chain, total))
+        !scr.get(&a.ch_drev, n_chains) || !scr.get(&a.ent, total) || !scr.get(&a.ent_chain, total) ||
+        !scr.get(&a.skey, n_lines) || !scr.get(&a.sidx, n_lines))
         return cuda_err(cudaErrorMemoryAllocation, "chain workspace");
     EMIT_CUDA(cudaMemsetAsync(a.ent_chain, 0xff, std::max<uint64_t>(total, 1) * sizeof(unsigned), s), "chain clear");
     if (a.vt && !scr.get(&a.cart, total)) return cuda_err(cudaErrorMemoryAllocation, "merge tree");
@@ -1004,13 +1012,11 @@ swg_status merge_graph(const unsigned long long *d_keys, const unsigned long lon
         }
     }
     // the nodes left, in key order
-    const uint64_t n_lines = n - h[4] + h[3];
     unsigned long long *skey2 = nullptr, *sidx2 = nullptr;
     uint64_t *lens = nullptr, *loff = nullptr;
-    if (!scr.get(&a.skey, n_lines) || !scr.get(&a.sidx, n_lines) || !scr.get(&lens, n_lines) || !scr.get(&loff, n_lines + 1))
+    unsigned *pos_of = nullptr;
+    if (!scr.get(&lens, n_lines) || !scr.get(&loff, n_lines + 1) || !scr.get(&pos_of, n))
         return cuda_err(cudaErrorMemoryAllocation, "line workspace");
-    k_mg_survivors<<<blocks(n), 256, 0, s>>>(a);
-    ++launches;
     uint64_t bytes = 0;
     // by splitters (three launches, 37 us for 6,000 lines; the library's passes
     // took eight and 61), or by the library's passes if there are more lines
@@ -1036,7 +1042,7 @@ swg_status merge_graph(const unsigned long long *d_keys, const unsigned long lon
         }
         if (over) EMIT_CUDA(cudaMemcpyAsync(&unordered, over, sizeof(unsigned), cudaMemcpyDeviceToHost, s), "sort status");
         if (n_lines) {
-            k_mg_line_len<<<blocks(8 * n_lines), 256, 0, s>>>(a, sidx2, n_lines, lens, over);
+            k_mg_line_len<<<blocks(8 * n_lines), 256, 0, s>>>(a, sidx2, n_lines, lens, over, pos_of);
             ++launches;
         }
         swg_status st = scan_lengths(lens, loff, n_lines, scr, s);
@@ -1049,14 +1055,11 @@ swg_status merge_graph(const unsigned long long *d_keys, const unsigned long lon
     if (gst) return gst;
     mg->k = k;
     mg->lines = n_lines;
-    unsigned *pos_of = nullptr;
-    if (!scr.get(&pos_of, n)) return cuda_err(cudaErrorMemoryAllocation, "line positions");
     if (n_lines) {
-        k_mg_pos<<<blocks(n_lines), 256, 0, s>>>(sidx2, n_lines, pos_of);
         k_mg_line_write<<<blocks(8 * n_lines), 256, 0, s>>>(a, sidx2, n_lines, loff, mg->text, pos_of, *mg);
     }
     k_mg_chars<<<blocks(n), 256, 0, s>>>(a, mg->text);
-    launches += 3;
+    launches += 2;
     EMIT_CUDA(cudaMemsetAsync(mg->text + bytes, '\n', 1, s), "merged text");
     EMIT_CUDA(cudaGetLastError(), "merge kernels");
     EMIT_CUDA(cudaMemcpyAsync(&herr, a.err, sizeof(unsigned), cudaMemcpyDeviceToHost, s), "merge status");
