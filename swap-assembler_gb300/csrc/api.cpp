@@ -1247,6 +1247,10 @@ swg_status super_plan(swg_graph *g, const swg_opts *o, const BuildArgs &a, uint6
     // buckets 17.5 ms, 524,288 16.7, in 1,048,576 and the small tables 17.4, but
     // the scan's and the preparation's share grows with them.)
     bucket_bits(o, N, 3072.0, b1, b2);
+    // up to 1024 buckets: the scan scatters to them and there is no second
+    // level (builds of 0.5M, 1.4M and 2.5M occurrences: 133 -> 129 us,
+    // 148 -> 144, 156 -> 147)
+    if (b1 + b2 <= swg::kPartBitsMax) b1 += b2, b2 = 0;
     const uint64_t P = 1ull << b1, NB = P << b2;
     const double scale_max = 2.0 * stride / share;
     // a random sequence has 2 / (w + 1) runs per k-mer and one more per read
@@ -1257,7 +1261,7 @@ swg_status super_plan(swg_graph *g, const swg_opts *o, const BuildArgs &a, uint6
     const uint64_t rec1 = rec_cap + rec_cap / 4 + rec_cap / 1000 + 1025 * P, rec2 = swg::super_bucket_room(rec_cap, NB, scale_max);
     if ((st = ensure(&g->d_part, &g->part_cap, 4 * P + 1, "partition table"))) return st;
     if ((st = ensure(&g->d_records, &g->records_cap, 2 * rec1, "records"))) return st;
-    if ((st = ensure(&g->d_rec2, &g->rec2_cap, 2 * rec2, "bucket records"))) return st;
+    if (b2 && (st = ensure(&g->d_rec2, &g->rec2_cap, 2 * rec2, "bucket records"))) return st;
     const uint64_t scratch = swg::gscan_scratch(NB);
     // d_bk: bucket samples / cursors [NB] | partition samples [P] | sample totals
     // [2] (cleared together) | regions [NB+1] | overflow lists [2 NB] | scan scratch
@@ -1290,6 +1294,11 @@ swg_status super_plan(swg_graph *g, const swg_opts *o, const BuildArgs &a, uint6
     SWG_CUDA(cudaMemsetAsync(sk.cursor2, 0, (NB + P + 2) * 8, s), "clear samples");
     g->launches += swg::launch_super_scan(a, sk, sk.n_pieces, stride, true, swg::kScatterResident, s);
     g->launches += swg::launch_super_caps(sk, NB, reinterpret_cast<uint64_t *>(pl.scr), s);
+    if (!b2) {  // the partitions are the buckets
+        sk.rec2 = sk.rec1;
+        sk.off2 = sk.part_start;
+        sk.cursor2 = sk.part_cursor;
+    }
     pl.b1 = b1;
     pl.b2 = b2;
     pl.P = P;
@@ -1390,7 +1399,7 @@ swg_status super_finish(swg_graph *g, const swg_opts *o, BuildArgs &a, cudaStrea
         a.host_written = &g->d_ctl->host_written;
         g->host_out_used = true;
     }
-    g->launches += swg::launch_super_sub(pl.sk, s);
+    if (pl.b2) g->launches += swg::launch_super_sub(pl.sk, s);
     SWG_CUDA(cudaGetLastError(), "bucket scatter launch");
     SWG_CUDA(cudaEventRecord(g->ev[3], s), "event");
     // (of a batch's per-sample tallies, only as many as there are samples sit beside the tables)
