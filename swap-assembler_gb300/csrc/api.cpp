@@ -925,6 +925,7 @@ struct BucketPlan {
     swg::BucketArgs bk;
     unsigned long long *scr = nullptr, *sampled = nullptr;
     bool super = false;  // sk instead of pa and bk: super-k-mer records
+    bool uniform = false, outgrown = false;  // regions of one size; one of them was too small
     swg::SkArgs sk;
 };
 
@@ -1238,7 +1239,8 @@ bool super_build(const swg_opts *o, const BuildArgs &a, uint64_t N) {
 // workspace and lays out the regions from every stride-th batch of a's reads,
 // which hold about `share` of the input.
 swg_status super_plan(swg_graph *g, const swg_opts *o, const BuildArgs &a, uint64_t N, uint64_t n_reads,
-                      uint32_t stride, double share, const swg::SkArgs &reads, cudaStream_t s, BucketPlan &pl) {
+                      uint32_t stride, double share, const swg::SkArgs &reads, cudaStream_t s, BucketPlan &pl,
+                      bool uniform = false) {
     swg_status st;
     int b1, b2;
     // sub-buckets of at most 3072 occurrences on average: the 2048-entry tables
@@ -1257,8 +1259,10 @@ swg_status super_plan(swg_graph *g, const swg_opts *o, const BuildArgs &a, uint6
     // (of those that have a k-mer)
     const uint64_t rec_cap =
         (uint64_t)(1.25 * ((double)std::min(n_reads, N) + 2.0 * (double)N / (swg::super_window(a.k, N) + 1))) + 65536;
+    uniform = uniform && !b2;
+    const uint64_t each = (rec_cap - 65536) * 8 / P + 256;  // a uniform region
     // (rec_cap / 1000: the partition regions are worked out in single precision)
-    const uint64_t rec1 = rec_cap + rec_cap / 4 + rec_cap / 1000 + 1025 * P, rec2 = swg::super_bucket_room(rec_cap, NB, scale_max);
+    const uint64_t rec1 = uniform ? P * each : rec_cap + rec_cap / 4 + rec_cap / 1000 + 1025 * P, rec2 = swg::super_bucket_room(rec_cap, NB, scale_max);
     if ((st = ensure(&g->d_part, &g->part_cap, 4 * P + 1, "partition table"))) return st;
     if ((st = ensure(&g->d_records, &g->records_cap, 2 * rec1, "records"))) return st;
     if (b2 && (st = ensure(&g->d_rec2, &g->rec2_cap, 2 * rec2, "bucket records"))) return st;
@@ -1291,9 +1295,13 @@ swg_status super_plan(swg_graph *g, const swg_opts *o, const BuildArgs &a, uint6
     sk.big_count = &g->d_ctl->pad;
     sk.big2_count = &g->d_ctl->pad2;
     sk.big_cap = (uint32_t)std::min<uint64_t>(NB, 0xffffffffu);
-    SWG_CUDA(cudaMemsetAsync(sk.cursor2, 0, (NB + P + 2) * 8, s), "clear samples");
-    g->launches += swg::launch_super_scan(a, sk, sk.n_pieces, stride, true, swg::kScatterResident, s);
-    g->launches += swg::launch_super_caps(sk, NB, reinterpret_cast<uint64_t *>(pl.scr), s);
+    if (uniform) {
+        g->launches += swg::launch_super_uniform(sk, each, s);
+    } else {
+        SWG_CUDA(cudaMemsetAsync(sk.cursor2, 0, (NB + P + 2) * 8, s), "clear samples");
+        g->launches += swg::launch_super_scan(a, sk, sk.n_pieces, stride, true, swg::kScatterResident, s);
+        g->launches += swg::launch_super_caps(sk, NB, reinterpret_cast<uint64_t *>(pl.scr), s);
+    }
     if (!b2) {  // the partitions are the buckets
         sk.rec2 = sk.rec1;
         sk.off2 = sk.part_start;
@@ -1304,6 +1312,7 @@ swg_status super_plan(swg_graph *g, const swg_opts *o, const BuildArgs &a, uint6
     pl.P = P;
     pl.NB = NB;
     pl.super = true;
+    pl.uniform = uniform;
     pl.sk = sk;
     return SWG_OK;
 }
@@ -1348,21 +1357,29 @@ swg_status build_super(swg_graph *g, const swg_opts *o, BuildArgs &a, cudaStream
         reads.pieces = true;
         as.read_range = reinterpret_cast<unsigned long long *>(range);
     }
-    BucketPlan pl;
     // the sample sizes the regions: a sixteenth of the reads, more of small
     // inputs (all below 4M occurrences: a batch of 256 reads is much of them)
     const uint32_t stride = a.total_occ >= (64ull << 20) ? 16 : (a.total_occ >= (4ull << 20) ? 4 : 1);
-    st = super_plan(g, o, as, a.total_occ, reads.n_pieces, stride, 1.0, reads, s, pl);
-    if (st == SWG_ERR_OOM) {
-        drop_records(g);
-        return build_bucketed(g, o, a, s, load);
+    // Up to a million occurrences, none: every bucket's region holds eight times
+    // the mean (at most 32 MB in all), and the sampled plan follows where that
+    // is too little, for repeats. Builds of 0.05M, 0.5M and 0.6M occurrences:
+    // 115 -> 97 us, 129 -> 98 and 123 -> 99 (of 0.8M, most of them of one base
+    // repeated, where the plan is made twice: 212 -> 351).
+    for (bool uniform = a.total_occ <= (1ull << 20);; uniform = false) {
+        BucketPlan pl;
+        st = super_plan(g, o, as, a.total_occ, reads.n_pieces, stride, 1.0, reads, s, pl, uniform);
+        if (st == SWG_ERR_OOM) {
+            drop_records(g);
+            return build_bucketed(g, o, a, s, load);
+        }
+        if (st) return st;
+        SWG_CUDA(cudaEventRecord(g->ev[1], s), "event");
+        g->launches += swg::launch_super_scan(as, pl.sk, reads.n_pieces, 1, false, swg::kScatterResident, s);
+        SWG_CUDA(cudaGetLastError(), "super-k-mer scan launch");
+        SWG_CUDA(cudaEventRecord(g->ev[2], s), "event");
+        st = super_finish(g, o, a, s, load, pl);
+        if (st || !pl.outgrown) return st;
     }
-    if (st) return st;
-    SWG_CUDA(cudaEventRecord(g->ev[1], s), "event");
-    g->launches += swg::launch_super_scan(as, pl.sk, reads.n_pieces, 1, false, swg::kScatterResident, s);
-    SWG_CUDA(cudaGetLastError(), "super-k-mer scan launch");
-    SWG_CUDA(cudaEventRecord(g->ev[2], s), "event");
-    return super_finish(g, o, a, s, load, pl);
 }
 
 // Output arrays of at least want k-molecules, the first keep kept.
@@ -1438,6 +1455,10 @@ swg_status super_finish(swg_graph *g, const swg_opts *o, BuildArgs &a, cudaStrea
         }
         if (again) {
             a = plain;
+            if (pl.uniform && g->d_records) {  // (not for want of memory)
+                pl.outgrown = true;
+                return SWG_OK;
+            }
             return build_bucketed(g, o, a, s, load, true);
         }
     }

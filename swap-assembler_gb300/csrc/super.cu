@@ -386,6 +386,13 @@ __global__ void __launch_bounds__(256) k_sk_bucket_caps(SkArgs s, const unsigned
     if (j < nb) caps[j] = bucket_cap(counts[j], x, nb);
 }
 
+// Regions of one size (one block).
+__global__ void __launch_bounds__(1024) k_sk_uniform(SkArgs s, uint64_t each) {
+    const uint32_t j = threadIdx.x;
+    if (j < s.n_parts) s.part_start[j] = s.part_cursor[j] = j * each;
+    if (j == 0) s.part_start[s.n_parts] = s.n_parts * each;
+}
+
 // Both kinds of regions of a plan of at most 1024 kRegionItems buckets, and
 // the cursors at their starts, by one block (six launches otherwise, most of a
 // small build's preparation). Single precision: 9 us for 2048 buckets, 25 in
@@ -1212,6 +1219,11 @@ int launch_super_pieces(const BuildArgs &a, uint64_t *count, uint64_t *first, ui
     const int n = launch_gscan(count, first, a.n_reads, scratch, total, st);
     k_sk_pieces_fill<<<(unsigned)((a.n_reads * 32 + 255) / 256), 256, 0, st>>>(a, first, off, len, seg);
     return 2 + n;
+}
+
+int launch_super_uniform(const SkArgs &s, uint64_t each, cudaStream_t st) {
+    k_sk_uniform<<<1, 1024, 0, st>>>(s, each);
+    return 1;
 }
 
 int launch_super_caps(const SkArgs &s, uint64_t nb, uint64_t *scratch, cudaStream_t st) {

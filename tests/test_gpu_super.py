@@ -93,6 +93,23 @@ def test_hot_buckets(copies):
     assert _check(reads, k, 2).info()["waves"] >= 1
 
 
+@pytest.mark.parametrize("repeats", [0, 4_000])
+@pytest.mark.parametrize("more", [-1, 0, 1])
+def test_around_a_million_occurrences(more, repeats):
+    """Up to 2^20 occurrences regions are of one size, unsampled; reads of one
+    base repeated outgrow theirs and the build goes on with sampled ones."""
+    rng = np.random.default_rng(9)
+    k = 21
+    reads = [b"A" * 100] * repeats
+    left = (1 << 20) + more - 80 * repeats
+    reads += _sampled(rng, _random(rng, 30_000), left // 80, [100])
+    if left % 80:
+        reads += [_random(rng, k - 1 + left % 80)]
+    reads = [reads[i] for i in rng.permutation(len(reads))]
+    g = _check(reads, k, 2)
+    assert g.info()["occurrences"] == (1 << 20) + more
+
+
 def test_few_survivors_and_many():
     """More survivors than the first output size (one per 8 occurrences):
     the count runs again into a larger one."""
