@@ -43,7 +43,10 @@ constexpr uint32_t kSkChunk = 256 * kSubItems;  // records per level-2 chunk
 // a bucket's records are counted this many at a time (16-bit counters: 3840 x
 // 17 + 255 occurrences cannot carry), the counters clamped to 255 in between
 constexpr uint32_t kSkClamp = 3840;
-constexpr uint64_t kSkBigRecords = 16384;  // larger buckets go to the global table
+// larger buckets go to the global table: one CTA alone counts a bucket, others
+// wait for it at the end (2.4G occurrences with 2% tandem repeats: count 17.5 ms
+// with 16384, 16.0 with 8192, 14.6 with 4096, the build 27.6, 26.1 and 26.7)
+constexpr uint64_t kSkBigRecords = 8192;
 
 __device__ __forceinline__ uint32_t sk_mix(uint32_t x) {  // bucket of a minimizer
     x ^= x >> 16;
