@@ -1260,7 +1260,7 @@ swg_status super_plan(swg_graph *g, const swg_opts *o, const BuildArgs &a, uint6
     const uint64_t rec_cap =
         (uint64_t)(1.25 * ((double)std::min(n_reads, N) + 2.0 * (double)N / (swg::super_window(a.k, N) + 1))) + 65536;
     uniform = uniform && !b2;
-    const uint64_t each = (rec_cap - 65536) * 8 / P + 256;  // a uniform region
+    const uint64_t each = (rec_cap - 65536) * 4 / P + 2048;  // a uniform region
     // (rec_cap / 1000: the partition regions are worked out in single precision)
     const uint64_t rec1 = uniform ? P * each : rec_cap + rec_cap / 4 + rec_cap / 1000 + 1025 * P, rec2 = swg::super_bucket_room(rec_cap, NB, scale_max);
     if ((st = ensure(&g->d_part, &g->part_cap, 4 * P + 1, "partition table"))) return st;
@@ -1360,12 +1360,13 @@ swg_status build_super(swg_graph *g, const swg_opts *o, BuildArgs &a, cudaStream
     // the sample sizes the regions: a sixteenth of the reads, more of small
     // inputs (all below 4M occurrences: a batch of 256 reads is much of them)
     const uint32_t stride = a.total_occ >= (64ull << 20) ? 16 : (a.total_occ >= (4ull << 20) ? 4 : 1);
-    // Up to a million occurrences, none: every bucket's region holds eight times
-    // the mean (at most 32 MB in all), and the sampled plan follows where that
-    // is too little, for repeats. Builds of 0.05M, 0.5M and 0.6M occurrences:
-    // 115 -> 97 us, 129 -> 98 and 123 -> 99 (of 0.8M, most of them of one base
-    // repeated, where the plan is made twice: 212 -> 351).
-    for (bool uniform = a.total_occ <= (1ull << 20);; uniform = false) {
+    // Where the scan scatters to the buckets, none: every region holds four
+    // times the mean and 2048 records (78 MB at most in all), and the sampled
+    // plan follows where that is too little, for repeats. Builds of 0.05M, 0.5M,
+    // 1.4M and 3.1M occurrences: 115 -> 97 us, 129 -> 100, 144 -> 110, 160 -> 125 (of
+    // 0.8M, most of them of one base repeated, where the plan is made twice:
+    // 212 -> 351).
+    for (bool uniform = true;; uniform = false) {
         BucketPlan pl;
         st = super_plan(g, o, as, a.total_occ, reads.n_pieces, stride, 1.0, reads, s, pl, uniform);
         if (st == SWG_ERR_OOM) {

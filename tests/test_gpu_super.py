@@ -94,20 +94,21 @@ def test_hot_buckets(copies):
 
 
 @pytest.mark.parametrize("repeats", [0, 4_000])
-@pytest.mark.parametrize("more", [-1, 0, 1])
-def test_around_a_million_occurrences(more, repeats):
-    """Up to 2^20 occurrences regions are of one size, unsampled; reads of one
-    base repeated outgrow theirs and the build goes on with sampled ones."""
+@pytest.mark.parametrize("total", [1 << 20, 1024 * 3072, 1024 * 3072 + 1])
+def test_regions_of_one_size(total, repeats):
+    """Up to 1024 buckets (of 3072 occurrences on average) there is no second
+    level and regions are of one size, unsampled; reads of one base repeated
+    outgrow theirs and the build goes on with sampled ones."""
     rng = np.random.default_rng(9)
     k = 21
     reads = [b"A" * 100] * repeats
-    left = (1 << 20) + more - 80 * repeats
+    left = total - 80 * repeats
     reads += _sampled(rng, _random(rng, 30_000), left // 80, [100])
     if left % 80:
         reads += [_random(rng, k - 1 + left % 80)]
     reads = [reads[i] for i in rng.permutation(len(reads))]
     g = _check(reads, k, 2)
-    assert g.info()["occurrences"] == (1 << 20) + more
+    assert g.info()["occurrences"] == total
 
 
 def test_few_survivors_and_many():
