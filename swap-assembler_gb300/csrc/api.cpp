@@ -1259,10 +1259,13 @@ swg_status super_plan(swg_graph *g, const swg_opts *o, const BuildArgs &a, uint6
     // (of those that have a k-mer)
     const uint64_t rec_cap =
         (uint64_t)(1.25 * ((double)std::min(n_reads, N) + 2.0 * (double)N / (swg::super_window(a.k, N) + 1))) + 65536;
-    uniform = uniform && !b2;
-    const uint64_t each = (rec_cap - 65536) * 4 / P + 2048;  // a uniform region
+    uniform = uniform && NB <= 8192;
+    // regions of one size: of a bucket, of a partition
+    const uint64_t bucket = (rec_cap - 65536) * (b2 ? 3 : 4) / NB + 2048;
+    const uint64_t part = b2 ? (rec_cap - 65536) * 3 / (2 * P) + 4096 : bucket;
     // (rec_cap / 1000: the partition regions are worked out in single precision)
-    const uint64_t rec1 = uniform ? P * each : rec_cap + rec_cap / 4 + rec_cap / 1000 + 1025 * P, rec2 = swg::super_bucket_room(rec_cap, NB, scale_max);
+    const uint64_t rec1 = uniform ? P * part : rec_cap + rec_cap / 4 + rec_cap / 1000 + 1025 * P,
+                   rec2 = uniform ? NB * bucket : swg::super_bucket_room(rec_cap, NB, scale_max);
     if ((st = ensure(&g->d_part, &g->part_cap, 4 * P + 1, "partition table"))) return st;
     if ((st = ensure(&g->d_records, &g->records_cap, 2 * rec1, "records"))) return st;
     if (b2 && (st = ensure(&g->d_rec2, &g->rec2_cap, 2 * rec2, "bucket records"))) return st;
@@ -1296,7 +1299,7 @@ swg_status super_plan(swg_graph *g, const swg_opts *o, const BuildArgs &a, uint6
     sk.big2_count = &g->d_ctl->pad2;
     sk.big_cap = (uint32_t)std::min<uint64_t>(NB, 0xffffffffu);
     if (uniform) {
-        g->launches += swg::launch_super_uniform(sk, each, s);
+        g->launches += swg::launch_super_uniform(sk, part, b2 ? NB : 0, bucket, s);
     } else {
         SWG_CUDA(cudaMemsetAsync(sk.cursor2, 0, (NB + P + 2) * 8, s), "clear samples");
         g->launches += swg::launch_super_scan(a, sk, sk.n_pieces, stride, true, swg::kScatterResident, s);
@@ -1357,20 +1360,22 @@ swg_status build_super(swg_graph *g, const swg_opts *o, BuildArgs &a, cudaStream
         reads.pieces = true;
         as.read_range = reinterpret_cast<unsigned long long *>(range);
     }
-    // the sample sizes the regions: a sixteenth of the reads, more of small
-    // inputs (all below 4M occurrences: a batch of 256 reads is much of them)
+    // the sample sizes the regions: a sixteenth of the reads, more of small inputs
     const uint32_t stride = a.total_occ >= (64ull << 20) ? 16 : (a.total_occ >= (4ull << 20) ? 4 : 1);
-    // Where the scan scatters to the buckets, none: every region holds four
-    // times the mean and 2048 records (78 MB at most in all), and the sampled
-    // plan follows where that is too little, for repeats. Builds of 0.05M, 0.5M,
-    // 1.4M and 3.1M occurrences: 115 -> 97 us, 129 -> 100, 144 -> 110, 160 -> 125 (of
-    // 0.8M, most of them of one base repeated, where the plan is made twice:
-    // 212 -> 351).
+    // Up to 8192 buckets (25M occurrences) no sample: every bucket's region
+    // holds three times the mean (four, where the scan scatters to the buckets)
+    // and 2048 records, every partition's half as much again as its mean: 0.7 GB
+    // at most in all. The sampled plan follows where that is too little, for
+    // repeats, or where there is no room. Builds of 0.05M, 0.5M, 1.4M, 3.1M, 9.6M
+    // and 24M occurrences: 115 -> 97 us, 129 -> 100, 144 -> 110, 160 -> 123,
+    // 223 -> 194, 369 -> 333 (of 0.8M, most of them of one base repeated, where
+    // the plan is made twice: 212 -> 351).
     for (bool uniform = true;; uniform = false) {
         BucketPlan pl;
         st = super_plan(g, o, as, a.total_occ, reads.n_pieces, stride, 1.0, reads, s, pl, uniform);
         if (st == SWG_ERR_OOM) {
             drop_records(g);
+            if (uniform) continue;
             return build_bucketed(g, o, a, s, load);
         }
         if (st) return st;

@@ -389,11 +389,13 @@ __global__ void __launch_bounds__(256) k_sk_bucket_caps(SkArgs s, const unsigned
     if (j < nb) caps[j] = bucket_cap(counts[j], x, nb);
 }
 
-// Regions of one size (one block).
-__global__ void __launch_bounds__(1024) k_sk_uniform(SkArgs s, uint64_t each) {
-    const uint32_t j = threadIdx.x;
-    if (j < s.n_parts) s.part_start[j] = s.part_cursor[j] = j * each;
-    if (j == 0) s.part_start[s.n_parts] = s.n_parts * each;
+// Regions of one size, of the partitions and of the buckets of a second level.
+__global__ void __launch_bounds__(1024) k_sk_uniform(SkArgs s, uint64_t part, uint32_t nb, uint64_t bucket) {
+    const uint32_t j = blockIdx.x * 1024 + threadIdx.x;
+    if (j < s.n_parts) s.part_start[j] = s.part_cursor[j] = j * part;
+    if (j == 0) s.part_start[s.n_parts] = s.n_parts * part;
+    if (j < nb) s.off2[j] = s.cursor2[j] = j * bucket;
+    if (j == 0 && nb) s.off2[nb] = nb * bucket;
 }
 
 // Both kinds of regions of a plan of at most 1024 kRegionItems buckets, and
@@ -1224,8 +1226,8 @@ int launch_super_pieces(const BuildArgs &a, uint64_t *count, uint64_t *first, ui
     return 2 + n;
 }
 
-int launch_super_uniform(const SkArgs &s, uint64_t each, cudaStream_t st) {
-    k_sk_uniform<<<1, 1024, 0, st>>>(s, each);
+int launch_super_uniform(const SkArgs &s, uint64_t part, uint64_t nb, uint64_t bucket, cudaStream_t st) {
+    k_sk_uniform<<<(unsigned)std::max<uint64_t>(1, (nb + 1023) / 1024), 1024, 0, st>>>(s, part, (uint32_t)nb, bucket);
     return 1;
 }
 

@@ -177,7 +177,7 @@ int launch_super_pieces(const BuildArgs &a, uint64_t *count, uint64_t *first, ui
 // bound: reads (pieces) at most; sample: sizes only, of every stride-th batch
 int launch_super_scan(const BuildArgs &a, const SkArgs &sk, uint64_t bound, uint32_t stride, bool sample,
                       int grid_mode, cudaStream_t s);
-int launch_super_uniform(const SkArgs &s, uint64_t each, cudaStream_t st);
+int launch_super_uniform(const SkArgs &s, uint64_t part, uint64_t nb, uint64_t bucket, cudaStream_t st);
 int launch_super_caps(const SkArgs &sk, uint64_t nb, uint64_t *scratch, cudaStream_t s);
 int launch_super_sub(const SkArgs &sk, cudaStream_t s);
 int launch_super_count(const BuildArgs &a, const SkArgs &sk, uint64_t nb, int table, cudaStream_t s);

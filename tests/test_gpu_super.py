@@ -97,8 +97,9 @@ def test_hot_buckets(copies):
 @pytest.mark.parametrize("total", [1 << 20, 1024 * 3072, 1024 * 3072 + 1])
 def test_regions_of_one_size(total, repeats):
     """Up to 1024 buckets (of 3072 occurrences on average) there is no second
-    level and regions are of one size, unsampled; reads of one base repeated
-    outgrow theirs and the build goes on with sampled ones."""
+    level; regions are of one size, unsampled, there and in somewhat larger
+    builds; reads of one base repeated outgrow theirs and the build goes on with
+    sampled ones."""
     rng = np.random.default_rng(9)
     k = 21
     reads = [b"A" * 100] * repeats
