@@ -1855,7 +1855,7 @@ __device__ void bucket_pass(const BuildArgs &a, const BucketArgs &b, uint64_t n_
 // Tier 1: tables of up to kBkTable entries, two persistent CTAs per SM over
 // all buckets; overflow to the big list.
 __global__ void __launch_bounds__(kBkThreads, 2) k_bucket_count(BuildArgs a, BucketArgs b, uint64_t n_buckets) {
-    if (*b.status & kStatusPartOverflow) return;  // a partition overflowed: the build recounts
+    if (block_reads_overflow(b.status)) return;  // a partition overflowed: the build recounts
     bucket_pass<kBkTable, kBkThreads>(a, b, n_buckets, nullptr, b.big, b.big_count, b.big_cap);
 }
 
@@ -1866,7 +1866,7 @@ __global__ void __launch_bounds__(kBkThreads, 2) k_bucket_count(BuildArgs a, Buc
 constexpr int kBkTableS = 2048, kBkThreadsS = 256;
 constexpr uint64_t kBkSmallRecords = 3072;
 __global__ void __launch_bounds__(kBkThreadsS, 4) k_bucket_count_small(BuildArgs a, BucketArgs b, uint64_t n_buckets) {
-    if (*b.status & kStatusPartOverflow) return;
+    if (block_reads_overflow(b.status)) return;
     bucket_pass<kBkTableS, kBkThreadsS, 4>(a, b, n_buckets, nullptr, b.big, b.big_count, b.big_cap);
 }
 
@@ -1874,7 +1874,7 @@ __global__ void __launch_bounds__(kBkThreadsS, 4) k_bucket_count_small(BuildArgs
 // tables of up to kBkTable2 entries; overflow to the second list (counted in
 // a global-memory table by the host-driven path).
 __global__ void __launch_bounds__(kBkThreads2, 1) k_bucket_count_large(BuildArgs a, BucketArgs b) {
-    if (*b.status & kStatusPartOverflow) return;
+    if (block_reads_overflow(b.status)) return;
     const unsigned n = umin64(*b.big_count, b.big_cap);
     bucket_pass<kBkTable2, kBkThreads2>(a, b, n, b.big, b.big2, b.big2_count, b.big_cap);
 }

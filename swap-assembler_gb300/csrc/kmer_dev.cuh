@@ -197,6 +197,15 @@ __device__ __forceinline__ uint64_t bucket_mult(const unsigned *cnt, uint32_t s,
     return cut_all ? 0 : m;
 }
 
+// Whether a region has been outgrown, so that the build will count again: one
+// answer for the whole block. The blocks of a counting kernel set the bit
+// themselves when they find a bucket outgrown, so threads that each read it
+// could disagree, and those that stayed would count with tables that the
+// others never cleared, at barriers the others never reach.
+__device__ __forceinline__ bool block_reads_overflow(const unsigned *status) {
+    return __syncthreads_or(threadIdx.x == 0 && (*(const volatile unsigned *)status & kStatusPartOverflow));
+}
+
 }  // namespace
 
 // Lets a kernel use up to `most` bytes of dynamic shared memory (its largest

@@ -1029,7 +1029,7 @@ __device__ void count_pass(const BuildArgs &a, const SkArgs &s, uint64_t n_items
 // CTA of 1024 threads an SM with 8192 entries, over tier 1's overflow list.
 template <int T, int NT, int kK>
 __global__ void __launch_bounds__(NT, 1024 / NT) k_sk_count(BuildArgs a, SkArgs s, uint64_t n) {
-    if ((*s.status & kStatusPartOverflow) || (T == 8192 && blockIdx.x >= *s.big_count)) return;
+    if (block_reads_overflow(s.status) || (T == 8192 && blockIdx.x >= *s.big_count)) return;
     if (T == 8192) {
         count_pass<T, NT, kK>(a, s, umin64(*s.big_count, s.big_cap), 1, s.big, s.big2, s.big2_count);
     } else {  // sets of four buckets, fewer where the CTAs would not get a dozen sets each
