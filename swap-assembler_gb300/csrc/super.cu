@@ -981,9 +981,11 @@ __device__ void count_pass(const BuildArgs &a, const SkArgs &s, uint64_t n_items
                 }
             }
             const unsigned m = __ballot_sync(kFull, keep);
+            __syncwarp();  // (a vote orders no memory: the lanes' slots are read before they are overwritten)
             if (keep) used[ns + __popc(m & lt)] = (unsigned short)sl;
             ns += __popc(m);
         }
+        __syncwarp();  // the list's front is written: other lanes read it below
         distinct += nu;
         unsigned long long out = 0;
         if (lane == 0 && ns) {
