@@ -133,22 +133,18 @@ swg_status scan_lengths(const uint64_t *len, uint64_t *off, uint64_t n, Scratch 
     return SWG_OK;
 }
 
-TextFile::~TextFile() {
-    if (fp) std::fclose(fp);
-}
-
-swg_status TextFile::open() {
-    fp = std::fopen(path, "wb");
-    if (fp) return SWG_OK;
-    set_error(std::string("cannot open ") + path);
-    return SWG_ERR_IO;
-}
-
-// 4 MiB chunks copied into two pinned buffers in turn; the copy of one chunk
-// overlaps the fwrite of the other. (Small buffers: pinning two of 64 MiB took
-// 4 ms a call, these 0.3 ms, and a chunk's write takes far longer than its
-// copy either way.)
-swg_status TextFile::write(const char *d_text, uint64_t bytes, cudaStream_t s) {
+// Writes text[0..bytes) to path: 4 MiB chunks copied into two pinned buffers
+// in turn; the copy of one chunk overlaps the fwrite of the other. (Small
+// buffers: pinning two of 64 MiB took 4 ms a call, these 0.3 ms, and a chunk's
+// write takes far longer than its copy either way.) Called once the text's
+// buffer is there and the kernels that fill it are launched: opening empties an
+// earlier file, which a call that fails before has to leave alone.
+swg_status stream_to_file(const char *d_text, uint64_t bytes, const char *path, cudaStream_t s) {
+    FILE *fp = std::fopen(path, "wb");
+    if (!fp) {
+        set_error(std::string("cannot open ") + path);
+        return SWG_ERR_IO;
+    }
     constexpr uint64_t kChunk = 4ull << 20;
     std::setvbuf(fp, nullptr, _IONBF, 0);
     char *h[2] = {nullptr, nullptr};
@@ -183,19 +179,12 @@ swg_status TextFile::write(const char *d_text, uint64_t bytes, cudaStream_t s) {
         if (h[b]) cudaFreeHost(h[b]);
     }
     const bool closed = std::fclose(fp) == 0;
-    fp = nullptr;
     if (e != cudaSuccess) return cuda_err(e, "streaming the text to the file");
     if (st != SWG_OK || !closed) {
         set_error(std::string("write failed: ") + path);
         return SWG_ERR_IO;
     }
     return SWG_OK;
-}
-
-swg_status stream_to_file(const char *d_text, uint64_t bytes, const char *path, cudaStream_t s) {
-    TextFile f(path);
-    const swg_status st = f.open();
-    return st ? st : f.write(d_text, bytes, s);
 }
 
 swg_status emit_node_lines(const unsigned long long *d_keys, const unsigned long long *d_mult, uint64_t n,
@@ -217,8 +206,6 @@ swg_status emit_node_lines(const unsigned long long *d_keys, const unsigned long
     }
     swg_status st = scan_lengths(len, off, n, scr, s);
     if (st) return st;
-    TextFile file(path);  // emptying an earlier file overlaps the kernels above
-    if ((st = file.open())) return st;
     uint64_t bytes = 0;
     EMIT_CUDA(cudaMemcpyAsync(&bytes, off + n, 8, cudaMemcpyDeviceToHost, s), "text size");
     EMIT_CUDA(cudaStreamSynchronize(s), "text size");
@@ -226,7 +213,7 @@ swg_status emit_node_lines(const unsigned long long *d_keys, const unsigned long
     if (!scr.get(&text, bytes)) return cuda_err(cudaErrorMemoryAllocation, "node-line text");
     if (n) k_node_write<<<blocks_for(n), 256, 0, s>>>(mult, keys, n, off, text);
     EMIT_CUDA(cudaGetLastError(), "node-line kernels");
-    return file.write(text, bytes, s);
+    return stream_to_file(text, bytes, path, s);
 }
 
 swg_status emit_kmer_graph(const unsigned long long *d_keys, const unsigned long long *d_mult, uint64_t n, int k,
@@ -262,8 +249,6 @@ swg_status emit_kmer_graph(const unsigned long long *d_keys, const unsigned long
     }
     st = scan_lengths(len, off, lines, scr, s);
     if (st) return st;
-    TextFile file(path);  // emptying an earlier file overlaps the kernels above
-    if ((st = file.open())) return st;
     uint64_t bytes = 0;
     EMIT_CUDA(cudaMemcpyAsync(&bytes, off + lines, 8, cudaMemcpyDeviceToHost, s), "text size");
     EMIT_CUDA(cudaStreamSynchronize(s), "text size");
@@ -271,7 +256,7 @@ swg_status emit_kmer_graph(const unsigned long long *d_keys, const unsigned long
     if (!scr.get(&text, bytes)) return cuda_err(cudaErrorMemoryAllocation, "kmerGraph text");
     if (lines) k_kg_write<<<blocks_for(lines), 256, 0, s>>>(tok2, idx2, lines, d_keys, d_mult, k, off, text);
     EMIT_CUDA(cudaGetLastError(), "kmerGraph kernels");
-    return file.write(text, bytes, s);
+    return stream_to_file(text, bytes, path, s);
 }
 
 }  // namespace swg

@@ -4,7 +4,6 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include <cstdio>
 #include <string>
 
 #include "swapgb.h"
@@ -324,19 +323,7 @@ swg_status copy_records_sorted(const unsigned long long *d_keys, const unsigned 
 uint64_t revcomp_host(uint64_t x, int k);
 // Device emission of the text outputs (emit.cu), byte-identical with the host
 // writers: records on the device, any order.
-// Device text -> file through two pinned buffers (emit.cu). Opened (and
-// emptied) on its own, so that this can overlap kernels in flight; write
-// closes it.
-struct TextFile {
-    const char *path;
-    FILE *fp = nullptr;
-    explicit TextFile(const char *p) : path(p) {}
-    ~TextFile();
-    TextFile(const TextFile &) = delete;
-    TextFile &operator=(const TextFile &) = delete;
-    swg_status open();
-    swg_status write(const char *d_text, uint64_t bytes, cudaStream_t s);
-};
+// Device text -> file through two pinned buffers (emit.cu).
 swg_status stream_to_file(const char *d_text, uint64_t bytes, const char *path, cudaStream_t s);
 // The merged graph on the device: the -d file's text (gathered node lines in
 // key order + final '\n') and, per line, its node key and per arc slot the
