@@ -262,25 +262,29 @@ swg_status build_partitioned(swg_graph *g, const swg_opts *o, BuildArgs &a, cuda
 swg_status build_bucketed(swg_graph *g, const swg_opts *o, BuildArgs &a, cudaStream_t s,
                           double load, bool counted = false);
 bool super_build(const swg_opts *o, const BuildArgs &a, uint64_t N);
-swg_status build_super(swg_graph *g, const swg_opts *o, BuildArgs &a, cudaStream_t s, double load, uint64_t longest);
+swg_status build_super(swg_graph *g, const swg_opts *o, BuildArgs &a, cudaStream_t s, double load, uint64_t longest,
+                       double room);
 
-// The default algorithm is the bucketed one while its worst-case workspace
-// (two record buffers of at most 1.5 x 8 bytes per occurrence, plus an
-// output of up to 16 bytes per occurrence) fits in 80% of the device memory
-// that is free or already held by this handle's record buffers; otherwise the
-// direct one, whose table grows with the distinct k-molecules instead of the
-// occurrences.
+// The default algorithm is the bucketed one while the worst-case workspace of
+// its build over single occurrences (two record buffers of at most 1.5 x 8
+// bytes per occurrence, plus an output of up to 16 bytes per occurrence) fits
+// in 80% of the device memory that is free or already held by this handle's
+// record buffers; otherwise the direct one, whose table grows with the
+// distinct k-molecules instead of the occurrences. *room: what that leaves for
+// the records of the build over super-k-mers (super_fits), in bytes.
 constexpr unsigned kBucketedMaxRead = 16384;  // longest read the default sends to the bucketed build
+constexpr double kAnyRoom = 1e300;            // bucketed because asked for: whatever can be allocated
 
-bool bucketed_fits(const swg_graph *g, uint64_t occurrences) {
+bool bucketed_fits(const swg_graph *g, uint64_t occurrences, double *room) {
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
     const double held = 8.0 * (double)(g->records_cap + g->rec2_cap);
-    const double need = 40.0 * (double)occurrences + (64 << 20);
-    return need <= 0.8 * ((double)free_b + held);
+    const double most = 0.8 * ((double)free_b + held);
+    *room = most - 16.0 * (double)occurrences;
+    return 40.0 * (double)occurrences + (64 << 20) <= most;
 }
 
 // NVTX range over one call, named after the reference's phase it replaces
@@ -348,9 +352,10 @@ swg_status build_impl(swg_graph *g, const swg_opts *o, const uint32_t *packed, u
     g->estimate = 0;
     // the bucketed build walks one read per thread: reads of more than 16 kbp
     // (long-read data) would leave the GPU waiting on a few threads
+    double room = kAnyRoom;
     const bool bucketed = o->algorithm == SWG_ALGO_BUCKETED ||
                           (o->algorithm == SWG_ALGO_DEFAULT && o->read_order == SWG_ORDER_INPUT &&
-                           g->h_ctl->max_len <= kBucketedMaxRead && bucketed_fits(g, a.total_occ));
+                           g->h_ctl->max_len <= kBucketedMaxRead && bucketed_fits(g, a.total_occ, &room));
     // the per-read occurrence prefix and the tiles of kTileOcc occurrences:
     // every algorithm but the bucketed build's thread-per-read scatter uses them
     if (!bucketed || swg::level1_shape(o->scatter_shape) == 4) {
@@ -363,7 +368,7 @@ swg_status build_impl(swg_graph *g, const swg_opts *o, const uint32_t *packed, u
         SWG_CUDA(cudaGetLastError(), "tile launch");
     }
     if (o->algorithm == SWG_ALGO_PARTITIONED) return build_partitioned(g, o, a, s, load);
-    if (bucketed && super_build(o, a, a.total_occ)) return build_super(g, o, a, s, load, g->h_ctl->max_len);
+    if (bucketed && super_build(o, a, a.total_occ)) return build_super(g, o, a, s, load, g->h_ctl->max_len, room);
     if (bucketed) return build_bucketed(g, o, a, s, load);
     return build_direct(g, o, a, s, load);
 }
@@ -602,7 +607,7 @@ swg_status build_partitioned(swg_graph *g, const swg_opts *o, BuildArgs &a, cuda
 // own sample cutoffs and counts per sample, and a final pass moves the
 // survivors into per-sample ranges with the tag stripped.
 swg_status batch_bucketed(swg_graph *g, const swg_opts *o, const swg_sample *sm, uint32_t S,
-                          BuildArgs &a, cudaStream_t s, double load, int tb, uint64_t longest) {
+                          BuildArgs &a, cudaStream_t s, double load, int tb, uint64_t longest, double room) {
     swg_status st;
     a.tag_bits = S > 1 ? tb : 0;
     a.cutoff = sm[0].cutoff;  // the single sample's, when untagged
@@ -611,7 +616,7 @@ swg_status batch_bucketed(swg_graph *g, const swg_opts *o, const swg_sample *sm,
     SWG_CUDA(cudaMemsetAsync(g->d_seg_counts, 0, 2ull * S * 8, s), "clear counters");
     bool same_k = true;  // one k for all: super-k-mer records
     for (uint32_t i = 1; i < S; i++) same_k = same_k && sm[i].k == sm[0].k;
-    st = same_k && super_build(o, a, a.total_occ) ? build_super(g, o, a, s, load, longest)
+    st = same_k && super_build(o, a, a.total_occ) ? build_super(g, o, a, s, load, longest, room)
                                                   : build_bucketed(g, o, a, s, load);
     if (st) return st;
     g->n_samples = S;
@@ -791,10 +796,11 @@ swg_status batch_impl(swg_graph *g, const swg_opts *o, const swg_sample *sm, uin
         int kmax = 1, tb = 0;
         for (uint32_t i = 0; i < S; i++) kmax = std::max(kmax, sm[i].k);
         while ((1u << tb) < S) tb++;
+        double room = kAnyRoom;
         if ((o->algorithm == SWG_ALGO_DEFAULT || o->algorithm == SWG_ALGO_BUCKETED) &&
             o->read_order == SWG_ORDER_INPUT && S <= swg::kMaxTagSamples && 2 * kmax + tb <= 64 &&
-            (o->algorithm == SWG_ALGO_BUCKETED || bucketed_fits(g, a.total_occ)))
-            return batch_bucketed(g, o, sm, S, a, s, load, tb, g->h_ctl->max_len);
+            (o->algorithm == SWG_ALGO_BUCKETED || bucketed_fits(g, a.total_occ, &room)))
+            return batch_bucketed(g, o, sm, S, a, s, load, tb, g->h_ctl->max_len, room);
     }
     a.n_tiles = (a.total_occ + swg::kTileOcc - 1) / swg::kTileOcc;
     if ((st = ensure(&g->d_tiles, &g->tiles_cap, a.n_tiles, "tile table"))) return st;
@@ -1235,13 +1241,18 @@ bool super_build(const swg_opts *o, const BuildArgs &a, uint64_t N) {
     return swg::super_window(a.k, N) && N && !swg::level1_shape(o->scatter_shape);
 }
 
-// Sizes the build for N occurrences of n_reads reads, allocates its
-// workspace and lays out the regions from every stride-th batch of a's reads,
-// which hold about `share` of the input.
-swg_status super_plan(swg_graph *g, const swg_opts *o, const BuildArgs &a, uint64_t N, uint64_t n_reads,
-                      uint32_t stride, double share, const swg::SkArgs &reads, cudaStream_t s, BucketPlan &pl,
-                      bool uniform = false) {
-    swg_status st;
+// Records that the buffers of a build over super-k-mers hold, for N occurrences
+// of n_reads reads.
+struct SuperSizes {
+    int b1, b2;
+    uint64_t rec_cap;       // records expected at most
+    bool uniform;           // regions of one size,
+    uint64_t part, bucket;  // ... of a partition, of a bucket
+    uint64_t rec1, rec2;    // level 1, level 2
+};
+
+SuperSizes super_sizes(const swg_opts *o, int k, uint64_t N, uint64_t n_reads, double scale_max, bool uniform) {
+    SuperSizes z;
     int b1, b2;
     // sub-buckets of at most 3072 occurrences on average: the 2048-entry tables
     // (four CTAs an SM) hold their k-molecules. (Past 800M occurrences they are
@@ -1254,21 +1265,50 @@ swg_status super_plan(swg_graph *g, const swg_opts *o, const BuildArgs &a, uint6
     // 148 -> 144, 156 -> 147)
     if (b1 + b2 <= swg::kPartBitsMax) b1 += b2, b2 = 0;
     const uint64_t P = 1ull << b1, NB = P << b2;
-    const double scale_max = 2.0 * stride / share;
     // a random sequence has 2 / (w + 1) runs per k-mer and one more per read
     // (of those that have a k-mer)
-    const uint64_t rec_cap =
-        (uint64_t)(1.25 * ((double)std::min(n_reads, N) + 2.0 * (double)N / (swg::super_window(a.k, N) + 1))) + 65536;
-    uniform = uniform && NB <= 8192;
-    // regions of one size: of a bucket, of a partition
-    const uint64_t bucket = (rec_cap - 65536) * (b2 ? 3 : 4) / NB + 2048;
-    const uint64_t part = b2 ? (rec_cap - 65536) * 3 / (2 * P) + 4096 : bucket;
+    z.rec_cap =
+        (uint64_t)(1.25 * ((double)std::min(n_reads, N) + 2.0 * (double)N / (swg::super_window(k, N) + 1))) + 65536;
+    z.b1 = b1;
+    z.b2 = b2;
+    z.uniform = uniform && NB <= 8192;
+    z.bucket = (z.rec_cap - 65536) * (b2 ? 3 : 4) / NB + 2048;
+    z.part = b2 ? (z.rec_cap - 65536) * 3 / (2 * P) + 4096 : z.bucket;
     // (rec_cap / 1000: the partition regions are worked out in single precision)
-    const uint64_t rec1 = uniform ? P * part : rec_cap + rec_cap / 4 + rec_cap / 1000 + 1025 * P,
-                   rec2 = uniform ? NB * bucket : swg::super_bucket_room(rec_cap, NB, scale_max);
+    z.rec1 = z.uniform ? P * z.part : z.rec_cap + z.rec_cap / 4 + z.rec_cap / 1000 + 1025 * P;
+    z.rec2 = !b2 ? 0 : (z.uniform ? NB * z.bucket : swg::super_bucket_room(z.rec_cap, NB, scale_max));
+    return z;
+}
+
+// The records of a build over super-k-mers take 16 bytes each, those over
+// single occurrences 8: for reads hardly longer than k, or regions of one size
+// much larger than their contents, they would take far more memory (25M
+// occurrences in reads of k bases: 119 bytes an occurrence, where single ones
+// take 24). So they are used while they take at most 37 bytes an occurrence and
+// `slack`, which with the output's 16 is what the request server charges for,
+// and fit in `room`. From a million occurrences and for reads of 50 bases and
+// more, sampled regions take 9 to 28 bytes an occurrence and regions of one
+// size 20 to 47, all of them within the line but k = 19 at 12.6M to 13.4M
+// occurrences; past it are also regions of one size for reads of 36 bases, 12.6M
+// to 18M occurrences, and any for reads within a base or two of k.
+constexpr uint64_t kSuperSlack = 64ull << 20;
+
+bool super_fits(const SuperSizes &z, uint64_t N, uint64_t slack, double room) {
+    const double need = 16.0 * (double)(z.rec1 + z.rec2);
+    return need <= 37.0 * (double)N + (double)slack && need <= room;
+}
+
+// Lays out the build for N occurrences in regions of sizes z: allocates its
+// workspace and works out the regions from every stride-th batch of a's reads
+// (unless they are of one size); scale_max: records per sampled record at most.
+swg_status super_plan(swg_graph *g, const SuperSizes &z, const BuildArgs &a, uint64_t N, uint32_t stride,
+                      double scale_max, const swg::SkArgs &reads, cudaStream_t s, BucketPlan &pl) {
+    swg_status st;
+    const int b1 = z.b1, b2 = z.b2;
+    const uint64_t P = 1ull << b1, NB = P << b2;
     if ((st = ensure(&g->d_part, &g->part_cap, 4 * P + 1, "partition table"))) return st;
-    if ((st = ensure(&g->d_records, &g->records_cap, 2 * rec1, "records"))) return st;
-    if (b2 && (st = ensure(&g->d_rec2, &g->rec2_cap, 2 * rec2, "bucket records"))) return st;
+    if ((st = ensure(&g->d_records, &g->records_cap, 2 * z.rec1, "records"))) return st;
+    if (b2 && (st = ensure(&g->d_rec2, &g->rec2_cap, 2 * z.rec2, "bucket records"))) return st;
     const uint64_t scratch = swg::gscan_scratch(NB);
     // d_bk: bucket samples / cursors [NB] | partition samples [P] | sample totals
     // [2] (cleared together) | regions [NB+1] | overflow lists [2 NB] | scan scratch
@@ -1293,13 +1333,13 @@ swg_status super_plan(swg_graph *g, const swg_opts *o, const BuildArgs &a, uint6
     sk.rec1 = reinterpret_cast<uint4 *>(g->d_records);
     sk.rec2 = reinterpret_cast<uint4 *>(g->d_rec2);
     sk.n_kmers = N;
-    sk.rec_cap = rec_cap;
+    sk.rec_cap = z.rec_cap;
     sk.scale_max = scale_max;
     sk.big_count = &g->d_ctl->pad;
     sk.big2_count = &g->d_ctl->pad2;
     sk.big_cap = (uint32_t)std::min<uint64_t>(NB, 0xffffffffu);
-    if (uniform) {
-        g->launches += swg::launch_super_uniform(sk, part, b2 ? NB : 0, bucket, s);
+    if (z.uniform) {
+        g->launches += swg::launch_super_uniform(sk, z.part, b2 ? NB : 0, z.bucket, s);
     } else {
         SWG_CUDA(cudaMemsetAsync(sk.cursor2, 0, (NB + P + 2) * 8, s), "clear samples");
         g->launches += swg::launch_super_scan(a, sk, sk.n_pieces, stride, true, swg::kScatterResident, s);
@@ -1315,7 +1355,7 @@ swg_status super_plan(swg_graph *g, const swg_opts *o, const BuildArgs &a, uint6
     pl.P = P;
     pl.NB = NB;
     pl.super = true;
-    pl.uniform = uniform;
+    pl.uniform = z.uniform;
     pl.sk = sk;
     return SWG_OK;
 }
@@ -1332,7 +1372,8 @@ void drop_records(swg_graph *g) {
     g->records_cap = g->rec2_cap = 0;
 }
 
-swg_status build_super(swg_graph *g, const swg_opts *o, BuildArgs &a, cudaStream_t s, double load, uint64_t longest) {
+swg_status build_super(swg_graph *g, const swg_opts *o, BuildArgs &a, cudaStream_t s, double load, uint64_t longest,
+                       double room) {
     swg_status st;
     g->algorithm = SWG_ALGO_BUCKETED;
     swg::SkArgs reads;
@@ -1364,15 +1405,22 @@ swg_status build_super(swg_graph *g, const swg_opts *o, BuildArgs &a, cudaStream
     const uint32_t stride = a.total_occ >= (64ull << 20) ? 16 : (a.total_occ >= (4ull << 20) ? 4 : 1);
     // Up to 8192 buckets (25M occurrences) no sample: every bucket's region
     // holds three times the mean (four, where the scan scatters to the buckets)
-    // and 2048 records, every partition's half as much again as its mean: 0.7 GB
-    // at most in all. The sampled plan follows where that is too little, for
-    // repeats, or where there is no room. Builds of 0.05M, 0.5M, 1.4M, 3.1M, 9.6M
+    // and 2048 records, every partition's half as much again as its mean (0.7 GB
+    // in all for 25M occurrences of 100 bp reads; super_fits bounds it). The
+    // sampled plan follows where that is too little, for repeats, or where there
+    // is no room, and single occurrences where the sampled plan does not fit. Builds of 0.05M, 0.5M, 1.4M, 3.1M, 9.6M
     // and 24M occurrences: 115 -> 97 us, 129 -> 100, 144 -> 110, 160 -> 123,
     // 223 -> 194, 369 -> 333 (of 0.8M, most of them of one base repeated, where
     // the plan is made twice: 212 -> 351).
+    const uint64_t slack = a.segs ? std::min<uint64_t>(kSuperSlack, (uint64_t)a.n_segs << 24) : kSuperSlack;
     for (bool uniform = true;; uniform = false) {
+        const SuperSizes z = super_sizes(o, a.k, a.total_occ, reads.n_pieces, 2.0 * stride, uniform);
+        if (!super_fits(z, a.total_occ, slack, room)) {
+            if (uniform) continue;
+            return build_bucketed(g, o, a, s, load);
+        }
         BucketPlan pl;
-        st = super_plan(g, o, as, a.total_occ, reads.n_pieces, stride, 1.0, reads, s, pl, uniform);
+        st = super_plan(g, z, as, a.total_occ, stride, 2.0 * stride, reads, s, pl);
         if (st == SWG_ERR_OOM) {
             drop_records(g);
             if (uniform) continue;
@@ -1745,7 +1793,8 @@ swg_status build_fasta_streamed(swg_graph *g, const swg_opts *o, const char *fir
         if (stream && c == 0) {
             // the first piece sizes the build: its occurrences per byte, and its reads as the sample
             const uint64_t N_est = occ_c ? (uint64_t)(scale * (double)occ_c * 1.02) + 65536 : 0;
-            if (!N_est || (o->algorithm == SWG_ALGO_DEFAULT && !bucketed_fits(g, N_est))) {
+            double room = kAnyRoom;
+            if (!N_est || (o->algorithm == SWG_ALGO_DEFAULT && !bucketed_fits(g, N_est, &room))) {
                 stream = false;
             } else {
                 SWG_CUDA(cudaStreamWaitEvent(s, packed_ev[0], 0), "build stream wait");
@@ -1759,14 +1808,15 @@ swg_status build_fasta_streamed(swg_graph *g, const swg_opts *o, const char *fir
                 g->algorithm = SWG_ALGO_BUCKETED;
                 // every stride-th batch of the first piece: 1/16 to 1/8 of all reads
                 const uint32_t stride = (uint32_t)std::max<uint64_t>(1, 16 * first_blocks / nc);
-                if (super_build(o, a0, N_est) && longest <= kSuperLongest) {
+                const double scale_max = 2.0 * stride * scale;
+                const SuperSizes z = super_sizes(o, a.k, N_est, (uint64_t)(scale * (double)reads_c * 1.02), scale_max, false);
+                if (super_build(o, a0, N_est) && longest <= kSuperLongest && super_fits(z, N_est, kSuperSlack, room)) {
                     swg::SkArgs reads;
                     std::memset(&reads, 0, sizeof(reads));
                     reads.off = g->d_off;
                     reads.len = g->d_len;
                     reads.n_pieces = reads_c;
-                    st = super_plan(g, o, a0, N_est, (uint64_t)(scale * (double)reads_c * 1.02), stride, 1.0 / scale,
-                                    reads, s, pl);
+                    st = super_plan(g, z, a0, N_est, stride, scale_max, reads, s, pl);
                     if (st == SWG_ERR_OOM) drop_records(g);
                 } else {
                     st = SWG_ERR_OOM;
@@ -1829,7 +1879,8 @@ swg_status build_fasta_streamed(swg_graph *g, const swg_opts *o, const char *fir
         swg::set_error("the last record has a header line but no sequence line");
         return SWG_ERR_BAD_INPUT;
     }
-    if (stream && o->algorithm == SWG_ALGO_DEFAULT && !bucketed_fits(g, occ)) stream = false;
+    double room = kAnyRoom;
+    if (stream && o->algorithm == SWG_ALGO_DEFAULT && !bucketed_fits(g, occ, &room)) stream = false;
     if (stream && pl.super && longest > kSuperLongest) stream = false;  // cut in pieces by the one-shot build
     if (!stream) {  // the one-shot build over the reads framed here
         st = build_impl(g, o, g->d_packed, words, g->d_off, g->d_len, reads);

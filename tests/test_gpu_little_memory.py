@@ -77,3 +77,43 @@ def test_failed_text_leaves_the_earlier_file(writer, tmp_path):
                 continue
             break
     assert failed >= 3 and path.read_bytes() == want
+
+
+def _random_reads(n_reads, length, genome, seed):
+    """Reads of one length at random places of a random genome, packed one over
+    another: the words, and every read's offset and length, on the device."""
+    import torch
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(seed)
+    words = torch.randint(-2**31, 2**31, ((genome + 15) // 16,), generator=gen, device="cuda", dtype=torch.int32)
+    off = torch.randint(0, genome - length + 1, (n_reads,), generator=gen, device="cuda")
+    return words, off, torch.full((n_reads,), length, device="cuda", dtype=torch.int32)
+
+
+def _build(g, opts, reads):
+    import torch
+    words, off, length = reads
+    torch.cuda.synchronize()
+    return g.build_device(opts, words.data_ptr(), words.numel(), off.data_ptr(), length.data_ptr(), off.numel())
+
+
+@pytest.mark.parametrize("k,length,occurrences", [(31, 31, 25_000_000), (21, 22, 20_000_000), (31, 33, 25_000_000),
+                                                  (21, 100, 24_000_000), (31, 31, 2_000_000), (31, 31, 70_000_000)])
+def test_workspace_of_short_reads_is_bounded(k, length, occurrences):
+    """53 bytes a k-mer occurrence and 64 MiB, the output included, however
+    many super-k-mers a read's k-mers make."""
+    import torch
+    reads = _random_reads(occurrences // (length - k + 1), length, 1_000_000, k + length)
+    g = swapgb.Graph()
+    swapgb.Graph().build_reads(swapgb.Opts(k=21, cutoff=1), swapgb.reads_from_fasta(b">r\n" + b"ACGT" * 20 + b"\n", 21))
+    torch.cuda.empty_cache()
+    before = torch.cuda.mem_get_info()[0]
+    _build(g, swapgb.Opts(k=k, cutoff=2), reads)
+    held = before - torch.cuda.mem_get_info()[0]
+    # a read's place in the build's prefix and scan arrays (8 B), tables of the buckets, allocations rounded up to 2 MiB
+    assert held <= 53 * occurrences + 64 * MB + 9 * reads[1].numel() + 64 * MB
+    want = swapgb.Graph()
+    _build(want, swapgb.Opts(k=k, cutoff=2, algorithm=swapgb.ALGO_DIRECT), reads)
+    assert g.distinct() == want.distinct() > 500_000  # (reads of k bases have no arcs: no k-molecule stays)
+    for a, b in zip(g.copy_out(), want.copy_out()):
+        assert np.array_equal(a, b)
