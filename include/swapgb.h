@@ -257,7 +257,8 @@ swg_status swg_batch_copy_out(const swg_graph *g, uint32_t s, uint64_t *keys, ui
 typedef struct swg_server swg_server;
 
 typedef struct swg_server_opts {
-    uint64_t memory_budget; /* device bytes for in-flight batches + resident results; 0 = 150 GiB */
+    uint64_t memory_budget; /* device bytes for in-flight batches, resident results and the sorting of
+                               fetched ones; 0 = 150 GiB */
     uint32_t workers;       /* batches in flight at once; 0 = 2 */
     uint32_t max_batch;     /* requests per batch; 0 = no limit */
     double load_factor;     /* 0 = 0.6 */
@@ -287,7 +288,10 @@ swg_status swg_server_wait(swg_server *srv, uint64_t ticket, double timeout_s);
 swg_status swg_server_result_info(swg_server *srv, uint64_t ticket, uint64_t *survivors,
                                   uint64_t *distinct);
 /* Copies the result to host memory (sorted by key when sorted != 0) and frees
- * it on the device; the ticket is then gone. */
+ * it on the device; the ticket is then gone. A sorted result is ordered on the
+ * device while the budget has room for the scratch (16 to 144 bytes a
+ * k-molecule; at most 256 MiB, or a sixteenth of the budget, of it stay mapped
+ * between fetches), else on the host. */
 swg_status swg_server_fetch(swg_server *srv, uint64_t ticket, uint64_t *keys, uint8_t *mult,
                             uint64_t cap, int sorted, uint64_t *n);
 /* Drops a finished result without copying it. */

@@ -54,6 +54,8 @@ struct Request {
 
 }  // namespace
 
+// Device memory that stays mapped between sorted fetches, and at most a
+// sixteenth of the budget.
 constexpr uint64_t kFetchKeep = 256ull << 20;
 
 struct swg_server {
@@ -64,7 +66,7 @@ struct swg_server {
     std::deque<Request *> queue;
     std::unordered_map<uint64_t, Request *> reqs;
     uint64_t next_ticket = 1;
-    uint64_t reserved = 0;  // in-flight footprints
+    uint64_t reserved = 0;  // in-flight footprints, scratch of sorted fetches under way
     uint64_t resident = 0;  // results waiting to be fetched
     uint64_t queued = 0;    // device bytes of the uploaded reads of queued requests (charged to the
                             // budget with the rest of the footprint once a worker takes the request)
@@ -76,7 +78,7 @@ struct swg_server {
     std::string dead_error;     // set when every worker failed its set-up
     std::vector<std::thread> workers;
     cudaStream_t fetch_stream = nullptr;
-    cudaMemPool_t pool = nullptr;  // scratch of sorted fetches; keeps at most kFetchKeep mapped between them
+    cudaMemPool_t pool = nullptr;  // scratch of sorted fetches
 };
 
 namespace {
@@ -287,7 +289,7 @@ swg_status swg_server_create(const swg_server_opts *o, swg_server **out) {
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = srv->device;
-    uint64_t keep = kFetchKeep;
+    uint64_t keep = std::min(kFetchKeep, srv->opts.memory_budget / 16);
     if (cudaMemPoolCreate(&srv->pool, &props) != cudaSuccess ||
         cudaMemPoolSetAttribute(srv->pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
         cudaGetLastError();
@@ -439,6 +441,7 @@ swg_status swg_server_fetch(swg_server *srv, uint64_t ticket, uint64_t *keys, ui
                             uint64_t cap, int sorted, uint64_t *n) {
     if (!srv) return SWG_ERR_BAD_INPUT;
     Request *r = nullptr;
+    uint64_t scratch = 0;  // of the device sort, where the budget has room for it
     {
         std::lock_guard<std::mutex> lock(srv->mu);
         auto it = srv->reqs.find(ticket);
@@ -455,14 +458,16 @@ swg_status swg_server_fetch(swg_server *srv, uint64_t ticket, uint64_t *keys, ui
             return SWG_ERR_BAD_INPUT;
         }
         srv->reqs.erase(it);  // the caller owns the result from here
+        const uint64_t want = sorted && r->n_out ? swg::sort_scratch_bytes(r->n_out) : 0;
+        if (srv->reserved + srv->resident + want <= srv->opts.memory_budget) scratch = want;
+        srv->reserved += scratch;
     }
     swg_status st = SWG_OK;
     cudaSetDevice(srv->device);
     if (r->n_out) {
         void *ws = nullptr;
-        const uint64_t want = swg::sort_scratch_bytes(r->n_out);
-        if (sorted && (srv->pool ? cudaMallocFromPoolAsync(&ws, want, srv->pool, srv->fetch_stream)
-                                 : cudaMallocAsync(&ws, want, srv->fetch_stream)) != cudaSuccess) {
+        if (scratch && (srv->pool ? cudaMallocFromPoolAsync(&ws, scratch, srv->pool, srv->fetch_stream)
+                                  : cudaMallocAsync(&ws, scratch, srv->fetch_stream)) != cudaSuccess) {
             cudaGetLastError();
             ws = nullptr;
         }
@@ -491,6 +496,7 @@ swg_status swg_server_fetch(swg_server *srv, uint64_t ticket, uint64_t *keys, ui
     {
         std::lock_guard<std::mutex> lock(srv->mu);
         srv->resident -= r->resident;
+        srv->reserved -= scratch;
     }
     srv->cv_work.notify_all();
     delete r;

@@ -117,3 +117,25 @@ def test_workspace_of_short_reads_is_bounded(k, length, occurrences):
     assert g.distinct() == want.distinct() > 500_000  # (reads of k bases have no arcs: no k-molecule stays)
     for a, b in zip(g.copy_out(), want.copy_out()):
         assert np.array_equal(a, b)
+
+
+def test_sorted_fetch_keeps_to_the_budget():
+    """The scratch of a fetch's sort (144 MB here) is charged to the server's
+    budget, or the host sorts."""
+    import torch
+    rng = np.random.default_rng(2)
+    read = np.frombuffer(b"ACGT", np.uint8)[rng.integers(0, 4, 1_000_000)].tobytes()
+    reads = swapgb.reads_from_fasta(b">r\n" + read + b"\n", 31)
+    want = swapgb.Graph().build_reads(swapgb.Opts(k=31, cutoff=1), reads).copy_out(sorted=True)
+    for budget, most in ((100 * MB, 100 * MB // 16), (4 << 30, 256 * MB)):
+        with_budget = swapgb.Server(memory_budget=budget, workers=1)
+        ticket = with_budget.submit(reads, 31, 1)
+        with_budget.wait(ticket, 60.0)
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        keys, mult = with_budget.fetch(ticket)
+        torch.cuda.synchronize()
+        assert before - torch.cuda.mem_get_info()[0] <= most + 4 * MB
+        assert with_budget.stats()["bytes_reserved"] == 0
+        assert np.array_equal(keys, want[0]) and np.array_equal(mult, want[1])
+        with_budget.close()
