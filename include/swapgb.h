@@ -438,9 +438,10 @@ swg_status swg_build_device_noalloc(const swg_opts *o, const uint32_t *d_packed,
 /* ---- autotuner ---------------------------------------------------------- */
 /* Times trial builds of a sample (device packed reads, as for
  * swg_graph_build_device) for each candidate: the bucketed build (the default
- * scheme) with records per bucket 2048 / 4096 / 8192 and each scatter block
- * shape (the level-1 partition count follows the input's size); the direct table at load factors
- * 0.5-0.8, in input and in minimizer order; hash-partitioned slices. Appends
+ * scheme) as it is planned without knobs, and with 2048 / 4096 / 8192
+ * occurrences per bucket and scatter block shapes 0 to 2 (the level-1 partition
+ * count follows the input's size); the direct table at load factors 0.5-0.8, in
+ * input and in minimizer order; hash-partitioned slices. Appends
  * the fastest to a cache file as one JSON line keyed by (k, read-length band
  * of read_len_hint). */
 typedef struct swg_tuning {

@@ -1,7 +1,9 @@
 // Autotuner: picks the counting scheme and its knobs for a (k, read-length
 // band) by timing trial builds of a sample on this GPU: the bucketed build
-// (the default) at several bucket sizes and scatter block shapes; the direct table at several load factors, in input and in
-// minimizer order; hash-partitioned slices. The choices go to a cache file,
+// as the default plans it, and at several bucket sizes and scatter block shapes
+// (any but 0 is a shape of the build over single occurrences); the direct table
+// at several load factors, in input and in minimizer order; hash-partitioned
+// slices. The choices go to a cache file,
 // one JSON object per line: {"k": K, "band": B, "load": X, "algorithm": A,
 // "read_order": O, "ms": T, "bucket_records": R, "part_bits": P,
 // "scatter_shape": S}.
@@ -66,7 +68,8 @@ swg_status swg_autotune(const swg_opts *base, const uint32_t *d_packed, uint64_t
     // bucketed: bucket size and scatter shape (the partition count follows the
     // input's size, so a count picked on a sample would not fit the full input)
     std::vector<Cand> cands;
-    for (uint32_t rec : {4096u, 2048u, 8192u})  // the default first: ties keep it
+    cands.push_back({0.6, SWG_ALGO_BUCKETED, SWG_ORDER_INPUT, 0, 0, 0});  // the default first: ties keep it
+    for (uint32_t rec : {4096u, 2048u, 8192u})
         for (int sh : {0, 1, 2}) cands.push_back({0.6, SWG_ALGO_BUCKETED, SWG_ORDER_INPUT, rec, 0, sh});
     for (double load : {0.5, 0.6, 0.7, 0.8}) cands.push_back({load, SWG_ALGO_DIRECT, SWG_ORDER_INPUT, 0, 0, 0});
     cands.push_back({0.6, SWG_ALGO_DIRECT, SWG_ORDER_MINIMIZER, 0, 0, 0});
