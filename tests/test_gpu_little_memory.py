@@ -139,3 +139,50 @@ def test_sorted_fetch_keeps_to_the_budget():
         assert with_budget.stats()["bytes_reserved"] == 0
         assert np.array_equal(keys, want[0]) and np.array_equal(mult, want[1])
         with_budget.close()
+
+
+def _same(g, k, cutoff, reads):
+    want = swapgb.Graph()
+    _build(want, swapgb.Opts(k=k, cutoff=cutoff, algorithm=swapgb.ALGO_DIRECT), reads)
+    assert g.size() == want.size() > 0
+    for a, b in zip(g.copy_out(), want.copy_out()):
+        assert np.array_equal(a, b)
+
+
+# 12.7M occurrences in reads of 100 bases at k = 31: super-k-mer records take
+# 409 MiB in regions of one size, 139 MiB in sampled ones, single occurrences
+# 291 MiB (204 MB counted exactly); the first output 24 MiB.
+N_READS = 181_429
+BUCKETED = dict(k=31, algorithm=swapgb.ALGO_BUCKETED)
+
+
+def test_regions_that_cannot_be_allocated():
+    """Regions of one size do not fit, sampled ones do; then nothing fits, and
+    the handle builds again once there is memory."""
+    reads = _random_reads(N_READS, 100, 400_000, 1)
+    g = swapgb.Graph()
+    with little_memory(270 * MB):
+        _build(g, swapgb.Opts(cutoff=2, **BUCKETED), reads)
+    assert g.info()["estimate"] == 0
+    _same(g, 31, 2, reads)
+    g = swapgb.Graph()
+    with little_memory(60 * MB):
+        with pytest.raises(swapgb.SwgError) as e:
+            _build(g, swapgb.Opts(cutoff=2, **BUCKETED), reads)
+        assert e.value.status == 3
+    _build(g, swapgb.Opts(cutoff=2, **BUCKETED), reads)
+    _same(g, 31, 2, reads)
+
+
+@pytest.mark.parametrize("genome,recounted", [(20_000, 0.0), (1_500_000, 1.0)])
+def test_output_that_cannot_be_allocated(genome, recounted):
+    """No room for the first guess of the output: the count alone says how much
+    is needed, and that fits, or fits only once the records are given back and
+    the build goes on over single occurrences."""
+    reads = _random_reads(N_READS, 100, genome, 2)
+    g = swapgb.Graph()
+    _build(g, swapgb.Opts(cutoff=255, **BUCKETED), reads)
+    with little_memory(8 * MB):
+        _build(g, swapgb.Opts(cutoff=2, **BUCKETED), reads)
+    assert g.info()["estimate"] == recounted
+    _same(g, 31, 2, reads)
