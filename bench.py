@@ -817,6 +817,29 @@ def main() -> int:
                 "unit": "GB/s", "frac": achieved / hbm, "peak_source": peak_src,
                 "traffic": (tpo * n_occ) if tpo else None, "traffic_source": tsrc,
                 "algorithmic_bytes": algo_bytes, "bytes_model": model, "kernel_ms": k_ms}
+    if kname.startswith(("k_bucket_count", "k_sk_count")) and not args.no_probe:
+        # the kernel's own ceiling is on chip: 64-bit shared CAS for the keys and
+        # 32-bit shared adds for the arcs, at the rates this GPU's shared-memory
+        # atomics reach. By single occurrences one CAS a record (a lower bound:
+        # linear probing adds some) and an add an arc. Super-k-mers are counted
+        # once for all equal records, which leaves between one CAS and add a
+        # distinct k-molecule and as many as there are occurrences and arcs.
+        r_add = swapgb.probe_shared_atomics("add_u32", 1 << 31, stream.cuda_stream)
+        r_cas = swapgb.probe_shared_atomics("cas_u64", 1 << 30, stream.cuda_stream)
+        n_arcs = 2 * n_occ - 2 * n_with_occ
+        merged = kname.startswith("k_sk_count")
+        cas, adds = (info["distinct"], info["distinct"]) if merged else (n_occ, n_arcs)
+        floor_ms = 1e3 * (cas / r_cas + adds / r_add)
+        roofline["on_chip"] = {"bound": "shared-memory atomics", "floor_ms": floor_ms,
+                               "frac": floor_ms / k_ms, "cas64_lane_ops_per_s": r_cas,
+                               "add32_lane_ops_per_s": r_add, "cas_per_build": cas,
+                               "adds_per_build": adds,
+                               "unmerged_ms": 1e3 * (n_occ / r_cas + n_arcs / r_add),
+                               "model": ("one 64-bit shared atomicCAS and one 32-bit shared atomicAdd per distinct "
+                                         "k-molecule (unmerged: per k-mer occurrence and per arc)" if merged else
+                                         "one 64-bit shared atomicCAS per record + one 32-bit shared atomicAdd per arc")
+                                        + ", at the rates swg_probe_shared_atomics measures in the same table "
+                                          "layout (this run)"}
     atomic = None
     if not args.no_probe and rank == 0:
         table_bytes = 16 << 30
