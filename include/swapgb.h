@@ -71,13 +71,18 @@ typedef enum swg_status {
 } swg_status;
 
 /* Counting algorithms (same results, different memory traffic). */
-#define SWG_ALGO_DEFAULT 0     /* bucketed when its workspace (at most 40 bytes per
-                                  k-mer occurrence) fits in device memory and no
-                                  read is longer than 16384 bases, else direct;
-                                  direct for SWG_ORDER_MINIMIZER */
+#define SWG_ALGO_DEFAULT 0     /* bucketed when 40 bytes per k-mer occurrence fit in
+                                  80% of the free device memory and no read is
+                                  longer than 16384 bases, else direct; direct for
+                                  SWG_ORDER_MINIMIZER */
 #define SWG_ALGO_DIRECT 1      /* one pass into a device-wide table in HBM */
 #define SWG_ALGO_PARTITIONED 2 /* hash-partitioned records, each partition counted in L2 */
-#define SWG_ALGO_BUCKETED 3    /* records split into buckets counted in shared memory */
+#define SWG_ALGO_BUCKETED 3    /* records split into buckets counted in shared memory:
+                                  super-k-mers (runs of k-mers with one minimizer) for
+                                  odd k from 19 to 31, one k for all reads, while their
+                                  workspace with the output is at most 53 bytes per
+                                  occurrence and 64 MiB; else single occurrences, at
+                                  most 40 bytes each and 64 MiB */
 
 /* Order in which the direct algorithm counts the reads (same results). */
 #define SWG_ORDER_INPUT 0     /* input order (default) */
@@ -93,10 +98,12 @@ typedef struct swg_opts {
     int algorithm;              /* SWG_ALGO_*; 0 = default */
     int read_order;             /* direct: SWG_ORDER_*; 0 = input order */
     /* Bucketed build knobs (0 = the default; swg_autotune picks them per k and
-     * read-length band): target records per bucket (64..65535), level-1
+     * read-length band): target k-mer occurrences per bucket (64..65535; by
+     * default 3072 of super-k-mers, 4096 of single occurrences), level-1
      * partition bits (8..10; more are used when the buckets would otherwise
-     * pass twice the target), block shape of the two scatter passes (the
-     * default is 256 threads x 16 records each; 1 = 512 x 8 for both, 2 =
+     * pass twice the target), block shape of the two scatter passes of single
+     * occurrences (any but 0 builds over those, for every k; 0 is 256 threads x
+     * 16 records each; 1 = 512 x 8 for both, 2 =
      * 256 x 8 for level 1 and 512 x 8 for level 2, 3 = level 2 staged by
      * bulk copies, 4 = level 1 with warp-cooperative extraction: the lanes of
      * a warp on consecutive k-mers, each cut from a window of the packed
@@ -124,11 +131,13 @@ typedef struct swg_build_info {
                              recounted in the larger (tier-2) shared-memory table */
     double estimate;      /* direct: distinct-count estimate used for sizing;
                              bucketed: 1 when a partition or bucket outgrew its
-                             sampled region and the build reran with exact counts */
+                             sampled region and the build reran with exact counts
+                             over single occurrences */
     float ms[5];          /* as swg_graph_last_timings */
     uint32_t bucket_table; /* bucketed: entries of the shared table the first
                               counting pass used (2048 when the buckets average
-                              at most 3072 records, else 4096); 0 otherwise */
+                              at most 3072 occurrences, else 4096; single
+                              occurrences of a batch: 4096); 0 otherwise */
 } swg_build_info;
 
 typedef struct swg_reads swg_reads; /* host-side packed reads */
