@@ -1234,7 +1234,7 @@ constexpr uint64_t kSuperWhole = 512;
 // Super-k-mers for every odd k that their records and minimizers serve (19 to
 // 31: a record holds 47 bases, and a shorter k has too few m-mers), at every
 // size: builds of 0.2M occurrences take 126 us, by single occurrences 178; of
-// 175M 2.14 ms and 3.01; of 2.4G, with repeats, 28.9 and 46.5. An even k-mer can
+// 175M 2.14 ms and 3.01; of 2.4G, with repeats, 25.0 and 46.5. An even k-mer can
 // be its own reverse complement, and a batch may mix k: single occurrences.
 bool super_build(const swg_opts *o, const BuildArgs &a, uint64_t N) {
     // (the other scatter shapes are shapes of the single-occurrence scatters)
@@ -1411,7 +1411,9 @@ swg_status build_super(swg_graph *g, const swg_opts *o, BuildArgs &a, cudaStream
     // is no room, and single occurrences where the sampled plan does not fit. Builds of 0.05M, 0.5M, 1.4M, 3.1M, 9.6M
     // and 24M occurrences: 115 -> 97 us, 129 -> 100, 144 -> 110, 160 -> 123,
     // 223 -> 194, 369 -> 333 (of 0.8M, most of them of one base repeated, where
-    // the plan is made twice: 212 -> 351).
+    // the build is made twice: 212 -> 351, by single occurrences 411). At the
+    // line the 2048 records (32 KB) of every bucket's region make 268 MB; larger
+    // builds were not tried without a sample.
     const uint64_t slack = a.segs ? std::min<uint64_t>(kSuperSlack, (uint64_t)a.n_segs << 24) : kSuperSlack;
     for (bool uniform = true;; uniform = false) {
         const SuperSizes z = super_sizes(o, a.k, a.total_occ, reads.n_pieces, 2.0 * stride, uniform);
@@ -1583,6 +1585,18 @@ constexpr uint64_t kStreamMin = 96ull << 20;    // shorter texts go up and are f
 constexpr uint64_t kStreamPiece = 40ull << 20;  // target bytes per piece
 constexpr uint64_t kStreamMaxPieces = 16;
 
+// Level-1 scatter of one piece's reads (a.read_range, or all of a's reads). Over
+// super-k-mers a thread takes a read whole, up to kSuperLongest bases: only the
+// one-shot build cuts long reads in pieces.
+int scatter_piece(const BuildArgs &a, const BucketPlan &pl, int grid_mode, cudaStream_t s) {
+    if (!pl.super) return swg::launch_part_scatter(a, pl.pa, s, grid_mode);
+    swg::SkArgs sk = pl.sk;
+    sk.off = a.read_off;
+    sk.len = a.read_len;
+    sk.n_pieces = a.n_reads;
+    return swg::launch_super_scan(a, sk, a.n_reads, 1, false, grid_mode, s);
+}
+
 // Streamed FASTA build (texts of kStreamMin bytes and more). The text goes
 // up in pieces on a copy stream; a framing stream frames each piece as it
 // lands — newline counts, newline positions, the records completed so far,
@@ -1600,16 +1614,6 @@ constexpr uint64_t kStreamMaxPieces = 16;
 // or read order, or a graph the bucketed workspace does not fit, falls back
 // to the one-shot build over the reads framed here. Results are those of the
 // one-shot build.
-// Level-1 scatter of one piece's reads (a.read_range, or all of a's reads).
-int scatter_piece(const BuildArgs &a, const BucketPlan &pl, int grid_mode, cudaStream_t s) {
-    if (!pl.super) return swg::launch_part_scatter(a, pl.pa, s, grid_mode);
-    swg::SkArgs sk = pl.sk;
-    sk.off = a.read_off;
-    sk.len = a.read_len;
-    sk.n_pieces = a.n_reads;
-    return swg::launch_super_scan(a, sk, a.n_reads, 1, false, grid_mode, s);
-}
-
 swg_status build_fasta_streamed(swg_graph *g, const swg_opts *o, const char *first, uint64_t n,
                                 cudaStream_t s, bool synced = false) {
     swg_status st;

@@ -1,10 +1,12 @@
 // Records (canonical key, 8 multiplicities) in key order on the device, for
-// the copies of a graph to the host that ask for it. Hand-written: one block
-// orders up to kOne records in shared memory in one launch; more take a
-// stable least-significant-digit radix sort, 8 bits a pass over the 2k bits
-// of a key. Bound by memory: a pass reads the keys twice and the records
-// once and writes them once (40 bytes a record), and by launches below about
-// a million records.
+// the copies of a graph to the host that ask for it, and for the merge's lines.
+// Hand-written, by size: one block orders up to kOne records in one launch; up
+// to kSplitMost are scattered to buckets between sampled splitters and ordered
+// by a block a bucket, in three launches; more, or a bucket that outgrows its
+// region, take a stable least-significant-digit radix sort, 8 bits a pass over
+// the 2k bits of a key. The first two are bound by launches and a block's steps,
+// a radix pass by memory: it reads the keys twice and the records once and
+// writes them once (40 bytes a record).
 #include <cuda_runtime.h>
 
 #include <algorithm>

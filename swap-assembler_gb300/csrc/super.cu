@@ -48,7 +48,8 @@ constexpr uint32_t kSkClamp = 3840;
 // with 16384, 16.0 with 8192, 14.6 with 4096, the build 27.6, 26.1 and 26.7)
 constexpr uint64_t kSkBigRecords = 8192;
 
-__device__ __forceinline__ uint32_t sk_mix(uint32_t x) {  // bucket of a minimizer
+// Bucket of a minimizer (lowbias32 of Wellons's hash-prospector).
+__device__ __forceinline__ uint32_t sk_mix(uint32_t x) {
     x ^= x >> 16;
     x *= 0x7feb352du;
     x ^= x >> 15;
@@ -87,7 +88,7 @@ __global__ void __launch_bounds__(256) k_sk_pieces_fill(BuildArgs a, const uint6
 // of W m-mers spans exactly K bases, one 64-bit window, so nothing but the
 // window minima is carried along a read: m-mers and their reverse complements
 // are cut from the top of the window at constant shifts. Window minima by the
-// two-scan scheme: arr holds the suffix minima of the previous block's hashes;
+// two-scan scheme of van Herk and of Gil and Werman: arr holds the suffix minima of the previous block's hashes;
 // with the running minimum of this block they give one minimum per k-mer at
 // three min operations each. A block leaves a bit mask of the positions where
 // the minimum changes; the runs that end there are queued after it, a warp's
